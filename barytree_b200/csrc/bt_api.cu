@@ -651,7 +651,6 @@ struct DevPlan {
     bool mixed = false, herm = false, need_src_clusters = false, need_tgt_grids = false;
     bool queue = false;     // mixed kernels on a device work queue
     int tpt = 2, tile = 1024;   // tile shape of the mixed particle-output kernel
-    int fp64_tb = 1;            // targets per thread of the FP64 particle-output kernel
     bool base_full = true;      // proxies at the base degree for every node (else only the selected
                                 // degrees' marked subtrees, the base degree among them)
     bool tc_up = false;         // leaf P2M on the tensor cores (bt_tc.cu)
@@ -690,6 +689,8 @@ struct DevPlan {
     int3 *d_hred = nullptr;                 // nodes with several chunks
     double *d_hpartial = nullptr;           // their partial moments
     int n_hchunks = 0, n_hred = 0;
+    // segment sums of the FP64 evaluation kernels where their items are few
+    double *d_evpart = nullptr, *d_gridpart = nullptr;
 };
 
 // BT_ERR_TIMEOUT if a tensor-core kernel of the last evaluation gave up
@@ -947,8 +948,9 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         g.c_off = d_ccoff; g.c_idx = d_ccidx; g.p_off = d_cpoff; g.p_idx = d_cpidx;
         g.s_ibeg = d_sibeg; g.s_numpar = d_snum; g.s_grid = d_sgrid; g.Q = d_Q;
         g.sx = d_sx; g.sy = d_sy; g.sz = d_sz; g.sq = d_sq; g.kp = v.kp; g.kp2 = v.kp2; g.Phi = d_Phi;
+        g.partial = v.d_gridpart; g.pstride = (size_t)v.T_n * P;
         bt::launch_eval_grids(v.kernel, herm, g, st);
-        launches++;
+        launches += g.partial ? 2 : 1;
     }
     CK(cudaGetLastError());
     if (ev) CK(record(2));
@@ -1015,9 +1017,10 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         a.t_ibeg = d_tibeg; a.t_numpar = d_tnum; a.a_off = d_aoff; a.a_idx = d_aidx; a.d_off = d_doff; a.d_idx = d_didx;
         a.s_ibeg = d_sibeg; a.s_numpar = d_snum; a.s_grid = d_sgrid; a.Q = d_Q;
         a.sx = d_sx; a.sy = d_sy; a.sz = d_sz; a.sq = d_sq; a.tx = d_tx; a.ty = d_ty; a.tz = d_tz;
-        a.kp = v.kp; a.kp2 = v.kp2; a.pot = d_pot; a.tb = v.fp64_tb;
+        a.kp = v.kp; a.kp2 = v.kp2; a.pot = d_pot;
+        a.partial = v.d_evpart; a.pstride = (size_t)nt;
         bt::launch_eval_targets(v.kernel, herm, a, st);
-        launches++;
+        launches += a.partial ? 2 : 1;
     }
     CK(cudaGetLastError());
     if (ev) CK(record(3));
@@ -1233,18 +1236,17 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
                     for (int v = T.leaves[u]; v >= 0 && !tnode_need[v]; v = T.parent[v]) tnode_need[v] = 1;
         }
     }
-    // FP64 particle-output kernel: two targets per thread where the items fill the GPU
-    const int fp64_tb = (!mixed && !ssm) ? bt::fp64_targets_per_thread(T.nleaves, leaf_count.data()) : 1;
     std::vector<int2> ev_items =
         make_items(T.nleaves, leaf_count.data(),
-                   mixed ? bt::mixed_targets_chunk() : ssm ? bt::ss_chunk() : bt::fp64_targets_chunk(fp64_tb),
+                   mixed ? bt::mixed_targets_chunk() : ssm ? bt::ss_chunk() : bt::EV_CHUNK,
                    leaf_cost);
     std::vector<int2> grid_items, l2p_items;
     if (need_tgt_grids) {
         std::vector<int> pcount(T.n, P);
         if (!tnode_need.empty())
             for (int i = 0; i < T.n; i++) pcount[i] = tnode_need[i] ? P : 0;
-        grid_items = make_items(T.n, pcount.data(), 128, gcost);
+        // points per item: the FP64 Lagrange kernel takes two per thread
+        grid_items = make_items(T.n, pcount.data(), mixed || ssm || herm ? 128 : bt::EV_CHUNK, gcost);
         std::vector<double> lcost(T.nleaves, 1.0);
         l2p_items = make_items(T.nleaves, leaf_count.data(), 128, lcost);
     }
@@ -1475,6 +1477,23 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     int3 *d_hred = nullptr;
     double *d_hpartial = nullptr;
 
+    // FP64: near-field entries whose box meets the target leaf's, the only
+    // ones where a source can coincide with a target, carry EV_MEETS
+    hvec<int> didx64;
+    if (!mixed && !ssm) {
+        didx64.resize((size_t)pl.t_direct.off[pl.t_direct.rows]);
+#pragma omp parallel for schedule(static)
+        for (int u = 0; u < T.nleaves; u++) {
+            const int t = T.leaves[u];
+            for (int64_t k = pl.t_direct.off[u]; k < pl.t_direct.off[u + 1]; k++) {
+                const int s = pl.t_direct.idx[k];
+                const bool meets = S.x0[s] <= T.x1[t] && T.x0[t] <= S.x1[s] && S.y0[s] <= T.y1[t] &&
+                                   T.y0[t] <= S.y1[s] && S.z0[s] <= T.z1[t] && T.z0[t] <= S.z1[s];
+                didx64[k] = meets ? s | bt::EV_MEETS : s;
+            }
+        }
+    }
+
     // device layout
     double *d_sx, *d_sy, *d_sz, *d_sq, *d_tx, *d_ty, *d_tz, *d_pot, *d_sgrid, *d_tgrid, *d_slen, *d_tlen, *d_ww;
     double *d_Q = nullptr, *d_Phi = nullptr;
@@ -1565,6 +1584,23 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         }
     }
 
+    // Segment sums of the FP64 evaluation kernels, where their work items are
+    // few (the results are the same without them): up to EV_SEGS doubles per
+    // target, or per grid point within a fixed bound.
+    double *d_evpart = nullptr, *d_gridpart = nullptr;
+    if (!mixed && !ssm) {
+        const size_t room = arena.fixed ? (arena.cap > L.total() ? arena.cap - L.total() : 0) : (size_t)1 << 30;
+        size_t need = 0;
+        auto want = [&](double **p, size_t count) {
+            if (need + sizeof(double) * count + 512 > room) return;
+            need += sizeof(double) * count + 512;
+            L.add(p, count);
+        };
+        if (bt::eval64_split(ev_items.size())) want(&d_evpart, (size_t)bt::EV_SEGS * nt);
+        if (need_tgt_grids && !herm && bt::eval64_split(grid_items.size()))
+            want(&d_gridpart, (size_t)bt::EV_SEGS * T.n * P);
+    }
+
     if (!arena.reserve(L.total())) {
         if (arena.fixed) {
             set_err("this call needs %zu bytes of device scratch; the static scratch holds %zu", L.total(), arena.cap);
@@ -1594,7 +1630,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         UP(d_tpar, T.parent, T.n); UP(d_tleaves, T.leaves, T.nleaves);
         if (T.lvl_off) UP(d_tlvl, T.lvl_nodes, T.lvl_off[T.max_depth]);
         UP(d_aoff, pl.t_approx.off, pl.t_approx.rows + 1); UP(d_aidx, pl.t_approx.idx, pl.t_approx.off[pl.t_approx.rows]);
-        UP(d_doff, pl.t_direct.off, pl.t_direct.rows + 1); UP(d_didx, pl.t_direct.idx, pl.t_direct.off[pl.t_direct.rows]);
+        UP(d_doff, pl.t_direct.off, pl.t_direct.rows + 1); UP(d_didx, didx64.empty() ? pl.t_direct.idx : didx64.data(), pl.t_direct.off[pl.t_direct.rows]);
         UP(d_ccoff, pl.g_cc.off, pl.g_cc.rows + 1); UP(d_ccidx, pl.g_cc.idx, pl.g_cc.off[pl.g_cc.rows]);
         UP(d_cpoff, pl.g_cp.off, pl.g_cp.rows + 1); UP(d_cpidx, pl.g_cp.idx, pl.g_cp.off[pl.g_cp.rows]);
         UP(d_evitems, ev_items.data(), ev_items.size());
@@ -1650,7 +1686,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         v.tile = shape.tile;
         v.tc_up = shape.tc_up && mixed;
         v.sharded = shape.nshards > 1;
-        v.fp64_tb = fp64_tb;
+        v.d_evpart = d_evpart; v.d_gridpart = d_gridpart;
         v.base_full = pl.a_deg == nullptr;
         v.sym_npairs = (int)sym_pairs.size();
         v.sym_far_pairs = (int)sym_far_pairs;
@@ -2410,9 +2446,11 @@ int bt_direct_full(int numTargets, int numSources, const double *targetX, const 
     if (rc != BT_OK) return rc;
     std::lock_guard<std::mutex> lk(ctx->mu);
     cudaStream_t st = ctx->stream;
-    double *d_t[4], *d_s[5], *d_o;
+    double *d_t[4], *d_s[5], *d_o, *d_part = nullptr;
+    const int parts = bt::direct_parts(numTargets, numSources);
     {
         Layout L;
+        if (!ss && parts > 1) L.add(&d_part, (size_t)parts * numTargets);
         for (int i = 0; i < 4; i++) L.add(&d_t[i], numTargets);
         for (int i = 0; i < 5; i++) L.add(&d_s[i], numSources);
         L.add(&d_o, numTargets);
@@ -2431,8 +2469,8 @@ int bt_direct_full(int numTargets, int numSources, const double *targetX, const 
             g_launches += 2;
         } else {
             bt::launch_direct(kernel, numTargets, numSources, d_t[0], d_t[1], d_t[2], d_s[0], d_s[1], d_s[2], d_s[3],
-                              kernelParam, d_o, st, kernelParam2);
-            g_launches += 1;
+                              kernelParam, kernelParam2, d_part, d_o, st);
+            g_launches += parts > 1 ? 2 : 1;
         }
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(outputArray, d_o, sizeof(double) * numTargets, cudaMemcpyDeviceToHost, st));

@@ -16,6 +16,7 @@
 #include <cstdint>
 
 #include "bt_device.h"
+#include "bt_eval64.h"
 #include "bt_kernels.cuh"
 
 namespace bt {
@@ -529,148 +530,19 @@ void launch_hermite_reduce(int n, int nred, const int3 *red, const double *parti
 }
 
 // ---------------------------------------------------------------------------
-// Particle-output evaluation: PC (clusters) + PP (particles) per target leaf.
-// One CTA per work item (target leaf, chunk of TB * EV_THREADS targets), TB
-// targets per thread (ti and ti + EV_THREADS, ...) so that every grid point
-// or source read from shared memory serves TB evaluations; FP64 accumulation
-// in registers in each target's own order (the same order for any TB);
-// exactly one writer per target.  TB = 2 where the work items fill the GPU
-// several times over, else 1 (fp64_targets_per_thread).
+// Hermite grid outputs: CP (source particles) onto the 8 moments of every grid
+// point of a target node, one grid point per thread.  The other evaluations
+// are in bt_eval64.cuh.
 // ---------------------------------------------------------------------------
-constexpr int EV_THREADS = 128;
 constexpr int PP_TILE = 512;
 
-template <int KT, bool HERM, int EV_TB>
+template <int KT>
 __global__ void __launch_bounds__(EV_THREADS)
-k_eval_targets(int n, const int2 *__restrict__ items, const int *__restrict__ leaf_node,
-               const int *__restrict__ t_ibeg, const int *__restrict__ t_numpar,
-               const int64_t *__restrict__ a_off, const int *__restrict__ a_idx,
-               const int64_t *__restrict__ d_off, const int *__restrict__ d_idx,
-               const int *__restrict__ s_ibeg, const int *__restrict__ s_numpar, const double *__restrict__ s_grid,
-               const double *__restrict__ Q, const double *__restrict__ sx, const double *__restrict__ sy,
-               const double *__restrict__ sz, const double *__restrict__ sq,
-               const double *__restrict__ tx, const double *__restrict__ ty, const double *__restrict__ tz,
-               double kp, double kp2, double *__restrict__ pot)
-{
-    extern __shared__ double sm[];
-    const int2 it = items[blockIdx.x];
-    const int u = it.x;
-    const int tnode = leaf_node[u];
-    const int tb = t_ibeg[tnode], tn = t_numpar[tnode];
-    bool active[EV_TB];
-    int t[EV_TB];
-    double x[EV_TB], y[EV_TB], z[EV_TB], acc[EV_TB];
-#pragma unroll
-    for (int b = 0; b < EV_TB; b++) {
-        const int ti = it.y * (EV_TB * EV_THREADS) + b * EV_THREADS + threadIdx.x;
-        active[b] = ti < tn;
-        t[b] = tb + (active[b] ? ti : 0);
-        x[b] = tx[t[b]]; y[b] = ty[t[b]]; z[b] = tz[t[b]];
-        acc[b] = 0.0;
-    }
-    const bool any = active[0];     // target b > 0 is active only if target 0 is
-    const int np1 = n + 1, P = np1 * np1 * np1;
-
-    // far field: source clusters
-    for (int64_t e = a_off[u]; e < a_off[u + 1]; e++) {
-        const int s = a_idx[e];
-        double *g = sm;
-        double *q = sm + 3 * np1;
-        const int nq = HERM ? 8 * P : P;
-        const double *Qs = Q + (size_t)s * nq;
-        for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) g[i] = s_grid[(size_t)s * 3 * np1 + i];
-        for (int i = threadIdx.x; i < nq; i += blockDim.x) q[i] = Qs[i];
-        __syncthreads();
-        if (any) {
-            int j = 0;
-            for (int k3 = 0; k3 < np1; k3++) {
-                const double gz = g[2 * np1 + k3];
-                for (int k2 = 0; k2 < np1; k2++) {
-                    const double gy = g[np1 + k2];
-                    if (!HERM && KT <= K_REGCOULOMB) {
-                        double dyz[EV_TB];
-#pragma unroll
-                        for (int b = 0; b < EV_TB; b++) {
-                            const double dz = z[b] - gz, dy = y[b] - gy;
-                            dyz[b] = dy * dy + dz * dz;
-                        }
-                        for (int k1 = 0; k1 < np1; k1++, j++) {
-                            const double gx = g[k1], qj = q[j];
-#pragma unroll
-                            for (int b = 0; b < EV_TB; b++) {
-                                const double dx = x[b] - gx;
-                                acc[b] += k_far<KT>(fma(dx, dx, dyz[b]), qj, kp);
-                            }
-                        }
-                    } else if (!HERM) {
-                        for (int k1 = 0; k1 < np1; k1++, j++) {
-#pragma unroll
-                            for (int b = 0; b < EV_TB; b++)
-                                acc[b] += k_any<KT, false>(x[b] - g[k1], y[b] - gy, z[b] - gz, q[j], kp, kp2);
-                        }
-                    } else {
-                        for (int k1 = 0; k1 < np1; k1++, j++) {
-#pragma unroll
-                            for (int b = 0; b < EV_TB; b++)
-                                acc[b] += k_pc_herm<KT>(x[b] - g[k1], y[b] - gy, z[b] - gz, q + j, P, kp);
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // near field: source particles
-    double4 *tile = reinterpret_cast<double4 *>(sm);
-    for (int64_t e = d_off[u]; e < d_off[u + 1]; e++) {
-        const int s = d_idx[e];
-        const int sb = s_ibeg[s], sn = s_numpar[s];
-        for (int c0 = 0; c0 < sn; c0 += PP_TILE) {
-            int cm = min(PP_TILE, sn - c0);
-            for (int i = threadIdx.x; i < cm; i += blockDim.x)
-                tile[i] = make_double4(sx[sb + c0 + i], sy[sb + c0 + i], sz[sb + c0 + i], sq[sb + c0 + i]);
-            __syncthreads();
-            if (any) {
-                for (int i = 0; i < cm; i++) {
-                    const double4 p = tile[i];
-#pragma unroll
-                    for (int b = 0; b < EV_TB; b++)
-                        acc[b] += k_any<KT, true>(x[b] - p.x, y[b] - p.y, z[b] - p.z, p.w, kp, kp2);
-                }
-            }
-            __syncthreads();
-        }
-    }
-#pragma unroll
-    for (int b = 0; b < EV_TB; b++)
-        if (active[b]) pot[t[b]] = acc[b];
-}
-
-int fp64_targets_chunk(int tb) { return tb * EV_THREADS; }
-
-int fp64_targets_per_thread(int nunits, const int *count)
-{
-    // work items of two targets per thread; under about four waves of
-    // resident blocks (16 blocks of 128 threads on each of ~148 SMs) one
-    // target per thread keeps twice as many blocks in flight
-    long long items = 0;
-    for (int u = 0; u < nunits; u++) items += (count[u] + 2 * EV_THREADS - 1) / (2 * EV_THREADS);
-    return items >= 4LL * 16 * 148 ? 2 : 1;
-}
-
-// ---------------------------------------------------------------------------
-// Grid-output evaluation: M2L (source clusters, CC) + CP (source particles)
-// onto the grid of a target node.  One thread per target grid point.
-// ---------------------------------------------------------------------------
-template <int KT, bool HERM>
-__global__ void __launch_bounds__(EV_THREADS)
-k_eval_grids(int n, const int2 *__restrict__ items, const double *__restrict__ t_grid,
-             const int64_t *__restrict__ c_off, const int *__restrict__ c_idx,
-             const int64_t *__restrict__ p_off, const int *__restrict__ p_idx,
-             const int *__restrict__ s_ibeg, const int *__restrict__ s_numpar, const double *__restrict__ s_grid,
-             const double *__restrict__ Q, const double *__restrict__ sx, const double *__restrict__ sy,
-             const double *__restrict__ sz, const double *__restrict__ sq, double kp, double kp2,
-             double *__restrict__ Phi)
+k_eval_grids_hermite(int n, const int2 *__restrict__ items, const double *__restrict__ t_grid,
+                     const int64_t *__restrict__ p_off, const int *__restrict__ p_idx,
+                     const int *__restrict__ s_ibeg, const int *__restrict__ s_numpar, const double *__restrict__ sx,
+                     const double *__restrict__ sy, const double *__restrict__ sz, const double *__restrict__ sq,
+                     double kp, double *__restrict__ Phi)
 {
     extern __shared__ double sm[];
     const int2 it = items[blockIdx.x];
@@ -681,40 +553,9 @@ k_eval_grids(int n, const int2 *__restrict__ items, const double *__restrict__ t
     const int jj = active ? j0 : 0;
     const double *tg = t_grid + (size_t)T * 3 * np1;
     const double x = tg[jj % np1], y = tg[np1 + (jj / np1) % np1], z = tg[2 * np1 + jj / (np1 * np1)];
-    double acc[HERM ? 8 : 1];
+    double acc[8];
 #pragma unroll
-    for (int m = 0; m < (HERM ? 8 : 1); m++) acc[m] = 0.0;
-
-    if (!HERM) {
-        for (int64_t e = c_off[T]; e < c_off[T + 1]; e++) {
-            const int s = c_idx[e];
-            double *g = sm;
-            double *q = sm + 3 * np1;
-            for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) g[i] = s_grid[(size_t)s * 3 * np1 + i];
-            for (int i = threadIdx.x; i < P; i += blockDim.x) q[i] = Q[(size_t)s * P + i];
-            __syncthreads();
-            if (active) {
-                int j = 0;
-                for (int k3 = 0; k3 < np1; k3++) {
-                    double dz = z - g[2 * np1 + k3];
-                    for (int k2 = 0; k2 < np1; k2++) {
-                        double dy = y - g[np1 + k2];
-                        if (KT <= K_REGCOULOMB) {
-                            double dyz = dy * dy + dz * dz;
-                            for (int k1 = 0; k1 < np1; k1++, j++) {
-                                double dx = x - g[k1];
-                                acc[0] += k_far<KT>(fma(dx, dx, dyz), q[j], kp);
-                            }
-                        } else {
-                            for (int k1 = 0; k1 < np1; k1++, j++)
-                                acc[0] += k_any<KT, false>(x - g[k1], dy, dz, q[j], kp, kp2);
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
+    for (int m = 0; m < 8; m++) acc[m] = 0.0;
     double4 *tile = reinterpret_cast<double4 *>(sm);
     for (int64_t e = p_off[T]; e < p_off[T + 1]; e++) {
         const int s = p_idx[e];
@@ -727,22 +568,47 @@ k_eval_grids(int n, const int2 *__restrict__ items, const double *__restrict__ t
             if (active) {
                 for (int i = 0; i < cm; i++) {
                     double4 p = tile[i];
-                    if (!HERM) {
-                        acc[0] += k_any<KT, false>(x - p.x, y - p.y, z - p.z, p.w, kp, kp2);
-                    } else {
-                        k_cp_herm<KT>(p.x - x, p.y - y, p.z - z, p.w, kp, acc);
-                    }
+                    k_cp_herm<KT>(p.x - x, p.y - y, p.z - z, p.w, kp, acc);
                 }
             }
             __syncthreads();
         }
     }
-    if (active) {
-        if (!HERM) Phi[(size_t)T * P + j0] = acc[0];
-        else
+    if (active)
 #pragma unroll
-            for (int m = 0; m < 8; m++) Phi[((size_t)T * 8 + m) * P + j0] = acc[m];
+        for (int m = 0; m < 8; m++) Phi[((size_t)T * 8 + m) * P + j0] = acc[m];
+}
+
+// Sums of the segments of a split launch, in order: the targets of an item
+// (its leaf's), or its grid points (leaf_node == nullptr: P points per node).
+__global__ void k_sum_segments(const int2 *__restrict__ items, const int *__restrict__ leaf_node,
+                               const int *__restrict__ ibeg, const int *__restrict__ numpar, int P,
+                               const double *__restrict__ partial, size_t pstride, double *__restrict__ out)
+{
+    const int2 it = items[blockIdx.x];
+    const int i = it.y * EV_CHUNK + threadIdx.x;
+    size_t t;
+    if (leaf_node) {
+        const int node = leaf_node[it.x];
+        if (i >= numpar[node]) return;
+        t = (size_t)ibeg[node] + i;
+    } else {
+        if (i >= P) return;
+        t = (size_t)it.x * P + i;
     }
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < EV_SEGS; k++) s += partial[(size_t)k * pstride + t];
+    out[t] = s;
+}
+
+__global__ void k_sum_parts(int n, int parts, const double *__restrict__ partial, double *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double s = 0.0;
+    for (int k = 0; k < parts; k++) s += partial[(size_t)k * n + i];
+    out[i] = s;
 }
 
 // ---------------------------------------------------------------------------
@@ -858,34 +724,6 @@ k_l2p_hermite(int n, const int2 *__restrict__ items, const int *__restrict__ lea
 #undef BZ
     }
     if (active) pot[t] += acc;
-}
-
-// ---------------------------------------------------------------------------
-// FP64 direct sum (InteractionCompute_Direct, src/interaction_compute/interaction_compute_direct.c:26-231)
-// ---------------------------------------------------------------------------
-template <int KT>
-__global__ void __launch_bounds__(EV_THREADS)
-k_direct(int nt, int ns, const double *__restrict__ tx, const double *__restrict__ ty, const double *__restrict__ tz,
-         const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
-         const double *__restrict__ sq, double kp, double kp2, double *__restrict__ out)
-{
-    __shared__ double4 tile[PP_TILE];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = t < nt;
-    const double x = active ? tx[t] : 0.0, y = active ? ty[t] : 0.0, z = active ? tz[t] : 0.0;
-    double acc = 0.0;
-    for (int c0 = 0; c0 < ns; c0 += PP_TILE) {
-        int cm = min(PP_TILE, ns - c0);
-        for (int i = threadIdx.x; i < cm; i += blockDim.x)
-            tile[i] = make_double4(sx[c0 + i], sy[c0 + i], sz[c0 + i], sq[c0 + i]);
-        __syncthreads();
-        for (int i = 0; i < cm; i++) {
-            double4 p = tile[i];
-            acc += k_any<KT, true>(x - p.x, y - p.y, z - p.z, p.w, kp, kp2);
-        }
-        __syncthreads();
-    }
-    if (active) out[t] = acc;
 }
 
 // Output in the caller's order (Particles_Targets_Reorder, src/particles/particles.c:58-94).
@@ -1014,71 +852,65 @@ void launch_l2l(int n, int nparents, const int *parents, const int *nchild, cons
     k_l2l<<<nparents, 256, sm, st>>>(n, parents, nchild, child, grid, Phi);
 }
 
-template <int KT, bool HERM>
-static void eval_targets_t(const EvalTargetsArgs &a, cudaStream_t st)
-{
-    int np1 = a.n + 1, P = np1 * np1 * np1;
-    size_t far = sizeof(double) * (size_t)(3 * np1 + (HERM ? 8 * P : P));
-    size_t near = sizeof(double4) * PP_TILE;
-    size_t sm = far > near ? far : near;
-    auto fn = a.tb == 2 ? k_eval_targets<KT, HERM, 2> : k_eval_targets<KT, HERM, 1>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    fn<<<a.nitems, EV_THREADS, sm, st>>>(a.n, a.items, a.leaf_node, a.t_ibeg, a.t_numpar, a.a_off, a.a_idx,
-                                         a.d_off, a.d_idx, a.s_ibeg, a.s_numpar, a.s_grid, a.Q, a.sx, a.sy,
-                                         a.sz, a.sq, a.tx, a.ty, a.tz, a.kp, a.kp2, a.pot);
-}
+// With fewer items than about four waves of resident blocks (8 blocks of
+// EV_THREADS threads on each of 148 SMs) the last wave is a large part of the
+// whole; a block per segment then gives the scheduler 16 times as many.
+bool eval64_split(size_t items) { return items < (size_t)4 * 8 * 148; }
 
 // Kernels with Hermite forms: Coulomb, Yukawa, regularized Coulomb, sin-over-r.
 void launch_eval_targets(int kernel, bool hermite, const EvalTargetsArgs &a, cudaStream_t st)
 {
     if (a.nitems <= 0) return;
     switch (kernel) {
-    case K_COULOMB: hermite ? eval_targets_t<K_COULOMB, true>(a, st) : eval_targets_t<K_COULOMB, false>(a, st); break;
-    case K_YUKAWA: hermite ? eval_targets_t<K_YUKAWA, true>(a, st) : eval_targets_t<K_YUKAWA, false>(a, st); break;
-    case K_REGCOULOMB:
-        hermite ? eval_targets_t<K_REGCOULOMB, true>(a, st) : eval_targets_t<K_REGCOULOMB, false>(a, st);
-        break;
-    case K_SINOVERR:
-        hermite ? eval_targets_t<K_SINOVERR, true>(a, st) : eval_targets_t<K_SINOVERR, false>(a, st);
-        break;
-    case K_REGYUKAWA: eval_targets_t<K_REGYUKAWA, false>(a, st); break;
-    case K_ATAN: eval_targets_t<K_ATAN, false>(a, st); break;
-    case K_MQ: eval_targets_t<K_MQ, false>(a, st); break;
-    case K_RBSU: eval_targets_t<K_RBSU, false>(a, st); break;
-    case K_RBSV: eval_targets_t<K_RBSV, false>(a, st); break;
-    default: eval_targets_t<K_USER, false>(a, st);
+    case K_COULOMB: eval_targets_kt<K_COULOMB>(hermite, a, st); break;
+    case K_YUKAWA: eval_targets_kt<K_YUKAWA>(hermite, a, st); break;
+    case K_REGCOULOMB: eval_targets_kt<K_REGCOULOMB>(hermite, a, st); break;
+    case K_SINOVERR: eval_targets_kt<K_SINOVERR>(hermite, a, st); break;
+    case K_REGYUKAWA: eval_targets_kt<K_REGYUKAWA>(false, a, st); break;
+    case K_ATAN: eval_targets_kt<K_ATAN>(false, a, st); break;
+    case K_MQ: eval_targets_kt<K_MQ>(false, a, st); break;
+    case K_RBSU: eval_targets_kt<K_RBSU>(false, a, st); break;
+    case K_RBSV: eval_targets_kt<K_RBSV>(false, a, st); break;
+    default: eval_targets_kt<K_USER>(false, a, st);
     }
+    if (a.partial)
+        k_sum_segments<<<a.nitems, EV_CHUNK, 0, st>>>(a.items, a.leaf_node, a.t_ibeg, a.t_numpar, 0, a.partial,
+                                                        a.pstride, a.pot);
 }
 
-template <int KT, bool HERM>
-static void eval_grids_t(const EvalGridsArgs &a, cudaStream_t st)
+template <int KT>
+static void eval_grids_hermite_t(const EvalGridsArgs &a, cudaStream_t st)
 {
-    int np1 = a.n + 1, P = np1 * np1 * np1;
-    size_t far = sizeof(double) * (size_t)(3 * np1 + P);
-    size_t near = sizeof(double4) * PP_TILE;
-    size_t sm = far > near ? far : near;
-    auto fn = k_eval_grids<KT, HERM>;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    fn<<<a.nitems, EV_THREADS, sm, st>>>(a.n, a.items, a.t_grid, a.c_off, a.c_idx, a.p_off, a.p_idx, a.s_ibeg,
-                                         a.s_numpar, a.s_grid, a.Q, a.sx, a.sy, a.sz, a.sq, a.kp, a.kp2, a.Phi);
+    k_eval_grids_hermite<KT><<<a.nitems, EV_THREADS, sizeof(double4) * PP_TILE, st>>>(
+        a.n, a.items, a.t_grid, a.p_off, a.p_idx, a.s_ibeg, a.s_numpar, a.sx, a.sy, a.sz, a.sq, a.kp, a.Phi);
 }
 
 // Grid outputs (CP, CC) exist for all but the periodic kernels (atan, MQ).
 void launch_eval_grids(int kernel, bool hermite, const EvalGridsArgs &a, cudaStream_t st)
 {
     if (a.nitems <= 0) return;
-    switch (kernel) {
-    case K_COULOMB: hermite ? eval_grids_t<K_COULOMB, true>(a, st) : eval_grids_t<K_COULOMB, false>(a, st); break;
-    case K_YUKAWA: hermite ? eval_grids_t<K_YUKAWA, true>(a, st) : eval_grids_t<K_YUKAWA, false>(a, st); break;
-    case K_REGCOULOMB:
-        hermite ? eval_grids_t<K_REGCOULOMB, true>(a, st) : eval_grids_t<K_REGCOULOMB, false>(a, st);
-        break;
-    case K_SINOVERR: hermite ? eval_grids_t<K_SINOVERR, true>(a, st) : eval_grids_t<K_SINOVERR, false>(a, st); break;
-    case K_REGYUKAWA: eval_grids_t<K_REGYUKAWA, false>(a, st); break;
-    case K_RBSU: eval_grids_t<K_RBSU, false>(a, st); break;
-    case K_RBSV: eval_grids_t<K_RBSV, false>(a, st); break;
-    default: eval_grids_t<K_USER, false>(a, st);
+    if (hermite) {
+        switch (kernel) {
+        case K_COULOMB: eval_grids_hermite_t<K_COULOMB>(a, st); break;
+        case K_YUKAWA: eval_grids_hermite_t<K_YUKAWA>(a, st); break;
+        case K_REGCOULOMB: eval_grids_hermite_t<K_REGCOULOMB>(a, st); break;
+        default: eval_grids_hermite_t<K_SINOVERR>(a, st);
+        }
+        return;
     }
+    switch (kernel) {
+    case K_COULOMB: eval_grids_kt<K_COULOMB>(a, st); break;
+    case K_YUKAWA: eval_grids_kt<K_YUKAWA>(a, st); break;
+    case K_REGCOULOMB: eval_grids_kt<K_REGCOULOMB>(a, st); break;
+    case K_SINOVERR: eval_grids_kt<K_SINOVERR>(a, st); break;
+    case K_REGYUKAWA: eval_grids_kt<K_REGYUKAWA>(a, st); break;
+    case K_RBSU: eval_grids_kt<K_RBSU>(a, st); break;
+    case K_RBSV: eval_grids_kt<K_RBSV>(a, st); break;
+    default: eval_grids_kt<K_USER>(a, st);
+    }
+    if (a.partial)
+        k_sum_segments<<<a.nitems, EV_CHUNK, 0, st>>>(a.items, nullptr, nullptr, nullptr,
+                                                        (a.n + 1) * (a.n + 1) * (a.n + 1), a.partial, a.pstride, a.Phi);
 }
 
 void launch_l2p(int n, bool hermite, int nitems, const int2 *items, const int *leaf_node, const int *parent,
@@ -1101,26 +933,29 @@ void launch_l2p(int n, bool hermite, int nitems, const int2 *items, const int *l
     }
 }
 
+// Enough parts for about three waves of resident blocks, each of at least one
+// source tile.
+int direct_parts(int nt, int ns)
+{
+    const int blocks = std::max(1, (nt + EV_CHUNK - 1) / EV_CHUNK);
+    return std::max(1, std::min(3 * 8 * 148 / blocks, ns / 512));
+}
+
 void launch_direct(int kernel, int nt, int ns, const double *tx, const double *ty, const double *tz,
-                   const double *sx, const double *sy, const double *sz, const double *sq, double kp, double *out,
-                   cudaStream_t st, double kp2)
+                   const double *sx, const double *sy, const double *sz, const double *sq, double kp, double kp2,
+                   double *partial, double *out, cudaStream_t st)
 {
     if (nt <= 0) return;
-    int grid = (nt + EV_THREADS - 1) / EV_THREADS;
-#define BT_DIRECT(K) k_direct<K><<<grid, EV_THREADS, 0, st>>>(nt, ns, tx, ty, tz, sx, sy, sz, sq, kp, kp2, out)
+    const int parts = direct_parts(nt, ns);
+    double *dst = parts > 1 ? partial : out;
+#define BT_DIRECT(K) case K: direct_kt<K>(nt, ns, parts, tx, ty, tz, sx, sy, sz, sq, kp, kp2, dst, st); break;
     switch (kernel) {
-    case K_COULOMB: BT_DIRECT(K_COULOMB); break;
-    case K_YUKAWA: BT_DIRECT(K_YUKAWA); break;
-    case K_REGCOULOMB: BT_DIRECT(K_REGCOULOMB); break;
-    case K_REGYUKAWA: BT_DIRECT(K_REGYUKAWA); break;
-    case K_ATAN: BT_DIRECT(K_ATAN); break;
-    case K_SINOVERR: BT_DIRECT(K_SINOVERR); break;
-    case K_MQ: BT_DIRECT(K_MQ); break;
-    case K_RBSU: BT_DIRECT(K_RBSU); break;
-    case K_RBSV: BT_DIRECT(K_RBSV); break;
-    default: BT_DIRECT(K_USER);
+        BT_DIRECT(K_COULOMB) BT_DIRECT(K_YUKAWA) BT_DIRECT(K_REGCOULOMB) BT_DIRECT(K_REGYUKAWA) BT_DIRECT(K_ATAN)
+        BT_DIRECT(K_SINOVERR) BT_DIRECT(K_MQ) BT_DIRECT(K_RBSU) BT_DIRECT(K_RBSV)
+    default: direct_kt<K_USER>(nt, ns, parts, tx, ty, tz, sx, sy, sz, sq, kp, kp2, dst, st);
     }
 #undef BT_DIRECT
+    if (parts > 1) k_sum_parts<<<(nt + 255) / 256, 256, 0, st>>>(nt, parts, partial, out);
 }
 
 }  // namespace bt

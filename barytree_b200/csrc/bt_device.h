@@ -8,25 +8,38 @@
 
 namespace bt {
 
+// FP64 evaluation kernels: outputs per work item, and the segments that each
+// output's interaction list is summed in.  With `partial` set, every segment
+// of an item has a block of its own and leaves its sums there (pstride outputs
+// per segment); the launcher adds them in order.  Without it one block sums
+// the segments.  Both give the same bits.
+constexpr int EV_THREADS = 128;
+constexpr int EV_CHUNK = 2 * EV_THREADS;
+constexpr int EV_SEGS = 16;
+// In a particle-output list: the source node's box meets the target leaf's, so
+// a source can coincide with a target and the skipping rule is tested.
+constexpr int EV_MEETS = (int)0x80000000;
+
 struct EvalTargetsArgs {
     int n, nitems;
-    const int2 *items;            // (target leaf unit, chunk), sorted by cost
+    const int2 *items;            // (target leaf unit, chunk of EV_CHUNK targets), sorted by cost
     const int *leaf_node;         // unit -> target node
     const int *t_ibeg, *t_numpar;
     const int64_t *a_off; const int *a_idx;   // source clusters per unit
-    const int64_t *d_off; const int *d_idx;   // source nodes per unit
+    const int64_t *d_off; const int *d_idx;   // source nodes per unit (with EV_MEETS)
     const int *s_ibeg, *s_numpar;
     const double *s_grid, *Q;
     const double *sx, *sy, *sz, *sq;
     const double *tx, *ty, *tz;
     double kp, kp2;                             // kernel_params[0], [1]
     double *pot;
-    int tb = 1;                                 // targets per thread (1 or 2): items of tb * 128 targets
+    double *partial = nullptr;
+    size_t pstride = 0;
 };
 
 struct EvalGridsArgs {
     int n, nitems;
-    const int2 *items;            // (target node, chunk of grid points)
+    const int2 *items;            // (target node, chunk of EV_CHUNK grid points (Hermite: EV_THREADS))
     const double *t_grid;
     const int64_t *c_off; const int *c_idx;   // source clusters (M2L) per target node
     const int64_t *p_off; const int *p_idx;   // source nodes (CP) per target node
@@ -35,6 +48,8 @@ struct EvalGridsArgs {
     const double *sx, *sy, *sz, *sq;
     double kp, kp2;                             // kernel_params[0], [1]
     double *Phi;
+    double *partial = nullptr;                  // Lagrange only
+    size_t pstride = 0;
 };
 
 void launch_p2m(int n, bool hermite, int nleaves, const int *leaves, int nnodes, const int *ibeg, const int *numpar,
@@ -59,10 +74,9 @@ void launch_m2m(int n, int nparents, const int *parents, const int *nchild, cons
 void launch_l2l(int n, int nparents, const int *parents, const int *nchild, const int *child, const double *grid,
                 double *Phi, cudaStream_t st);
 void launch_eval_targets(int kernel, bool hermite, const EvalTargetsArgs &a, cudaStream_t st);
-// Targets per work item of launch_eval_targets with tb targets per thread, and
-// the tb to use for target leaves with count[u] targets.
-int fp64_targets_chunk(int tb);
-int fp64_targets_per_thread(int nunits, const int *count);
+// Whether `items` work items are too few to fill the GPU with one block each
+// (then every segment gets its own block).
+bool eval64_split(size_t items);
 void launch_eval_grids(int kernel, bool hermite, const EvalGridsArgs &a, cudaStream_t st);
 void launch_l2p(int n, bool hermite, int nitems, const int2 *items, const int *leaf_node, const int *parent,
                 const int *t_ibeg, const int *t_numpar, const double *t_grid, const double *box_len,
@@ -72,8 +86,11 @@ void launch_scatter(int n, const int *order, const double *src, double *dst, cud
 // dst[i] = src[order[i]] (inputs in caller order -> tree order)
 void launch_gather(int n, const int *order, const double *src, double *dst, cudaStream_t st);
 float run_probe(int which, int sms, double *ops, void *scratch, cudaStream_t st);
+// Parts that the direct sum splits its sources into (partial sums: parts * nt
+// doubles when parts > 1).
+int direct_parts(int nt, int ns);
 void launch_direct(int kernel, int nt, int ns, const double *tx, const double *ty, const double *tz,
-                   const double *sx, const double *sy, const double *sz, const double *sq, double kp, double *out,
-                   cudaStream_t st, double kp2 = 0.0);
+                   const double *sx, const double *sy, const double *sz, const double *sq, double kp, double kp2,
+                   double *partial, double *out, cudaStream_t st);
 
 }  // namespace bt

@@ -1,0 +1,8 @@
+// bt_eval64_coulomb.cu -- FP64 evaluation kernels: Coulomb.
+#include "bt_eval64.cuh"
+
+namespace bt {
+
+BT_EVAL64_INSTANTIATE(K_COULOMB)
+
+}  // namespace bt
