@@ -87,43 +87,38 @@ __constant__ const double2 exp64_table[EXP64_TAB] = {      // {2^(j/64) rounded,
 
 struct Exp64 {
     double chi, clo;        // -kappa * 64 / ln2 in two parts
+    int rmax;               // upper half of the r where exp is 2^-1101
     const double2 *tab;     // the table in shared memory
 };
 
+// kappa >= 0
 __device__ __forceinline__ Exp64 exp64_make(double kappa, const double2 *tab)
 {
     constexpr double hi = 92.33248261689366, lo = 1.3027375194195861e-15;     // 64 / ln2
     Exp64 c;
     c.chi = -kappa * hi;
     c.clo = fma(-kappa, hi, -c.chi) - kappa * lo;
+    c.rmax = __double2hiint(1101.0 * 0.6931471805599453 / kappa);             // kappa 0: infinity
     c.tab = tab;
     return c;
 }
 
-// v 2^(n/64 rounded down) outside the exponent range of the integer addition
-static __device__ __noinline__ double exp64_edge(double v, double n, double t)
-{
-    if (!(fabs(n) < 1.0e9)) return t < 0.0 ? 0.0 : t > 0.0 ? HUGE_VAL : t;   // t NaN: NaN
-    const int k = max(-2000, min(2000, (int)n >> 6)), k1 = k / 2, k2 = k - k1;
-    // two exact powers of two, so that a subnormal result is rounded once
-    return v * __hiloint2double((k1 + 1023) << 20, 0) * __hiloint2double((k2 + 1023) << 20, 0);
-}
-
+// r >= 0 (a NaN may give any value).  No branch, so that the compiler can
+// interleave several values: r is cut off where exp is below every normal
+// number, and a result below 2^-1021 is replaced by one below 2^-1021.
 __device__ __forceinline__ double exp64(double r, const Exp64 &c)
 {
     constexpr double magic = 6755399441055744.0;            // 1.5 * 2^52
     constexpr double c1 = 0.010830424696249145, c2 = 5.86490495505617e-05, c3 = 2.1173137155464776e-07,
                      c4 = 5.732851688640402e-10, c5 = 1.2417843701716925e-12;   // (ln2 / 64)^i / i!
+    r = __hiloint2double(min(__double2hiint(r), c.rmax), __double2loint(r));
     const double m = fma(r, c.chi, magic), n = m - magic;
     const double f = fma(r, c.clo, fma(r, c.chi, -n));
     const double p = f * fma(f, fma(f, fma(f, fma(f, c5, c4), c3), c2), c1);
-    const int lo = __double2loint(m), k = lo >> 6;
+    const int lo = __double2loint(m);
     const double2 T = c.tab[lo & (EXP64_TAB - 1)];
     const double v = T.x + fma(T.x, p, T.y);
-    // n does not fit 32 bits, or v 2^k is not a normal number
-    if ((__double2hiint(m) - 0x43380000) != (lo >> 31) || (unsigned)(k + 1021) > 2043u)
-        return exp64_edge(v, n, r * c.chi);
-    return __hiloint2double(__double2hiint(v) + (k << 20), __double2loint(v));
+    return __hiloint2double(__double2hiint(v) + (max(lo >> 6, -1022) << 20), __double2loint(v));
 }
 
 }  // namespace bt
