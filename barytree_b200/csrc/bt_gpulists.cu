@@ -31,13 +31,30 @@ namespace bt {
 
 namespace {
 
-constexpr int GL_THREADS = 64;
-constexpr int GL_MAX_STACK = 384;          // shared-memory stack slots per thread (98 KB per block)
+constexpr int GL_THREADS = 32;           // one warp: the batches of a small system spread over more SMs
+constexpr int GL_MAX_STACK = 384;          // shared-memory stack slots per thread (49 KB per block)
 
+// What a node is to the batch; in the upper bits of a stack entry.
+enum { GL_OPEN = 0, GL_CLUSTER = 1, GL_DIRECT = 2 };
+constexpr int GL_SHIFT = 29, GL_NODE = (1 << GL_SHIFT) - 1;      // node numbers fit 29 bits (checked by the host)
+
+__device__ __forceinline__ int gl_class(const double4 B, const double4 g, const int2 cn, double theta, double thr)
+{
+    const double tx = __dsub_rn(B.x, g.x), ty = __dsub_rn(B.y, g.y), tz = __dsub_rn(B.z, g.z);
+    const double dist = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(tx, tx), __dmul_rn(ty, ty)), __dmul_rn(tz, tz)));
+    if (__dadd_rn(g.w, B.w) < __dmul_rn(dist, theta) && g.w != 0.0 && thr < (double)cn.x) return GL_CLUSTER;
+    return cn.y == 0 ? GL_DIRECT : GL_OPEN;
+}
+
+// Opening a node classifies all its children at once, so that up to eight
+// nodes' loads and square roots are in flight together; the stack holds
+// classified nodes.  Classifying each node when it was popped made the walk
+// one chain of memory latencies (125 us for 5,000 particles in 133 leaves,
+// 330 us for 250,000 targets; the list order is the same).
 template <bool FILL>
 __global__ void __launch_bounds__(GL_THREADS)
 k_pc_traverse(int nb, const double4 *__restrict__ bat, const int *__restrict__ broot,
-              const double4 *__restrict__ geo, const int2 *__restrict__ cnt_nc, const int *__restrict__ child,
+              const double4 *__restrict__ geo, const int2 *__restrict__ cnt_nc, const int4 *__restrict__ child,
               double theta, double thr, int depth_cap, int *__restrict__ counts, const int64_t *__restrict__ aoff,
               const int64_t *__restrict__ poff, int *__restrict__ aidx, int *__restrict__ pidx,
               int *__restrict__ overflow)
@@ -49,26 +66,38 @@ k_pc_traverse(int nb, const double4 *__restrict__ bat, const int *__restrict__ b
     int sp = 0, na = 0, np = 0;
     int *a_out = FILL ? aidx + aoff[b] : nullptr, *p_out = FILL ? pidx + poff[b] : nullptr;
     const int root = broot[b];
-    if (root >= 0) stk[threadIdx.x] = root, sp = 1;
+    if (root >= 0) stk[threadIdx.x] = root | gl_class(B, geo[root], cnt_nc[root], theta, thr) << GL_SHIFT, sp = 1;
     while (sp) {
         sp--;
-        const int node = stk[sp * GL_THREADS + threadIdx.x];
-        const double4 g = geo[node];
-        const double tx = __dsub_rn(B.x, g.x), ty = __dsub_rn(B.y, g.y), tz = __dsub_rn(B.z, g.z);
-        const double dist = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(tx, tx), __dmul_rn(ty, ty)), __dmul_rn(tz, tz)));
-        const int2 cn = cnt_nc[node];      // numpar, nchild
-        if (__dadd_rn(g.w, B.w) < __dmul_rn(dist, theta) && g.w != 0.0 && thr < (double)cn.x) {
+        const int entry = stk[sp * GL_THREADS + threadIdx.x], node = entry & GL_NODE, cls = entry >> GL_SHIFT;
+        if (cls == GL_CLUSTER) {
             if (FILL) a_out[na] = node;
             na++;
-        } else if (cn.y == 0) {
+        } else if (cls == GL_DIRECT) {
             if (FILL) p_out[np] = node;
             np++;
         } else {
-            if (sp + cn.y > depth_cap) {
+            const int nc = cnt_nc[node].y;
+            if (sp + nc > depth_cap) {
                 atomicExch(overflow, 1);
                 return;
             }
-            for (int i = cn.y - 1; i >= 0; i--) stk[(sp++) * GL_THREADS + threadIdx.x] = child[8 * (size_t)node + i];
+            const int4 c0 = child[2 * (size_t)node], c1 = child[2 * (size_t)node + 1];
+            const int id[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+            double4 g[8];
+            int2 cn[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (i < nc) {
+                    g[i] = geo[id[i]];
+                    cn[i] = cnt_nc[id[i]];
+                }
+#pragma unroll
+            for (int i = 0; i < 8; i++)       // child i to slot nc - 1 - i: the first child is popped first
+                if (i < nc)
+                    stk[(sp + nc - 1 - i) * GL_THREADS + threadIdx.x] =
+                        id[i] | gl_class(B, g[i], cn[i], theta, thr) << GL_SHIFT;
+            sp += nc;
         }
     }
     if (!FILL) {
@@ -83,7 +112,7 @@ int gpu_pc_lists(const bt_tree *trav, const bt_tree *bat, const bt_params *o, vo
                  bt_csr *ap, bt_csr *pp, cudaStream_t st, long long *launches)
 {
     const int nb = bat->nleaves, nn = trav->n;
-    if (nb <= 0 || nn <= 0) return -1;
+    if (nb <= 0 || nn <= 0 || nn > GL_NODE) return -1;
     const int cap = 7 * trav->max_depth + 8;
     if (cap > GL_MAX_STACK) return -1;
     // device layout: geometry, counts/children, batches, roots, counts,
@@ -96,7 +125,7 @@ int gpu_pc_lists(const bt_tree *trav, const bt_tree *bat, const bt_params *o, vo
     };
     double4 *d_geo = (double4 *)take(sizeof(double4) * (size_t)nn);
     int2 *d_cn = (int2 *)take(sizeof(int2) * (size_t)nn);
-    int *d_child = (int *)take(sizeof(int) * 8 * (size_t)nn);
+    int4 *d_child = (int4 *)take(sizeof(int) * 8 * (size_t)nn);
     double4 *d_bat = (double4 *)take(sizeof(double4) * (size_t)nb);
     int *d_root = (int *)take(sizeof(int) * (size_t)nb);
     int *d_cnt = (int *)take(sizeof(int) * 2 * (size_t)nb);
