@@ -7,6 +7,7 @@
 //   charges:   Lagrange Q[node*P + j], Hermite Q[(node*8 + m)*P + j], with
 //              j = k1 + (n+1)*(k2 + (n+1)*k3) (x fastest, src/clusters/clusters.c:929-933)
 //   potentials on target grids: same layout as charges.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,6 +21,8 @@
 #include "bt_kernels.cuh"
 
 namespace bt {
+
+namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------------------
 // Upward pass
@@ -156,15 +159,36 @@ k_p2m_sep(const int *__restrict__ leaves, const int *__restrict__ ibeg, const in
 }
 
 // Per-axis basis matrix M[i][k] = L_k(child node i) of a parent grid
-// evaluated at a child's grid coordinates, for all three axes, into smem.
-__device__ void axis_matrices(int n, const double *pnodes, const double *cnodes, double *M)
+// evaluated at a child's grid coordinates, for all three axes, into smem:
+// lagrange_basis with a thread per entry (the divisions), then per row (the
+// sum in k order and its reciprocal), then per entry again.
+struct BasisScratch {
+    double inv[3 * MAXNP];
+    int ex[3 * MAXNP];
+};
+
+__device__ void axis_matrices(int n, const double *pnodes, const double *cnodes, double *M, BasisScratch &b)
 {
-    const int np1 = n + 1;
-    for (int w = threadIdx.x; w < 3 * np1; w += blockDim.x) {
-        int a = w / np1, i = w % np1;
-        double L[MAXNP];
-        lagrange_basis(n, pnodes + a * np1, cnodes[a * np1 + i], L);
-        for (int k = 0; k <= n; k++) M[(a * np1 + i) * np1 + k] = L[k];
+    const int np1 = n + 1, rows = 3 * np1;
+    for (int r = threadIdx.x; r < rows; r += blockDim.x) b.ex[r] = -1;
+    __syncthreads();
+    for (int w = threadIdx.x; w < rows * np1; w += blockDim.x) {
+        const int r = w / np1, k = w - r * np1, ax = r / np1;
+        const double d = cnodes[r] - pnodes[ax * np1 + k];
+        if (fabs(d) < DBL_MIN) atomicMax(&b.ex[r], k);
+        const double wk = ((k & 1) ? -1.0 : 1.0) * ((k == 0 || k == n) ? 0.5 : 1.0);
+        M[w] = wk / d;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+        double sum = 0.0;
+        for (int k = 0; k < np1; k++) sum += M[r * np1 + k];
+        b.inv[r] = 1.0 / sum;
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < rows * np1; w += blockDim.x) {
+        const int r = w / np1, k = w - r * np1;
+        M[w] = b.ex[r] >= 0 ? (k == b.ex[r] ? 1.0 : 0.0) : M[w] * b.inv[r];
     }
 }
 
@@ -212,50 +236,67 @@ __device__ void kron_apply(int n, const double *M, const double *in, double *t1,
 
 // M2M for the parents of one level (pc_comp_ms_modifiedF_child_to_parent,
 // src/clusters/clusters.c:379-582): Q[parent] = sum_children kron(M^T) Q[child].
-__global__ void k_m2m(int n, const int *__restrict__ parents, const int *__restrict__ nchild,
-                      const int *__restrict__ child, const double *__restrict__ grid, double *__restrict__ Q)
+// A cluster of eight blocks per parent, one per child: the children's terms
+// are formed side by side in the blocks' shared memory and added, in child
+// order, through distributed shared memory.  The upper levels hold few
+// parents, and one block per parent with its children in turn took 60 us a
+// level there (the chain of eight basis evaluations and contractions).
+constexpr int KRON_CHILDREN = 8;
+
+__global__ void __cluster_dims__(KRON_CHILDREN, 1, 1)
+k_m2m(int n, const int *__restrict__ parents, const int *__restrict__ nchild, const int *__restrict__ child,
+      const double *__restrict__ grid, double *__restrict__ Q)
 {
     extern __shared__ double sm[];
+    __shared__ BasisScratch bs;
     const int np1 = n + 1, P = np1 * np1 * np1;
-    const int p = parents[blockIdx.x];
+    const int p = parents[blockIdx.x / KRON_CHILDREN], c = blockIdx.x % KRON_CHILDREN, nc = nchild[p];
     double *M = sm;                        // 3*np1*np1
     double *in = M + 3 * np1 * np1;        // P
     double *t1 = in + P, *t2 = t1 + P, *acc = t2 + P;
-    for (int j = threadIdx.x; j < P; j += blockDim.x) acc[j] = 0.0;
-    const double *pn = grid + (size_t)p * 3 * np1;
-    for (int c = 0; c < nchild[p]; c++) {
-        int ch = child[8 * p + c];
-        axis_matrices(n, pn, grid + (size_t)ch * 3 * np1, M);
-        for (int j = threadIdx.x; j < P; j += blockDim.x) in[j] = Q[(size_t)ch * P + j];
+    cg::cluster_group cluster = cg::this_cluster();
+    if (c < nc) {
+        const int ch = child[8 * p + c];
+        for (int j = threadIdx.x; j < P; j += blockDim.x) {
+            in[j] = Q[(size_t)ch * P + j];
+            acc[j] = 0.0;
+        }
+        axis_matrices(n, grid + (size_t)p * 3 * np1, grid + (size_t)ch * 3 * np1, M, bs);
         __syncthreads();
         kron_apply(n, M, in, t1, t2, acc, true);
     }
-    for (int j = threadIdx.x; j < P; j += blockDim.x) Q[(size_t)p * P + j] = acc[j];
+    cluster.sync();
+    for (int j = c * blockDim.x + threadIdx.x; j < P; j += KRON_CHILDREN * blockDim.x) {
+        double s = 0.0;
+        for (int k = 0; k < nc; k++) s += *cluster.map_shared_rank(acc + j, k);
+        Q[(size_t)p * P + j] = s;
+    }
+    cluster.sync();                        // a block's shared memory stays until all have read it
 }
 
 // L2L for the parents of one level (cp_comp_pot_parent_to_child,
 // src/interaction_compute/interaction_compute_downpass.c:151-323):
-// Phi[child] += kron(M) Phi[parent].
+// Phi[child] += kron(M) Phi[parent], one block per child.
 __global__ void k_l2l(int n, const int *__restrict__ parents, const int *__restrict__ nchild,
                       const int *__restrict__ child, const double *__restrict__ grid, double *__restrict__ Phi)
 {
     extern __shared__ double sm[];
+    __shared__ BasisScratch bs;
     const int np1 = n + 1, P = np1 * np1 * np1;
-    const int p = parents[blockIdx.x];
+    const int p = parents[blockIdx.x / KRON_CHILDREN], c = blockIdx.x % KRON_CHILDREN;
+    if (c >= nchild[p]) return;
+    const int ch = child[8 * p + c];
     double *M = sm;
     double *in = M + 3 * np1 * np1;
     double *t1 = in + P, *t2 = t1 + P, *acc = t2 + P;
-    for (int j = threadIdx.x; j < P; j += blockDim.x) in[j] = Phi[(size_t)p * P + j];
-    const double *pn = grid + (size_t)p * 3 * np1;
-    for (int c = 0; c < nchild[p]; c++) {
-        int ch = child[8 * p + c];
-        axis_matrices(n, pn, grid + (size_t)ch * 3 * np1, M);
-        for (int j = threadIdx.x; j < P; j += blockDim.x) acc[j] = Phi[(size_t)ch * P + j];
-        __syncthreads();
-        kron_apply(n, M, in, t1, t2, acc, false);
-        for (int j = threadIdx.x; j < P; j += blockDim.x) Phi[(size_t)ch * P + j] = acc[j];
-        __syncthreads();
+    for (int j = threadIdx.x; j < P; j += blockDim.x) {
+        in[j] = Phi[(size_t)p * P + j];
+        acc[j] = Phi[(size_t)ch * P + j];
     }
+    axis_matrices(n, grid + (size_t)p * 3 * np1, grid + (size_t)ch * 3 * np1, M, bs);
+    __syncthreads();
+    kron_apply(n, M, in, t1, t2, acc, false);
+    for (int j = threadIdx.x; j < P; j += blockDim.x) Phi[(size_t)ch * P + j] = acc[j];
 }
 
 // Hermite P2M at every source node (pc_comp_ms_modifiedF_hermite,
@@ -586,7 +627,7 @@ __global__ void k_sum_segments(const int2 *__restrict__ items, const int *__rest
                                const double *__restrict__ partial, size_t pstride, double *__restrict__ out)
 {
     const int2 it = items[blockIdx.x];
-    const int i = it.y * EV_CHUNK + threadIdx.x;
+    const int i = it.y * blockDim.x + threadIdx.x;
     size_t t;
     if (leaf_node) {
         const int node = leaf_node[it.x];
@@ -840,7 +881,7 @@ void launch_m2m(int n, int nparents, const int *parents, const int *nchild, cons
     if (nparents <= 0) return;
     size_t sm = kron_smem(n);
     cudaFuncSetAttribute(k_m2m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_m2m<<<nparents, 256, sm, st>>>(n, parents, nchild, child, grid, Q);
+    k_m2m<<<KRON_CHILDREN * nparents, 256, sm, st>>>(n, parents, nchild, child, grid, Q);
 }
 
 void launch_l2l(int n, int nparents, const int *parents, const int *nchild, const int *child, const double *grid,
@@ -849,7 +890,7 @@ void launch_l2l(int n, int nparents, const int *parents, const int *nchild, cons
     if (nparents <= 0) return;
     size_t sm = kron_smem(n);
     cudaFuncSetAttribute(k_l2l, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_l2l<<<nparents, 256, sm, st>>>(n, parents, nchild, child, grid, Phi);
+    k_l2l<<<KRON_CHILDREN * nparents, 256, sm, st>>>(n, parents, nchild, child, grid, Phi);
 }
 
 // With fewer items than about four waves of resident blocks (8 blocks of
@@ -874,8 +915,13 @@ void launch_eval_targets(int kernel, bool hermite, const EvalTargetsArgs &a, cud
     default: eval_targets_kt<K_USER>(false, a, st);
     }
     if (a.partial)
-        k_sum_segments<<<a.nitems, EV_CHUNK, 0, st>>>(a.items, a.leaf_node, a.t_ibeg, a.t_numpar, 0, a.partial,
-                                                        a.pstride, a.pot);
+        launch_sum_segments(a.nitems, a.items, EV_CHUNK, a.leaf_node, a.t_ibeg, a.t_numpar, a.partial, a.pstride, a.pot, st);
+}
+
+void launch_sum_segments(int nitems, const int2 *items, int chunk, const int *leaf_node, const int *ibeg,
+                         const int *numpar, const double *partial, size_t pstride, double *out, cudaStream_t st)
+{
+    if (nitems > 0) k_sum_segments<<<nitems, chunk, 0, st>>>(items, leaf_node, ibeg, numpar, 0, partial, pstride, out);
 }
 
 template <int KT>

@@ -16,6 +16,8 @@ namespace bt {
 constexpr int EV_THREADS = 128;
 constexpr int EV_CHUNK = 2 * EV_THREADS;
 constexpr int EV_SEGS = 16;
+// Part s of EV_SEGS of the list [b, e).
+__host__ __device__ inline int64_t seg_begin(int64_t b, int64_t e, int s) { return b + (e - b) * s / EV_SEGS; }
 // In a particle-output list: the source node's box meets the target leaf's, so
 // a source can coincide with a target and the skipping rule is tested.
 constexpr int EV_MEETS = (int)0x80000000;
@@ -77,6 +79,10 @@ void launch_eval_targets(int kernel, bool hermite, const EvalTargetsArgs &a, cud
 // Whether `items` work items are too few to fill the GPU with one block each
 // (then every segment gets its own block).
 bool eval64_split(size_t items);
+// out = the sums of the segments, in order, for the items' targets (chunk a
+// multiple of 32 up to 1024).
+void launch_sum_segments(int nitems, const int2 *items, int chunk, const int *leaf_node, const int *ibeg,
+                         const int *numpar, const double *partial, size_t pstride, double *out, cudaStream_t st);
 void launch_eval_grids(int kernel, bool hermite, const EvalGridsArgs &a, cudaStream_t st);
 void launch_l2p(int n, bool hermite, int nitems, const int2 *items, const int *leaf_node, const int *parent,
                 const int *t_ibeg, const int *t_numpar, const double *t_grid, const double *box_len,

@@ -339,9 +339,6 @@ __device__ __noinline__ double again64(int n, const int *a_idx, int64_t a0, int6
     return acc;
 }
 
-// Part s of EV_SEGS of the list [b, e).
-__device__ __forceinline__ int64_t seg_begin(int64_t b, int64_t e, int s) { return b + (e - b) * s / EV_SEGS; }
-
 // acc of slice 0: the sum over the slices in order (all threads call).
 __device__ __forceinline__ void sum_slices(double *acc, double *red, const Lanes &w)
 {

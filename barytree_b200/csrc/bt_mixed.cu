@@ -22,6 +22,7 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "bt_device.h"
 #include "bt_f2.cuh"
 #include "bt_kernels.cuh"
 #include "bt_mixed.h"
@@ -515,7 +516,11 @@ __device__ __noinline__ float pp_tile_close(const Tile tl, int cm, float x, floa
 }
 
 // Particle-output evaluation, mixed precision.  Each thread owns TPT
-// targets of a work item (target leaf, chunk of MX_CHUNK targets).
+// targets of a work item (target leaf, chunk of MX_CHUNK targets), each warp
+// 32 * TPT consecutive ones; a warp beyond the leaf's last target only helps
+// to stage, so a leaf costs its targets rounded up to a warp's.  Each target's
+// lists are summed in EV_SEGS segments and the segments in order, as in the
+// FP64 kernels: a launch with few items runs one block per (item, segment).
 // Blocks of a work-queue launch take items (cost-sorted, longest first) from
 // a device counter until the queue is empty; without a queue, block b
 // evaluates item b.
@@ -529,7 +534,8 @@ __device__ __forceinline__ int next_item(int *queue, int *slot)
 }
 
 template <int KT, bool HERM, int TPT>
-__device__ __forceinline__ void targets_item(const MixedTargetsArgs &a, const int2 it, float *smf)
+__device__ __forceinline__ void targets_item(const MixedTargetsArgs &a, const int2 it, int seg0, int seg1, float *smf,
+                                             double *tot)
 {
     const int u = it.x;
     const int tnode = a.leaf_node[u];
@@ -539,119 +545,141 @@ __device__ __forceinline__ void targets_item(const MixedTargetsArgs &a, const in
     int tid[TPT];
 #pragma unroll
     for (int t = 0; t < TPT; t++) {
-        int ti = it.y * MX_CHUNK + t * (MX_CHUNK / TPT) + threadIdx.x;
+        const int ti = it.y * MX_CHUNK + (threadIdx.x >> 5) * 32 * TPT + t * 32 + (threadIdx.x & 31);
         act[t] = ti < tn;
+        tot[t * (MX_CHUNK / TPT) + threadIdx.x] = 0.0;
         tid[t] = tb + (act[t] ? ti : 0);
         float4 tp = a.tpos[tid[t]];
         x[t] = tp.x; y[t] = tp.y; z[t] = tp.z;
     }
+    const bool warp_on = it.y * MX_CHUNK + (int)(threadIdx.x >> 5) * 32 * TPT < tn;
     const double trad = a.t_rad[tnode];
     const double cx = a.t_ctr[3 * tnode], cy = a.t_ctr[3 * tnode + 1], cz = a.t_ctr[3 * tnode + 2];
     const float kc = (float)a.kc;
-    double acc[TPT];
+    const int64_t ab = a.a_off[u], ae = a.a_off[u + 1], db = a.d_off[u], de = a.d_off[u + 1];
+    for (int seg = seg0; seg < seg1; seg++) {
+        double acc[TPT];
 #pragma unroll
-    for (int t = 0; t < TPT; t++) acc[t] = 0.0;
-
-    // far field: source clusters
-    for (int64_t e = a.a_off[u]; e < a.a_off[u + 1]; e++) {
-        const int s = a.a_idx[e];
-        const int deg = a.a_deg ? a.a_deg[e] : a.n;
-        const int np1 = deg + 1, P = np1 * np1 * np1;
-        float *g = smf;
-        float *q = smf + 3 * 16;
-        const double *gs = a.s_grid[deg] + (size_t)s * 3 * np1;
-        for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) {
-            int ax = i / np1;
-            double c = ax == 0 ? cx : ax == 1 ? cy : cz;
-            g[ax * np1 + (i % np1)] = (float)(gs[i] - c);
-        }
-        float v[TPT];
-        if (HERM) {
-            const float *Qs = a.Q32[deg] + (size_t)s * 8 * P;
-            for (int i = threadIdx.x; i < 8 * P; i += blockDim.x) {
-                const int m = i / P;
-                const float v = Qs[i] * (m == 7 ? 15.0f : m >= 4 ? 3.0f : 1.0f);
-                if constexpr (far_packed<KT, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(v, v);
-                else q[i] = v;
+        for (int t = 0; t < TPT; t++) acc[t] = 0.0;
+        // far field: source clusters
+        for (int64_t e = seg_begin(ab, ae, seg), e1 = seg_begin(ab, ae, seg + 1); e < e1; e++) {
+            const int s = a.a_idx[e];
+            const int deg = a.a_deg ? a.a_deg[e] : a.n;
+            const int np1 = deg + 1, P = np1 * np1 * np1;
+            float *g = smf;
+            float *q = smf + 3 * 16;
+            const double *gs = a.s_grid[deg] + (size_t)s * 3 * np1;
+            for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) {
+                int ax = i / np1;
+                double c = ax == 0 ? cx : ax == 1 ? cy : cz;
+                g[ax * np1 + (i % np1)] = (float)(gs[i] - c);
             }
-            __syncthreads();
-            pc_cluster_herm_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, (float)a.kp, v);
-        } else {
-            const float *Qs = a.Q32[deg] + (size_t)s * P;
-            for (int i = threadIdx.x; i < P; i += blockDim.x) {
-                if constexpr (far_packed<KT, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(Qs[i], Qs[i]);
-                else q[i] = Qs[i];
-            }
-            __syncthreads();
-            pc_cluster_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, v);
-        }
-#pragma unroll
-        for (int t = 0; t < TPT; t++) acc[t] += (double)v[t];
-        __syncthreads();
-    }
-    // near field: source leaves, particles relative to their leaf centre
-    // fixed array strides (the tile length only bounds the loop): a runtime
-    // stride costs the Coulomb kernel 16 registers and a resident block
-    const int tile = a.tile;
-    const Tile tl{smf, smf + MX_TILE_MAX, smf + 2 * MX_TILE_MAX, smf + 3 * MX_TILE_MAX};
-    for (int64_t e = a.d_off[u]; e < a.d_off[u + 1]; e++) {
-        const int s = a.d_idx[e];
-        const bool near = a.d_flag[e] != 0;
-        const int sb = a.s_ibeg[s], sn = a.s_numpar[s];
-        const float ox = (float)(a.s_ctr[3 * s] - cx), oy = (float)(a.s_ctr[3 * s + 1] - cy),
-                    oz = (float)(a.s_ctr[3 * s + 2] - cz);
-        float xs[TPT], ys[TPT], zs[TPT];   // targets in the source leaf's frame
-#pragma unroll
-        for (int t = 0; t < TPT; t++) { xs[t] = x[t] - ox; ys[t] = y[t] - oy; zs[t] = z[t] - oz; }
-        // at least the smallest normal float, so that a coincident pair (r2
-        // == 0 after flushing) always takes the FP64 path with the skipping
-        // rule, also between single-particle leaves of radius 0
-        const double rr = MX_CLOSE_FRAC * (trad + a.s_rad[s]);
-        const float thr2 = fmaxf((float)(rr * rr), FLT_MIN);
-        for (int c0 = 0; c0 < sn; c0 += tile) {
-            const int cm = min(tile, sn - c0), cm4 = (cm + 3) & ~3;
-            for (int i = threadIdx.x; i < cm4; i += blockDim.x) {
-                const float4 p = i < cm ? a.spos[sb + c0 + i] : make_float4(MX_PAD_POS, MX_PAD_POS, MX_PAD_POS, 0.0f);
-                tl.x[i] = p.x; tl.y[i] = p.y; tl.z[i] = p.z; tl.q[i] = p.w;
-            }
-            __syncthreads();
-            float sum[TPT], mn[TPT];
-            if (near) {
-#pragma unroll
-                for (int t = 0; t < TPT; t++) mn[t] = FLT_MAX;
-                pp_tile<KT, true, TPT>(tl, cm4, xs, ys, zs, kc, sum, mn);
-                bool close = false;
-#pragma unroll
-                for (int t = 0; t < TPT; t++) close |= act[t] && mn[t] < thr2;
-                if (__any_sync(0xffffffffu, close)) {
-#pragma unroll
-                    for (int t = 0; t < TPT; t++)
-                        if (act[t] && mn[t] < thr2)
-                            sum[t] = pp_tile_close<KT>(tl, cm, xs[t], ys[t], zs[t], kc, thr2, a.tx64[tid[t]],
-                                                       a.ty64[tid[t]], a.tz64[tid[t]], a.sx64, a.sy64, a.sz64,
-                                                       a.sq64, sb + c0, a.kp, &acc[t]);
+            float v[TPT];
+            if (HERM) {
+                const float *Qs = a.Q32[deg] + (size_t)s * 8 * P;
+                for (int i = threadIdx.x; i < 8 * P; i += blockDim.x) {
+                    const int m = i / P;
+                    const float v = Qs[i] * (m == 7 ? 15.0f : m >= 4 ? 3.0f : 1.0f);
+                    if constexpr (far_packed<KT, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(v, v);
+                    else q[i] = v;
                 }
+                __syncthreads();
+                if (warp_on) pc_cluster_herm_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, (float)a.kp, v);
             } else {
-                pp_tile<KT, false, TPT>(tl, cm4, xs, ys, zs, kc, sum, mn);
+                const float *Qs = a.Q32[deg] + (size_t)s * P;
+                for (int i = threadIdx.x; i < P; i += blockDim.x) {
+                    if constexpr (far_packed<KT, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(Qs[i], Qs[i]);
+                    else q[i] = Qs[i];
+                }
+                __syncthreads();
+                if (warp_on) pc_cluster_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, v);
             }
 #pragma unroll
-            for (int t = 0; t < TPT; t++) acc[t] += (double)sum[t];
+            for (int t = 0; t < TPT; t++)
+                if (warp_on) acc[t] += (double)v[t];
             __syncthreads();
         }
-    }
+        // near field: source leaves, particles relative to their leaf centre
+        // fixed array strides (the tile length only bounds the loop): a runtime
+        // stride costs the Coulomb kernel 16 registers and a resident block
+        const int tile = a.tile;
+        const Tile tl{smf, smf + MX_TILE_MAX, smf + 2 * MX_TILE_MAX, smf + 3 * MX_TILE_MAX};
+        for (int64_t e = seg_begin(db, de, seg), e1 = seg_begin(db, de, seg + 1); e < e1; e++) {
+            const int s = a.d_idx[e];
+            const bool near = a.d_flag[e] != 0;
+            const int sb = a.s_ibeg[s], sn = a.s_numpar[s];
+            const float ox = (float)(a.s_ctr[3 * s] - cx), oy = (float)(a.s_ctr[3 * s + 1] - cy),
+                        oz = (float)(a.s_ctr[3 * s + 2] - cz);
+            float xs[TPT], ys[TPT], zs[TPT];   // targets in the source leaf's frame
 #pragma unroll
-    for (int t = 0; t < TPT; t++)
-        if (act[t]) a.pot[tid[t]] = acc[t];
+            for (int t = 0; t < TPT; t++) { xs[t] = x[t] - ox; ys[t] = y[t] - oy; zs[t] = z[t] - oz; }
+            // at least the smallest normal float, so that a coincident pair (r2
+            // == 0 after flushing) always takes the FP64 path with the skipping
+            // rule, also between single-particle leaves of radius 0
+            const double rr = MX_CLOSE_FRAC * (trad + a.s_rad[s]);
+            const float thr2 = fmaxf((float)(rr * rr), FLT_MIN);
+            for (int c0 = 0; c0 < sn; c0 += tile) {
+                const int cm = min(tile, sn - c0), cm4 = (cm + 3) & ~3;
+                for (int i = threadIdx.x; i < cm4; i += blockDim.x) {
+                    const float4 p = i < cm ? a.spos[sb + c0 + i] : make_float4(MX_PAD_POS, MX_PAD_POS, MX_PAD_POS, 0.0f);
+                    tl.x[i] = p.x; tl.y[i] = p.y; tl.z[i] = p.z; tl.q[i] = p.w;
+                }
+                __syncthreads();
+                float sum[TPT], mn[TPT];
+                if (!warp_on) {
+#pragma unroll
+                    for (int t = 0; t < TPT; t++) sum[t] = 0.0f;
+                } else if (near) {
+#pragma unroll
+                    for (int t = 0; t < TPT; t++) mn[t] = FLT_MAX;
+                    pp_tile<KT, true, TPT>(tl, cm4, xs, ys, zs, kc, sum, mn);
+                    bool close = false;
+#pragma unroll
+                    for (int t = 0; t < TPT; t++) close |= act[t] && mn[t] < thr2;
+                    if (__any_sync(0xffffffffu, close)) {
+#pragma unroll
+                        for (int t = 0; t < TPT; t++)
+                            if (act[t] && mn[t] < thr2)
+                                sum[t] = pp_tile_close<KT>(tl, cm, xs[t], ys[t], zs[t], kc, thr2, a.tx64[tid[t]],
+                                                           a.ty64[tid[t]], a.tz64[tid[t]], a.sx64, a.sy64, a.sz64,
+                                                           a.sq64, sb + c0, a.kp, &acc[t]);
+                    }
+                } else {
+                    pp_tile<KT, false, TPT>(tl, cm4, xs, ys, zs, kc, sum, mn);
+                }
+#pragma unroll
+                for (int t = 0; t < TPT; t++) acc[t] += (double)sum[t];
+                __syncthreads();
+            }
+        }
+        // the segment's sums: to the launch's partial array, or onto the total
+#pragma unroll
+        for (int t = 0; t < TPT; t++) {
+            if (a.partial) {
+                if (act[t]) a.partial[(size_t)seg * a.pstride + tid[t]] = acc[t];
+            } else {
+                tot[t * (MX_CHUNK / TPT) + threadIdx.x] += acc[t];
+            }
+        }
+    }
+    if (!a.partial)
+#pragma unroll
+        for (int t = 0; t < TPT; t++)
+            if (act[t]) a.pot[tid[t]] = tot[t * (MX_CHUNK / TPT) + threadIdx.x];
 }
 
 template <int KT, bool HERM, int TPT>
 __device__ __forceinline__ void eval_targets_mixed_body(const MixedTargetsArgs &a)
 {
     extern __shared__ float smf[];
+    __shared__ double tot[MX_CHUNK];
     __shared__ int slot;
     int w = a.queue ? next_item(a.queue, &slot) : blockIdx.x;
-    while (w < a.nitems) {
-        targets_item<KT, HERM, TPT>(a, a.items[w], smf);
+    // split: item-major within a segment, so the items stay longest first
+    const int nwork = a.partial ? a.nitems * EV_SEGS : a.nitems;
+    while (w < nwork) {
+        const int seg = w / a.nitems;
+        targets_item<KT, HERM, TPT>(a, a.items[w - seg * a.nitems], seg, a.partial ? seg + 1 : EV_SEGS, smf, tot);
         if (!a.queue) break;
         w = next_item(a.queue, &slot);
     }
@@ -807,7 +835,8 @@ static void eval_targets_mixed_t(const MixedTargetsArgs &a, cudaStream_t st)
     auto kernel = k_eval_targets_mixed<KT, HERM, TPT>;
     if constexpr (TPT == 2 && rb_blocks<KT, HERM>() > 0) kernel = k_eval_targets_mixed_rb<KT, HERM, TPT>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    int grid = a.queue ? queue_grid(kernel, MX_CHUNK / TPT, sm, a.nitems) : a.nitems;
+    const int nwork = a.partial ? a.nitems * EV_SEGS : a.nitems;
+    int grid = a.queue ? queue_grid(kernel, MX_CHUNK / TPT, sm, nwork) : nwork;
     kernel<<<grid, MX_CHUNK / TPT, sm, st>>>(a);
 }
 
@@ -825,7 +854,13 @@ void launch_eval_targets_mixed(int kernel, const MixedTargetsArgs &a, cudaStream
     if (kernel == 1) a.herm ? eval_targets_mixed_h<1, true>(a, st) : eval_targets_mixed_h<1, false>(a, st);
     else if (kernel == 2) a.herm ? eval_targets_mixed_h<2, true>(a, st) : eval_targets_mixed_h<2, false>(a, st);
     else a.herm ? eval_targets_mixed_h<3, true>(a, st) : eval_targets_mixed_h<3, false>(a, st);
+    if (a.partial)
+        launch_sum_segments(a.nitems, a.items, MX_CHUNK, a.leaf_node, a.t_ibeg, a.t_numpar, a.partial, a.pstride, a.pot, st);
 }
+
+// Below about four waves of resident blocks (6 on each of 148 SMs) every
+// segment of an item gets its own block.
+bool mixed_split(size_t items) { return items < (size_t)4 * 6 * 148; }
 
 template <int KT>
 static void eval_grids_mixed_t(const MixedGridsArgs &a, cudaStream_t st)

@@ -50,6 +50,8 @@ struct MixedTargetsArgs {
     double kp;                                  // kernel parameter (FP64 close pairs)
     double *pot;
     int tpt, tile;                              // targets per thread, near-field source tile
+    double *partial;                            // a block per (item, segment) leaves its sums here (or nullptr)
+    size_t pstride;
 };
 
 struct MixedGridsArgs {
@@ -73,6 +75,7 @@ void launch_rel_positions(int nleaves, const int *leaves, const int *ibeg, const
 void launch_to_f32(size_t n, const double *src, float *dst, cudaStream_t st);
 void launch_eval_targets_mixed(int kernel, const MixedTargetsArgs &a, cudaStream_t st);
 void launch_eval_grids_mixed(int kernel, const MixedGridsArgs &a, cudaStream_t st);
+bool mixed_split(size_t items);                               // few items: split them by segment
 int mixed_targets_chunk();                                   // targets per work item
 double mixed_kernel_constant(int kernel, double kernel_param);
 
