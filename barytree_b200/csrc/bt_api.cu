@@ -504,6 +504,26 @@ bool same_host(const double *a, const double *b, size_t n)
     return !diff;
 }
 
+// A batch whose systems are not all their own targets: which ones are (their
+// target and source trees are the same from the roots on).
+bool same_systems_possible(const bt_plan &pl, const Systems &sys)
+{
+    return sys.n > 1 && pl.prm.maxs == pl.prm.maxt && pl.prm.precision == BT_PRECISION_FP64;
+}
+
+void same_systems_host(bt_plan &pl, const Systems &sys, const double *tx, const double *ty, const double *tz,
+                       const double *sx, const double *sy, const double *sz)
+{
+    if (!same_systems_possible(pl, sys)) return;
+    pl.sys_same = (unsigned char *)calloc((size_t)sys.n, 1);
+    for (int k = 0; k < sys.n; k++) {
+        const size_t n = (size_t)(sys.toff[k + 1] - sys.toff[k]);
+        if (sys.soff[k + 1] - sys.soff[k] != (int64_t)n) continue;
+        const int64_t t = sys.toff[k], q = sys.soff[k];
+        pl.sys_same[k] = same_host(tx + t, sx + q, n) && same_host(ty + t, sy + q, n) && same_host(tz + t, sz + q, n);
+    }
+}
+
 // Build the host plan: copies, trees, lists.
 void build_plan(bt_plan &pl, const Systems &sys, const double *tx, const double *ty, const double *tz,
                 const double *sx, const double *sy, const double *sz, const double *sq)
@@ -524,6 +544,7 @@ void build_plan(bt_plan &pl, const Systems &sys, const double *tx, const double 
     } else {
         bt_parts_init(&pl.tgt, nt, tx, ty, tz, nullptr);
         bt_forest_build(&pl.tt, &pl.tgt, sys.n, sys.toff.data(), pl.prm.maxt);
+        same_systems_host(pl, sys, tx, ty, tz, sx, sy, sz);
     }
     bt_plan_lists(&pl);
 }
@@ -600,6 +621,14 @@ int build_plan_gpu(DeviceCtx *ctx, Arena &tarena, bt_plan &pl, const Systems &sy
         which = "target";
         e = bt::gpu_build_forest(sys.n, sys.toff.data(), tx, ty, tz, nullptr, o.maxt, ta, d_work, wbytes, &pl.tt, st,
                                  &launches);
+        if (!e && !inputs_on_device) {
+            same_systems_host(pl, sys, tx, ty, tz, sx, sy, sz);
+        } else if (!e && same_systems_possible(pl, sys)) {
+            pl.sys_same = (unsigned char *)calloc((size_t)sys.n, 1);
+            e = bt::gpu_systems_equal(sys.n, sys.toff.data(), sys.soff.data(), tx, ty, tz, sx, sy, sz, d_work, wbytes,
+                                      pl.sys_same, st);
+            launches++;
+        }
     }
     g_launches += launches;
     if (e) {
@@ -656,12 +685,13 @@ struct DevPlan {
     bool tc_up = false;         // leaf P2M on the tensor cores (bt_tc.cu)
     bool sharded = false;       // this call evaluates a share of the target leaves (others get 0)
     // symmetric near-field pairs (bt_sym.cu)
-    int sym_npairs = 0;
-    int sym_far_pairs = 0;      // the first pairs: boxes apart by more than the close-pair distance
+    int sym_nblocks = 0;
+    int sym_far_blocks = 0;     // the first blocks: pairs whose boxes are apart by more than the close-pair distance
     double *d_sbox = nullptr;   // node boxes (x0 x1 y0 y1 z0 z1) for the pairs within it
-    int2 *d_sym_pairs = nullptr;
+    int2 *d_sym_pairs = nullptr, *d_sym_blocks = nullptr;
     int64_t *d_sym_slot = nullptr, *d_sym_in_off = nullptr, *d_sym_in_slot = nullptr;
     float *d_sym_partial = nullptr;
+    double *d_sym_partial64 = nullptr;      // FP64 path
     int *d_err = nullptr;       // set by a tensor-core kernel whose bounded wait expired
     int n = 0, P = 0, ns = 0, nt = 0, max_np1 = 0, kernel = 0;
     double kp = 0.0;
@@ -689,7 +719,7 @@ struct DevPlan {
     int3 *d_hred = nullptr;                 // nodes with several chunks
     double *d_hpartial = nullptr;           // their partial moments
     int n_hchunks = 0, n_hred = 0;
-    // segment sums of the FP64 evaluation kernels where their items are few
+    // segment sums of the evaluation kernels where their items are few
     double *d_evpart = nullptr, *d_gridpart = nullptr;
 };
 
@@ -730,6 +760,8 @@ bt::MixedTargetsArgs mixed_targets_args(const DevPlan &v)
     a.t_rad = v.d_trad; a.s_rad = v.d_srad;
     a.tx64 = v.d_tx; a.ty64 = v.d_ty; a.tz64 = v.d_tz; a.sx64 = v.d_sx; a.sy64 = v.d_sy; a.sz64 = v.d_sz; a.sq64 = v.d_sq;
     a.kp = v.kp;
+    a.partial = v.d_evpart;
+    a.pstride = (size_t)v.nt;
     return a;
 }
 
@@ -970,7 +1002,7 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         // the symmetric pairs write only their own partial sums: their two
         // kernels run beside the particle-output kernel on two more streams,
         // joined before the gather adds them into the potentials
-        const bool fork = v.sym_npairs > 0 && fk && fk->side && fk->side2;
+        const bool fork = v.sym_nblocks > 0 && fk && fk->side && fk->side2;
         cudaStream_t sst = st, sst2 = st;
         if (fork) {
             CK(cudaEventRecord(fk->fork, st));
@@ -979,24 +1011,24 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
             sst = fk->side;
             sst2 = fk->side2;
         }
-        if (v.sym_npairs > 0) {
+        if (v.sym_nblocks > 0) {
             bt::SymArgs y;
-            y.npairs = v.sym_npairs; y.pair = v.d_sym_pairs; y.slot = v.d_sym_slot;
+            y.pair = v.d_sym_pairs; y.slot = v.d_sym_slot;
             y.ibeg = v.d_sibeg; y.numpar = v.d_snum; y.ctr = v.d_sctr; y.pos = v.d_spos;
             y.partial = v.d_sym_partial; y.kc = (float)bt::mixed_kernel_constant(v.kernel, v.kp);
             y.rad = v.d_srad; y.box = v.d_sbox; y.x64 = v.d_sx; y.y64 = v.d_sy; y.z64 = v.d_sz; y.q64 = v.d_sq;
             y.kp = v.kp;
             bt::SymArgs yc = y;
-            y.npairs = v.sym_far_pairs;
-            yc.npairs = v.sym_npairs - v.sym_far_pairs;
-            yc.pair += v.sym_far_pairs;
-            yc.slot += v.sym_far_pairs;
+            y.nblocks = v.sym_far_blocks;
+            y.block = v.d_sym_blocks;
+            yc.nblocks = v.sym_nblocks - v.sym_far_blocks;
+            yc.block = v.d_sym_blocks + v.sym_far_blocks;
             bt::launch_pp_sym(v.kernel, y, sst);
             bt::launch_pp_sym_close(v.kernel, yc, sst2);
-            launches += (y.npairs > 0) + (yc.npairs > 0);
+            launches += (y.nblocks > 0) + (yc.nblocks > 0);
         }
         bt::launch_eval_targets_mixed(v.kernel, a, st);
-        launches++;
+        launches += a.partial ? 2 : 1;
         if (fork) {
             CK(cudaGetLastError());
             CK(cudaEventRecord(fk->join, sst));
@@ -1004,7 +1036,7 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
             CK(cudaStreamWaitEvent(st, fk->join, 0));
             CK(cudaStreamWaitEvent(st, fk->join2, 0));
         }
-        if (v.sym_npairs > 0) {
+        if (v.sym_nblocks > 0) {
             bt::SymGatherArgs g;
             g.nleaves = v.T_nleaves; g.leaf_node = v.d_tleaves; g.ibeg = v.d_sibeg; g.numpar = v.d_snum;
             g.in_off = v.d_sym_in_off; g.in_slot = v.d_sym_in_slot; g.partial = v.d_sym_partial; g.pot = d_pot;
@@ -1019,8 +1051,34 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         a.sx = d_sx; a.sy = d_sy; a.sz = d_sz; a.sq = d_sq; a.tx = d_tx; a.ty = d_ty; a.tz = d_tz;
         a.kp = v.kp; a.kp2 = v.kp2; a.pot = d_pot;
         a.partial = v.d_evpart; a.pstride = (size_t)nt;
+        // the symmetric pairs beside the particle-output kernel, joined before
+        // the gather adds their slices
+        const bool fork = v.sym_nblocks > 0 && fk && fk->side;
+        if (fork) {
+            CK(cudaEventRecord(fk->fork, st));
+            CK(cudaStreamWaitEvent(fk->side, fk->fork, 0));
+        }
+        if (v.sym_nblocks > 0) {
+            bt::Sym64Args y;
+            y.nblocks = v.sym_nblocks; y.block = v.d_sym_blocks; y.pair = v.d_sym_pairs; y.slot = v.d_sym_slot; y.ibeg = d_sibeg; y.numpar = d_snum;
+            y.x = d_sx; y.y = d_sy; y.z = d_sz; y.q = d_sq; y.partial = v.d_sym_partial64; y.kp = v.kp;
+            bt::launch_pp_sym64(v.kernel, y, fork ? fk->side : st);
+            launches++;
+        }
         bt::launch_eval_targets(v.kernel, herm, a, st);
         launches += a.partial ? 2 : 1;
+        if (fork) {
+            CK(cudaGetLastError());
+            CK(cudaEventRecord(fk->join, fk->side));
+            CK(cudaStreamWaitEvent(st, fk->join, 0));
+        }
+        if (v.sym_nblocks > 0) {
+            bt::SymGather64Args g;
+            g.nleaves = v.T_nleaves; g.leaf_node = v.d_tleaves; g.ibeg = d_tibeg; g.numpar = d_tnum;
+            g.in_off = v.d_sym_in_off; g.in_slot = v.d_sym_in_slot; g.partial = v.d_sym_partial64; g.pot = d_pot;
+            bt::launch_sym_gather64(g, st);
+            launches++;
+        }
     }
     CK(cudaGetLastError());
     if (ev) CK(record(3));
@@ -1258,16 +1316,29 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     std::vector<int64_t> mx_doff, mx_cpoff;
     hvec<int> mx_didx, mx_cpidx;
     hvec<unsigned char> mx_dflag;
+    int max_leaf = 0;
+    for (int u = 0; u < T.nleaves; u++) max_leaf = std::max(max_leaf, T.numpar[T.leaves[u]]);
+    // targets that are the sources, and a kernel that is symmetric in r: the
+    // symmetric near-field pass.  FP64 takes it pair by pair (leaves of
+    // SYM64_MIN_LEAF to SYM_MAX_LEAF particles); a shard in FP64 evaluates
+    // all of its targets' potentials itself, and the static scratch holds no
+    // partial sums.
+    const bool sym_kernel = shape.sym && T.nleaves > 1 && o.kernel >= COULOMB && o.kernel <= REGULARIZED_COULOMB;
+    const bool sym_ok = pl.same_tree && sym_kernel;
+    const bool sym64 = (pl.same_tree || pl.sys_same) && sym_kernel && !mixed && !ssm && shape.nshards == 1 &&
+                       !arena.fixed && max_leaf >= bt::SYM64_MIN_LEAF;
+    if (mixed || sym64) {
+        std::vector<int> lf, lc;
+        leaf_ranges(S, lf, lc);
+        expand_to_leaves(pl.t_direct, S, lf, lc, mx_doff, mx_didx);
+        if (mixed) expand_to_leaves(pl.g_cp, S, lf, lc, mx_cpoff, mx_cpidx);
+        mx_dflag.resize(mx_didx.size());
+    }
     if (mixed) {
         sctr.resize(3 * (size_t)S.n);
         tctr.resize(3 * (size_t)T.n);
         for (int i = 0; i < S.n; i++) { sctr[3 * i] = S.xm[i]; sctr[3 * i + 1] = S.ym[i]; sctr[3 * i + 2] = S.zm[i]; }
         for (int i = 0; i < T.n; i++) { tctr[3 * i] = T.xm[i]; tctr[3 * i + 1] = T.ym[i]; tctr[3 * i + 2] = T.zm[i]; }
-        std::vector<int> lf, lc;
-        leaf_ranges(S, lf, lc);
-        expand_to_leaves(pl.t_direct, S, lf, lc, mx_doff, mx_didx);
-        expand_to_leaves(pl.g_cp, S, lf, lc, mx_cpoff, mx_cpidx);
-        mx_dflag.resize(mx_didx.size());
 #pragma omp parallel for schedule(static)
         for (int u = 0; u < T.nleaves; u++) {
             int t = T.leaves[u];
@@ -1281,6 +1352,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             }
         }
     }
+    if (sym64) std::fill(mx_dflag.begin(), mx_dflag.end(), (unsigned char)0);     // one group of pairs
     pt.mark("plan: work items and near-field lists");
     // Symmetric near-field pairs: with the targets being the sources and a
     // symmetric kernel, leaf pairs {A, B} (A != B) that hold each other as
@@ -1290,17 +1362,25 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     // first, then the pairs within it (their own kernel); each group is
     // numbered by head unit (A < B), then by partner node, so the numbering
     // does not depend on the thread count.
-    hvec<int2> sym_pairs;
+    hvec<int2> sym_pairs, sym_blocks;
+    int64_t sym_far_blocks = 0;
     hvec<int64_t> sym_slot, sym_in_slot;
     std::vector<int64_t> sym_in_off;
     int64_t sym_total = 0, sym_far_pairs = 0;
-    int max_leaf = 0;
-    for (int u = 0; u < T.nleaves; u++) max_leaf = std::max(max_leaf, T.numpar[T.leaves[u]]);
-    if (mixed && pl.same_tree && shape.sym && max_leaf <= bt::SYM_MAX_LEAF &&
-        (o.kernel == COULOMB || o.kernel == YUKAWA || o.kernel == REGULARIZED_COULOMB) && T.nleaves > 1) {
+    bool sym_dropped = false;      // the pairs have left the per-target lists
+    auto sym64_leaf = [&](int v) { return S.numpar[v] >= bt::SYM64_MIN_LEAF && S.numpar[v] <= bt::SYM_MAX_LEAF; };
+    if ((mixed && sym_ok && max_leaf <= bt::SYM_MAX_LEAF) || sym64) {
         const int NU = T.nleaves;
-        std::vector<int> unit_of(T.n, -1);
-        for (int u = 0; u < NU; u++) unit_of[T.leaves[u]] = u;
+        // the source node that a unit's leaf is: the trees are one, or (FP64,
+        // a batch) the trees of a system whose targets are its sources have
+        // the same nodes from their roots on
+        std::vector<int> sleaf(NU), unit_of(S.n, -1);
+        for (int k = 0; k < T.nroots; k++)
+            for (int u = T.leaf_off[k]; u < T.leaf_off[k + 1]; u++)
+                sleaf[u] = pl.same_tree ? T.leaves[u]
+                           : pl.sys_same[k] ? T.leaves[u] - T.roots[k] + S.roots[k] : -1;
+        for (int u = 0; u < NU; u++)
+            if (sleaf[u] >= 0) unit_of[sleaf[u]] = u;
         // a pair belongs to the shard that owns its head (the lower leaf):
         // that shard evaluates it and gathers both sides, the partner's side
         // into targets another shard owns (the combining sum adds them)
@@ -1319,11 +1399,12 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             std::vector<uint64_t> keys;
 #pragma omp for schedule(static)
             for (int u = 0; u < NU; u++) {
-                const int A = T.leaves[u];
+                const int A = sleaf[u];
                 keys.clear();
                 for (int64_t k = mx_doff[u]; k < mx_doff[u + 1]; k++) {
                     const int B = mx_didx[k];
-                    if (B == A || unit_of[B] < 0) continue;
+                    if (A < 0 || B == A || unit_of[B] < 0) continue;
+                    if (sym64 && !(sym64_leaf(A) && sym64_leaf(B))) continue;
                     keys.push_back(((uint64_t)(uint32_t)B << 32) | (uint64_t)(k - mx_doff[u]));
                 }
                 std::sort(keys.begin(), keys.end());
@@ -1349,7 +1430,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         // both entries; every entry is written by one head at most
 #pragma omp parallel for schedule(static)
         for (int u = 0; u < NU; u++) {
-            const int A = T.leaves[u];
+            const int A = sleaf[u];
             for (int64_t j = mx_doff[u]; j < far_end[u]; j++) {
                 const int B = far[j], ub = unit_of[B];
                 if (B < A) continue;
@@ -1365,13 +1446,14 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         int64_t npaired = 0;       // entries in a pair, whichever shard evaluates it
 #pragma omp parallel for schedule(static) reduction(+ : npaired)
         for (int u = 0; u < NU; u++) {
-            const int A = T.leaves[u];
+            const int A = sleaf[u];
             int64_t heads[2] = {0, 0}, all = 0;
             for (int64_t j = mx_doff[u]; j < far_end[u]; j++)
                 if (rev[j] >= 0) {
                     npaired++;
                     const bool head = A < far[j];
-                    if (head ? owned[u] : owned[unit_of[far[j]]]) all++;
+                    // one slice from a pair this leaf heads, one per part of a head's particles
+                    if (head ? owned[u] : owned[unit_of[far[j]]]) all += head ? 1 : bt::sym_parts(S.numpar[far[j]]);
                     heads[fnear[j]] += head && owned[u] ? 1 : 0;
                 }
             poff0[u + 1] = heads[0];
@@ -1387,21 +1469,22 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         for (int u = 0; u < NU; u++) poff1[u + 1] += poff1[u];
         pt.mark("plan: symmetric: reverse look-ups");
         const int64_t npairs = poff1[NU];
+        hvec<int64_t> pid;
+        std::vector<int64_t> usz0(NU + 1, 0), usz1(NU + 1, 0);
         if (npaired > 0) {
             // pairs headed by each unit, and the pair number of each head entry
             sym_pairs.resize((size_t)npairs);
-            hvec<int64_t> pid(ne);
-            std::vector<int64_t> usz0(NU + 1, 0), usz1(NU + 1, 0);
+            pid.resize((size_t)ne);
 #pragma omp parallel for schedule(static)
             for (int u = 0; u < NU; u++) {
-                const int A = T.leaves[u];
+                const int A = sleaf[u];
                 int64_t p[2] = {poff0[u], poff1[u]}, sz[2] = {0, 0};
                 for (int64_t j = mx_doff[u]; j < far_end[u]; j++)
                     if (rev[j] >= 0 && A < far[j] && owned[u]) {
                         const int g = fnear[j];
                         pid[j] = p[g];
                         sym_pairs[p[g]++] = make_int2(A, far[j]);
-                        sz[g] += S.numpar[A] + S.numpar[far[j]];
+                        sz[g] += S.numpar[A] + (int64_t)bt::sym_parts(S.numpar[A]) * S.numpar[far[j]];
                     }
                 usz0[u + 1] = sz[0];
                 usz1[u + 1] = sz[1];
@@ -1410,17 +1493,38 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             usz1[0] = usz0[NU];
             for (int u = 0; u < NU; u++) usz1[u + 1] += usz1[u];
             sym_total = usz1[NU];
-            // each pair's partial sums: A's particles, then B's
+            // FP64 slices up to 32 GB; a larger system (some 70M particles)
+            // evaluates every direction
+            sym_dropped = !sym64 || sym_total <= (int64_t)1 << 32;
+        }
+        if (!sym_dropped) {
+            sym_pairs.clear();
+            sym_total = 0;
+        } else {
+            // each pair's partial sums: A's particles, then B's for every part
+            // of A; and its blocks, one per part.  All pairs of a unit's group
+            // have the unit's leaf as A, so their blocks are consecutive.
             sym_slot.resize((size_t)npairs);
+            std::vector<int64_t> boff0(NU + 1, 0), boff1(NU + 1, 0);
+            for (int u = 0; u < NU; u++) {
+                const int parts = sleaf[u] >= 0 ? bt::sym_parts(S.numpar[sleaf[u]]) : 0;
+                boff0[u + 1] = boff0[u] + (poff0[u + 1] - poff0[u]) * parts;
+                boff1[u + 1] = (poff1[u + 1] - poff1[u]) * parts;
+            }
+            boff1[0] = sym_far_blocks = boff0[NU];
+            for (int u = 0; u < NU; u++) boff1[u + 1] += boff1[u];
+            sym_blocks.resize((size_t)boff1[NU]);
 #pragma omp parallel for schedule(static)
             for (int u = 0; u < NU; u++) {
                 const int64_t pb[2] = {poff0[u], poff1[u]}, pe[2] = {poff0[u + 1], poff1[u + 1]};
-                const int64_t sb[2] = {usz0[u], usz1[u]};
+                const int64_t sb[2] = {usz0[u], usz1[u]}, bb[2] = {boff0[u], boff1[u]};
+                const int parts = sleaf[u] >= 0 ? bt::sym_parts(S.numpar[sleaf[u]]) : 0;
                 for (int g = 0; g < 2; g++) {
-                    int64_t s = sb[g];
+                    int64_t s = sb[g], w = bb[g];
                     for (int64_t p = pb[g]; p < pe[g]; p++) {
                         sym_slot[p] = s;
-                        s += S.numpar[sym_pairs[p].x] + S.numpar[sym_pairs[p].y];
+                        s += S.numpar[sym_pairs[p].x] + (int64_t)parts * S.numpar[sym_pairs[p].y];
+                        for (int k = 0; k < parts; k++) sym_blocks[w++] = make_int2((int)p, k);
                     }
                 }
             }
@@ -1432,7 +1536,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             hvec<unsigned char> drop(ne);
 #pragma omp parallel for schedule(static)
             for (int u = 0; u < NU; u++) {
-                const int A = T.leaves[u];
+                const int A = sleaf[u];
                 int64_t w = ioff[u];
                 std::fill(drop.begin() + mx_doff[u], drop.begin() + mx_doff[u + 1], (unsigned char)0);
                 for (int64_t j = mx_doff[u]; j < far_end[u]; j++) {
@@ -1441,7 +1545,12 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
                     // both directions leave the lists; only this shard's pairs are gathered
                     drop[mx_doff[u] + fent[j]] = 1;
                     if (!(A < B ? owned[u] : owned[unit_of[B]])) continue;
-                    sym_in_slot[w++] = A < B ? sym_slot[pid[j]] : sym_slot[pid[rev[j]]] + S.numpar[B];
+                    if (A < B) {
+                        sym_in_slot[w++] = sym_slot[pid[j]];
+                        continue;
+                    }
+                    for (int k = 0; k < bt::sym_parts(S.numpar[B]); k++)
+                        sym_in_slot[w++] = sym_slot[pid[rev[j]]] + S.numpar[B] + (int64_t)k * S.numpar[A];
                 }
             }
             pt.mark("plan: symmetric: pairs and slots");
@@ -1477,21 +1586,25 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     int3 *d_hred = nullptr;
     double *d_hpartial = nullptr;
 
-    // FP64: near-field entries whose box meets the target leaf's, the only
-    // ones where a source can coincide with a target, carry EV_MEETS
+    // The near field of the FP64 kernels: what the symmetric pairs leave, or
+    // the plan's own list.  Entries whose box meets the target leaf's, the
+    // only ones where a source can coincide with a target, carry EV_MEETS.
+    const int64_t *near_off = sym64 && sym_dropped ? mx_doff.data() : pl.t_direct.off;
+    const int *near_idx = sym64 && sym_dropped ? mx_didx.data() : pl.t_direct.idx;
     hvec<int> didx64;
     if (!mixed && !ssm) {
-        didx64.resize((size_t)pl.t_direct.off[pl.t_direct.rows]);
+        didx64.resize((size_t)near_off[T.nleaves]);
 #pragma omp parallel for schedule(static)
         for (int u = 0; u < T.nleaves; u++) {
             const int t = T.leaves[u];
-            for (int64_t k = pl.t_direct.off[u]; k < pl.t_direct.off[u + 1]; k++) {
-                const int s = pl.t_direct.idx[k];
+            for (int64_t k = near_off[u]; k < near_off[u + 1]; k++) {
+                const int s = near_idx[k];
                 const bool meets = S.x0[s] <= T.x1[t] && T.x0[t] <= S.x1[s] && S.y0[s] <= T.y1[t] &&
                                    T.y0[t] <= S.y1[s] && S.z0[s] <= T.z1[t] && T.z0[t] <= S.z1[s];
                 didx64[k] = meets ? s | bt::EV_MEETS : s;
             }
         }
+        near_idx = didx64.data();
     }
 
     // device layout
@@ -1523,7 +1636,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     L.add(&d_tibeg, T.n); L.add(&d_tnum, T.n); L.add(&d_tnch, T.n); L.add(&d_tch, 8 * (size_t)T.n);
     L.add(&d_tpar, T.n); L.add(&d_tleaves, T.nleaves); L.add(&d_tlvl, T.lvl_off ? T.lvl_off[T.max_depth] : 0);
     L.add(&d_aoff, pl.t_approx.rows + 1); L.add(&d_aidx, pl.t_approx.off[pl.t_approx.rows]);
-    L.add(&d_doff, pl.t_direct.rows + 1); L.add(&d_didx, pl.t_direct.off[pl.t_direct.rows]);
+    L.add(&d_doff, pl.t_direct.rows + 1); L.add(&d_didx, near_off[pl.t_direct.rows]);
     L.add(&d_ccoff, pl.g_cc.rows + 1); L.add(&d_ccidx, pl.g_cc.off[pl.g_cc.rows]);
     L.add(&d_cpoff, pl.g_cp.rows + 1); L.add(&d_cpidx, pl.g_cp.off[pl.g_cp.rows]);
     L.add(&d_evitems, ev_items.size()); L.add(&d_griditems, grid_items.size()); L.add(&d_l2pitems, l2p_items.size());
@@ -1556,10 +1669,17 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     double *d_srad = nullptr, *d_trad = nullptr;
     float *d_xQ32[BT_MAX_DEGREE + 1] = {};
     int *d_xleaves[BT_MAX_DEGREE + 1] = {}, *d_xlvl[BT_MAX_DEGREE + 1] = {};
-    int2 *d_sym_pairs = nullptr;
+    int2 *d_sym_pairs = nullptr, *d_sym_blocks = nullptr;
     int64_t *d_sym_slot = nullptr, *d_sym_in_off = nullptr, *d_sym_in_slot = nullptr;
     float *d_sym_partial = nullptr;
     double *d_sbox = nullptr;
+    double *d_sym_partial64 = nullptr;
+    if (!sym_pairs.empty()) {
+        L.add(&d_sym_blocks, sym_blocks.size());
+        L.add(&d_sym_pairs, sym_pairs.size()); L.add(&d_sym_slot, sym_slot.size());
+        L.add(&d_sym_in_off, sym_in_off.size()); L.add(&d_sym_in_slot, sym_in_slot.size());
+        if (!mixed) L.add(&d_sym_partial64, (size_t)sym_total);
+    }
     if (mixed) {
         L.add(&d_spos, ns); L.add(&d_tpos, nt);
         if (need_src_clusters) L.add(&d_Q32, (size_t)S.n * P * nq);
@@ -1568,12 +1688,8 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         L.add(&d_mxcpoff, mx_cpoff.size()); L.add(&d_mxcpidx, mx_cpidx.size());
         if (pl.a_deg) L.add(&d_adeg, n_approx);
         L.add(&d_srad, S.n); L.add(&d_trad, T.n);
-        if ((int64_t)sym_pairs.size() > sym_far_pairs) L.add(&d_sbox, 6 * (size_t)S.n);
-        if (!sym_pairs.empty()) {
-            L.add(&d_sym_pairs, sym_pairs.size()); L.add(&d_sym_slot, sym_slot.size());
-            L.add(&d_sym_in_off, sym_in_off.size()); L.add(&d_sym_in_slot, sym_in_slot.size());
-            L.add(&d_sym_partial, (size_t)sym_total);
-        }
+        if ((int64_t)sym_blocks.size() > sym_far_blocks) L.add(&d_sbox, 6 * (size_t)S.n);
+        if (!sym_pairs.empty()) L.add(&d_sym_partial, (size_t)sym_total);
         for (size_t i = 0; i < xdeg.size(); i++) {
             size_t Pd = (size_t)(xdeg[i] + 1) * (xdeg[i] + 1) * (xdeg[i] + 1);
             L.add(&d_xgrid[i], xgrid[i].size());
@@ -1584,11 +1700,11 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         }
     }
 
-    // Segment sums of the FP64 evaluation kernels, where their work items are
+    // Segment sums of the evaluation kernels, where their work items are
     // few (the results are the same without them): up to EV_SEGS doubles per
     // target, or per grid point within a fixed bound.
     double *d_evpart = nullptr, *d_gridpart = nullptr;
-    if (!mixed && !ssm) {
+    if (!ssm) {
         const size_t room = arena.fixed ? (arena.cap > L.total() ? arena.cap - L.total() : 0) : (size_t)1 << 30;
         size_t need = 0;
         auto want = [&](double **p, size_t count) {
@@ -1596,8 +1712,8 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             need += sizeof(double) * count + 512;
             L.add(p, count);
         };
-        if (bt::eval64_split(ev_items.size())) want(&d_evpart, (size_t)bt::EV_SEGS * nt);
-        if (need_tgt_grids && !herm && bt::eval64_split(grid_items.size()))
+        if (mixed ? bt::mixed_split(ev_items.size()) : bt::eval64_split(ev_items.size())) want(&d_evpart, (size_t)bt::EV_SEGS * nt);
+        if (!mixed && need_tgt_grids && !herm && bt::eval64_split(grid_items.size()))
             want(&d_gridpart, (size_t)bt::EV_SEGS * T.n * P);
     }
 
@@ -1630,7 +1746,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         UP(d_tpar, T.parent, T.n); UP(d_tleaves, T.leaves, T.nleaves);
         if (T.lvl_off) UP(d_tlvl, T.lvl_nodes, T.lvl_off[T.max_depth]);
         UP(d_aoff, pl.t_approx.off, pl.t_approx.rows + 1); UP(d_aidx, pl.t_approx.idx, pl.t_approx.off[pl.t_approx.rows]);
-        UP(d_doff, pl.t_direct.off, pl.t_direct.rows + 1); UP(d_didx, didx64.empty() ? pl.t_direct.idx : didx64.data(), pl.t_direct.off[pl.t_direct.rows]);
+        UP(d_doff, near_off, pl.t_direct.rows + 1); UP(d_didx, near_idx, near_off[pl.t_direct.rows]);
         UP(d_ccoff, pl.g_cc.off, pl.g_cc.rows + 1); UP(d_ccidx, pl.g_cc.idx, pl.g_cc.off[pl.g_cc.rows]);
         UP(d_cpoff, pl.g_cp.off, pl.g_cp.rows + 1); UP(d_cpidx, pl.g_cp.idx, pl.g_cp.off[pl.g_cp.rows]);
         UP(d_evitems, ev_items.data(), ev_items.size());
@@ -1651,6 +1767,11 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             bt::launch_mul(ns, d_sq, d_sw, d_qw, st);
             launches += 3;
         }
+        if (!sym_pairs.empty()) {
+            UP(d_sym_blocks, sym_blocks.data(), sym_blocks.size());
+            UP(d_sym_pairs, sym_pairs.data(), sym_pairs.size()); UP(d_sym_slot, sym_slot.data(), sym_slot.size());
+            UP(d_sym_in_off, sym_in_off.data(), sym_in_off.size()); UP(d_sym_in_slot, sym_in_slot.data(), sym_in_slot.size());
+        }
         if (mixed) {
             UP(d_sctr, sctr.data(), sctr.size()); UP(d_tctr, tctr.data(), tctr.size());
             UP(d_mxdoff, mx_doff.data(), mx_doff.size()); UP(d_mxdidx, mx_didx.data(), mx_didx.size());
@@ -1663,10 +1784,6 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
                     b[0] = S.x0[i]; b[1] = S.x1[i]; b[2] = S.y0[i]; b[3] = S.y1[i]; b[4] = S.z0[i]; b[5] = S.z1[i];
                 }
                 UP(d_sbox, sbox.data(), sbox.size());
-            }
-            if (!sym_pairs.empty()) {
-                UP(d_sym_pairs, sym_pairs.data(), sym_pairs.size()); UP(d_sym_slot, sym_slot.data(), sym_slot.size());
-                UP(d_sym_in_off, sym_in_off.data(), sym_in_off.size()); UP(d_sym_in_slot, sym_in_slot.data(), sym_in_slot.size());
             }
             if (pl.a_deg) UP(d_adeg, pl.a_deg, n_approx);
             UP(d_srad, S.rad, S.n); UP(d_trad, T.rad, T.n);
@@ -1688,11 +1805,12 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         v.sharded = shape.nshards > 1;
         v.d_evpart = d_evpart; v.d_gridpart = d_gridpart;
         v.base_full = pl.a_deg == nullptr;
-        v.sym_npairs = (int)sym_pairs.size();
-        v.sym_far_pairs = (int)sym_far_pairs;
+        v.sym_nblocks = (int)sym_blocks.size();
+        v.sym_far_blocks = (int)sym_far_blocks;
+        v.d_sym_blocks = d_sym_blocks;
         v.d_sbox = d_sbox;
         v.d_sym_pairs = d_sym_pairs; v.d_sym_slot = d_sym_slot; v.d_sym_in_off = d_sym_in_off;
-        v.d_sym_in_slot = d_sym_in_slot; v.d_sym_partial = d_sym_partial;
+        v.d_sym_in_slot = d_sym_in_slot; v.d_sym_partial = d_sym_partial; v.d_sym_partial64 = d_sym_partial64;
         v.n = n; v.P = P; v.ns = ns; v.nt = nt; v.max_np1 = max_np1; v.kernel = o.kernel; v.kp = o.kp;
         v.S_n = S.n; v.S_nleaves = S.nleaves; v.S_max_depth = S.max_depth;
         v.T_n = T.n; v.T_nleaves = T.nleaves; v.T_max_depth = T.max_depth;

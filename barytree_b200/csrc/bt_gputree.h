@@ -41,4 +41,10 @@ int gpu_arrays_equal(const double *a, const double *b, size_t n, unsigned long l
 // Source line (bt_gputree.cu) of the last failing CUDA call of a build.
 int gpu_tree_fail_line();
 
+// equal[k] = 1 where system k's targets are its sources, bit for bit (device
+// arrays; synchronises).
+int gpu_systems_equal(int nsys, const int64_t *toff, const int64_t *soff, const double *tx, const double *ty,
+                      const double *tz, const double *sx, const double *sy, const double *sz, void *work,
+                      size_t work_bytes, unsigned char *equal, cudaStream_t st);
+
 }  // namespace bt

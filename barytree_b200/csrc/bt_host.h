@@ -73,6 +73,7 @@ typedef struct {
     unsigned char *a_deg;   /* per t_approx entry: interpolation degree (NULL: prm.degree) */
     long long sel_hist[14]; /* learned selection: entries per degree, [13] = direct instead */
     int same_tree;          /* the targets are the sources: tt is a copy of st            */
+    unsigned char *sys_same; /* else, per system of a batch: its targets are its sources (or NULL) */
 } bt_plan;
 
 /* bt_params.c */

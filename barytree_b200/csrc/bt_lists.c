@@ -250,4 +250,6 @@ void bt_plan_free(bt_plan *pl)
     for (int i = 0; i < 8; i++) bt_csr_free(c[i]);
     free(pl->a_deg);
     pl->a_deg = NULL;
+    free(pl->sys_same);
+    pl->sys_same = NULL;
 }

@@ -20,16 +20,21 @@
 // both sides' slices.  The main loop's sums are added to these at the end.
 // Self pairs (A with A) stay in the particle-output kernel.
 //
-// Work: one block per pair.  The block's threads hold A's targets, four per
-// thread in two packed FP32 pairs, in chunks of 512; B's particles stream
-// through shared memory, staged as {v, v} pairs.  Every 1/r feeds the
-// thread's A-side sums and, through a per-thread register per source, the
-// B side: each group of 16 sources is reduced across the warp by a
+// Work: one block per pair and part of SYM_PART of A's targets.  B's particles
+// stream through shared memory in tiles, staged as {v, v} pairs; the block's
+// warps divide a tile's sources, and each takes them against the part's
+// targets 128 at a time, four per thread in two packed FP32 pairs.  Every 1/r
+// feeds the thread's A-side sums and, through a per-thread register per
+// source, the B side: each group of 16 sources is reduced across the warp by a
 // reduce-scatter (16 shuffles for 16 sources; lanes 2i and 2i+1 end with
-// source i), then across the block's warps in a fixed order.  Both sides go to the
-// pair's own slices of a partial-sum array; k_sym_gather adds each leaf's
-// slices in FP64 in pair order.  No atomics: the potentials are the same bit
-// for bit on every run.
+// source i).  The warps' A-side sums are added in a fixed order.  Both sides
+// go to the pair's own slices of a partial-sum array (A's once, B's per part);
+// k_sym_gather adds each leaf's slices in FP64 in pair order.  No atomics: the
+// potentials are the same bit for bit on every run.
+// With the targets divided over the warps instead (512 per block and pass) a
+// leaf of 1,560 cost the lanes of 2,048; now it costs those of 1,664, every
+// warp has work, and a block is a quarter as long, which is what small
+// systems lack.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -58,8 +63,8 @@ constexpr int SY_THREADS = 128;
 #endif
 constexpr int SY_TPT = BT_SYM_TPT;
 constexpr int SY_NP = SY_TPT / 2;
-constexpr int SY_CHUNK = SY_TPT * SY_THREADS;  // targets of A per pass
-constexpr int SY_TILE = 512;                   // sources of B per shared-memory tile
+constexpr int SY_CHUNK = SY_TPT * 32;          // targets of A a warp holds at a time
+constexpr int SY_TILE = 256;                   // sources of B per shared-memory tile
 constexpr int SY_SB = 16;                      // sources per warp reduction
 constexpr int SY_WARPS = SY_THREADS / 32;
 constexpr float SY_PAD_POS = 1.0e18f;          // padding sources: far away, no charge
@@ -143,18 +148,19 @@ __device__ int near_box(int *out, int n, int base, const double *__restrict__ x,
 }
 
 template <int KT, bool CLAMP>
-__global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(SymArgs a)
+__global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(const __grid_constant__ SymArgs a)
 {
     __shared__ __align__(16) f2_t tile[SY_TILE][4];     // {x, x}, {y, y}, {z, z}, {q, q}
-    __shared__ float red[SY_WARPS][SY_TILE];
     __shared__ float accB[SYM_MAX_LEAF];
-    __shared__ double accA[SY_TPT][SY_THREADS];          // A side: each tile's FP32 sums, added in FP64
+    __shared__ double accA[SY_WARPS][SYM_PART];          // each warp's A side: FP32 sums per tile, added in FP64
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int2 pr = a.pair[blockIdx.x];
+    const int2 work = a.block[blockIdx.x];
+    const int2 pr = a.pair[work.x];
     const int A = pr.x, B = pr.y;
-    const int ia = a.ibeg[A], na = a.numpar[A], ib = a.ibeg[B], nb = a.numpar[B];
-    float *outA = a.partial + a.slot[blockIdx.x];
-    float *outB = outA + na;
+    const int a0 = work.y * SYM_PART, na = a.numpar[A], nb = a.numpar[B], pa = min(SYM_PART, na - a0);
+    const int ia = a.ibeg[A] + a0, ib = a.ibeg[B];
+    float *outA = a.partial + a.slot[work.x] + a0;
+    float *outB = a.partial + a.slot[work.x] + na + (size_t)work.y * nb;
     // A's targets in B's frame: positions relative to A's centre minus the offset of B's
     const float ox = (float)(a.ctr[3 * B] - a.ctr[3 * A]), oy = (float)(a.ctr[3 * B + 1] - a.ctr[3 * A + 1]),
                 oz = (float)(a.ctr[3 * B + 2] - a.ctr[3 * A + 2]);
@@ -165,13 +171,14 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(SymArg
         const double rr = MX_CLOSE_FRAC * (a.rad[A] + a.rad[B]);
         thr2 = fmaxf((float)(rr * rr), FLT_MIN);
         __shared__ int wcnt[SY_WARPS];
-        int *candA = reinterpret_cast<int *>(&tile[0][0]), *candB = candA + SYM_MAX_LEAF;
-        for (int i = threadIdx.x; i < na; i += SY_THREADS) outA[i] = 0.0f;
+        int *candA = reinterpret_cast<int *>(&accA[0][0]), *candB = candA + SYM_PART;
+        static_assert(sizeof(int) * (SYM_PART + SYM_MAX_LEAF) <= sizeof(accA), "the candidate lists live in accA");
+        for (int i = threadIdx.x; i < pa; i += SY_THREADS) outA[i] = 0.0f;
         for (int j = threadIdx.x; j < nb; j += SY_THREADS) outB[j] = 0.0f;
         // every pair with FP32 r^2 below thr2 lies within 1.01 thr of both boxes
         const double d = 1.01 * sqrt((double)thr2);
-        const int nca = near_box(candA, na, ia, a.x64, a.y64, a.z64, a.box + 6 * B, d, wcnt);
-        const int ncb = near_box(candB, nb, ib, a.x64, a.y64, a.z64, a.box + 6 * A, d, wcnt);
+        const int nca = near_box(candA, pa, ia, a.x64, a.y64, a.z64, a.box + 6 * B, d, wcnt);
+        const int ncb = nca > 0 ? near_box(candB, nb, ib, a.x64, a.y64, a.z64, a.box + 6 * A, d, wcnt) : 0;
         if (nca > 0 && ncb > 0) {
             float kcl, unused;
             f2_split(sym_kval<KT>(f2_make(thr2, thr2), kc2), kcl, unused);   // the clamped term's kernel value
@@ -199,39 +206,38 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(SymArg
                 (sideA ? outA[i] : outB[i]) = (float)c;
             }
         }
-        __syncthreads();                                  // the candidate lists live in the tile
+        __syncthreads();                                  // the candidate lists are done with
     }
+    const int nch = (pa + SY_CHUNK - 1) / SY_CHUNK;
     for (int j = threadIdx.x; j < nb; j += SY_THREADS) accB[j] = 0.0f;
-    for (int c0 = 0; c0 < na; c0 += SY_CHUNK) {
-        // targets c0 + threadIdx.x + k * SY_THREADS, k = 0..SY_TPT-1, packed as (0, 1), (2, 3), ...
-        f2_t X[SY_NP], Y[SY_NP], Z[SY_NP], QT[SY_NP], S[SY_NP];
-        bool act[SY_TPT];
-#pragma unroll
-        for (int p = 0; p < SY_NP; p++) {
-            const int t0 = c0 + threadIdx.x + (2 * p) * SY_THREADS, t1 = t0 + SY_THREADS;
-            act[2 * p] = t0 < na;
-            act[2 * p + 1] = t1 < na;
-            const float4 p0 = a.pos[ia + (act[2 * p] ? t0 : 0)], p1 = a.pos[ia + (act[2 * p + 1] ? t1 : 0)];
-            X[p] = f2_make(p0.x - ox, p1.x - ox);
-            Y[p] = f2_make(p0.y - oy, p1.y - oy);
-            Z[p] = f2_make(p0.z - oz, p1.z - oz);
-            QT[p] = f2_make(act[2 * p] ? p0.w : 0.0f, act[2 * p + 1] ? p1.w : 0.0f);   // absent targets add nothing
-            S[p] = f2_make(0.0f, 0.0f);
+    for (int i = lane; i < nch * SY_CHUNK; i += 32) accA[warp][i] = 0.0;
+    for (int s0 = 0; s0 < nb; s0 += SY_TILE) {
+        const int cm = min(SY_TILE, nb - s0), groups = (cm + SY_SB - 1) / SY_SB;
+        __syncthreads();                                  // the previous tile is done with
+        for (int i = threadIdx.x; i < groups * SY_SB; i += SY_THREADS) {
+            const float4 p = i < cm ? a.pos[ib + s0 + i] : make_float4(SY_PAD_POS, SY_PAD_POS, SY_PAD_POS, 0.0f);
+            tile[i][0] = f2_make(p.x, p.x);
+            tile[i][1] = f2_make(p.y, p.y);
+            tile[i][2] = f2_make(p.z, p.z);
+            tile[i][3] = f2_make(p.w, p.w);
         }
+        __syncthreads();
+        // the warp's sources of the tile, against every chunk of the part
+        const int b0 = groups * warp / SY_WARPS * SY_SB, b1 = groups * (warp + 1) / SY_WARPS * SY_SB;
+        for (int c = 0; c < nch && b0 < b1; c++) {
+            // targets c * SY_CHUNK + lane + 32 k, k = 0..SY_TPT-1, packed as (0, 1), (2, 3), ...
+            f2_t X[SY_NP], Y[SY_NP], Z[SY_NP], QT[SY_NP], S[SY_NP];
 #pragma unroll
-        for (int k = 0; k < SY_TPT; k++) accA[k][threadIdx.x] = 0.0;
-        for (int s0 = 0; s0 < nb; s0 += SY_TILE) {
-            const int cm = min(SY_TILE, nb - s0), cmb = (cm + SY_SB - 1) & ~(SY_SB - 1);
-            __syncthreads();                              // the previous tile is done with
-            for (int i = threadIdx.x; i < cmb; i += SY_THREADS) {
-                const float4 p = i < cm ? a.pos[ib + s0 + i] : make_float4(SY_PAD_POS, SY_PAD_POS, SY_PAD_POS, 0.0f);
-                tile[i][0] = f2_make(p.x, p.x);
-                tile[i][1] = f2_make(p.y, p.y);
-                tile[i][2] = f2_make(p.z, p.z);
-                tile[i][3] = f2_make(p.w, p.w);
+            for (int p = 0; p < SY_NP; p++) {
+                const int t0 = c * SY_CHUNK + lane + 64 * p, t1 = t0 + 32;
+                const float4 p0 = a.pos[ia + (t0 < pa ? t0 : 0)], p1 = a.pos[ia + (t1 < pa ? t1 : 0)];
+                X[p] = f2_make(p0.x - ox, p1.x - ox);
+                Y[p] = f2_make(p0.y - oy, p1.y - oy);
+                Z[p] = f2_make(p0.z - oz, p1.z - oz);
+                QT[p] = f2_make(t0 < pa ? p0.w : 0.0f, t1 < pa ? p1.w : 0.0f);   // absent targets add nothing
+                S[p] = f2_make(0.0f, 0.0f);
             }
-            __syncthreads();
-            for (int sb = 0; sb < cmb; sb += SY_SB) {
+            for (int sb = b0; sb < b1; sb += SY_SB) {
                 float v[SY_SB];
 #pragma unroll
                 for (int s = 0; s < SY_SB; s++) {
@@ -262,33 +268,29 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(SymArg
                 rs_stage<2, 4>(v, lane);
                 rs_stage<1, 2>(v, lane);
                 v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-                if ((lane & 1) == 0) red[warp][sb + (lane >> 1)] = v[0];
+                if ((lane & 1) == 0) {
+                    const int j = s0 + sb + (lane >> 1);
+                    if (j < nb) accB[j] += v[0];          // the source is this warp's alone
+                }
             }
-            // the tile's A-side sums into FP64 (FP32 chains of at most one tile)
+            // the chunk's A-side sums into FP64 (FP32 chains of at most a quarter of a tile)
 #pragma unroll
             for (int p = 0; p < SY_NP; p++) {
                 float lo, hi;
                 f2_split(S[p], lo, hi);
-                accA[2 * p][threadIdx.x] += (double)lo;
-                accA[2 * p + 1][threadIdx.x] += (double)hi;
-                S[p] = f2_make(0.0f, 0.0f);
+                accA[warp][c * SY_CHUNK + lane + 64 * p] += (double)lo;
+                accA[warp][c * SY_CHUNK + lane + 64 * p + 32] += (double)hi;
             }
-            __syncthreads();
-            // the block's B-side sum per source, warps in a fixed order
-            for (int j = threadIdx.x; j < cm; j += SY_THREADS) {
-                float r = red[0][j];
-#pragma unroll
-                for (int w = 1; w < SY_WARPS; w++) r += red[w][j];
-                accB[s0 + j] += r;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < SY_TPT; k++) {
-            const int t = c0 + threadIdx.x + k * SY_THREADS;
-            if (act[k]) outA[t] = (float)(CLAMP ? accA[k][threadIdx.x] + (double)outA[t] : accA[k][threadIdx.x]);
         }
     }
     __syncthreads();
+    // the warps' sums in a fixed order
+    for (int i = threadIdx.x; i < pa; i += SY_THREADS) {
+        double r = accA[0][i];
+#pragma unroll
+        for (int w = 1; w < SY_WARPS; w++) r += accA[w][i];
+        outA[i] = (float)(CLAMP ? r + (double)outA[i] : r);
+    }
     for (int j = threadIdx.x; j < nb; j += SY_THREADS) outB[j] = CLAMP ? accB[j] + outB[j] : accB[j];
 }
 
@@ -299,8 +301,9 @@ __global__ void k_sym_gather(SymGatherArgs a)
     if (k0 == k1) return;
     const int node = a.leaf_node[u];
     const int ib = a.ibeg[node], nb = a.numpar[node];
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) {
+    for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < nb; j += gridDim.y * blockDim.x) {
         double s = 0.0;
+#pragma unroll 4
         for (int64_t k = k0; k < k1; k++) s += (double)a.partial[a.in_slot[k] + j];
         a.pot[ib + j] += s;
     }
@@ -310,23 +313,23 @@ __global__ void k_sym_gather(SymGatherArgs a)
 
 void launch_pp_sym(int kernel, const SymArgs &a, cudaStream_t st)
 {
-    if (a.npairs <= 0) return;
-    if (kernel == 3) k_pp_sym<3, false><<<a.npairs, SY_THREADS, 0, st>>>(a);
-    else if (kernel == 2) k_pp_sym<2, false><<<a.npairs, SY_THREADS, 0, st>>>(a);
-    else k_pp_sym<1, false><<<a.npairs, SY_THREADS, 0, st>>>(a);
+    if (a.nblocks <= 0) return;
+    if (kernel == 3) k_pp_sym<3, false><<<a.nblocks, SY_THREADS, 0, st>>>(a);
+    else if (kernel == 2) k_pp_sym<2, false><<<a.nblocks, SY_THREADS, 0, st>>>(a);
+    else k_pp_sym<1, false><<<a.nblocks, SY_THREADS, 0, st>>>(a);
 }
 
 void launch_pp_sym_close(int kernel, const SymArgs &a, cudaStream_t st)
 {
-    if (a.npairs <= 0) return;
-    if (kernel == 3) k_pp_sym<3, true><<<a.npairs, SY_THREADS, 0, st>>>(a);
-    else if (kernel == 2) k_pp_sym<2, true><<<a.npairs, SY_THREADS, 0, st>>>(a);
-    else k_pp_sym<1, true><<<a.npairs, SY_THREADS, 0, st>>>(a);
+    if (a.nblocks <= 0) return;
+    if (kernel == 3) k_pp_sym<3, true><<<a.nblocks, SY_THREADS, 0, st>>>(a);
+    else if (kernel == 2) k_pp_sym<2, true><<<a.nblocks, SY_THREADS, 0, st>>>(a);
+    else k_pp_sym<1, true><<<a.nblocks, SY_THREADS, 0, st>>>(a);
 }
 
 void launch_sym_gather(const SymGatherArgs &a, cudaStream_t st)
 {
-    if (a.nleaves > 0) k_sym_gather<<<a.nleaves, 128, 0, st>>>(a);
+    if (a.nleaves > 0) k_sym_gather<<<dim3(a.nleaves, 4), 128, 0, st>>>(a);
 }
 
 }  // namespace bt

@@ -1,4 +1,4 @@
-// bt_sym.h -- symmetric near-field pairs of the mixed path (internal).
+// bt_sym.h -- symmetric near-field pairs (internal).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -8,15 +8,30 @@ namespace bt {
 
 // Largest leaf the symmetric pass takes (particles).
 constexpr int SYM_MAX_LEAF = 2048;
+// Smallest leaf whose pairs the FP64 path's symmetric pass takes (a rule per
+// pair, so that a batch takes the pairs its systems take in separate calls).
+// Measured, uniform systems, whole calls without and with the pass: leaves of
+// 195 particles 5.7 and 6.0 ms (Yukawa 10.9 and 10.8 ms; the pairs' planning
+// eats the gain), of 390 particles 10.4 and 9.3 ms (26.2 and 22.6 ms), of 1560
+// particles 5.8 and 5.0 ms (13.4 and 10.3 ms).  Leaves below 512, where the
+// gain is small, keep the sums of every direction.
+constexpr int SYM64_MIN_LEAF = 512;
+
+// Particles of A per block: a pair of leaves (A, B) is evaluated by
+// sym_parts(numpar[A]) blocks.
+constexpr int SYM_PART = 512;
+inline int sym_parts(int na) { return (na + SYM_PART - 1) / SYM_PART; }
 
 struct SymArgs {
-    int npairs;
+    int nblocks;
+    const int2 *block;            // (pair, part of A)
     const int2 *pair;             // (A, B) leaf nodes, A != B
-    const int64_t *slot;          // per pair: A side at slot[p], B side at slot[p] + numpar[A]
+    // per pair: A's sums at slot[p], B's from part k at slot[p] + numpar[A] + k numpar[B]
+    const int64_t *slot;
     const int *ibeg, *numpar;     // per node (the target tree is the source tree)
     const double *ctr;            // node centres, 3 per node
     const float4 *pos;            // particles relative to their leaf centre, with charge
-    float *partial;               // per pair, per particle of A then of B: the pair's potential there
+    float *partial;               // the pairs' potentials at their particles
     float kc;                     // mixed_kernel_constant()
     // pairs of leaves within the close-pair distance of each other (launch_pp_sym_close)
     const double *rad;            // node radii
@@ -42,5 +57,28 @@ void launch_pp_sym(int kernel, const SymArgs &a, cudaStream_t st);
 // by FP64 ones (from the FP64 particles) before the slices are written.
 void launch_pp_sym_close(int kernel, const SymArgs &a, cudaStream_t st);
 void launch_sym_gather(const SymGatherArgs &a, cudaStream_t st);
+
+// The FP64 path's pairs (bt_sym64.cu): one kernel for all of them, FP64 slices.
+struct Sym64Args {
+    int nblocks;
+    const int2 *block, *pair;
+    const int64_t *slot;
+    const int *ibeg, *numpar;
+    const double *x, *y, *z, *q;  // particles in tree order
+    double *partial;
+    double kp;
+};
+
+struct SymGather64Args {
+    int nleaves;
+    const int *leaf_node;
+    const int *ibeg, *numpar;
+    const int64_t *in_off, *in_slot;
+    const double *partial;
+    double *pot;
+};
+
+void launch_pp_sym64(int kernel, const Sym64Args &a, cudaStream_t st);
+void launch_sym_gather64(const SymGather64Args &a, cudaStream_t st);
 
 }  // namespace bt

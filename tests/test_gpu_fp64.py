@@ -1,0 +1,112 @@
+"""FP64 evaluation kernels at the sizes where their work division changes:
+chunks of 256 targets, lanes by powers of two, segments of the interaction
+lists, every degree, the symmetric pairs' leaf range, and arguments outside
+the kernels' short forms.  Against the CPU oracle (a restatement of the
+reference in FP64) or the same sums in numpy, at the FP64 parity bar."""
+import numpy as np
+import pytest
+
+import barytree_b200 as B
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def _rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+def _cube(seed, n):
+    rng = np.random.default_rng(seed)
+    return (*(rng.uniform(-1, 1, n) for _ in range(3)), rng.uniform(-1, 1, n))
+
+
+def _direct(t, s, q, kernel, kp):
+    d2 = sum((a[:, None] - b[None, :]) ** 2 for a, b in zip(t, s))
+    if kernel == 3:
+        return (1.0 / np.sqrt(d2 + kp * kp)) @ q
+    with np.errstate(divide="ignore"):
+        k = np.exp(-kp * np.sqrt(d2)) / np.sqrt(d2) if kernel == 2 else 1.0 / np.sqrt(d2)
+    return np.where(d2 > 0, k, 0.0) @ q
+
+
+@pytest.mark.parametrize("kernel,kp", [(1, 0.0), (2, 0.7), (3, 1e-2)])
+@pytest.mark.parametrize("nt", [1, 2, 3, 31, 33, 64, 65, 127, 128, 129, 255, 256, 257, 700])
+def test_direct_sum_at_every_lane_split(kernel, kp, nt):
+    x, y, z, q = _cube(nt, 3001)
+    t = [x[:nt], y[:nt], z[:nt]]                    # targets among the sources: skipped pairs
+    ref = _direct(t, (x, y, z), q, kernel, kp)
+    assert _rel(B.direct(*t, x, y, z, q, kernel, kp), ref) <= TOL
+
+
+@pytest.mark.parametrize("ctype", [1, 2, 3])
+@pytest.mark.parametrize("degree", range(1, 13))
+def test_every_degree(ctype, degree):
+    x, y, z, q = _cube(degree, 5000)
+    kernel, kp = (degree % 3) + 1, 0.3
+    kw = dict(compute_type=ctype, degree=degree, theta=0.8, max_source_leaf=150, max_target_leaf=90)
+    ref = O.treecode(x, y, z, None, x, y, z, q, None, kernel, [kp], 1, 1, ctype, 0.8, degree, 150, 90, 1.0, -1.0, 0)
+    assert _rel(B.treecode(x, y, z, x, y, z, q, kernel=kernel, kernel_param=kp, **kw), ref) <= TOL
+
+
+@pytest.mark.parametrize("kernel,kp", [(1, 0.0), (2, 0.7), (3, 1e-2)])
+@pytest.mark.parametrize("n,leaf", [(4200, 600), (6000, 800), (9000, 1200), (14000, 2048)])
+def test_symmetric_pairs(kernel, kp, n, leaf):
+    """Leaves of 512 to 2048 particles in pairs; the rest direction by direction."""
+    x, y, z, q = _cube(n, n)
+    kw = dict(kernel=kernel, kernel_param=kp, degree=6, theta=0.7, max_source_leaf=leaf, max_target_leaf=leaf)
+    sym, rep = B.treecode(x, y, z, x, y, z, q, return_report=True, **kw)
+    off = B.treecode(x, y, z, x, y, z, q, symmetry=B.SYMMETRY_OFF, **kw)
+    assert rep["sym_ptwise"] > 0
+    assert _rel(sym, off) <= 1e-13
+    assert np.array_equal(sym, B.treecode(x, y, z, x.copy(), y.copy(), z.copy(), q, **kw))
+    # beside a system with targets of its own: the same bits as alone
+    other = _cube(n + 1, 3000)
+    systems = [(*other[:3], x, y, z, q), (x, y, z, x, y, z, q)]
+    assert np.array_equal(B.treecode_batch(systems, **kw)[1], sym)
+    assert np.array_equal(B.treecode_batch(systems, tree_build=B.TREE_HOST, **kw)[1], sym)
+
+
+@pytest.mark.parametrize("approx", [1, 2])
+def test_few_items_and_many_items_give_the_same_bits(approx):
+    """A system evaluated alone (a block per list segment) and inside a batch
+    with enough work items for one block per item."""
+    rng = np.random.default_rng(7)
+    one = _cube(1, 20000)
+    big = tuple(rng.uniform(-1, 1, 1_300_000) for _ in range(4))
+    kw = dict(approximation=approx, degree=3, theta=0.9, max_source_leaf=500, max_target_leaf=500,
+              size_check=1.0 if approx == 1 else 4.0)
+    sys_of = lambda p: (*p[:3], *p[:3], p[3])  # noqa: E731
+    alone = B.treecode(*sys_of(one), **kw)
+    assert np.array_equal(B.treecode_batch([sys_of(one), sys_of(big)], **kw)[0], alone)
+
+
+@pytest.mark.parametrize("kernel,kp,scale", [(1, 0.0, 1e160), (1, 0.0, 1e-160), (3, 0.0, 1e-160), (2, -0.4, 1.0),
+                                              (2, 900.0, 1.0), (2, 0.0, 1.0), (2, 1e-3, 1e160)])
+def test_arguments_outside_the_short_forms(kernel, kp, scale):
+    """Squares that overflow or underflow, a growing exponential, one that
+    underflows: what the library functions give, term by term."""
+    x, y, z, q = _cube(3, 1500)
+    x, y, z = x * scale, y * scale, z * scale
+    with np.errstate(all="ignore"):
+        d2 = sum((a[:, None] - a[None, :]) ** 2 for a in (x, y, z))
+        if kernel == 2:
+            r = np.sqrt(d2)
+            ref = np.where(r > np.finfo(float).tiny, np.exp(-kp * r) / r, 0.0) @ q
+        elif kernel == 3:
+            ref = (1.0 / np.sqrt(d2)) @ q
+        else:
+            ref = np.where(d2 > np.finfo(float).tiny, 1.0 / np.sqrt(d2), 0.0) @ q
+    got = [B.direct(x, y, z, x, y, z, q, kernel, kp)]
+    kw = dict(kernel=kernel, kernel_param=kp, degree=3, max_source_leaf=400, max_target_leaf=400, theta=1e-9)
+    got.append(B.treecode(x, y, z, x, y, z, q, **kw))                               # near field only, pairs
+    got.append(B.treecode(x, y, z, x, y, z, q, symmetry=B.SYMMETRY_OFF, **kw))
+    for g in got:
+        ok = np.isfinite(ref)
+        assert np.array_equal(np.isfinite(g), ok)
+        if ok.any() and np.linalg.norm(ref[ok]) > 0:
+            assert _rel(g[ok], ref[ok]) <= 1e-12
+        else:
+            assert np.all(g[ok] == ref[ok])
