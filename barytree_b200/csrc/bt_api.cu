@@ -995,8 +995,9 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         a.s_ibeg = d_sibeg; a.s_numpar = d_snum; a.s_grid = d_sgrid; a.Q = d_Q; a.W = v.d_W;
         a.sx = d_sx; a.sy = d_sy; a.sz = d_sz; a.sq = d_sq; a.sw = v.d_sw;
         a.tx = d_tx; a.ty = d_ty; a.tz = d_tz; a.tq = v.d_tq; a.kp = v.kp; a.kp2 = v.kp2; a.pot = d_pot;
+        a.partial = v.d_evpart; a.pstride = (size_t)nt;
         bt::launch_ss_targets(v.kernel, herm, a, st);
-        launches++;
+        launches += a.partial ? 2 : 1;
     } else if (nt > 0 && mixed) {
         const bt::MixedTargetsArgs a = mixed_targets_args(v);
         // the symmetric pairs write only their own partial sums: their two
@@ -1704,7 +1705,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     // few (the results are the same without them): up to EV_SEGS doubles per
     // target, or per grid point within a fixed bound.
     double *d_evpart = nullptr, *d_gridpart = nullptr;
-    if (!ssm) {
+    {
         const size_t room = arena.fixed ? (arena.cap > L.total() ? arena.cap - L.total() : 0) : (size_t)1 << 30;
         size_t need = 0;
         auto want = [&](double **p, size_t count) {
@@ -1713,7 +1714,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             L.add(p, count);
         };
         if (mixed ? bt::mixed_split(ev_items.size()) : bt::eval64_split(ev_items.size())) want(&d_evpart, (size_t)bt::EV_SEGS * nt);
-        if (!mixed && need_tgt_grids && !herm && bt::eval64_split(grid_items.size()))
+        if (!mixed && !ssm && need_tgt_grids && !herm && bt::eval64_split(grid_items.size()))
             want(&d_gridpart, (size_t)bt::EV_SEGS * T.n * P);
     }
 
@@ -2568,7 +2569,7 @@ int bt_direct_full(int numTargets, int numSources, const double *targetX, const 
     const int parts = bt::direct_parts(numTargets, numSources);
     {
         Layout L;
-        if (!ss && parts > 1) L.add(&d_part, (size_t)parts * numTargets);
+        if (parts > 1) L.add(&d_part, (size_t)parts * numTargets);
         for (int i = 0; i < 4; i++) L.add(&d_t[i], numTargets);
         for (int i = 0; i < 5; i++) L.add(&d_s[i], numSources);
         L.add(&d_o, numTargets);
@@ -2582,9 +2583,9 @@ int bt_direct_full(int numTargets, int numSources, const double *targetX, const 
             for (int i = 0; i < nsc; i++) CK(cudaMemcpyAsync(d_s[i], hs[i], sizeof(double) * numSources, cudaMemcpyHostToDevice, st));
         if (ss) {
             bt::launch_ss_direct(kernel, numTargets, numSources, d_t[0], d_t[1], d_t[2], d_t[3], d_s[0], d_s[1], d_s[2],
-                                 d_s[3], d_s[4], kernelParam, kernelParam2, d_o, st);
+                                 d_s[3], d_s[4], kernelParam, kernelParam2, d_part, d_o, st);
             bt::launch_ss_correction(numTargets, bt::ss_correction_constant(kernel, kernelParam), d_t[3], d_o, st);
-            g_launches += 2;
+            g_launches += parts > 1 ? 3 : 2;
         } else {
             bt::launch_direct(kernel, numTargets, numSources, d_t[0], d_t[1], d_t[2], d_s[0], d_s[1], d_s[2], d_s[3],
                               kernelParam, kernelParam2, d_part, d_o, st);

@@ -1001,7 +1001,12 @@ void launch_direct(int kernel, int nt, int ns, const double *tx, const double *t
     default: direct_kt<K_USER>(nt, ns, parts, tx, ty, tz, sx, sy, sz, sq, kp, kp2, dst, st);
     }
 #undef BT_DIRECT
-    if (parts > 1) k_sum_parts<<<(nt + 255) / 256, 256, 0, st>>>(nt, parts, partial, out);
+    if (parts > 1) launch_sum_parts(nt, parts, partial, out, st);
+}
+
+void launch_sum_parts(int n, int parts, const double *partial, double *out, cudaStream_t st)
+{
+    k_sum_parts<<<(n + 255) / 256, 256, 0, st>>>(n, parts, partial, out);
 }
 
 }  // namespace bt

@@ -95,6 +95,8 @@ float run_probe(int which, int sms, double *ops, void *scratch, cudaStream_t st)
 // Parts that the direct sum splits its sources into (partial sums: parts * nt
 // doubles when parts > 1).
 int direct_parts(int nt, int ns);
+// out = the sum of `parts` arrays of n values, in order.
+void launch_sum_parts(int n, int parts, const double *partial, double *out, cudaStream_t st);
 void launch_direct(int kernel, int nt, int ns, const double *tx, const double *ty, const double *tz,
                    const double *sx, const double *sy, const double *sz, const double *sq, double kp, double kp2,
                    double *partial, double *out, cudaStream_t st);

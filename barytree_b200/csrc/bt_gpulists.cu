@@ -7,9 +7,8 @@
 // whose radius is not zero and which holds more particles than size check
 // times the grid size becomes a cluster (approximation) entry; otherwise a
 // leaf becomes a direct entry and an internal node is opened, children in
-// order.  Here one thread walks one batch with an explicit stack in shared
-// memory (interleaved by thread, so lanes at the same depth hit different
-// banks); popping the top and pushing the children last-first visits nodes
+// order.  Here eight lanes walk one batch with an explicit stack in shared
+// memory; popping the top and pushing the children last-first visits nodes
 // in the recursion's order.  The comparisons use __dsub_rn / __dmul_rn /
 // __dadd_rn / __dsqrt_rn, so nothing is contracted into an FMA and every
 // value equals the host's IEEE FP64 result: membership and order are the
@@ -31,8 +30,9 @@ namespace bt {
 
 namespace {
 
-constexpr int GL_THREADS = 32;           // one warp: the batches of a small system spread over more SMs
-constexpr int GL_MAX_STACK = 384;          // shared-memory stack slots per thread (49 KB per block)
+constexpr int GL_LANES = 8;               // lanes per batch
+constexpr int GL_THREADS = 64;
+constexpr int GL_MAX_STACK = 384;          // shared-memory stack slots per batch
 
 // What a node is to the batch; in the upper bits of a stack entry.
 enum { GL_OPEN = 0, GL_CLUSTER = 1, GL_DIRECT = 2 };
@@ -46,61 +46,68 @@ __device__ __forceinline__ int gl_class(const double4 B, const double4 g, const 
     return cn.y == 0 ? GL_DIRECT : GL_OPEN;
 }
 
-// Opening a node classifies all its children at once, so that up to eight
-// nodes' loads and square roots are in flight together; the stack holds
-// classified nodes.  Classifying each node when it was popped made the walk
-// one chain of memory latencies (125 us for 5,000 particles in 133 leaves,
-// 330 us for 250,000 targets; the list order is the same).
+// Eight lanes walk a batch: the top eight stack entries are read together,
+// those above the topmost node to open are emitted in stack order by ballots,
+// and that node's children are loaded and classified by a lane each, onto a
+// stack of classified nodes.  With one lane per batch and a node per step the
+// walk was one chain of memory latencies and square roots (125 us for 5,000
+// particles in 133 leaves); a lane opening eight children by itself took
+// about as long, for the lanes of a warp seldom open at the same step.
 template <bool FILL>
 __global__ void __launch_bounds__(GL_THREADS)
 k_pc_traverse(int nb, const double4 *__restrict__ bat, const int *__restrict__ broot,
-              const double4 *__restrict__ geo, const int2 *__restrict__ cnt_nc, const int4 *__restrict__ child,
+              const double4 *__restrict__ geo, const int2 *__restrict__ cnt_nc, const int *__restrict__ child,
               double theta, double thr, int depth_cap, int *__restrict__ counts, const int64_t *__restrict__ aoff,
               const int64_t *__restrict__ poff, int *__restrict__ aidx, int *__restrict__ pidx,
               int *__restrict__ overflow)
 {
-    extern __shared__ int stk[];
-    const int b = blockIdx.x * GL_THREADS + threadIdx.x;
-    if (b >= nb) return;
+    extern __shared__ int stacks[];
+    const int lane = threadIdx.x & (GL_LANES - 1), group = threadIdx.x / GL_LANES;
+    const int b = blockIdx.x * (GL_THREADS / GL_LANES) + group;
+    if (b >= nb) return;                          // whole groups
+    const int shift = (threadIdx.x & 31) & ~(GL_LANES - 1);
+    const unsigned mask = 0xffu << shift;
+    int *stk = stacks + (size_t)group * depth_cap;
     const double4 B = bat[b];
     int sp = 0, na = 0, np = 0;
     int *a_out = FILL ? aidx + aoff[b] : nullptr, *p_out = FILL ? pidx + poff[b] : nullptr;
     const int root = broot[b];
-    if (root >= 0) stk[threadIdx.x] = root | gl_class(B, geo[root], cnt_nc[root], theta, thr) << GL_SHIFT, sp = 1;
-    while (sp) {
-        sp--;
-        const int entry = stk[sp * GL_THREADS + threadIdx.x], node = entry & GL_NODE, cls = entry >> GL_SHIFT;
-        if (cls == GL_CLUSTER) {
-            if (FILL) a_out[na] = node;
-            na++;
-        } else if (cls == GL_DIRECT) {
-            if (FILL) p_out[np] = node;
-            np++;
-        } else {
-            const int nc = cnt_nc[node].y;
-            if (sp + nc > depth_cap) {
-                atomicExch(overflow, 1);
-                return;
-            }
-            const int4 c0 = child[2 * (size_t)node], c1 = child[2 * (size_t)node + 1];
-            const int id[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            double4 g[8];
-            int2 cn[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (i < nc) {
-                    g[i] = geo[id[i]];
-                    cn[i] = cnt_nc[id[i]];
-                }
-#pragma unroll
-            for (int i = 0; i < 8; i++)       // child i to slot nc - 1 - i: the first child is popped first
-                if (i < nc)
-                    stk[(sp + nc - 1 - i) * GL_THREADS + threadIdx.x] =
-                        id[i] | gl_class(B, g[i], cn[i], theta, thr) << GL_SHIFT;
-            sp += nc;
-        }
+    if (root >= 0) {
+        if (lane == 0) stk[0] = root | gl_class(B, geo[root], cnt_nc[root], theta, thr) << GL_SHIFT;
+        sp = 1;
     }
-    if (!FILL) {
+    __syncwarp(mask);
+    while (sp) {
+        const int top = min(sp, GL_LANES);
+        const int entry = lane < top ? stk[sp - 1 - lane] : GL_CLUSTER << GL_SHIFT, cls = entry >> GL_SHIFT;
+        int node = entry & GL_NODE;
+        const unsigned open = (__ballot_sync(mask, cls == GL_OPEN) >> shift) & 0xffu;
+        const int first = open ? __ffs(open) - 1 : top;
+        const unsigned cb = (__ballot_sync(mask, lane < first && cls == GL_CLUSTER) >> shift) & 0xffu;
+        const unsigned db = (__ballot_sync(mask, lane < first && cls == GL_DIRECT) >> shift) & 0xffu;
+        if (FILL && lane < first) {
+            const unsigned below = (1u << lane) - 1u;
+            if (cls == GL_CLUSTER) a_out[na + __popc(cb & below)] = node;
+            else p_out[np + __popc(db & below)] = node;
+        }
+        na += __popc(cb);
+        np += __popc(db);
+        sp -= first;
+        if (!open) continue;
+        node = __shfl_sync(mask, node, first, GL_LANES);
+        sp--;
+        const int nc = cnt_nc[node].y, id = child[8 * (size_t)node + lane];
+        if (sp + nc > depth_cap) {
+            if (lane == 0) atomicExch(overflow, 1);
+            return;
+        }
+        __syncwarp(mask);                         // the entries have been read
+        // the first child on top: it is visited first
+        if (lane < nc) stk[sp + nc - 1 - lane] = id | gl_class(B, geo[id], cnt_nc[id], theta, thr) << GL_SHIFT;
+        sp += nc;
+        __syncwarp(mask);
+    }
+    if (!FILL && lane == 0) {
         counts[b] = na;
         counts[nb + b] = np;
     }
@@ -125,7 +132,7 @@ int gpu_pc_lists(const bt_tree *trav, const bt_tree *bat, const bt_params *o, vo
     };
     double4 *d_geo = (double4 *)take(sizeof(double4) * (size_t)nn);
     int2 *d_cn = (int2 *)take(sizeof(int2) * (size_t)nn);
-    int4 *d_child = (int4 *)take(sizeof(int) * 8 * (size_t)nn);
+    int *d_child = (int *)take(sizeof(int) * 8 * (size_t)nn);
     double4 *d_bat = (double4 *)take(sizeof(double4) * (size_t)nb);
     int *d_root = (int *)take(sizeof(int) * (size_t)nb);
     int *d_cnt = (int *)take(sizeof(int) * 2 * (size_t)nb);
@@ -156,11 +163,11 @@ int gpu_pc_lists(const bt_tree *trav, const bt_tree *bat, const bt_params *o, vo
     GL_CK(cudaMemcpyAsync(d_bat, bg.data(), sizeof(double4) * (size_t)nb, cudaMemcpyHostToDevice, st));
     GL_CK(cudaMemcpyAsync(d_root, root.data(), sizeof(int) * (size_t)nb, cudaMemcpyHostToDevice, st));
     GL_CK(cudaMemsetAsync(d_ovf, 0, sizeof(int), st));
-    const size_t smem = sizeof(int) * (size_t)GL_THREADS * (size_t)cap;
+    const size_t smem = sizeof(int) * (size_t)(GL_THREADS / GL_LANES) * (size_t)cap;
     GL_CK(cudaFuncSetAttribute(k_pc_traverse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     GL_CK(cudaFuncSetAttribute(k_pc_traverse<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const double thr = o->size_check * o->P;
-    const int blocks = (nb + GL_THREADS - 1) / GL_THREADS;
+    const int per = GL_THREADS / GL_LANES, blocks = (nb + per - 1) / per;
     k_pc_traverse<false><<<blocks, GL_THREADS, smem, st>>>(nb, d_bat, d_root, d_geo, d_cn, d_child, o->theta, thr,
                                                            cap, d_cnt, nullptr, nullptr, nullptr, nullptr, d_ovf);
     GL_CK(cudaGetLastError());

@@ -28,6 +28,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "bt_eval64.cuh"
 #include "bt_kernels.cuh"
 #include "bt_ss.h"
 
@@ -36,7 +37,6 @@ namespace bt {
 namespace {
 
 constexpr int SS_THREADS = 128;
-constexpr int SS_TILE = 256;
 
 // SS near-field pair (PP): target charge tq, source (q, w).
 template <int KT>
@@ -123,73 +123,217 @@ __device__ __forceinline__ void ss_grid(double dx, double dy, double dz, double 
     }
 }
 
-// Particle-output evaluation with SS: PC + PP per target leaf chunk, one
-// target per thread (FP64).
-template <int KT, bool HERM>
-__global__ void __launch_bounds__(SS_THREADS) k_ss_targets(SsTargetsArgs a)
+// The short forms (bt_fp64.cuh), used for every kernel; the functions above
+// form a sum again where it is not finite.  exp64 takes r (kappa) for the
+// Yukawa kernels and r^2 (1 / alpha^2) for the others.
+struct SsKern {
+    double eps2;
+    Exp64 ex;
+    bool lib;               // parameters outside exp64's range
+};
+
+template <int KT>
+__device__ __forceinline__ SsKern ss_kern(double kp, double kp2, double2 *tab)
 {
-    __shared__ double g[3 * MAXNP];
-    __shared__ double tile[5][SS_TILE];
-    const int2 it = a.items[blockIdx.x];
-    const int u = it.x;
-    const int tnode = a.leaf_node[u];
-    const int tb = a.t_ibeg[tnode], tn = a.t_numpar[tnode];
-    const int ti = it.y * SS_THREADS + threadIdx.x;
-    const bool active = ti < tn;
-    const int t = tb + (active ? ti : 0);
-    const double x = a.tx[t], y = a.ty[t], z = a.tz[t], tq = a.tq[t];
-    const int np1 = a.n + 1, P = np1 * np1 * np1, nq = HERM ? 8 * P : P;
-    double acc = 0.0;
-    for (int64_t e = a.a_off[u]; e < a.a_off[u + 1]; e++) {
-        const int s = a.a_idx[e];
-        for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) g[i] = a.s_grid[(size_t)s * 3 * np1 + i];
+    SsKern k;
+    k.eps2 = KT == K_REGCOULOMB || KT == K_REGYUKAWA ? kp2 * kp2 : 0.0;
+    const double kappa = KT == K_YUKAWA || KT == K_REGYUKAWA ? kp : 1.0 / (kp * kp);
+    k.lib = !(kappa >= 0.0 && kappa < 1.0e300);
+    for (int i = threadIdx.x; i < EXP64_TAB; i += blockDim.x) tab[i] = exp64_table[i];
+    k.ex = exp64_make(kappa, tab);
+    return k;
+}
+
+// K(r) with the exponential of the Yukawa kernels (kv), and the subtraction
+// factor g (1 for those).
+template <int KT>
+__device__ __forceinline__ void ss_values(double r2, const SsKern &k, double &kv, double &g)
+{
+    if (KT == K_YUKAWA) {
+        double r;
+        const double y = rsqrt_sqrt_n(r2, r);
+        kv = y * exp64(r, k.ex);
+        g = 1.0;
+    } else if (KT == K_REGYUKAWA) {
+        // r of a coincident pair from a tiny r^2 instead of zero
+        const double c = __hiloint2double(max(__double2hiint(r2), 0x01a00000), __double2loint(r2));
+        double r;
+        rsqrt_sqrt_n(c, r);
+        kv = rsqrt_n(r2 + k.eps2) * exp64(r, k.ex);
+        g = 1.0;
+    } else {
+        kv = rsqrt_n(KT == K_REGCOULOMB ? r2 + k.eps2 : r2);
+        g = exp64(r2, k.ex);
+    }
+}
+
+// Near-field tile: x, y; z, q; w of each source.
+struct SsTile {
+    double2 *xy, *zq;
+    double *w;
+};
+constexpr size_t SS_TILE_BYTES = (2 * sizeof(double2) + sizeof(double)) * EV_TILE;
+
+__device__ __forceinline__ SsTile ss_tile(double *sm)
+{
+    double2 *p = reinterpret_cast<double2 *>(sm);
+    return SsTile{p, p + EV_TILE, reinterpret_cast<double *>(p + 2 * EV_TILE)};
+}
+
+// acc += the SS pair terms of sources sb .. sb + sn - 1 (all threads call).
+template <int KT>
+__device__ __forceinline__ void ss_near(double *acc, const SsTile &t, int sb, int sn, const double *__restrict__ sx,
+                                        const double *__restrict__ sy, const double *__restrict__ sz,
+                                        const double *__restrict__ sq, const double *__restrict__ sw, const Out2 &o,
+                                        const double *tq, const Lanes &w, const SsKern &k)
+{
+    for (int c0 = 0; c0 < sn; c0 += EV_TILE) {
+        const int cm = min(EV_TILE, sn - c0);
+        for (int i = threadIdx.x; i < cm; i += EV_THREADS) {
+            const int j = sb + c0 + i;
+            t.xy[i] = make_double2(sx[j], sy[j]);
+            t.zq[i] = make_double2(sz[j], sq[j]);
+            t.w[i] = sw[j];
+        }
         __syncthreads();
-        if (active) {
-            const double *Qs = a.Q + (size_t)s * nq, *Ws = a.W + (size_t)s * nq;
-            int j = 0;
-            for (int k3 = 0; k3 < np1; k3++) {
-                const double dz = z - g[2 * np1 + k3];
-                for (int k2 = 0; k2 < np1; k2++) {
-                    const double dy = y - g[np1 + k2];
-                    for (int k1 = 0; k1 < np1; k1++, j++) {
-                        const double dx = x - g[k1];
-                        if (HERM) acc += ss_pc_herm<KT>(dx, dy, dz, Qs + j, Ws + j, P, tq, a.kp, a.kp2);
-                        else acc += ss_pc<KT>(dx, dy, dz, Qs[j], Ws[j], tq, a.kp, a.kp2);
-                    }
+        if (w.active[0])
+#pragma unroll 2
+            for (int i = w.slice; i < cm; i += w.slices) {
+                const double2 p = t.xy[i], s = t.zq[i];
+                const double sw_i = t.w[i];
+#pragma unroll
+                for (int b = 0; b < 2; b++) {
+                    const double dx = o.x[b] - p.x, dy = o.y[b] - p.y, dz = o.z[b] - s.x;
+                    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                    double kv, g;
+                    ss_values<KT>(r2, k, kv, g);
+                    // r <= DBL_MIN is skipped by Coulomb and Yukawa: every r^2 but zero counts
+                    if ((KT == K_COULOMB || KT == K_YUKAWA) && __double_as_longlong(r2) <= 0) kv = 0.0;
+                    acc[b] = fma(fma(-tq[b], g, s.y) * sw_i, kv, acc[b]);
                 }
             }
-        }
         __syncthreads();
     }
-    for (int64_t e = a.d_off[u]; e < a.d_off[u + 1]; e++) {
-        const int s = a.d_idx[e];
-        const int sb = a.s_ibeg[s], sn = a.s_numpar[s];
-        for (int c0 = 0; c0 < sn; c0 += SS_TILE) {
-            const int cm = min(SS_TILE, sn - c0);
-            for (int i = threadIdx.x; i < cm; i += blockDim.x) {
-                const int k = sb + c0 + i;
-                tile[0][i] = a.sx[k]; tile[1][i] = a.sy[k]; tile[2][i] = a.sz[k];
-                tile[3][i] = a.sq[k]; tile[4][i] = a.sw[k];
-            }
+}
+
+// Particle-output evaluation with SS: PC + PP per chunk of a target leaf; the
+// division of a block and of the lists is that of bt_eval64.cuh.
+template <int KT, bool HERM>
+__global__ void __launch_bounds__(EV_THREADS, 4) k_ss_targets(const __grid_constant__ SsTargetsArgs a)
+{
+    extern __shared__ __align__(16) double sm[];
+    __shared__ double red[2 * EV_THREADS];
+    __shared__ double2 tab[EXP64_TAB];
+    const SsKern k = ss_kern<KT>(a.kp, a.kp2, tab);
+    const int2 it = a.items[blockIdx.x];
+    const int u = it.x, tnode = a.leaf_node[u];
+    const Lanes w(min(EV_CHUNK, a.t_numpar[tnode] - it.y * EV_CHUNK));
+    const int t0 = a.t_ibeg[tnode] + it.y * EV_CHUNK;
+    Out2 o;
+    double tq[2];
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+        const int t = t0 + w.out(b);
+        o.x[b] = a.tx[t]; o.y[b] = a.ty[t]; o.z[b] = a.tz[t]; tq[b] = a.tq[t];
+    }
+    const int np1 = a.n + 1, P = np1 * np1 * np1, nq = HERM ? 8 * P : P;
+    const int64_t ab = a.a_off[u], ae = a.a_off[u + 1], db = a.d_off[u], de = a.d_off[u + 1];
+    const int seg0 = a.partial ? blockIdx.y : 0, seg1 = a.partial ? blockIdx.y + 1 : EV_SEGS;
+    double total[2] = {0.0, 0.0};
+    for (int seg = seg0; seg < seg1; seg++) {
+        const int64_t a0 = seg_begin(ab, ae, seg), a1 = seg_begin(ab, ae, seg + 1);
+        const int64_t d0 = seg_begin(db, de, seg), d1 = seg_begin(db, de, seg + 1);
+        double acc[2] = {0.0, 0.0};
+        for (int64_t e = k.lib && !HERM ? a1 : a0; e < a1; e++) {
+            const int s = a.a_idx[e];
+            double *g = sm, *q = sm + 3 * np1, *wq = q + P;
+            for (int i = threadIdx.x; i < 3 * np1; i += EV_THREADS) g[i] = a.s_grid[(size_t)s * 3 * np1 + i];
+            if (!HERM)
+                for (int i = threadIdx.x; i < P; i += EV_THREADS) {
+                    q[i] = a.Q[(size_t)s * P + i];
+                    wq[i] = a.W[(size_t)s * P + i];
+                }
             __syncthreads();
-            if (active)
-                for (int i = 0; i < cm; i++)
-                    acc += ss_pp<KT>(x - tile[0][i], y - tile[1][i], z - tile[2][i], tile[3][i], tile[4][i], tq, a.kp,
-                                     a.kp2);
+            if (w.active[0])
+                for (int row = w.slice; row < np1 * np1; row += w.slices) {
+                    const int k3 = row / np1, k2 = row - k3 * np1;
+                    double dy[2], dz[2], dyz[2];
+#pragma unroll
+                    for (int b = 0; b < 2; b++) {
+                        dy[b] = o.y[b] - g[np1 + k2];
+                        dz[b] = o.z[b] - g[2 * np1 + k3];
+                        dyz[b] = fma(dy[b], dy[b], dz[b] * dz[b]);
+                    }
+#pragma unroll 2
+                    for (int i = 0; i < np1; i++) {
+                        const int j = row * np1 + i;
+#pragma unroll
+                        for (int b = 0; b < 2; b++) {
+                            const double dx = o.x[b] - g[i];
+                            if (HERM) {
+                                acc[b] += ss_pc_herm<KT>(dx, dy[b], dz[b], a.Q + (size_t)s * nq + j,
+                                                         a.W + (size_t)s * nq + j, P, tq[b], a.kp, a.kp2);
+                            } else {
+                                double kv, f;
+                                ss_values<KT>(fma(dx, dx, dyz[b]), k, kv, f);
+                                acc[b] = fma(fma(-tq[b] * f, wq[j], q[j]), kv, acc[b]);
+                            }
+                        }
+                    }
+                }
             __syncthreads();
         }
+        const SsTile tile = ss_tile(sm);
+        for (int64_t e = k.lib ? d1 : d0; e < d1; e++) {
+            const int s = a.d_idx[e];
+            ss_near<KT>(acc, tile, a.s_ibeg[s], a.s_numpar[s], a.sx, a.sy, a.sz, a.sq, a.sw, o, tq, w, k);
+        }
+#pragma unroll 1
+        for (int b = 0; b < 2; b++) {
+            if (!w.active[b] || (!k.lib && isfinite(acc[b]))) continue;
+            // again with the library functions, the thread's share
+            double s = 0.0;
+            const double x = o.x[b], y = o.y[b], z = o.z[b];
+            for (int64_t e = a0; e < a1; e++) {
+                const double *g = a.s_grid + (size_t)a.a_idx[e] * 3 * np1, *Qs = a.Q + (size_t)a.a_idx[e] * nq,
+                             *Ws = a.W + (size_t)a.a_idx[e] * nq;
+                for (int row = w.slice; row < np1 * np1; row += w.slices)
+                    for (int i = 0; i < np1; i++) {
+                        const int k3 = row / np1, k2 = row - k3 * np1, j = row * np1 + i;
+                        const double dx = x - g[i], dy = y - g[np1 + k2], dz = z - g[2 * np1 + k3];
+                        if (HERM) s += ss_pc_herm<KT>(dx, dy, dz, Qs + j, Ws + j, P, tq[b], a.kp, a.kp2);
+                        else s += ss_pc<KT>(dx, dy, dz, Qs[j], Ws[j], tq[b], a.kp, a.kp2);
+                    }
+            }
+            for (int64_t e = d0; e < d1; e++) {
+                const int n = a.d_idx[e], sb = a.s_ibeg[n], sn = a.s_numpar[n];
+                for (int c0 = 0; c0 < sn; c0 += EV_TILE)
+                    for (int i = sb + c0 + w.slice; i < sb + min(sn, c0 + EV_TILE); i += w.slices)
+                        s += ss_pp<KT>(x - a.sx[i], y - a.sy[i], z - a.sz[i], a.sq[i], a.sw[i], tq[b], a.kp, a.kp2);
+            }
+            acc[b] = s;
+        }
+        sum_slices(acc, red, w);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            total[b] += acc[b];
+            if (a.partial && w.active[b] && w.slice == 0) a.partial[(size_t)seg * a.pstride + t0 + w.out(b)] = acc[b];
+        }
     }
-    if (active) a.pot[t] = acc;
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+        if (!a.partial && w.active[b] && w.slice == 0) a.pot[t0 + w.out(b)] = total[b];
 }
 
 // Grid-output evaluation with SS (Lagrange): M2L from source clusters (Q, W)
 // and CP from source particles (q*w, w) onto both fields of a target node's
-// grid, one grid point per thread.
+// grid, one grid point per thread, Coulomb and Yukawa.
 template <int KT>
-__global__ void __launch_bounds__(SS_THREADS) k_ss_grids(SsGridsArgs a)
+__global__ void __launch_bounds__(SS_THREADS) k_ss_grids(const __grid_constant__ SsGridsArgs a)
 {
-    __shared__ double g[3 * MAXNP];
-    __shared__ double tile[5][SS_TILE];
+    extern __shared__ __align__(16) double sm[];
+    __shared__ double2 tab[EXP64_TAB];
+    const SsKern k = ss_kern<KT>(a.kp, 0.0, tab);
     const int2 it = a.items[blockIdx.x];
     const int T = it.x;
     const int np1 = a.n + 1, P = np1 * np1 * np1;
@@ -199,35 +343,69 @@ __global__ void __launch_bounds__(SS_THREADS) k_ss_grids(SsGridsArgs a)
     const double *tg = a.t_grid + (size_t)T * 3 * np1;
     const double x = tg[jj % np1], y = tg[np1 + (jj / np1) % np1], z = tg[2 * np1 + jj / (np1 * np1)];
     double fq = 0.0, fw = 0.0;
-    for (int64_t e = a.c_off[T]; e < a.c_off[T + 1]; e++) {
+    for (int64_t e = k.lib ? a.c_off[T + 1] : a.c_off[T]; e < a.c_off[T + 1]; e++) {
         const int s = a.c_idx[e];
-        for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) g[i] = a.s_grid[(size_t)s * 3 * np1 + i];
-        __syncthreads();
-        if (active) {
-            const double *Qs = a.Q + (size_t)s * P, *Ws = a.W + (size_t)s * P;
-            int j = 0;
-            for (int k3 = 0; k3 < np1; k3++)
-                for (int k2 = 0; k2 < np1; k2++)
-                    for (int k1 = 0; k1 < np1; k1++, j++)
-                        ss_grid<KT>(x - g[k1], y - g[np1 + k2], z - g[2 * np1 + k3], Qs[j], Ws[j], a.kp, fq, fw);
+        double *g = sm, *q = sm + 3 * np1, *w = q + P;
+        for (int i = threadIdx.x; i < 3 * np1; i += SS_THREADS) g[i] = a.s_grid[(size_t)s * 3 * np1 + i];
+        for (int i = threadIdx.x; i < P; i += SS_THREADS) {
+            q[i] = a.Q[(size_t)s * P + i];
+            w[i] = a.W[(size_t)s * P + i];
         }
         __syncthreads();
+        if (active)
+            for (int row = 0; row < np1 * np1; row++) {
+                const int k3 = row / np1, k2 = row - k3 * np1;
+                const double dy = y - g[np1 + k2], dz = z - g[2 * np1 + k3], dyz = fma(dy, dy, dz * dz);
+#pragma unroll 4
+                for (int i = 0; i < np1; i++) {
+                    const double dx = x - g[i];
+                    double kv, f;
+                    ss_values<KT>(fma(dx, dx, dyz), k, kv, f);
+                    fq = fma(q[row * np1 + i], kv, fq);
+                    fw = fma(f * w[row * np1 + i], kv, fw);
+                }
+            }
+        __syncthreads();
     }
-    for (int64_t e = a.p_off[T]; e < a.p_off[T + 1]; e++) {
+    const SsTile t = ss_tile(sm);
+    for (int64_t e = k.lib ? a.p_off[T + 1] : a.p_off[T]; e < a.p_off[T + 1]; e++) {
         const int s = a.p_idx[e];
         const int sb = a.s_ibeg[s], sn = a.s_numpar[s];
-        for (int c0 = 0; c0 < sn; c0 += SS_TILE) {
-            const int cm = min(SS_TILE, sn - c0);
-            for (int i = threadIdx.x; i < cm; i += blockDim.x) {
-                const int k = sb + c0 + i;
-                tile[0][i] = a.sx[k]; tile[1][i] = a.sy[k]; tile[2][i] = a.sz[k];
-                tile[3][i] = a.sq[k] * a.sw[k]; tile[4][i] = a.sw[k];
+        for (int c0 = 0; c0 < sn; c0 += EV_TILE) {
+            const int cm = min(EV_TILE, sn - c0);
+            for (int i = threadIdx.x; i < cm; i += SS_THREADS) {
+                const int j = sb + c0 + i;
+                t.xy[i] = make_double2(a.sx[j], a.sy[j]);
+                t.zq[i] = make_double2(a.sz[j], a.sq[j] * a.sw[j]);
+                t.w[i] = a.sw[j];
             }
             __syncthreads();
             if (active)
-                for (int i = 0; i < cm; i++)
-                    ss_grid<KT>(x - tile[0][i], y - tile[1][i], z - tile[2][i], tile[3][i], tile[4][i], a.kp, fq, fw);
+#pragma unroll 4
+                for (int i = 0; i < cm; i++) {
+                    const double2 p = t.xy[i], v = t.zq[i];
+                    const double dx = x - p.x, dy = y - p.y, dz = z - v.x;
+                    double kv, f;
+                    ss_values<KT>(fma(dx, dx, fma(dy, dy, dz * dz)), k, kv, f);
+                    fq = fma(v.y, kv, fq);
+                    fw = fma(f * t.w[i], kv, fw);
+                }
             __syncthreads();
+        }
+    }
+    if (active && (k.lib || !isfinite(fq) || !isfinite(fw))) {
+        fq = fw = 0.0;
+        for (int64_t e = a.c_off[T]; e < a.c_off[T + 1]; e++) {
+            const double *g = a.s_grid + (size_t)a.c_idx[e] * 3 * np1, *Qs = a.Q + (size_t)a.c_idx[e] * P,
+                         *Ws = a.W + (size_t)a.c_idx[e] * P;
+            for (int j = 0; j < P; j++)
+                ss_grid<KT>(x - g[j % np1], y - g[np1 + (j / np1) % np1], z - g[2 * np1 + j / (np1 * np1)], Qs[j], Ws[j],
+                            a.kp, fq, fw);
+        }
+        for (int64_t e = a.p_off[T]; e < a.p_off[T + 1]; e++) {
+            const int s = a.p_idx[e];
+            for (int i = a.s_ibeg[s]; i < a.s_ibeg[s] + a.s_numpar[s]; i++)
+                ss_grid<KT>(x - a.sx[i], y - a.sy[i], z - a.sz[i], a.sq[i] * a.sw[i], a.sw[i], a.kp, fq, fw);
         }
     }
     if (active) {
@@ -264,45 +442,65 @@ __global__ void k_axpy_items(const int2 *__restrict__ items, int chunk, const in
     }
 }
 
-// SS direct sum over all sources (InteractionCompute_Direct with
-// singularity subtraction, src/interaction_compute/interaction_compute_direct.c:26-231):
-// one target per thread, sources staged through shared memory.
+// SS direct sum (InteractionCompute_Direct with singularity subtraction,
+// src/interaction_compute/interaction_compute_direct.c:26-231): sources
+// blockIdx.y of gridDim.y parts onto EV_CHUNK targets, as k_direct.
 template <int KT>
-__global__ void __launch_bounds__(SS_THREADS)
+__global__ void __launch_bounds__(EV_THREADS, 4)
 k_ss_direct(int nt, int ns, const double *__restrict__ tx, const double *__restrict__ ty,
             const double *__restrict__ tz, const double *__restrict__ tq, const double *__restrict__ sx,
             const double *__restrict__ sy, const double *__restrict__ sz, const double *__restrict__ sq,
             const double *__restrict__ sw, double kp, double kp2, double *__restrict__ out)
 {
-    __shared__ double s_x[SS_TILE], s_y[SS_TILE], s_z[SS_TILE], s_q[SS_TILE], s_w[SS_TILE];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = t < nt;
-    const double x = active ? tx[t] : 0.0, y = active ? ty[t] : 0.0, z = active ? tz[t] : 0.0;
-    const double q = active ? tq[t] : 0.0;
-    double acc = 0.0;
-    for (int c0 = 0; c0 < ns; c0 += SS_TILE) {
-        const int cm = min(SS_TILE, ns - c0);
-        for (int i = threadIdx.x; i < cm; i += blockDim.x) {
-            s_x[i] = sx[c0 + i]; s_y[i] = sy[c0 + i]; s_z[i] = sz[c0 + i];
-            s_q[i] = sq[c0 + i]; s_w[i] = sw[c0 + i];
-        }
-        __syncthreads();
-        for (int i = 0; i < cm; i++)
-            acc += ss_pp<KT>(x - s_x[i], y - s_y[i], z - s_z[i], s_q[i], s_w[i], q, kp, kp2);
-        __syncthreads();
+    extern __shared__ __align__(16) double sm[];
+    __shared__ double red[2 * EV_THREADS];
+    __shared__ double2 tab[EXP64_TAB];
+    const SsKern k = ss_kern<KT>(kp, kp2, tab);
+    const int t0 = blockIdx.x * EV_CHUNK;
+    const Lanes w(min(EV_CHUNK, nt - t0));
+    Out2 o;
+    double q[2], acc[2] = {0.0, 0.0};
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+        const int t = t0 + w.out(b);
+        o.x[b] = tx[t]; o.y[b] = ty[t]; o.z[b] = tz[t]; q[b] = tq[t];
     }
-    if (active) out[t] = acc;
+    const int s0 = (int)((int64_t)ns * blockIdx.y / gridDim.y), s1 = (int)((int64_t)ns * (blockIdx.y + 1) / gridDim.y);
+    ss_near<KT>(acc, ss_tile(sm), s0, k.lib ? 0 : s1 - s0, sx, sy, sz, sq, sw, o, q, w, k);
+#pragma unroll 1
+    for (int b = 0; b < 2; b++)
+        if (w.active[b] && (k.lib || !isfinite(acc[b]))) {
+            acc[b] = 0.0;
+            for (int c0 = s0; c0 < s1; c0 += EV_TILE)
+                for (int i = c0 + w.slice; i < min(s1, c0 + EV_TILE); i += w.slices)
+                    acc[b] += ss_pp<KT>(o.x[b] - sx[i], o.y[b] - sy[i], o.z[b] - sz[i], sq[i], sw[i], q[b], kp, kp2);
+        }
+    sum_slices(acc, red, w);
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+        if (w.active[b] && w.slice == 0) out[(size_t)blockIdx.y * nt + t0 + w.out(b)] = acc[b];
+}
+
+// Dynamic shared memory: a cluster's grid and both proxy arrays (Lagrange), or a tile.
+size_t ss_smem(int n, bool hermite)
+{
+    const size_t np1 = n + 1, far = sizeof(double) * (3 * np1 + (hermite ? 0 : 2 * np1 * np1 * np1));
+    return far > SS_TILE_BYTES ? far : SS_TILE_BYTES;
 }
 
 template <int KT, bool HERM>
 void ss_targets_t(const SsTargetsArgs &a, cudaStream_t st)
 {
-    k_ss_targets<KT, HERM><<<a.nitems, SS_THREADS, 0, st>>>(a);
+    const size_t sm = ss_smem(a.n, HERM);
+    cudaFuncSetAttribute(k_ss_targets<KT, HERM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_ss_targets<KT, HERM><<<dim3(a.nitems, a.partial ? EV_SEGS : 1), EV_THREADS, sm, st>>>(a);
+    if (a.partial)
+        launch_sum_segments(a.nitems, a.items, EV_CHUNK, a.leaf_node, a.t_ibeg, a.t_numpar, a.partial, a.pstride, a.pot, st);
 }
 
 }  // namespace
 
-int ss_chunk() { return SS_THREADS; }
+int ss_chunk() { return EV_CHUNK; }
 
 void launch_ss_targets(int kernel, bool hermite, const SsTargetsArgs &a, cudaStream_t st)
 {
@@ -313,11 +511,19 @@ void launch_ss_targets(int kernel, bool hermite, const SsTargetsArgs &a, cudaStr
     else hermite ? ss_targets_t<K_REGCOULOMB, true>(a, st) : ss_targets_t<K_REGCOULOMB, false>(a, st);
 }
 
+template <int KT>
+static void ss_grids_t(const SsGridsArgs &a, cudaStream_t st)
+{
+    const size_t sm = ss_smem(a.n, false);
+    cudaFuncSetAttribute(k_ss_grids<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_ss_grids<KT><<<a.nitems, SS_THREADS, sm, st>>>(a);
+}
+
 void launch_ss_grids(int kernel, const SsGridsArgs &a, cudaStream_t st)
 {
     if (a.nitems <= 0) return;
-    if (kernel == K_COULOMB) k_ss_grids<K_COULOMB><<<a.nitems, SS_THREADS, 0, st>>>(a);
-    else k_ss_grids<K_YUKAWA><<<a.nitems, SS_THREADS, 0, st>>>(a);
+    if (kernel == K_COULOMB) ss_grids_t<K_COULOMB>(a, st);
+    else ss_grids_t<K_YUKAWA>(a, st);
 }
 
 bool ss_direct_kernel(int kernel)
@@ -327,16 +533,20 @@ bool ss_direct_kernel(int kernel)
 
 void launch_ss_direct(int kernel, int nt, int ns, const double *tx, const double *ty, const double *tz,
                       const double *tq, const double *sx, const double *sy, const double *sz, const double *sq,
-                      const double *sw, double kp, double kp2, double *out, cudaStream_t st)
+                      const double *sw, double kp, double kp2, double *partial, double *out, cudaStream_t st)
 {
     if (nt <= 0) return;
-    const int grid = (nt + SS_THREADS - 1) / SS_THREADS;
-#define BT_SSD(K) k_ss_direct<K><<<grid, SS_THREADS, 0, st>>>(nt, ns, tx, ty, tz, tq, sx, sy, sz, sq, sw, kp, kp2, out)
+    const int parts = direct_parts(nt, ns);
+    double *dst = parts > 1 ? partial : out;
+    const dim3 grid((nt + EV_CHUNK - 1) / EV_CHUNK, parts);
+#define BT_SSD(K)                                                                                                   \
+    k_ss_direct<K><<<grid, EV_THREADS, SS_TILE_BYTES, st>>>(nt, ns, tx, ty, tz, tq, sx, sy, sz, sq, sw, kp, kp2, dst)
     if (kernel == K_COULOMB) BT_SSD(K_COULOMB);
     else if (kernel == K_YUKAWA) BT_SSD(K_YUKAWA);
     else if (kernel == K_REGYUKAWA) BT_SSD(K_REGYUKAWA);
     else BT_SSD(K_REGCOULOMB);
 #undef BT_SSD
+    if (parts > 1) launch_sum_parts(nt, parts, partial, out, st);
 }
 
 void launch_mul(int n, const double *a, const double *b, double *c, cudaStream_t st)

@@ -18,6 +18,8 @@ struct SsTargetsArgs {
     const double *tx, *ty, *tz, *tq;
     double kp, kp2;                             // kernel_params[0], [1]
     double *pot;
+    double *partial = nullptr;                  // a block per segment of an item (EvalTargetsArgs)
+    size_t pstride = 0;
 };
 
 struct SsGridsArgs {
@@ -39,10 +41,11 @@ void launch_ss_grids(int kernel, const SsGridsArgs &a, cudaStream_t st);
 // Kernels with a singularity-subtraction direct sum (Coulomb, Yukawa and
 // their regularized forms); the others ignore the singularity setting.
 bool ss_direct_kernel(int kernel);
-// out[t] = sum_j of the SS pair term over all sources (no correction term)
+// out[t] = sum_j of the SS pair term over all sources (no correction term);
+// partial as in launch_direct
 void launch_ss_direct(int kernel, int nt, int ns, const double *tx, const double *ty, const double *tz,
                       const double *tq, const double *sx, const double *sy, const double *sz, const double *sq,
-                      const double *sw, double kp, double kp2, double *out, cudaStream_t st);
+                      const double *sw, double kp, double kp2, double *partial, double *out, cudaStream_t st);
 void launch_mul(int n, const double *a, const double *b, double *c, cudaStream_t st);
 // pot[i] += c tq[i]
 void launch_ss_correction(int n, double c, const double *tq, double *pot, cudaStream_t st);
