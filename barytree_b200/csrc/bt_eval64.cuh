@@ -29,6 +29,10 @@
 #include "bt_fp64.cuh"
 #include "bt_kernels.cuh"
 
+#ifndef BT_EV_MINB
+#define BT_EV_MINB 4
+#endif
+
 namespace bt {
 
 constexpr int EV_TILE = 512;        // sources per shared-memory tile
@@ -152,7 +156,7 @@ __device__ __forceinline__ void far64_any(double *acc, int np1, const double *g,
     }
 }
 
-// Hermite far field: q holds the 8 moments P apart, qxy, qyz, qxz times 3 and
+// Hermite far field: q holds each point's 8 moments, qxy, qyz, qxz times 3 and
 // qxyz times 15 (K_*_PC_Hermite, src/kernels/coulomb/coulomb_pc.c:66-138).
 // With u = 1/r^2 the value is
 //   1/r [ q + u (qx dx + qy dy + qz dz) + u^2 (qxy dx dy + qyz dy dz + qxz dx dz) + u^3 qxyz dx dy dz ]
@@ -162,7 +166,6 @@ template <int KT>
 __device__ __forceinline__ void herm64(double *acc, int np1, const double *g, const double *q, const Out2 &o,
                                        const Lanes &w, const Kern64 &k)
 {
-    const int P = np1 * np1 * np1;
     for (int row = w.slice; row < np1 * np1; row += w.slices) {
         const int k3 = row / np1, k2 = row - k3 * np1;
         double dy[2], dz[2], dydz[2], dyz[2];
@@ -175,7 +178,9 @@ __device__ __forceinline__ void herm64(double *acc, int np1, const double *g, co
             if (KT == K_REGCOULOMB) dyz[b] += k.eps2;
         }
         for (int i = 0; i < np1; i++) {
-            const double *m = q + row * np1 + i;
+            const double2 *qp = reinterpret_cast<const double2 *>(q + 8 * (row * np1 + i));
+            const double2 qa = qp[0], qb = qp[1], qc = qp[2], qd = qp[3];
+            const double m[8] = {qa.x, qa.y, qb.x, qb.y, qc.x, qc.y, qd.x, qd.y};
 #pragma unroll
             for (int b = 0; b < 2; b++) {
                 const double dx = o.x[b] - g[i], r2 = fma(dx, dx, dyz[b]);
@@ -184,15 +189,15 @@ __device__ __forceinline__ void herm64(double *acc, int np1, const double *g, co
                     const double rinv = rsqrt_sqrt_n(r2, r), u = rinv * rinv;
                     const double kr = k.kp * r, kr2 = kr * kr, p1 = 1.0 + kr, p2 = fma(kr2, 1.0 / 3.0, p1),
                                  p3 = fma(kr2 * kr, 1.0 / 15.0, fma(kr2, 0.4, p1));
-                    const double e = fma(u * p2, m[5 * P] * dydz[b], p1 * fma(m[3 * P], dz[b], m[2 * P] * dy[b]));
-                    const double c = fma(u * p3, m[7 * P] * dydz[b], p2 * fma(m[6 * P], dz[b], m[4 * P] * dy[b]));
-                    const double v = fma(dx * u, fma(u, c, p1 * m[P]), fma(u, e, m[0]));
+                    const double e = fma(u * p2, m[5] * dydz[b], p1 * fma(m[3], dz[b], m[2] * dy[b]));
+                    const double c = fma(u * p3, m[7] * dydz[b], p2 * fma(m[6], dz[b], m[4] * dy[b]));
+                    const double v = fma(dx * u, fma(u, c, p1 * m[1]), fma(u, e, m[0]));
                     acc[b] = fma(rinv * v, exp64(r, k.ex), acc[b]);
                 } else {
                     const double rinv = rsqrt_n(r2), u = rinv * rinv, v = u * dydz[b];
-                    const double e = fma(m[5 * P], v, fma(m[3 * P], dz[b], m[2 * P] * dy[b]));
-                    const double c = fma(m[7 * P], v, fma(m[6 * P], dz[b], m[4 * P] * dy[b]));
-                    acc[b] = fma(rinv, fma(dx * u, fma(u, c, m[P]), fma(u, e, m[0])), acc[b]);
+                    const double e = fma(m[5], v, fma(m[3], dz[b], m[2] * dy[b]));
+                    const double c = fma(m[7], v, fma(m[6], dz[b], m[4] * dy[b]));
+                    acc[b] = fma(rinv, fma(dx * u, fma(u, c, m[1]), fma(u, e, m[0])), acc[b]);
                 }
             }
         }
@@ -356,7 +361,7 @@ __device__ __forceinline__ void sum_slices(double *acc, double *red, const Lanes
 // Particle outputs: PC (clusters) + PP (particles) onto a chunk of a target
 // leaf.  NP1 = n + 1 (Lagrange with a short form), else 0.
 template <int KT, int NP1, bool HERM>
-__global__ void __launch_bounds__(EV_THREADS, 4) k_eval_targets(const __grid_constant__ EvalTargetsArgs a)
+__global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB) k_eval_targets(const __grid_constant__ EvalTargetsArgs a)
 {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[2 * EV_THREADS];
@@ -384,8 +389,14 @@ __global__ void __launch_bounds__(EV_THREADS, 4) k_eval_targets(const __grid_con
             const int s = a.a_idx[e];
             double *g = sm, *q = sm + 3 * np1;
             for (int i = threadIdx.x; i < 3 * np1; i += EV_THREADS) g[i] = a.s_grid[(size_t)s * 3 * np1 + i];
-            for (int i = threadIdx.x; i < nq; i += EV_THREADS)
-                q[i] = a.Q[(size_t)s * nq + i] * (HERM && fast64<KT>() ? herm64_scale(i / P) : 1.0);
+            if constexpr (HERM && fast64<KT>()) {
+                // a point's moments side by side, after the grid's 3 np1 rounded up to 16 bytes
+                q = sm + 3 * np1 + (np1 & 1);
+                for (int i = threadIdx.x; i < nq; i += EV_THREADS)
+                    q[i] = a.Q[(size_t)s * nq + (i & 7) * P + (i >> 3)] * herm64_scale(i & 7);
+            } else {
+                for (int i = threadIdx.x; i < nq; i += EV_THREADS) q[i] = a.Q[(size_t)s * nq + i];
+            }
             __syncthreads();
             if (w.active[0]) {
                 if constexpr (HERM && fast64<KT>()) herm64<KT>(acc, np1, g, q, o, w, k);
@@ -424,7 +435,7 @@ __global__ void __launch_bounds__(EV_THREADS, 4) k_eval_targets(const __grid_con
 // Grid outputs: M2L (clusters, Lagrange) + CP (particles) onto a chunk of a
 // target node's grid points.
 template <int KT, int NP1>
-__global__ void __launch_bounds__(EV_THREADS, 4) k_eval_grids(const __grid_constant__ EvalGridsArgs a)
+__global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB) k_eval_grids(const __grid_constant__ EvalGridsArgs a)
 {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[2 * EV_THREADS];
@@ -488,7 +499,7 @@ __global__ void __launch_bounds__(EV_THREADS, 4) k_eval_grids(const __grid_const
 // Direct sum: sources blockIdx.y of gridDim.y parts onto EV_CHUNK targets;
 // several parts go to `out` nt apart and are added by k_sum_parts.
 template <int KT>
-__global__ void __launch_bounds__(EV_THREADS, 4)
+__global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB)
 k_direct(int nt, int ns, const double *__restrict__ tx, const double *__restrict__ ty, const double *__restrict__ tz,
          const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
          const double *__restrict__ sq, double kp, double kp2, double *__restrict__ out)
@@ -542,7 +553,7 @@ void eval_targets_kt(bool hermite, const EvalTargetsArgs &a, cudaStream_t st)
     const size_t np1 = a.n + 1, P = np1 * np1 * np1;
     if constexpr (fast64<KT>() || KT == K_SINOVERR)
         if (hermite) {
-            eval64_launch(k_eval_targets<KT, 0, true>, a, 3 * np1 + 8 * P, st);
+            eval64_launch(k_eval_targets<KT, 0, true>, a, 3 * np1 + 1 + 8 * P, st);
             return;
         }
     if constexpr (fast64<KT>()) {

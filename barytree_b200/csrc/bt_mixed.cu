@@ -153,18 +153,22 @@ __device__ __forceinline__ void pc_cluster(const float *x, const float *y, const
 }
 
 // Hermite far field of one source cluster for NT targets (FP32; moments
-// q[m * P + j], m = 0..7 in the reference's order q, qx, qy, qz, qxy, qyz,
-// qxz, qxyz, with qxy..qxz pre-multiplied by 3 and qxyz by 15 when staged).
+// q[8 * j + m] of grid point j, m = 0..7 in the reference's order q, qx, qy,
+// qz, qxy, qyz, qxz, qxyz, with qxy..qxz pre-multiplied by 3 and qxyz by 15
+// when staged).  Moments P apart took eight shared-memory reads per point,
+// which the load pipe served more slowly than the FP32 pipe its arithmetic.
 // The terms of K_*_PC_Hermite (src/kernels/coulomb/coulomb_pc.c:66-138,
 // yukawa/yukawa_pc.c, regularized-coulomb/regularized-coulomb_pc.c):
 //   r^-1 q + r^-3 (qx dx + qy dy + qz dz) + 3 r^-5 (qxy dx dy + qyz dy dz
 //   + qxz dx dz) + 15 r^-7 qxyz dx dy dz, Yukawa with exp(-kappa r) and the
-//   polynomials in kappa r.  Kahan-compensated per grid row.
+//   polynomials in kappa r.  Evaluated as 1/r (E + dx u F) with u = 1/r^2 and
+//   E, F nested in u: 14 FP32 operations besides 1/r (19 when every term
+//   formed its power of 1/r and its product of differences).
+//   Kahan-compensated per grid row.
 template <int KT, int NP1, int NT>
 __device__ __forceinline__ void pc_cluster_herm(const float *x, const float *y, const float *z, const float *g,
                                                 const float *q, float kc, float kp, float *out)
 {
-    constexpr int P = NP1 * NP1 * NP1;
     float gx[NT][NP1];
 #pragma unroll
     for (int t = 0; t < NT; t++)
@@ -191,18 +195,16 @@ __device__ __forceinline__ void pc_cluster_herm(const float *x, const float *y, 
 #pragma unroll
             for (int k1 = 0; k1 < NP1; k1++) {
                 const int jj = j + k1;
-                const float q0 = q[jj], q1 = q[P + jj], q2 = q[2 * P + jj], q3 = q[3 * P + jj];
-                const float q4 = q[4 * P + jj], q5 = q[5 * P + jj], q6 = q[6 * P + jj], q7 = q[7 * P + jj];
+                const float4 qa = *reinterpret_cast<const float4 *>(q + 8 * jj),
+                             qb = *reinterpret_cast<const float4 *>(q + 8 * jj + 4);
+                const float q0 = qa.x, q1 = qa.y, q2 = qa.z, q3 = qa.w, q4 = qb.x, q5 = qb.y, q6 = qb.z, q7 = qb.w;
 #pragma unroll
                 for (int t = 0; t < NT; t++) {
                     const float dx = gx[t][k1];
                     const float r2 = fmaf(dx, dx, dyz[t]);
                     const float rinv = rsqrt_apx(r2);
-                    const float rinv2 = rinv * rinv;
-                    const float dxdy = dx * dy[t], dxdz = dx * dz[t];
-                    const float a1 = fmaf(q1, dx, fmaf(q2, dy[t], q3 * dz[t]));
-                    const float a2 = fmaf(q4, dxdy, fmaf(q5, dydz[t], q6 * dxdz));
-                    const float a3 = q7 * dxdy * dz[t];
+                    // sorted by powers of dx: E + dx u F, u = 1/r^2
+                    const float u = rinv * rinv, du = dx * u;
                     if (KT == 2) {
                         // Yukawa: exp(-kappa r) (r^-1 q + r^-3 (1 + kr) a1 + r^-5 (3 + 3kr + k^2r^2) a2
                         // + r^-7 (15 + 15kr + 6k^2r^2 + k^3r^3) a3), with a2, a3 staged x3, x15
@@ -211,11 +213,14 @@ __device__ __forceinline__ void pc_cluster_herm(const float *x, const float *y, 
                         const float p1 = 1.0f + kr;
                         const float p2 = fmaf(kr2, 1.0f / 3.0f, p1);                    // (3 + 3kr + k^2r^2) / 3
                         const float p3 = fmaf(kr2 * kr, 1.0f / 15.0f, fmaf(kr2, 0.4f, p1));  // (15 + 15kr + 6k^2r^2 + k^3r^3) / 15
-                        const float r3 = rinv * rinv2, r5 = r3 * rinv2, r7 = r5 * rinv2;
-                        row[t] = fmaf(e, fmaf(rinv, q0, fmaf(r3 * p1, a1, fmaf(r5 * p2, a2, r7 * p3 * a3))), row[t]);
+                        const float b1 = fmaf(u * p2, q5 * dydz[t], p1 * fmaf(q3, dz[t], q2 * dy[t]));
+                        const float b2 = fmaf(u * p3, q7 * dydz[t], p2 * fmaf(q6, dz[t], q4 * dy[t]));
+                        row[t] = fmaf(rinv * e, fmaf(du, fmaf(u, b2, p1 * q1), fmaf(u, b1, q0)), row[t]);
                     } else {
-                        const float r3 = rinv * rinv2, r5 = r3 * rinv2, r7 = r5 * rinv2;
-                        row[t] = fmaf(rinv, q0, fmaf(r3, a1, fmaf(r5, a2, fmaf(r7, a3, row[t]))));
+                        const float v = u * dydz[t];
+                        const float E = fmaf(u, fmaf(q5, v, fmaf(q3, dz[t], q2 * dy[t])), q0);
+                        const float F = fmaf(u, fmaf(q7, v, fmaf(q6, dz[t], q4 * dy[t])), q1);
+                        row[t] = fmaf(rinv, fmaf(du, F, E), row[t]);
                     }
                 }
             }
@@ -307,7 +312,7 @@ template <int KT, int NP1, int NT>
 __device__ __forceinline__ void pc_cluster_herm_f2(const float *x, const float *y, const float *z, const float *g,
                                                    const f2_t *qd, float kc, float *out)
 {
-    constexpr int P = NP1 * NP1 * NP1, NPR = NT / 2;
+    constexpr int NPR = NT / 2;
     f2_t gx[NPR][NP1];
 #pragma unroll
     for (int p = 0; p < NPR; p++)
@@ -335,8 +340,9 @@ __device__ __forceinline__ void pc_cluster_herm_f2(const float *x, const float *
 #pragma unroll
             for (int k1 = 0; k1 < NP1; k1++) {
                 const int jj = j + k1;
-                const f2_t q0 = qd[jj], q1 = qd[P + jj], q2 = qd[2 * P + jj], q3 = qd[3 * P + jj];
-                const f2_t q4 = qd[4 * P + jj], q5 = qd[5 * P + jj], q6 = qd[6 * P + jj], q7 = qd[7 * P + jj];
+                const ulonglong2 *qv = reinterpret_cast<const ulonglong2 *>(qd + 8 * jj);
+                const ulonglong2 qa = qv[0], qb = qv[1], qc = qv[2], qe = qv[3];
+                const f2_t q0 = qa.x, q1 = qa.y, q2 = qb.x, q3 = qb.y, q4 = qc.x, q5 = qc.y, q6 = qe.x, q7 = qe.y;
 #pragma unroll
                 for (int p = 0; p < NPR; p++) {
                     const f2_t dx = gx[p][k1];
@@ -344,13 +350,10 @@ __device__ __forceinline__ void pc_cluster_herm_f2(const float *x, const float *
                     float ra, rb;
                     f2_split(r2, ra, rb);
                     const f2_t rinv = f2_make(rsqrt_apx(ra), rsqrt_apx(rb));
-                    const f2_t rinv2 = f2_mul(rinv, rinv);
-                    const f2_t dxdy = f2_mul(dx, dy[p]), dxdz = f2_mul(dx, dz[p]);
-                    const f2_t a1 = f2_fma(q1, dx, f2_fma(q2, dy[p], f2_mul(q3, dz[p])));
-                    const f2_t a2 = f2_fma(q4, dxdy, f2_fma(q5, dydz[p], f2_mul(q6, dxdz)));
-                    const f2_t a3 = f2_mul(f2_mul(q7, dxdy), dz[p]);
-                    const f2_t r3 = f2_mul(rinv, rinv2), r5 = f2_mul(r3, rinv2), r7 = f2_mul(r5, rinv2);
-                    row[p] = f2_fma(rinv, q0, f2_fma(r3, a1, f2_fma(r5, a2, f2_fma(r7, a3, row[p]))));
+                    const f2_t u = f2_mul(rinv, rinv), v = f2_mul(u, dydz[p]);
+                    const f2_t E = f2_fma(u, f2_fma(q5, v, f2_fma(q3, dz[p], f2_mul(q2, dy[p]))), q0);
+                    const f2_t F = f2_fma(u, f2_fma(q7, v, f2_fma(q6, dz[p], f2_mul(q4, dy[p]))), q1);
+                    row[p] = f2_fma(rinv, f2_fma(f2_mul(dx, u), F, E), row[p]);
                 }
             }
             j += NP1;
@@ -578,8 +581,9 @@ __device__ __forceinline__ void targets_item(const MixedTargetsArgs &a, const in
             if (HERM) {
                 const float *Qs = a.Q32[deg] + (size_t)s * 8 * P;
                 for (int i = threadIdx.x; i < 8 * P; i += blockDim.x) {
-                    const int m = i / P;
-                    const float v = Qs[i] * (m == 7 ? 15.0f : m >= 4 ? 3.0f : 1.0f);
+                    // a point's moments side by side: the loop reads them in 128-bit words
+                    const int m = i & 7;
+                    const float v = Qs[m * P + (i >> 3)] * (m == 7 ? 15.0f : m >= 4 ? 3.0f : 1.0f);
                     if constexpr (far_packed<KT, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(v, v);
                     else q[i] = v;
                 }

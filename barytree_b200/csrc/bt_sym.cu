@@ -64,7 +64,10 @@ constexpr int SY_THREADS = 128;
 constexpr int SY_TPT = BT_SYM_TPT;
 constexpr int SY_NP = SY_TPT / 2;
 constexpr int SY_CHUNK = SY_TPT * 32;          // targets of A a warp holds at a time
-constexpr int SY_TILE = 256;                   // sources of B per shared-memory tile
+#ifndef BT_SYM_TILE
+#define BT_SYM_TILE 256
+#endif
+constexpr int SY_TILE = BT_SYM_TILE;                   // sources of B per shared-memory tile
 constexpr int SY_SB = 16;                      // sources per warp reduction
 constexpr int SY_WARPS = SY_THREADS / 32;
 constexpr float SY_PAD_POS = 1.0e18f;          // padding sources: far away, no charge
@@ -294,19 +297,27 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(const 
     for (int j = threadIdx.x; j < nb; j += SY_THREADS) outB[j] = CLAMP ? accB[j] + outB[j] : accB[j];
 }
 
-__global__ void k_sym_gather(SymGatherArgs a)
+// One block per leaf and GATHER_THREADS of its particles; the slices' offsets
+// go through shared memory, so that a thread's loads do not wait for them.
+__global__ void __launch_bounds__(GATHER_THREADS) k_sym_gather(SymGatherArgs a)
 {
+    __shared__ int64_t slot[GATHER_THREADS];
     const int u = blockIdx.x;
     const int64_t k0 = a.in_off[u], k1 = a.in_off[u + 1];
-    if (k0 == k1) return;
     const int node = a.leaf_node[u];
-    const int ib = a.ibeg[node], nb = a.numpar[node];
-    for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < nb; j += gridDim.y * blockDim.x) {
-        double s = 0.0;
-#pragma unroll 4
-        for (int64_t k = k0; k < k1; k++) s += (double)a.partial[a.in_slot[k] + j];
-        a.pot[ib + j] += s;
+    const int nb = a.numpar[node], j = blockIdx.y * GATHER_THREADS + threadIdx.x;
+    if (k0 == k1 || (int)blockIdx.y * GATHER_THREADS >= nb) return;
+    double s = 0.0;
+    for (int64_t b = k0; b < k1; b += GATHER_THREADS) {
+        const int m = (int)min((int64_t)GATHER_THREADS, k1 - b);
+        __syncthreads();
+        if ((int)threadIdx.x < m) slot[threadIdx.x] = a.in_slot[b + threadIdx.x];
+        __syncthreads();
+        if (j < nb)
+#pragma unroll 8
+            for (int k = 0; k < m; k++) s += (double)a.partial[slot[k] + j];
     }
+    if (j < nb) a.pot[a.ibeg[node] + j] += s;
 }
 
 }  // namespace
@@ -329,7 +340,7 @@ void launch_pp_sym_close(int kernel, const SymArgs &a, cudaStream_t st)
 
 void launch_sym_gather(const SymGatherArgs &a, cudaStream_t st)
 {
-    if (a.nleaves > 0) k_sym_gather<<<dim3(a.nleaves, 4), 128, 0, st>>>(a);
+    if (a.nleaves > 0) k_sym_gather<<<dim3(a.nleaves, SYM_MAX_LEAF / GATHER_THREADS), GATHER_THREADS, 0, st>>>(a);
 }
 
 }  // namespace bt

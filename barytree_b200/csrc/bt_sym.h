@@ -17,6 +17,9 @@ constexpr int SYM_MAX_LEAF = 2048;
 // gain is small, keep the sums of every direction.
 constexpr int SYM64_MIN_LEAF = 512;
 
+// Threads (particles) per block of the gathers.
+constexpr int GATHER_THREADS = 128;
+
 // Particles of A per block: a pair of leaves (A, B) is evaluated by
 // sym_parts(numpar[A]) blocks.
 constexpr int SYM_PART = 512;

@@ -25,6 +25,10 @@
 #include "bt_eval64.cuh"
 #include "bt_sym.h"
 
+#ifndef BT_S64_MINB
+#define BT_S64_MINB 3
+#endif
+
 namespace bt {
 
 namespace {
@@ -60,7 +64,7 @@ __device__ __noinline__ double leaf_again(const Sym64Args &a, int i, int jb, int
 }
 
 template <int KT>
-__global__ void __launch_bounds__(S64_THREADS, 4) k_pp_sym64(const __grid_constant__ Sym64Args a)
+__global__ void __launch_bounds__(S64_THREADS, BT_S64_MINB) k_pp_sym64(const __grid_constant__ Sym64Args a)
 {
     __shared__ double2 xy[S64_TILE], zq[S64_TILE];
     __shared__ double accB[SYM_MAX_LEAF];
@@ -140,19 +144,27 @@ __global__ void __launch_bounds__(S64_THREADS, 4) k_pp_sym64(const __grid_consta
     }
 }
 
-__global__ void k_sym_gather64(SymGather64Args a)
+// One block per leaf and GATHER_THREADS of its particles; the slices' offsets
+// go through shared memory, so that a thread's loads do not wait for them.
+__global__ void __launch_bounds__(GATHER_THREADS) k_sym_gather64(SymGather64Args a)
 {
+    __shared__ int64_t slot[GATHER_THREADS];
     const int u = blockIdx.x;
     const int64_t k0 = a.in_off[u], k1 = a.in_off[u + 1];
-    if (k0 == k1) return;
     const int node = a.leaf_node[u];
-    const int ib = a.ibeg[node], nb = a.numpar[node];
-    for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < nb; j += gridDim.y * blockDim.x) {
-        double s = 0.0;
-#pragma unroll 4
-        for (int64_t k = k0; k < k1; k++) s += a.partial[a.in_slot[k] + j];
-        a.pot[ib + j] += s;
+    const int nb = a.numpar[node], j = blockIdx.y * GATHER_THREADS + threadIdx.x;
+    if (k0 == k1 || (int)blockIdx.y * GATHER_THREADS >= nb) return;
+    double s = 0.0;
+    for (int64_t b = k0; b < k1; b += GATHER_THREADS) {
+        const int m = (int)min((int64_t)GATHER_THREADS, k1 - b);
+        __syncthreads();
+        if ((int)threadIdx.x < m) slot[threadIdx.x] = a.in_slot[b + threadIdx.x];
+        __syncthreads();
+        if (j < nb)
+#pragma unroll 8
+            for (int k = 0; k < m; k++) s += a.partial[slot[k] + j];
     }
+    if (j < nb) a.pot[a.ibeg[node] + j] += s;
 }
 
 }  // namespace
@@ -167,7 +179,7 @@ void launch_pp_sym64(int kernel, const Sym64Args &a, cudaStream_t st)
 
 void launch_sym_gather64(const SymGather64Args &a, cudaStream_t st)
 {
-    if (a.nleaves > 0) k_sym_gather64<<<dim3(a.nleaves, 4), 128, 0, st>>>(a);
+    if (a.nleaves > 0) k_sym_gather64<<<dim3(a.nleaves, SYM_MAX_LEAF / GATHER_THREADS), GATHER_THREADS, 0, st>>>(a);
 }
 
 }  // namespace bt
