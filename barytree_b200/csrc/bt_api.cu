@@ -250,6 +250,50 @@ struct Layout {
     }
 };
 
+// Host-to-device copies of one plan.  Each async copy costs the host some
+// microseconds, and a small system has about 35 of a few KB: neighbouring
+// small arrays (in device order) are gathered on the host and go in one copy.
+// Large arrays are copied from where they are.
+struct Uploads {
+    struct Item {
+        char *dst;
+        const char *src;
+        size_t bytes;
+    };
+    static constexpr size_t SMALL = 32 * 1024, GAP = 512;
+    std::vector<Item> items;
+    std::vector<char> buf;
+    void add(void *dst, const void *src, size_t bytes)
+    {
+        if (bytes > 0) items.push_back(Item{(char *)dst, (const char *)src, bytes});
+    }
+    cudaError_t run(cudaStream_t st)
+    {
+        std::sort(items.begin(), items.end(), [](const Item &a, const Item &b) { return a.dst < b.dst; });
+        cudaError_t e = cudaSuccess;
+        for (size_t i = 0; i < items.size() && e == cudaSuccess;) {
+            size_t j = i + 1;
+            if (items[i].bytes <= SMALL)
+                while (j < items.size() && items[j].bytes <= SMALL &&
+                       (size_t)(items[j].dst - (items[j - 1].dst + items[j - 1].bytes)) <= GAP)
+                    j++;
+            if (j == i + 1) {
+                e = cudaMemcpyAsync(items[i].dst, items[i].src, items[i].bytes, cudaMemcpyHostToDevice, st);
+            } else {
+                char *d0 = items[i].dst;
+                const size_t span = (size_t)(items[j - 1].dst + items[j - 1].bytes - d0);
+                buf.resize(std::max(buf.size(), span));
+                for (size_t k = i; k < j; k++) memcpy(buf.data() + (items[k].dst - d0), items[k].src, items[k].bytes);
+                // pageable memory: the buffer has been read when the call returns
+                e = cudaMemcpyAsync(d0, buf.data(), span, cudaMemcpyHostToDevice, st);
+            }
+            i = j;
+        }
+        items.clear();
+        return e;
+    }
+};
+
 #define CK(call)                                                                      \
     do {                                                                              \
         cudaError_t e_ = (call);                                                      \
@@ -1304,8 +1348,9 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         std::vector<int> pcount(T.n, P);
         if (!tnode_need.empty())
             for (int i = 0; i < T.n; i++) pcount[i] = tnode_need[i] ? P : 0;
-        // points per item: the FP64 Lagrange kernel takes two per thread
-        grid_items = make_items(T.n, pcount.data(), mixed || ssm || herm ? 128 : bt::EV_CHUNK, gcost);
+        // points per item: the Lagrange kernels take two per thread
+        static_assert(bt::MX_CHUNK == bt::EV_CHUNK, "one chunk of grid points for both precisions");
+        grid_items = make_items(T.n, pcount.data(), ssm || herm ? 128 : bt::EV_CHUNK, gcost);
         std::vector<double> lcost(T.nleaves, 1.0);
         l2p_items = make_items(T.nleaves, leaf_count.data(), 128, lcost);
     }
@@ -1619,7 +1664,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     int *d_order;
     double *d_out;
     pt.mark("plan: Hermite chunks, device layout");
-    Layout L;
+    Layout L, W;       // arrays that are uploaded, side by side; work arrays after them
     if (dp) {
         d_sx = (double *)dp->sx; d_sy = (double *)dp->sy; d_sz = (double *)dp->sz; d_sq = (double *)dp->sq;
         d_tx = (double *)dp->tx; d_ty = (double *)dp->ty; d_tz = (double *)dp->tz; d_order = (int *)dp->order;
@@ -1627,11 +1672,11 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         L.add(&d_sx, ns); L.add(&d_sy, ns); L.add(&d_sz, ns); L.add(&d_sq, ns);
         L.add(&d_tx, nt); L.add(&d_ty, nt); L.add(&d_tz, nt); L.add(&d_order, nt);
     }
-    L.add(&d_pot, nt);
+    W.add(&d_pot, nt);
     L.add(&d_sgrid, sgrid.size()); L.add(&d_tgrid, tgrid.size());
     L.add(&d_slen, slen.size()); L.add(&d_tlen, tlen.size()); L.add(&d_ww, BT_MAX_DEGREE + 1);
-    if (need_src_clusters) L.add(&d_Q, (size_t)S.n * P * nq);
-    if (need_tgt_grids) L.add(&d_Phi, (size_t)T.n * P * nq);
+    if (need_src_clusters) W.add(&d_Q, (size_t)S.n * P * nq);
+    if (need_tgt_grids) W.add(&d_Phi, (size_t)T.n * P * nq);
     L.add(&d_sibeg, S.n); L.add(&d_snum, S.n); L.add(&d_snch, S.n); L.add(&d_sch, 8 * (size_t)S.n);
     L.add(&d_sleaves, S.nleaves); L.add(&d_slvl, S.lvl_off ? S.lvl_off[S.max_depth] : 0);
     L.add(&d_tibeg, T.n); L.add(&d_tnum, T.n); L.add(&d_tnch, T.n); L.add(&d_tch, 8 * (size_t)T.n);
@@ -1641,24 +1686,24 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     L.add(&d_ccoff, pl.g_cc.rows + 1); L.add(&d_ccidx, pl.g_cc.off[pl.g_cc.rows]);
     L.add(&d_cpoff, pl.g_cp.rows + 1); L.add(&d_cpidx, pl.g_cp.off[pl.g_cp.rows]);
     L.add(&d_evitems, ev_items.size()); L.add(&d_griditems, grid_items.size()); L.add(&d_l2pitems, l2p_items.size());
-    L.add(&d_out, nt);
+    W.add(&d_out, nt);
     int *d_queue;           // work-queue counters of the two evaluation kernels, then the error flag
-    L.add(&d_queue, 3);
+    W.add(&d_queue, 3);
     // subtraction: target charges and source weights in tree order, q*w,
     // the weight proxies and the weight field, a staging buffer for the
     // caller-order inputs, and the source order when the host built the tree
     double *d_tq = nullptr, *d_sw = nullptr, *d_qw = nullptr, *d_W = nullptr, *d_Phiw = nullptr, *d_ssin = nullptr;
     int *d_sordh = nullptr;
     if (ssm) {
-        L.add(&d_tq, nt); L.add(&d_sw, ns); L.add(&d_qw, ns); L.add(&d_ssin, std::max(nt, ns));
-        if (need_src_clusters) L.add(&d_W, (size_t)S.n * P * nq);
-        if (need_tgt_grids) L.add(&d_Phiw, (size_t)T.n * P);
+        W.add(&d_tq, nt); W.add(&d_sw, ns); W.add(&d_qw, ns); W.add(&d_ssin, std::max(nt, ns));
+        if (need_src_clusters) W.add(&d_W, (size_t)S.n * P * nq);
+        if (need_tgt_grids) W.add(&d_Phiw, (size_t)T.n * P);
         if (!dp) L.add(&d_sordh, ns);
     }
     if (herm && need_src_clusters) {
         L.add(&d_hchunks, hchunks.size());
         L.add(&d_hred, hred.size());
-        L.add(&d_hpartial, (size_t)hslots * 8 * P);
+        W.add(&d_hpartial, (size_t)hslots * 8 * P);
     }
     float4 *d_spos = nullptr, *d_tpos = nullptr;
     float *d_Q32 = nullptr;
@@ -1679,27 +1724,29 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         L.add(&d_sym_blocks, sym_blocks.size());
         L.add(&d_sym_pairs, sym_pairs.size()); L.add(&d_sym_slot, sym_slot.size());
         L.add(&d_sym_in_off, sym_in_off.size()); L.add(&d_sym_in_slot, sym_in_slot.size());
-        if (!mixed) L.add(&d_sym_partial64, (size_t)sym_total);
+        if (!mixed) W.add(&d_sym_partial64, (size_t)sym_total);
     }
     if (mixed) {
-        L.add(&d_spos, ns); L.add(&d_tpos, nt);
-        if (need_src_clusters) L.add(&d_Q32, (size_t)S.n * P * nq);
+        W.add(&d_spos, ns); W.add(&d_tpos, nt);
+        if (need_src_clusters) W.add(&d_Q32, (size_t)S.n * P * nq);
         L.add(&d_sctr, sctr.size()); L.add(&d_tctr, tctr.size());
         L.add(&d_mxdoff, mx_doff.size()); L.add(&d_mxdidx, mx_didx.size()); L.add(&d_mxdflag, mx_dflag.size());
         L.add(&d_mxcpoff, mx_cpoff.size()); L.add(&d_mxcpidx, mx_cpidx.size());
         if (pl.a_deg) L.add(&d_adeg, n_approx);
         L.add(&d_srad, S.n); L.add(&d_trad, T.n);
         if ((int64_t)sym_blocks.size() > sym_far_blocks) L.add(&d_sbox, 6 * (size_t)S.n);
-        if (!sym_pairs.empty()) L.add(&d_sym_partial, (size_t)sym_total);
+        if (!sym_pairs.empty()) W.add(&d_sym_partial, (size_t)sym_total);
         for (size_t i = 0; i < xdeg.size(); i++) {
             size_t Pd = (size_t)(xdeg[i] + 1) * (xdeg[i] + 1) * (xdeg[i] + 1);
             L.add(&d_xgrid[i], xgrid[i].size());
-            L.add(&d_xQ[i], (size_t)S.n * Pd);
-            L.add(&d_xQ32[i], (size_t)S.n * Pd);
+            W.add(&d_xQ[i], (size_t)S.n * Pd);
+            W.add(&d_xQ32[i], (size_t)S.n * Pd);
             L.add(&d_xleaves[i], xleaves[i].size());
             L.add(&d_xlvl[i], xlvl[i].size());
         }
     }
+
+    L.reqs.insert(L.reqs.end(), W.reqs.begin(), W.reqs.end());
 
     // Segment sums of the evaluation kernels, where their work items are
     // few (the results are the same without them): up to EV_SEGS doubles per
@@ -1730,8 +1777,9 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
 
     double t_setup = now_ms();
     {
-#define UP(dst, src, cnt)                                                                              \
-    if ((cnt) > 0) CK(cudaMemcpyAsync(dst, src, sizeof(*(src)) * (size_t)(cnt), cudaMemcpyHostToDevice, st))
+        Uploads ups;
+        std::vector<double> sbox;
+#define UP(dst, src, cnt) ups.add(dst, src, sizeof(*(src)) * (size_t)(cnt))
         if (!dp) {
             UP(d_sx, pl.src.x, ns); UP(d_sy, pl.src.y, ns); UP(d_sz, pl.src.z, ns); UP(d_sq, pl.src.q, ns);
             UP(d_tx, pl.tgt.x, nt); UP(d_ty, pl.tgt.y, nt); UP(d_tz, pl.tgt.z, nt);
@@ -1757,17 +1805,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         }
         UP(d_griditems, grid_items.data(), grid_items.size());
         UP(d_l2pitems, l2p_items.data(), l2p_items.size());
-        if (ssm) {
-            const cudaMemcpyKind kin = ss->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-            const int *sorder = dp ? dp->sorder : d_sordh;
-            if (!dp) UP(d_sordh, pl.src.order, ns);
-            if (nt > 0) CK(cudaMemcpyAsync(d_ssin, ss->tq, sizeof(double) * (size_t)nt, kin, st));
-            bt::launch_gather(nt, d_order, d_ssin, d_tq, st);
-            if (ns > 0) CK(cudaMemcpyAsync(d_ssin, ss->sw, sizeof(double) * (size_t)ns, kin, st));
-            bt::launch_gather(ns, sorder, d_ssin, d_sw, st);
-            bt::launch_mul(ns, d_sq, d_sw, d_qw, st);
-            launches += 3;
-        }
+        if (ssm && !dp) UP(d_sordh, pl.src.order, ns);
         if (!sym_pairs.empty()) {
             UP(d_sym_blocks, sym_blocks.data(), sym_blocks.size());
             UP(d_sym_pairs, sym_pairs.data(), sym_pairs.size()); UP(d_sym_slot, sym_slot.data(), sym_slot.size());
@@ -1777,7 +1815,6 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             UP(d_sctr, sctr.data(), sctr.size()); UP(d_tctr, tctr.data(), tctr.size());
             UP(d_mxdoff, mx_doff.data(), mx_doff.size()); UP(d_mxdidx, mx_didx.data(), mx_didx.size());
             UP(d_mxdflag, mx_dflag.data(), mx_dflag.size());
-            std::vector<double> sbox;
             if (d_sbox) {
                 sbox.resize(6 * (size_t)S.n);
                 for (int i = 0; i < S.n; i++) {
@@ -1794,6 +1831,17 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
                 UP(d_xlvl[i], xlvl[i].data(), xlvl[i].size());
             }
             UP(d_mxcpoff, mx_cpoff.data(), mx_cpoff.size()); UP(d_mxcpidx, mx_cpidx.data(), mx_cpidx.size());
+        }
+        CK(ups.run(st));
+        if (ssm) {
+            const cudaMemcpyKind kin = ss->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+            const int *sorder = dp ? dp->sorder : d_sordh;
+            if (nt > 0) CK(cudaMemcpyAsync(d_ssin, ss->tq, sizeof(double) * (size_t)nt, kin, st));
+            bt::launch_gather(nt, d_order, d_ssin, d_tq, st);
+            if (ns > 0) CK(cudaMemcpyAsync(d_ssin, ss->sw, sizeof(double) * (size_t)ns, kin, st));
+            bt::launch_gather(ns, sorder, d_ssin, d_sw, st);
+            bt::launch_mul(ns, d_sq, d_sw, d_qw, st);
+            launches += 3;
         }
 #undef UP
         cudaEvent_t *ev = ctx->ev;

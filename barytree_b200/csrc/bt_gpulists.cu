@@ -32,6 +32,7 @@ namespace {
 
 constexpr int GL_LANES = 8;               // lanes per batch
 constexpr int GL_THREADS = 64;
+constexpr size_t GL_PACK = 256 * 1024;     // uploads below this go in one copy
 constexpr int GL_MAX_STACK = 384;          // shared-memory stack slots per batch
 
 // What a node is to the batch; in the upper bits of a stack entry.
@@ -135,8 +136,9 @@ int gpu_pc_lists(const bt_tree *trav, const bt_tree *bat, const bt_params *o, vo
     int *d_child = (int *)take(sizeof(int) * 8 * (size_t)nn);
     double4 *d_bat = (double4 *)take(sizeof(double4) * (size_t)nb);
     int *d_root = (int *)take(sizeof(int) * (size_t)nb);
-    int *d_cnt = (int *)take(sizeof(int) * 2 * (size_t)nb);
-    int *d_ovf = (int *)take(sizeof(int));
+    const size_t up_bytes = (size_t)(p - (char *)work);       // everything uploaded lies before here
+    int *d_cnt = (int *)take(sizeof(int) * (2 * (size_t)nb + 1));
+    int *d_ovf = d_cnt + 2 * (size_t)nb;
     int64_t *d_off = (int64_t *)take(sizeof(int64_t) * 2 * ((size_t)nb + 1));
     if (!d_off) return -1;
 
@@ -157,11 +159,19 @@ int gpu_pc_lists(const bt_tree *trav, const bt_tree *bat, const bt_params *o, vo
 
     cudaError_t e;
 #define GL_CK(x) do { if ((e = (x)) != cudaSuccess) return (int)e; } while (0)
-    GL_CK(cudaMemcpyAsync(d_geo, geo.data(), sizeof(double4) * (size_t)nn, cudaMemcpyHostToDevice, st));
-    GL_CK(cudaMemcpyAsync(d_cn, cn.data(), sizeof(int2) * (size_t)nn, cudaMemcpyHostToDevice, st));
-    GL_CK(cudaMemcpyAsync(d_child, trav->child, sizeof(int) * 8 * (size_t)nn, cudaMemcpyHostToDevice, st));
-    GL_CK(cudaMemcpyAsync(d_bat, bg.data(), sizeof(double4) * (size_t)nb, cudaMemcpyHostToDevice, st));
-    GL_CK(cudaMemcpyAsync(d_root, root.data(), sizeof(int) * (size_t)nb, cudaMemcpyHostToDevice, st));
+    // small trees: one copy instead of five
+    std::vector<char> hup(up_bytes <= GL_PACK ? up_bytes : 0);
+    auto upload = [&](void *dst, const void *src, size_t bytes) {
+        if (hup.empty()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+        memcpy(hup.data() + ((char *)dst - (char *)work), src, bytes);
+        return cudaSuccess;
+    };
+    GL_CK(upload(d_geo, geo.data(), sizeof(double4) * (size_t)nn));
+    GL_CK(upload(d_cn, cn.data(), sizeof(int2) * (size_t)nn));
+    GL_CK(upload(d_child, trav->child, sizeof(int) * 8 * (size_t)nn));
+    GL_CK(upload(d_bat, bg.data(), sizeof(double4) * (size_t)nb));
+    GL_CK(upload(d_root, root.data(), sizeof(int) * (size_t)nb));
+    if (!hup.empty()) GL_CK(cudaMemcpyAsync(work, hup.data(), up_bytes, cudaMemcpyHostToDevice, st));
     GL_CK(cudaMemsetAsync(d_ovf, 0, sizeof(int), st));
     const size_t smem = sizeof(int) * (size_t)(GL_THREADS / GL_LANES) * (size_t)cap;
     GL_CK(cudaFuncSetAttribute(k_pc_traverse<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -172,8 +182,7 @@ int gpu_pc_lists(const bt_tree *trav, const bt_tree *bat, const bt_params *o, vo
                                                            cap, d_cnt, nullptr, nullptr, nullptr, nullptr, d_ovf);
     GL_CK(cudaGetLastError());
     std::vector<int> cnt(2 * (size_t)nb + 1);
-    GL_CK(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * 2 * (size_t)nb, cudaMemcpyDeviceToHost, st));
-    GL_CK(cudaMemcpyAsync(cnt.data() + 2 * (size_t)nb, d_ovf, sizeof(int), cudaMemcpyDeviceToHost, st));
+    GL_CK(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * (2 * (size_t)nb + 1), cudaMemcpyDeviceToHost, st));
     GL_CK(cudaStreamSynchronize(st));
     *launches += 1;
     if (cnt[2 * (size_t)nb]) return -1;

@@ -62,8 +62,7 @@ struct ChunkArgs {
 };
 
 __global__ void k_boxes(ChunkArgs c, const double *__restrict__ x, const double *__restrict__ y,
-                        const double *__restrict__ z, unsigned long long *__restrict__ kmin,
-                        unsigned long long *__restrict__ kmax)
+                        const double *__restrict__ z, unsigned long long *__restrict__ key)
 {
     const int ch = blockIdx.x, node = c.chunk_node[ch], b = c.chunk_begin[ch], n = c.chunk_len[ch];
     unsigned long long mn[3] = {~0ULL, ~0ULL, ~0ULL}, mx[3] = {0, 0, 0};
@@ -81,8 +80,8 @@ __global__ void k_boxes(ChunkArgs c, const double *__restrict__ x, const double 
     }
     if ((threadIdx.x & 31) == 0) {
         for (int a = 0; a < 3; a++) {
-            atomicMin(&kmin[3 * node + a], mn[a]);
-            atomicMax(&kmax[3 * node + a], mx[a]);
+            atomicMin(&key[6 * node + a], mn[a]);
+            atomicMin(&key[6 * node + 3 + a], ~mx[a]);       // the largest, complemented: one fill serves both
         }
     }
 }
@@ -266,7 +265,7 @@ size_t gpu_tree_work_bytes(int n, int maxpar, bool with_q, int nsys)
     return per * (size_t)n + (size_t)n            // second copy of the particles, slot codes
            + L * (2 * 3 * 8 + 4 * 8 * 4 + 3 * 8 + 3)  // boxes, part counts, mids, axes
            + C * (3 * 4 + 2 * 8 * 4)              // chunk descriptors, histograms, offsets
-           + 24 * 256;
+           + 24 * 256 + 16;
 }
 
 int gpu_build_tree(int n, const double *x, const double *y, const double *z, const double *q, int maxpar,
@@ -299,16 +298,13 @@ int gpu_build_forest(int nsys, const int64_t *sys_off, const double *x, const do
     if (!with_q) A.q = nullptr;
     unsigned char *code = (unsigned char *)take((size_t)n);
     const size_t nodes_max = level_nodes_max(n, maxpar, nsys), chunks_max = (size_t)n / GT_CHUNK + nodes_max;
-    unsigned long long *kmin = (unsigned long long *)take(3 * 8 * nodes_max);
-    unsigned long long *kmax = (unsigned long long *)take(3 * 8 * nodes_max);
-    int *cnt[3];
-    for (int k = 0; k < 3; k++) cnt[k] = (int *)take(8 * 4 * nodes_max);
-    int *cnt0 = (int *)take(8 * 4 * nodes_max);
-    double *mid = (double *)take(3 * 8 * nodes_max);
-    signed char *axis = (signed char *)take(3 * nodes_max);
-    int *c_node = (int *)take(4 * chunks_max), *c_begin = (int *)take(4 * chunks_max), *c_len = (int *)take(4 * chunks_max);
+    unsigned long long *key = (unsigned long long *)take(6 * 8 * nodes_max);
+    int *cnt = (int *)take(3 * 8 * 4 * nodes_max);
+    // what a level uploads lies side by side: one copy for the chunks and, for
+    // a split, the mids, first part counts and axes
+    unsigned char *up = (unsigned char *)take((3 * 8 + 8 * 4 + 3) * nodes_max + 16 + 3 * 4 * chunks_max);
+    std::vector<unsigned char> hup;
     int *c_hist = (int *)take(8 * 4 * chunks_max), *c_off = (int *)take(8 * 4 * chunks_max);
-    ChunkArgs ca{c_node, c_begin, c_len};
 
     GT_CK(cudaMemcpyAsync(A.x, x, 8 * (size_t)n, cudaMemcpyDefault, st));
     GT_CK(cudaMemcpyAsync(A.y, y, 8 * (size_t)n, cudaMemcpyDefault, st));
@@ -326,7 +322,7 @@ int gpu_build_forest(int nsys, const int64_t *sys_off, const double *x, const do
     }
     int lo = 0, hi = (int)nodes.size(), depth = 1;
     std::vector<int> hc_node, hc_begin, hc_len, hc_off;
-    std::vector<unsigned long long> hkmin, hkmax;
+    std::vector<unsigned long long> hkey;
     std::vector<int> hcnt, hchist;
     std::vector<double> hmid;
     std::vector<signed char> haxis;
@@ -343,17 +339,25 @@ int gpu_build_forest(int nsys, const int64_t *sys_off, const double *x, const do
             }
         }
         int nch = (int)hc_node.size();
-        GT_CK(cudaMemcpyAsync(c_node, hc_node.data(), 4 * (size_t)nch, cudaMemcpyHostToDevice, st));
-        GT_CK(cudaMemcpyAsync(c_begin, hc_begin.data(), 4 * (size_t)nch, cudaMemcpyHostToDevice, st));
-        GT_CK(cudaMemcpyAsync(c_len, hc_len.data(), 4 * (size_t)nch, cudaMemcpyHostToDevice, st));
-        GT_CK(cudaMemsetAsync(kmin, 0xff, 3 * 8 * (size_t)L, st));
-        GT_CK(cudaMemsetAsync(kmax, 0x00, 3 * 8 * (size_t)L, st));
-        k_boxes<<<nch, GT_THREADS, 0, st>>>(ca, A.x, A.y, A.z, kmin, kmax);
+        // the chunk arrays at offset `at` of the upload area
+        ChunkArgs ca;
+        auto put_chunks = [&](size_t at) {
+            const size_t b = 4 * (size_t)nch;
+            hup.resize(at + 3 * b);
+            memcpy(hup.data() + at, hc_node.data(), b);
+            memcpy(hup.data() + at + b, hc_begin.data(), b);
+            memcpy(hup.data() + at + 2 * b, hc_len.data(), b);
+            ca.chunk_node = (const int *)(up + at);
+            ca.chunk_begin = (const int *)(up + at + b);
+            ca.chunk_len = (const int *)(up + at + 2 * b);
+        };
+        put_chunks(0);
+        GT_CK(cudaMemcpyAsync(up, hup.data(), hup.size(), cudaMemcpyHostToDevice, st));
+        GT_CK(cudaMemsetAsync(key, 0xff, 6 * 8 * (size_t)L, st));
+        k_boxes<<<nch, GT_THREADS, 0, st>>>(ca, A.x, A.y, A.z, key);
         (*launches)++;
-        hkmin.resize(3 * (size_t)L);
-        hkmax.resize(3 * (size_t)L);
-        GT_CK(cudaMemcpyAsync(hkmin.data(), kmin, 3 * 8 * (size_t)L, cudaMemcpyDeviceToHost, st));
-        GT_CK(cudaMemcpyAsync(hkmax.data(), kmax, 3 * 8 * (size_t)L, cudaMemcpyDeviceToHost, st));
+        hkey.resize(6 * (size_t)L);
+        GT_CK(cudaMemcpyAsync(hkey.data(), key, 6 * 8 * (size_t)L, cudaMemcpyDeviceToHost, st));
         GT_CK(cudaStreamSynchronize(st));
         // 2. split decisions on the host (same arithmetic as bt_tree.c)
         std::vector<int> split;               // level-local indices of nodes to split
@@ -363,8 +367,8 @@ int gpu_build_forest(int nsys, const int64_t *sys_off, const double *x, const do
         for (int i = 0; i < L; i++) {
             HNode &nd = nodes[lo + i];
             for (int a = 0; a < 3; a++) {
-                nd.box[2 * a] = dkey_inv(hkmin[3 * i + a]);
-                nd.box[2 * a + 1] = dkey_inv(hkmax[3 * i + a]);
+                nd.box[2 * a] = dkey_inv(hkey[6 * (size_t)i + a]);
+                nd.box[2 * a + 1] = dkey_inv(~hkey[6 * (size_t)i + 3 + a]);
             }
             if (nd.np <= maxpar) continue;
             double xl = nd.box[1] - nd.box[0], yl = nd.box[3] - nd.box[2], zl = nd.box[5] - nd.box[4];
@@ -391,19 +395,24 @@ int gpu_build_forest(int nsys, const int64_t *sys_off, const double *x, const do
             }
         }
         nch = (int)hc_node.size();
-        GT_CK(cudaMemcpyAsync(c_node, hc_node.data(), 4 * (size_t)nch, cudaMemcpyHostToDevice, st));
-        GT_CK(cudaMemcpyAsync(c_begin, hc_begin.data(), 4 * (size_t)nch, cudaMemcpyHostToDevice, st));
-        GT_CK(cudaMemcpyAsync(c_len, hc_len.data(), 4 * (size_t)nch, cudaMemcpyHostToDevice, st));
-        GT_CK(cudaMemcpyAsync(mid, hmid.data(), 3 * 8 * (size_t)L, cudaMemcpyHostToDevice, st));
-        GT_CK(cudaMemcpyAsync(axis, haxis.data(), 3 * (size_t)L, cudaMemcpyHostToDevice, st));
-        // 3. slot bits, one divided axis per pass
-        for (int k = 0; k < 3; k++) GT_CK(cudaMemsetAsync(cnt[k], 0, 8 * 4 * (size_t)L, st));
-        // part counts before the first pass: the whole node is one part
+        // 3. slot bits, one divided axis per pass; part counts before the
+        // first pass: the whole node is one part
         hcnt.assign(8 * (size_t)L, 0);
         for (int i : split) hcnt[8 * i] = nodes[lo + i].np;
-        GT_CK(cudaMemcpyAsync(cnt0, hcnt.data(), 8 * 4 * (size_t)L, cudaMemcpyHostToDevice, st));
+        const size_t mid_b = 3 * 8 * (size_t)L, cnt_b = 8 * 4 * (size_t)L, axis_b = 3 * (size_t)L;
+        const double *mid = (const double *)up;
+        const int *cnt0 = (const int *)(up + mid_b);
+        const signed char *axis = (const signed char *)(up + mid_b + cnt_b);
+        put_chunks((mid_b + cnt_b + axis_b + 15) & ~size_t(15));
+        memcpy(hup.data(), hmid.data(), mid_b);
+        memcpy(hup.data() + mid_b, hcnt.data(), cnt_b);
+        memcpy(hup.data() + mid_b + cnt_b, haxis.data(), axis_b);
+        GT_CK(cudaMemcpyAsync(up, hup.data(), hup.size(), cudaMemcpyHostToDevice, st));
+        GT_CK(cudaMemsetAsync(cnt, 0, 3 * cnt_b, st));
         for (int k = 0; k < 3; k++) {
-            k_codes<<<nch, GT_THREADS, 0, st>>>(ca, k, axis, mid, k == 0 ? cnt0 : cnt[k - 1], A.x, A.y, A.z, code, cnt[k]);
+            int *now = cnt + 8 * (size_t)L * k;
+            k_codes<<<nch, GT_THREADS, 0, st>>>(ca, k, axis, mid, k == 0 ? cnt0 : now - 8 * (size_t)L, A.x, A.y, A.z, code,
+                                                now);
             (*launches)++;
         }
         k_chunk_hist<<<nch, GT_THREADS, 0, st>>>(ca, code, c_hist);

@@ -58,13 +58,11 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
 }
 
 constexpr int MX_THREADS = 128;                 // threads of the grid-output kernel
-// Register budget of the grid-output kernel: BT_MX_MIN_BLOCKS resident blocks
-// per SM (unset: the compiler's choice).
-#ifdef BT_MX_MIN_BLOCKS
-#define BT_MX_BOUNDS __launch_bounds__(MX_THREADS, BT_MX_MIN_BLOCKS)
-#else
-#define BT_MX_BOUNDS __launch_bounds__(MX_THREADS)
+// Register budget of the grid-output kernel: BT_MX_MIN_BLOCKS resident blocks per SM.
+#ifndef BT_MX_MIN_BLOCKS
+#define BT_MX_MIN_BLOCKS 6
 #endif
+#define BT_MX_BOUNDS __launch_bounds__(MX_THREADS, BT_MX_MIN_BLOCKS)
 constexpr int MX_TILE = 1024;                   // sources per tile of the grid-output kernel
 // Register budget of the 2-targets-per-thread Lagrange particle-output
 // kernel (Coulomb, regularised Coulomb): room for 6 resident blocks per SM.
@@ -105,6 +103,25 @@ __host__ __device__ constexpr int rb_blocks()
 #endif
 __host__ __device__ constexpr bool far_sw(int k1) { return k1 < BT_FAR_SW; }
 
+// Yukawa: row + q exp(-kappa r) / r, one Newton step on the MUFU's 1/r (its
+// error would otherwise enter both 1/r and the exponent).
+__device__ __forceinline__ float far_yukawa(float r2, float q, float kc, float row)
+{
+    const float rinv = rsqrt_apx(r2), h = r2 * rinv;
+    const float t = fmaf(-0.5f * h, rinv, 1.5f);
+    return fmaf(q * (rinv * t), ex2_apx(kc * (h * t)), row);
+}
+__device__ __forceinline__ f2_t f2_far_yukawa(f2_t r2, f2_t q, f2_t kc, f2_t row)
+{
+    float a, b;
+    f2_split(r2, a, b);
+    const f2_t rinv = f2_make(rsqrt_apx(a), rsqrt_apx(b)), h = f2_mul(r2, rinv);
+    const f2_t t = f2_fma(f2_mul(f2_make(-0.5f, -0.5f), h), rinv, f2_make(1.5f, 1.5f));
+    f2_split(f2_mul(kc, f2_mul(h, t)), a, b);
+    const f2_t e = f2_make(ex2_apx(a), ex2_apx(b));
+    return f2_fma(f2_mul(q, f2_mul(rinv, t)), e, row);
+}
+
 // Far field of one source cluster (degree NP1-1) for NT targets at (x,y,z),
 // relative to the target centre; g = grid coordinates relative to the same
 // centre, q = proxy charges (shared memory, FP32).
@@ -129,7 +146,7 @@ __device__ __forceinline__ void pc_cluster(const float *x, const float *y, const
 #pragma unroll
             for (int t = 0; t < NT; t++) {
                 float dy = y[t] - gy, dz = z[t] - gz;
-                dyz[t] = fmaf(dy, dy, dz * dz);
+                dyz[t] = fmaf(dy, dy, KT == 3 ? fmaf(dz, dz, kc) : dz * dz);     // regularised: + eps^2
                 row[t] = 0.f;
             }
 #pragma unroll
@@ -138,9 +155,8 @@ __device__ __forceinline__ void pc_cluster(const float *x, const float *y, const
 #pragma unroll
                 for (int t = 0; t < NT; t++) {
                     const float r2 = fmaf(gx[t][k1], gx[t][k1], dyz[t]);
-                    if (KT == 2) row[t] += kf_far<KT>(r2, qq, kc);
-                    else if (far_sw(k1)) row[t] = fmaf(qq, rsqrt_sw(KT == 3 ? r2 + kc : r2), row[t]);
-                    else row[t] = fmaf(qq, rsqrt_apx(KT == 3 ? r2 + kc : r2), row[t]);
+                    if (KT == 2) row[t] = far_yukawa(r2, qq, kc, row[t]);
+                    else row[t] = fmaf(qq, far_sw(k1) ? rsqrt_sw(r2) : rsqrt_apx(r2), row[t]);
                 }
             }
             j += NP1;
@@ -244,8 +260,7 @@ __device__ __forceinline__ void pc_cluster_herm(const float *x, const float *y, 
 // boxes lie within that distance (flagged per near-field entry); the other
 // entries run pp_tile_far with no test at all.
 
-// Lagrange far field with the targets in packed pairs (NT even, Coulomb and
-// regularised Coulomb): pc_cluster's operations lane by lane in f32x2
+// Lagrange far field with the targets in packed pairs (NT even): pc_cluster's operations lane by lane in f32x2
 // instructions (identical results); qd holds each proxy charge twice.
 template <int KT, int NP1, int NT>
 __device__ __forceinline__ void pc_cluster_f2(const float *x, const float *y, const float *z, const float *g,
@@ -260,7 +275,7 @@ __device__ __forceinline__ void pc_cluster_f2(const float *x, const float *y, co
     float s[NT], c[NT];
 #pragma unroll
     for (int t = 0; t < NT; t++) { s[t] = 0.f; c[t] = 0.f; }
-    const f2_t kc2 = f2_make(kc, kc), one = f2_make(1.0f, 1.0f), zero = f2_make(0.0f, 0.0f);
+    const f2_t kc2 = f2_make(kc, kc), zero = f2_make(0.0f, 0.0f);
     int j = 0;
     for (int k3 = 0; k3 < NP1; k3++) {
         const float gz = g[2 * NP1 + k3];
@@ -270,7 +285,7 @@ __device__ __forceinline__ void pc_cluster_f2(const float *x, const float *y, co
 #pragma unroll
             for (int p = 0; p < NPR; p++) {
                 const f2_t dy = f2_make(y[2 * p] - gy, y[2 * p + 1] - gy), dz = f2_make(z[2 * p] - gz, z[2 * p + 1] - gz);
-                dyz[p] = f2_fma(dy, dy, f2_mul(dz, dz));
+                dyz[p] = f2_fma(dy, dy, KT == 3 ? f2_fma(dz, dz, kc2) : f2_mul(dz, dz));
                 row[p] = zero;
             }
 #pragma unroll
@@ -278,9 +293,10 @@ __device__ __forceinline__ void pc_cluster_f2(const float *x, const float *y, co
                 const f2_t qq = qd[j + k1];
 #pragma unroll
                 for (int p = 0; p < NPR; p++) {
-                    f2_t r2 = f2_fma(gx[p][k1], gx[p][k1], dyz[p]);
-                    if (KT == 3) r2 = f2_fma(one, kc2, r2);
-                    if (far_sw(k1)) {             // resolved at compile time: k1 is unrolled
+                    const f2_t r2 = f2_fma(gx[p][k1], gx[p][k1], dyz[p]);
+                    if (KT == 2) {
+                        row[p] = f2_far_yukawa(r2, qq, kc2, row[p]);
+                    } else if (far_sw(k1)) {      // resolved at compile time: k1 is unrolled
                         row[p] = f2_fma(qq, f2_rsqrt_sw(r2), row[p]);
                     } else {
                         float a, b;
@@ -370,11 +386,11 @@ __device__ __forceinline__ void pc_cluster_herm_f2(const float *x, const float *
     for (int t = 0; t < NT; t++) out[t] = s[t] - c[t];
 }
 
-// Packed far field (Lagrange and Hermite) for this kernel type and target count?
-template <int KT, int NT>
-__host__ __device__ constexpr bool far_packed() { return KT != 2 && NT % 2 == 0; }
+// Packed far field for this kernel type and target count?  (Hermite: not for Yukawa.)
+template <int KT, bool HERM, int NT>
+__host__ __device__ constexpr bool far_packed() { return !(HERM && KT == 2) && NT % 2 == 0; }
 
-// q: the staged proxy charges, as {q, q} pairs when far_packed<KT, NT>().
+// q: the staged proxy charges, as {q, q} pairs when far_packed().
 template <int KT, int NT>
 __device__ void pc_cluster_dispatch(int np1, const float *x, const float *y, const float *z, const float *g,
                                     const float *q, float kc, float *out)
@@ -382,7 +398,7 @@ __device__ void pc_cluster_dispatch(int np1, const float *x, const float *y, con
     switch (np1) {
 #define BT_CASE(N)                                                                                         \
     case N:                                                                                                \
-        if constexpr (far_packed<KT, NT>())                                                                \
+        if constexpr (far_packed<KT, false, NT>())                                                         \
             pc_cluster_f2<KT, N, NT>(x, y, z, g, reinterpret_cast<const f2_t *>(q), kc, out);              \
         else                                                                                               \
             pc_cluster<KT, N, NT>(x, y, z, g, q, kc, out);                                                 \
@@ -396,7 +412,7 @@ __device__ void pc_cluster_dispatch(int np1, const float *x, const float *y, con
 }
 
 
-// q: the staged moments, as {q, q} pairs when far_packed<KT, NT>().
+// q: the staged moments, as {q, q} pairs when far_packed().
 template <int KT, int NT>
 __device__ void pc_cluster_herm_dispatch(int np1, const float *x, const float *y, const float *z, const float *g,
                                          const float *q, float kc, float kp, float *out)
@@ -404,7 +420,7 @@ __device__ void pc_cluster_herm_dispatch(int np1, const float *x, const float *y
     switch (np1) {
 #define BT_CASE(N)                                                                                         \
     case N:                                                                                                \
-        if constexpr (far_packed<KT, NT>())                                                               \
+        if constexpr (far_packed<KT, true, NT>())                                                         \
             pc_cluster_herm_f2<KT, N, NT>(x, y, z, g, reinterpret_cast<const f2_t *>(q), kc, out);         \
         else                                                                                               \
             pc_cluster_herm<KT, N, NT>(x, y, z, g, q, kc, kp, out);                                        \
@@ -427,11 +443,11 @@ struct Tile {
 constexpr float MX_PAD_POS = 1.0e18f;   // r2 ~ 1e36 < FLT_MAX; with q = 0 it adds nothing
 
 // Two sources (a pair) against one target, accumulated into the pair sum S.
+// r2: with eps^2 for the regularised kernel (folded into the squared distance);
 // kc: mixed_kernel_constant(); kc2 = {kc, kc}.
 template <int KT>
 __device__ __forceinline__ f2_t kf2_acc(f2_t r2, f2_t q, f2_t S, f2_t kc2)
 {
-    if (KT == 3) r2 = f2_fma(f2_make(1.0f, 1.0f), kc2, r2);   // r2 + eps^2
     float a, b;
     f2_split(r2, a, b);
     const f2_t rinv = f2_make(rsqrt_apx(a), rsqrt_apx(b));
@@ -473,7 +489,7 @@ __device__ __forceinline__ void pp_tile(const Tile tl, int cm4, const float *x, 
 #pragma unroll
             for (int t = 0; t < TPT; t++) {
                 const f2_t dx = f2_sub(X[t], px), dy = f2_sub(Y[t], py), dz = f2_sub(Z[t], pz);
-                const f2_t r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+                const f2_t r2 = f2_fma(dx, dx, f2_fma(dy, dy, KT == 3 ? f2_fma(dz, dz, kc2) : f2_mul(dz, dz)));
                 if (NEAR) {
                     float a, b;
                     f2_split(r2, a, b);
@@ -494,7 +510,8 @@ __device__ __forceinline__ void pp_tile(const Tile tl, int cm4, const float *x, 
 // A tile holding a close pair for this target, again in scalar form: the
 // FP32 sum over the pairs at or beyond the close distance (which also drops
 // coincident pairs, r2 == 0), and the close pairs in FP64 from the FP64
-// coordinates and charges with the reference's skipping rule (k_pp).
+// coordinates and charges with the reference's skipping rule (k_pp).  thr2:
+// the close distance squared, plus eps^2 for the regularised kernel.
 template <int KT>
 __device__ __noinline__ float pp_tile_close(const Tile tl, int cm, float x, float y, float z, float kc, float thr2,
                                             double xd, double yd, double zd, const double *__restrict__ sx,
@@ -505,9 +522,9 @@ __device__ __noinline__ float pp_tile_close(const Tile tl, int cm, float x, floa
     double a = 0.0;
     for (int i = 0; i < cm; i++) {
         const float dx = x - tl.x[i], dy = y - tl.y[i], dz = z - tl.z[i];
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, KT == 3 ? fmaf(dz, dz, kc) : dz * dz));
         if (r2 >= thr2) {
-            s += kf_far<KT>(r2, tl.q[i], kc);
+            s += KT == 3 ? tl.q[i] * rsqrt_apx(r2) : kf_far<KT>(r2, tl.q[i], kc);
         } else {
             const int gi = base + i;
             const double ex = xd - sx[gi], ey = yd - sy[gi], ez = zd - sz[gi];
@@ -534,6 +551,13 @@ __device__ __forceinline__ int next_item(int *queue, int *slot)
     const int w = *slot;
     __syncthreads();
     return w;
+}
+
+// Shared-memory floats of one staged cluster: its grid, and its proxies
+// (moments) as pairs; a multiple of four.
+__host__ __device__ inline int far_floats(int np1, bool herm)
+{
+    return 3 * 16 + ((herm ? 16 : 2) * np1 * np1 * np1 + 3 & ~3);
 }
 
 template <int KT, bool HERM, int TPT>
@@ -565,42 +589,58 @@ __device__ __forceinline__ void targets_item(const MixedTargetsArgs &a, const in
 #pragma unroll
         for (int t = 0; t < TPT; t++) acc[t] = 0.0;
         // far field: source clusters
-        for (int64_t e = seg_begin(ab, ae, seg), e1 = seg_begin(ab, ae, seg + 1); e < e1; e++) {
-            const int s = a.a_idx[e];
-            const int deg = a.a_deg ? a.a_deg[e] : a.n;
-            const int np1 = deg + 1, P = np1 * np1 * np1;
-            float *g = smf;
-            float *q = smf + 3 * 16;
-            const double *gs = a.s_grid[deg] + (size_t)s * 3 * np1;
-            for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) {
-                int ax = i / np1;
-                double c = ax == 0 ? cx : ax == 1 ? cy : cz;
-                g[ax * np1 + (i % np1)] = (float)(gs[i] - c);
-            }
-            float v[TPT];
-            if (HERM) {
-                const float *Qs = a.Q32[deg] + (size_t)s * 8 * P;
-                for (int i = threadIdx.x; i < 8 * P; i += blockDim.x) {
-                    // a point's moments side by side: the loop reads them in 128-bit words
-                    const int m = i & 7;
-                    const float v = Qs[m * P + (i >> 3)] * (m == 7 ? 15.0f : m >= 4 ? 3.0f : 1.0f);
-                    if constexpr (far_packed<KT, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(v, v);
-                    else q[i] = v;
+        // As many clusters as the tile's memory holds are staged together
+        // (Hermite: one), so that their loads are in flight together and a
+        // pair of barriers serves several clusters: 64 systems of degree 7,
+        // 37.7 -> 35.4 ms with eps^2 folded into the squared distances.
+        for (int64_t e = seg_begin(ab, ae, seg), e1 = seg_begin(ab, ae, seg + 1); e < e1;) {
+            const int64_t eb = e;
+            int used = 0;
+            do {
+                const int s = a.a_idx[e];
+                const int np1 = (a.a_deg ? a.a_deg[e] : a.n) + 1, P = np1 * np1 * np1;
+                float *g = smf + used, *q = g + 3 * 16;
+                const double *gs = a.s_grid[np1 - 1] + (size_t)s * 3 * np1;
+                for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) {
+                    int ax = i / np1;
+                    double c = ax == 0 ? cx : ax == 1 ? cy : cz;
+                    g[i] = (float)(gs[i] - c);
                 }
-                __syncthreads();
-                if (warp_on) pc_cluster_herm_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, (float)a.kp, v);
-            } else {
-                const float *Qs = a.Q32[deg] + (size_t)s * P;
-                for (int i = threadIdx.x; i < P; i += blockDim.x) {
-                    if constexpr (far_packed<KT, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(Qs[i], Qs[i]);
-                    else q[i] = Qs[i];
+                if (HERM) {
+                    const float *Qs = a.Q32[np1 - 1] + (size_t)s * 8 * P;
+                    for (int i = threadIdx.x; i < 8 * P; i += blockDim.x) {
+                        // a point's moments side by side: the loop reads them in 128-bit words
+                        const int m = i & 7;
+                        const float v = Qs[m * P + (i >> 3)] * (m == 7 ? 15.0f : m >= 4 ? 3.0f : 1.0f);
+                        if constexpr (far_packed<KT, HERM, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(v, v);
+                        else q[i] = v;
+                    }
+                } else {
+                    const float *Qs = a.Q32[np1 - 1] + (size_t)s * P;
+#pragma unroll 4
+                    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+                        const float v = Qs[i];
+                        if constexpr (far_packed<KT, HERM, TPT>()) reinterpret_cast<f2_t *>(q)[i] = f2_make(v, v);
+                        else q[i] = v;
+                    }
                 }
-                __syncthreads();
-                if (warp_on) pc_cluster_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, v);
-            }
+                used += far_floats(np1, HERM);
+                e++;
+            } while (!HERM && e < e1 && used + far_floats((a.a_deg ? a.a_deg[e] : a.n) + 1, HERM) <= a.smem_floats);
+            __syncthreads();
+            if (warp_on) {
+                used = 0;
+                for (int64_t f = eb; f < e; f++) {
+                    const int np1 = (a.a_deg ? a.a_deg[f] : a.n) + 1;
+                    const float *g = smf + used, *q = g + 3 * 16;
+                    float v[TPT];
+                    if (HERM) pc_cluster_herm_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, (float)a.kp, v);
+                    else pc_cluster_dispatch<KT, TPT>(np1, x, y, z, g, q, kc, v);
 #pragma unroll
-            for (int t = 0; t < TPT; t++)
-                if (warp_on) acc[t] += (double)v[t];
+                    for (int t = 0; t < TPT; t++) acc[t] += (double)v[t];
+                    used += far_floats(np1, HERM);
+                }
+            }
             __syncthreads();
         }
         // near field: source leaves, particles relative to their leaf centre
@@ -621,7 +661,7 @@ __device__ __forceinline__ void targets_item(const MixedTargetsArgs &a, const in
             // == 0 after flushing) always takes the FP64 path with the skipping
             // rule, also between single-particle leaves of radius 0
             const double rr = MX_CLOSE_FRAC * (trad + a.s_rad[s]);
-            const float thr2 = fmaxf((float)(rr * rr), FLT_MIN);
+            const float thr2 = fmaxf((float)(rr * rr), FLT_MIN) + (KT == 3 ? kc : 0.0f);   // as r2 has it
             for (int c0 = 0; c0 < sn; c0 += tile) {
                 const int cm = min(tile, sn - c0), cm4 = (cm + 3) & ~3;
                 for (int i = threadIdx.x; i < cm4; i += blockDim.x) {
@@ -704,62 +744,89 @@ __global__ void __launch_bounds__(MX_CHUNK / TPT, rb_blocks<KT, HERM>()) k_eval_
 }
 
 // Grid-output evaluation (M2L from source clusters + CP from source leaves)
-// onto the grid of a target node, mixed precision, Lagrange.  One thread per
-// target grid point.
+// onto the grid of a target node, mixed precision, Lagrange.  Two grid points
+// per thread (packed pairs), each warp 64 consecutive ones; a warp beyond the
+// grid's last point only stages.
 template <int KT>
 __device__ __forceinline__ void grids_item(const MixedGridsArgs &a, const int2 it, float *smf)
 {
+    constexpr int NT = 2;
     const int T = it.x;
     const int np1 = a.n + 1, P = np1 * np1 * np1;
-    const int j0 = it.y * MX_THREADS + threadIdx.x;
-    const bool active = j0 < P;
-    const int jj = active ? j0 : 0;
+    const int first = it.y * MX_CHUNK + (threadIdx.x >> 5) * 32 * NT;
+    const bool warp_on = first < P;
     const double *tg = a.t_grid + (size_t)T * 3 * np1;
     const double cx = a.t_ctr[3 * T], cy = a.t_ctr[3 * T + 1], cz = a.t_ctr[3 * T + 2];
-    float x[1] = {(float)(tg[jj % np1] - cx)}, y[1] = {(float)(tg[np1 + (jj / np1) % np1] - cy)},
-          z[1] = {(float)(tg[2 * np1 + jj / (np1 * np1)] - cz)};
+    float x[NT], y[NT], z[NT];
+    double acc[NT];
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+        const int j0 = first + 32 * t + (threadIdx.x & 31), j = j0 < P ? j0 : 0;
+        x[t] = (float)(tg[j % np1] - cx);
+        y[t] = (float)(tg[np1 + (j / np1) % np1] - cy);
+        z[t] = (float)(tg[2 * np1 + j / (np1 * np1)] - cz);
+        acc[t] = 0.0;
+    }
     const float kc = (float)a.kc;
-    double acc = 0.0;
-    for (int64_t e = a.c_off[T]; e < a.c_off[T + 1]; e++) {
-        const int s = a.c_idx[e];
-        float *g = smf;
-        float *q = smf + 3 * 16;
-        const double *gs = a.s_grid + (size_t)s * 3 * np1;
-        for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) {
-            int ax = i / np1;
-            double c = ax == 0 ? cx : ax == 1 ? cy : cz;
-            g[ax * np1 + (i % np1)] = (float)(gs[i] - c);
+    const int need = far_floats(np1, false);
+    for (int64_t e = a.c_off[T], e1 = a.c_off[T + 1]; e < e1;) {
+        const int64_t eb = e;
+        for (int used = 0; e < e1 && (e == eb || used + need <= a.smem_floats); e++, used += need) {
+            const int s = a.c_idx[e];
+            float *g = smf + used;
+            f2_t *q = reinterpret_cast<f2_t *>(g + 3 * 16);
+            const double *gs = a.s_grid + (size_t)s * 3 * np1;
+            for (int i = threadIdx.x; i < 3 * np1; i += blockDim.x) {
+                int ax = i / np1;
+                double c = ax == 0 ? cx : ax == 1 ? cy : cz;
+                g[i] = (float)(gs[i] - c);
+            }
+#pragma unroll 4
+            for (int i = threadIdx.x; i < P; i += blockDim.x) {
+                const float v = a.Q32[(size_t)s * P + i];
+                q[i] = f2_make(v, v);
+            }
         }
-        for (int i = threadIdx.x; i < P; i += blockDim.x) q[i] = a.Q32[(size_t)s * P + i];
         __syncthreads();
-        float v[1];
-        pc_cluster_dispatch<KT, 1>(np1, x, y, z, g, q, kc, v);
-        acc += (double)v[0];
+        if (warp_on)
+            for (int k = 0; k < (int)(e - eb); k++) {
+                float v[NT];
+                pc_cluster_dispatch<KT, NT>(np1, x, y, z, smf + k * need, smf + k * need + 3 * 16, kc, v);
+#pragma unroll
+                for (int t = 0; t < NT; t++) acc[t] += (double)v[t];
+            }
         __syncthreads();
     }
-    float4 *tile = reinterpret_cast<float4 *>(smf);
+    const Tile tl{smf, smf + MX_TILE, smf + 2 * MX_TILE, smf + 3 * MX_TILE};
     for (int64_t e = a.p_off[T]; e < a.p_off[T + 1]; e++) {
         const int s = a.p_idx[e];
         const int sb = a.s_ibeg[s], sn = a.s_numpar[s];
         const float ox = (float)(a.s_ctr[3 * s] - cx), oy = (float)(a.s_ctr[3 * s + 1] - cy),
                     oz = (float)(a.s_ctr[3 * s + 2] - cz);
-        const float xs = x[0] - ox, ys = y[0] - oy, zs = z[0] - oz;
+        float xs[NT], ys[NT], zs[NT];
+#pragma unroll
+        for (int t = 0; t < NT; t++) { xs[t] = x[t] - ox; ys[t] = y[t] - oy; zs[t] = z[t] - oz; }
         for (int c0 = 0; c0 < sn; c0 += MX_TILE) {
-            int cm = min(MX_TILE, sn - c0);
-            for (int i = threadIdx.x; i < cm; i += blockDim.x) tile[i] = a.spos[sb + c0 + i];
-            __syncthreads();
-            float s0 = 0.f;
-#pragma unroll 4
-            for (int i = 0; i < cm; i++) {
-                float4 p = tile[i];
-                float dx = xs - p.x, dy = ys - p.y, dz = zs - p.z;
-                s0 += kf_far<KT>(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), p.w, kc);
+            const int cm = min(MX_TILE, sn - c0), cm4 = (cm + 3) & ~3;
+            for (int i = threadIdx.x; i < cm4; i += blockDim.x) {
+                const float4 p = i < cm ? a.spos[sb + c0 + i] : make_float4(MX_PAD_POS, MX_PAD_POS, MX_PAD_POS, 0.0f);
+                tl.x[i] = p.x; tl.y[i] = p.y; tl.z[i] = p.z; tl.q[i] = p.w;
             }
-            acc += (double)s0;
+            __syncthreads();
+            if (warp_on) {
+                float sum[NT];
+                pp_tile<KT, false, NT>(tl, cm4, xs, ys, zs, kc, sum, nullptr);
+#pragma unroll
+                for (int t = 0; t < NT; t++) acc[t] += (double)sum[t];
+            }
             __syncthreads();
         }
     }
-    if (active) a.Phi[(size_t)T * P + j0] = acc;
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+        const int j = first + 32 * t + (threadIdx.x & 31);
+        if (j < P) a.Phi[(size_t)T * P + j] = acc[t];
+    }
 }
 
 template <int KT>
@@ -815,7 +882,7 @@ int mixed_targets_chunk() { return MX_CHUNK; }
 static size_t mixed_smem(int max_np1, bool herm, int tile_stride)
 {
     // proxy charges are staged as {q, q} pairs (packed far field)
-    size_t far = sizeof(float) * (size_t)(3 * 16 + (herm ? 16 : 2) * max_np1 * max_np1 * max_np1);
+    size_t far = sizeof(float) * (size_t)far_floats(max_np1, herm);
     size_t near = sizeof(float4) * (size_t)tile_stride;
     return far > near ? far : near;
 }
@@ -833,9 +900,10 @@ static int queue_grid(K kernel, int threads, size_t smem, int nitems)
 }
 
 template <int KT, bool HERM, int TPT>
-static void eval_targets_mixed_t(const MixedTargetsArgs &a, cudaStream_t st)
+static void eval_targets_mixed_t(MixedTargetsArgs a, cudaStream_t st)
 {
     size_t sm = mixed_smem(a.max_np1, HERM, MX_TILE_MAX);
+    a.smem_floats = (int)(sm / sizeof(float));
     auto kernel = k_eval_targets_mixed<KT, HERM, TPT>;
     if constexpr (TPT == 2 && rb_blocks<KT, HERM>() > 0) kernel = k_eval_targets_mixed_rb<KT, HERM, TPT>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -867,9 +935,10 @@ void launch_eval_targets_mixed(int kernel, const MixedTargetsArgs &a, cudaStream
 bool mixed_split(size_t items) { return items < (size_t)4 * 6 * 148; }
 
 template <int KT>
-static void eval_grids_mixed_t(const MixedGridsArgs &a, cudaStream_t st)
+static void eval_grids_mixed_t(MixedGridsArgs a, cudaStream_t st)
 {
     size_t sm = mixed_smem(a.n + 1, false, MX_TILE);
+    a.smem_floats = (int)(sm / sizeof(float));
     cudaFuncSetAttribute(k_eval_grids_mixed<KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     int grid = a.queue ? queue_grid(k_eval_grids_mixed<KT>, MX_THREADS, sm, a.nitems) : a.nitems;
     k_eval_grids_mixed<KT><<<grid, MX_THREADS, sm, st>>>(a);

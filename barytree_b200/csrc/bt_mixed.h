@@ -50,13 +50,14 @@ struct MixedTargetsArgs {
     double kp;                                  // kernel parameter (FP64 close pairs)
     double *pot;
     int tpt, tile;                              // targets per thread, near-field source tile
+    int smem_floats;                            // set by the launcher: room for staged clusters
     double *partial;                            // a block per (item, segment) leaves its sums here (or nullptr)
     size_t pstride;
 };
 
 struct MixedGridsArgs {
     int n, nitems;
-    const int2 *items;
+    const int2 *items;                          // (target node, chunk of MX_CHUNK grid points)
     int *queue;                                 // work-queue counter (zeroed), or nullptr: one block per item
     const double *t_grid, *t_ctr;
     const int64_t *c_off; const int *c_idx;     // M2L source clusters per target node
@@ -67,6 +68,7 @@ struct MixedGridsArgs {
     const float4 *spos;
     double kc;                                  // mixed_kernel_constant()
     double *Phi;
+    int smem_floats;                            // set by the launcher: room for staged clusters
 };
 
 void launch_rel_positions(int nleaves, const int *leaves, const int *ibeg, const int *numpar, const double *ctr,

@@ -87,13 +87,12 @@ __device__ __forceinline__ void rs_stage(float *v, int lane)
     }
 }
 
-// The kernel value of a packed pair of r^2 (the particle-output kernel's
-// arithmetic): Coulomb 1/r; regularised Coulomb 1/sqrt(r^2 + eps^2);
+// The kernel value of a packed pair of r^2, which holds eps^2 for the
+// regularised kernel (the particle-output kernel's arithmetic): 1/r;
 // Yukawa with one Newton step on 1/r, then exp(-kappa r) by ex2.
 template <int KT>
 __device__ __forceinline__ f2_t sym_kval(f2_t r2, f2_t kc2)
 {
-    if (KT == 3) r2 = f2_fma(f2_make(1.0f, 1.0f), kc2, r2);
     float ra, rb;
     f2_split(r2, ra, rb);
     f2_t k = f2_make(rsqrt_apx(ra), rsqrt_apx(rb));
@@ -109,12 +108,18 @@ __device__ __forceinline__ f2_t sym_kval(f2_t r2, f2_t kc2)
 
 // The main loop's FP32 r^2 of one pair, with its instructions: x, y, z the
 // target in the source leaf's frame, p the source.
-__device__ __forceinline__ float sym_r2(float x, float y, float z, float4 p)
+template <int KT>
+__device__ __forceinline__ f2_t sym_r2p(f2_t dx, f2_t dy, f2_t dz, f2_t kc2)
+{
+    return f2_fma(dx, dx, f2_fma(dy, dy, KT == 3 ? f2_fma(dz, dz, kc2) : f2_mul(dz, dz)));
+}
+template <int KT>
+__device__ __forceinline__ float sym_r2(float x, float y, float z, float4 p, f2_t kc2)
 {
     const f2_t dx = f2_sub(f2_make(x, x), f2_make(p.x, p.x)), dy = f2_sub(f2_make(y, y), f2_make(p.y, p.y)),
                dz = f2_sub(f2_make(z, z), f2_make(p.z, p.z));
     float r2, unused;
-    f2_split(f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz))), r2, unused);
+    f2_split(sym_r2p<KT>(dx, dy, dz, kc2), r2, unused);
     return r2;
 }
 
@@ -172,14 +177,17 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(const 
     float thr2 = 0.0f;
     if (CLAMP) {
         const double rr = MX_CLOSE_FRAC * (a.rad[A] + a.rad[B]);
-        thr2 = fmaxf((float)(rr * rr), FLT_MIN);
+        const float cut2 = fmaxf((float)(rr * rr), FLT_MIN);
+        thr2 = cut2 + (KT == 3 ? a.kc : 0.0f);               // as r^2 has it
         __shared__ int wcnt[SY_WARPS];
         int *candA = reinterpret_cast<int *>(&accA[0][0]), *candB = candA + SYM_PART;
         static_assert(sizeof(int) * (SYM_PART + SYM_MAX_LEAF) <= sizeof(accA), "the candidate lists live in accA");
         for (int i = threadIdx.x; i < pa; i += SY_THREADS) outA[i] = 0.0f;
         for (int j = threadIdx.x; j < nb; j += SY_THREADS) outB[j] = 0.0f;
-        // every pair with FP32 r^2 below thr2 lies within 1.01 thr of both boxes
-        const double d = 1.01 * sqrt((double)thr2);
+        // every pair with FP32 r^2 below thr2 lies within 1.01 of the close
+        // distance of both boxes (with eps^2 far above its square the clamp
+        // changes r^2 by less than its rounding)
+        const double d = 1.01 * sqrt((double)cut2);
         const int nca = near_box(candA, pa, ia, a.x64, a.y64, a.z64, a.box + 6 * B, d, wcnt);
         const int ncb = nca > 0 ? near_box(candB, nb, ib, a.x64, a.y64, a.z64, a.box + 6 * A, d, wcnt) : 0;
         if (nca > 0 && ncb > 0) {
@@ -198,8 +206,8 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(const 
                     const int gj = (sideA ? ib : ia) + j;
                     const float4 pj = a.pos[gj];
                     // the pair's r^2 as the main loop forms it: A's target in B's frame
-                    const float r2 = sideA ? sym_r2(pi.x - ox, pi.y - oy, pi.z - oz, pj)
-                                           : sym_r2(pj.x - ox, pj.y - oy, pj.z - oz, pi);
+                    const float r2 = sideA ? sym_r2<KT>(pi.x - ox, pi.y - oy, pi.z - oz, pj, kc2)
+                                           : sym_r2<KT>(pj.x - ox, pj.y - oy, pj.z - oz, pi, kc2);
                     if (r2 < thr2) {
                         const double ex = a.x64[gi] - a.x64[gj], ey = a.y64[gi] - a.y64[gj],
                                      ez = a.z64[gi] - a.z64[gj];
@@ -250,7 +258,7 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(const 
 #pragma unroll
                     for (int p = 0; p < SY_NP; p++) {
                         const f2_t dx = f2_sub(X[p], xy.x), dy = f2_sub(Y[p], xy.y), dz = f2_sub(Z[p], zq.x);
-                        f2_t r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+                        f2_t r2 = sym_r2p<KT>(dx, dy, dz, kc2);
                         if (CLAMP) {
                             float ra, rb;
                             f2_split(r2, ra, rb);
