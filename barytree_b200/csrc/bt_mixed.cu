@@ -537,8 +537,10 @@ __device__ __noinline__ float pp_tile_close(const Tile tl, int cm, float x, floa
 
 // Particle-output evaluation, mixed precision.  Each thread owns TPT
 // targets of a work item (target leaf, chunk of MX_CHUNK targets), each warp
-// 32 * TPT consecutive ones; a warp beyond the leaf's last target only helps
-// to stage, so a leaf costs its targets rounded up to a warp's.  Each target's
+// 32 * TPT consecutive ones.  In the Hermite kernel, which the FP32 pipe
+// bounds, a warp beyond the leaf's last target only helps to stage (2M system
+// 152.7 -> 149.7 ms); in the Lagrange kernel it evaluates like the others (the
+// 16M system took 895 ms so and 904 ms with the warps skipped).  Each target's
 // lists are summed in EV_SEGS segments and the segments in order, as in the
 // FP64 kernels: a launch with few items runs one block per (item, segment).
 // Blocks of a work-queue launch take items (cost-sorted, longest first) from
@@ -579,7 +581,7 @@ __device__ __forceinline__ void targets_item(const MixedTargetsArgs &a, const in
         float4 tp = a.tpos[tid[t]];
         x[t] = tp.x; y[t] = tp.y; z[t] = tp.z;
     }
-    const bool warp_on = it.y * MX_CHUNK + (int)(threadIdx.x >> 5) * 32 * TPT < tn;
+    const bool warp_on = !HERM || it.y * MX_CHUNK + (int)(threadIdx.x >> 5) * 32 * TPT < tn;
     const double trad = a.t_rad[tnode];
     const double cx = a.t_ctr[3 * tnode], cy = a.t_ctr[3 * tnode + 1], cz = a.t_ctr[3 * tnode + 2];
     const float kc = (float)a.kc;
