@@ -1539,9 +1539,10 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             usz1[0] = usz0[NU];
             for (int u = 0; u < NU; u++) usz1[u + 1] += usz1[u];
             sym_total = usz1[NU];
-            // FP64 slices up to 32 GB; a larger system (some 70M particles)
-            // evaluates every direction
-            sym_dropped = !sym64 || sym_total <= (int64_t)1 << 32;
+            // Slices within 32 GB (FP64, some 70M particles) or 64 GB (mixed);
+            // a larger system evaluates every direction.  Shards of one
+            // system have to decide alike, so they always take the pairs.
+            sym_dropped = shape.nshards > 1 || sym_total <= (sym64 ? (int64_t)1 << 32 : (int64_t)1 << 34);
         }
         if (!sym_dropped) {
             sym_pairs.clear();
