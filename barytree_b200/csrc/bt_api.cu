@@ -1414,6 +1414,11 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     std::vector<int64_t> sym_in_off;
     int64_t sym_total = 0, sym_far_pairs = 0;
     bool sym_dropped = false;      // the pairs have left the per-target lists
+    // FP64: the units of systems that have pairs, whose near field is what is
+    // left of the leaf-expanded list.  The other systems of a batch keep the
+    // plan's list, as in a call of their own: the segments of the sums are cut
+    // by list entries, and cluster-cluster lists hold interior nodes.
+    std::vector<unsigned char> unit_expanded;
     auto sym64_leaf = [&](int v) { return S.numpar[v] >= bt::SYM64_MIN_LEAF && S.numpar[v] <= bt::SYM_MAX_LEAF; };
     if ((mixed && sym_ok && max_leaf <= bt::SYM_MAX_LEAF) || sym64) {
         const int NU = T.nleaves;
@@ -1513,6 +1518,15 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         sym_far_pairs = poff0[NU];
         poff1[0] = sym_far_pairs;
         for (int u = 0; u < NU; u++) poff1[u + 1] += poff1[u];
+        if (sym64) {
+            unit_expanded.assign(NU, 0);
+            for (int k = 0; k < T.nroots; k++) {
+                bool has = false;
+                for (int u = T.leaf_off[k]; u < T.leaf_off[k + 1] && !has; u++)
+                    for (int64_t j = mx_doff[u]; j < far_end[u] && !has; j++) has = rev[j] >= 0;
+                if (has) std::fill(unit_expanded.begin() + T.leaf_off[k], unit_expanded.begin() + T.leaf_off[k + 1], 1);
+            }
+        }
         pt.mark("plan: symmetric: reverse look-ups");
         const int64_t npairs = poff1[NU];
         hvec<int64_t> pid;
@@ -1636,21 +1650,30 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     // The near field of the FP64 kernels: what the symmetric pairs leave, or
     // the plan's own list.  Entries whose box meets the target leaf's, the
     // only ones where a source can coincide with a target, carry EV_MEETS.
-    const int64_t *near_off = sym64 && sym_dropped ? mx_doff.data() : pl.t_direct.off;
-    const int *near_idx = sym64 && sym_dropped ? mx_didx.data() : pl.t_direct.idx;
+    const int64_t *near_off = pl.t_direct.off;
+    const int *near_idx = pl.t_direct.idx;
+    std::vector<int64_t> doff64;
     hvec<int> didx64;
     if (!mixed && !ssm) {
-        didx64.resize((size_t)near_off[T.nleaves]);
+        auto expanded = [&](int u) { return sym_dropped && unit_expanded[u]; };
+        doff64.assign((size_t)T.nleaves + 1, 0);
+        for (int u = 0; u < T.nleaves; u++) {
+            const int64_t *off = expanded(u) ? mx_doff.data() : pl.t_direct.off;
+            doff64[u + 1] = doff64[u] + (off[u + 1] - off[u]);
+        }
+        didx64.resize((size_t)doff64[T.nleaves]);
 #pragma omp parallel for schedule(static)
         for (int u = 0; u < T.nleaves; u++) {
             const int t = T.leaves[u];
-            for (int64_t k = near_off[u]; k < near_off[u + 1]; k++) {
-                const int s = near_idx[k];
+            const int *from = expanded(u) ? mx_didx.data() + mx_doff[u] : pl.t_direct.idx + pl.t_direct.off[u];
+            for (int64_t k = doff64[u]; k < doff64[u + 1]; k++) {
+                const int s = from[k - doff64[u]];
                 const bool meets = S.x0[s] <= T.x1[t] && T.x0[t] <= S.x1[s] && S.y0[s] <= T.y1[t] &&
                                    T.y0[t] <= S.y1[s] && S.z0[s] <= T.z1[t] && T.z0[t] <= S.z1[s];
                 didx64[k] = meets ? s | bt::EV_MEETS : s;
             }
         }
+        near_off = doff64.data();
         near_idx = didx64.data();
     }
 

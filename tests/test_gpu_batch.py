@@ -42,6 +42,34 @@ def test_batch_equals_separate_calls(ctype, precision):
         assert np.array_equal(p, ref)
 
 
+# FP64 systems whose lists differ in kind: leaves below the symmetric pairs'
+# 512 particles and interior nodes in the direct lists of cluster-cluster
+# (44,800 points in leaves of about 90 under nodes of about 700, fewer than
+# the degree's 729 grid points), pairs of leaves of about 550, and targets of
+# its own.
+def _kinds():
+    small, = _systems(21, [(44800, 44800)])
+    pairs, = _systems(22, [(4400, 4400)])
+    own, = _systems(23, [(4400, 4400)], same=False)
+    return small, pairs, own
+
+
+@pytest.mark.parametrize("ctype", [1, 2, 3])
+@pytest.mark.parametrize("tree_build", [B.TREE_GPU, B.TREE_HOST])
+def test_fp64_batch_of_systems_with_and_without_pairs_equals_separate_calls(ctype, tree_build):
+    """What one system of a batch is summed in does not depend on the others:
+    with the symmetric pairs on, each has the bits of its own call."""
+    systems = _kinds()
+    kw = dict(kernel=2, kernel_param=0.5, compute_type=ctype, degree=8, theta=0.8, max_source_leaf=600,
+              max_target_leaf=600, tree_build=tree_build)
+    alone, reps = zip(*[B.treecode(*s, return_report=True, **kw) for s in systems])
+    assert [r["sym_ptwise"] > 0 for r in reps] == [False, True, False]
+    for order in ([0, 1, 2], [1, 0], [0, 2]):
+        pots = B.treecode_batch([systems[k] for k in order], **kw)
+        for k, p in zip(order, pots):
+            assert np.array_equal(p, alone[k]), (order, k)
+
+
 def test_batch_host_and_gpu_tree_builds_agree():
     systems = _systems(2, SIZES)
     kw = dict(kernel=1, degree=6, max_source_leaf=200, max_target_leaf=200, precision=B.PRECISION_MIXED)
