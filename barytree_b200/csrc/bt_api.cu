@@ -548,11 +548,23 @@ bool same_host(const double *a, const double *b, size_t n)
     return !diff;
 }
 
+// Whether a call runs the mixed-precision kernels: Lagrange, and Hermite
+// particle-cluster (its far field in FP32 over the 8 moments).  Hermite grid
+// outputs, subtraction and the other kernels evaluate in FP64 whatever
+// precision is asked for.
+bool mixed_path(const bt_params &o)
+{
+    return o.precision == BT_PRECISION_MIXED && o.sing != SUBTRACTION &&
+           (o.approx != HERMITE || o.ctype == PARTICLE_CLUSTER) && o.kernel <= REGULARIZED_COULOMB;
+}
+
 // A batch whose systems are not all their own targets: which ones are (their
-// target and source trees are the same from the roots on).
+// target and source trees are the same from the roots on), for the FP64
+// path's symmetric pairs.
 bool same_systems_possible(const bt_plan &pl, const Systems &sys)
 {
-    return sys.n > 1 && pl.prm.maxs == pl.prm.maxt && pl.prm.precision == BT_PRECISION_FP64;
+    const bt_params &o = pl.prm;
+    return sys.n > 1 && o.maxs == o.maxt && !mixed_path(o) && o.sing != SUBTRACTION && o.kernel <= REGULARIZED_COULOMB;
 }
 
 void same_systems_host(bt_plan &pl, const Systems &sys, const double *tx, const double *ty, const double *tz,
@@ -1290,11 +1302,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         leaf_cost[u] = c;
     }
     const bool ssm = ss != nullptr;
-    // mixed precision: Lagrange, and Hermite particle-cluster (its far field
-    // in FP32 over the 8 moments); Hermite grid outputs and subtraction
-    // evaluate in FP64
-    const bool mixed = o.precision == BT_PRECISION_MIXED && !ssm && (!herm || o.ctype == PARTICLE_CLUSTER) &&
-                       o.kernel <= REGULARIZED_COULOMB;
+    const bool mixed = mixed_path(o);
     // grid-output cost per target node (CP and CC): the work-item order of
     // the grid evaluation, and for a sharded call the share of the leaves
     // under the node

@@ -70,6 +70,19 @@ def test_fp64_batch_of_systems_with_and_without_pairs_equals_separate_calls(ctyp
             assert np.array_equal(p, alone[k]), (order, k)
 
 
+def test_mixed_hermite_cluster_particle_batch_equals_separate_calls():
+    """A mixed request that evaluates in FP64 (Hermite grid outputs) takes the
+    FP64 pairs in a batch as it does alone."""
+    _, pairs, own = _kinds()
+    kw = dict(kernel=1, approximation=2, compute_type=2, degree=4, theta=0.7, max_source_leaf=600,
+              max_target_leaf=600, size_check=4.0, precision=B.PRECISION_MIXED)
+    ref, rep = B.treecode(*pairs, return_report=True, **kw)
+    assert rep["sym_ptwise"] > 0
+    pots = B.treecode_batch([own, pairs], **kw)
+    assert np.array_equal(pots[1], ref)
+    assert np.array_equal(pots[0], B.treecode(*own, **kw))
+
+
 def test_batch_host_and_gpu_tree_builds_agree():
     systems = _systems(2, SIZES)
     kw = dict(kernel=1, degree=6, max_source_leaf=200, max_target_leaf=200, precision=B.PRECISION_MIXED)
