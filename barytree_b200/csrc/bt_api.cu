@@ -237,6 +237,12 @@ struct Layout {
     std::vector<std::pair<void **, size_t>> reqs;
     template <typename T>
     void add(T **p, size_t count) { reqs.push_back({(void **)p, sizeof(T) * (count > 0 ? count : 1)}); }
+    template <typename T>
+    void resize(T **p, size_t count)
+    {
+        for (auto &r : reqs)
+            if (r.first == (void **)p) r.second = sizeof(T) * (count > 0 ? count : 1);
+    }
     size_t total() const
     {
         size_t s = 0;
@@ -730,6 +736,14 @@ int build_plan_gpu(DeviceCtx *ctx, Arena &tarena, bt_plan &pl, const Systems &sy
     return BT_OK;
 }
 
+// Blocks of one round of the symmetric pairs: those of the pairs whose boxes
+// are apart by more than the close-pair distance, and of the others.
+struct SymRound {
+    int64_t far0, far1, near0, near1;
+};
+// Device memory of the pairs' slices (a round's).
+constexpr size_t SYM_SLICE_BYTES = (size_t)8 << 30;
+
 // Everything the device sequence of one evaluation needs: the device arrays
 // of a prepared plan and the few host-side sizes that shape the launches.
 struct DevPlan {
@@ -741,8 +755,8 @@ struct DevPlan {
     bool tc_up = false;         // leaf P2M on the tensor cores (bt_tc.cu)
     bool sharded = false;       // this call evaluates a share of the target leaves (others get 0)
     // symmetric near-field pairs (bt_sym.cu)
-    int sym_nblocks = 0;
-    int sym_far_blocks = 0;     // the first blocks: pairs whose boxes are apart by more than the close-pair distance
+    std::vector<SymRound> sym_rounds;
+    double *d_sym_run = nullptr;        // several rounds: the leaves' running sums
     double *d_sbox = nullptr;   // node boxes (x0 x1 y0 y1 z0 z1) for the pairs within it
     int2 *d_sym_pairs = nullptr, *d_sym_blocks = nullptr;
     int64_t *d_sym_slot = nullptr, *d_sym_in_off = nullptr, *d_sym_in_slot = nullptr;
@@ -1059,7 +1073,8 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         // the symmetric pairs write only their own partial sums: their two
         // kernels run beside the particle-output kernel on two more streams,
         // joined before the gather adds them into the potentials
-        const bool fork = v.sym_nblocks > 0 && fk && fk->side && fk->side2;
+        const int nrounds = (int)v.sym_rounds.size();
+        const bool fork = nrounds > 0 && fk && fk->side && fk->side2;
         cudaStream_t sst = st, sst2 = st;
         if (fork) {
             CK(cudaEventRecord(fk->fork, st));
@@ -1068,7 +1083,12 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
             sst = fk->side;
             sst2 = fk->side2;
         }
-        if (v.sym_nblocks > 0) {
+        bt::SymGatherArgs g;
+        g.nleaves = v.T_nleaves; g.leaf_node = v.d_tleaves; g.ibeg = v.d_sibeg; g.numpar = v.d_snum;
+        g.in_off = v.d_sym_in_off; g.in_slot = v.d_sym_in_slot; g.partial = v.d_sym_partial; g.pot = d_pot;
+        g.run = v.d_sym_run; g.nrounds = nrounds;
+        for (int r = 0; r < nrounds; r++) {
+            const SymRound &w = v.sym_rounds[r];
             bt::SymArgs y;
             y.pair = v.d_sym_pairs; y.slot = v.d_sym_slot;
             y.ibeg = v.d_sibeg; y.numpar = v.d_snum; y.ctr = v.d_sctr; y.pos = v.d_spos;
@@ -1076,13 +1096,26 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
             y.rad = v.d_srad; y.box = v.d_sbox; y.x64 = v.d_sx; y.y64 = v.d_sy; y.z64 = v.d_sz; y.q64 = v.d_sq;
             y.kp = v.kp;
             bt::SymArgs yc = y;
-            y.nblocks = v.sym_far_blocks;
-            y.block = v.d_sym_blocks;
-            yc.nblocks = v.sym_nblocks - v.sym_far_blocks;
-            yc.block = v.d_sym_blocks + v.sym_far_blocks;
+            y.nblocks = (int)(w.far1 - w.far0);
+            y.block = v.d_sym_blocks + w.far0;
+            yc.nblocks = (int)(w.near1 - w.near0);
+            yc.block = v.d_sym_blocks + w.near0;
             bt::launch_pp_sym(v.kernel, y, sst);
             bt::launch_pp_sym_close(v.kernel, yc, sst2);
             launches += (y.nblocks > 0) + (yc.nblocks > 0);
+            if (r + 1 == nrounds) break;
+            // the next round reuses the slices: gathered before it starts
+            if (fork) {
+                CK(cudaEventRecord(fk->join2, sst2));
+                CK(cudaStreamWaitEvent(sst, fk->join2, 0));
+            }
+            g.round = r;
+            bt::launch_sym_gather(g, sst);
+            launches++;
+            if (fork) {
+                CK(cudaEventRecord(fk->join, sst));
+                CK(cudaStreamWaitEvent(sst2, fk->join, 0));
+            }
         }
         bt::launch_eval_targets_mixed(v.kernel, a, st);
         launches += a.partial ? 2 : 1;
@@ -1093,10 +1126,8 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
             CK(cudaStreamWaitEvent(st, fk->join, 0));
             CK(cudaStreamWaitEvent(st, fk->join2, 0));
         }
-        if (v.sym_nblocks > 0) {
-            bt::SymGatherArgs g;
-            g.nleaves = v.T_nleaves; g.leaf_node = v.d_tleaves; g.ibeg = v.d_sibeg; g.numpar = v.d_snum;
-            g.in_off = v.d_sym_in_off; g.in_slot = v.d_sym_in_slot; g.partial = v.d_sym_partial; g.pot = d_pot;
+        if (nrounds > 0) {
+            g.round = nrounds - 1;
             bt::launch_sym_gather(g, st);
             launches++;
         }
@@ -1110,16 +1141,28 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         a.partial = v.d_evpart; a.pstride = (size_t)nt;
         // the symmetric pairs beside the particle-output kernel, joined before
         // the gather adds their slices
-        const bool fork = v.sym_nblocks > 0 && fk && fk->side;
+        const int nrounds = (int)v.sym_rounds.size();
+        const bool fork = nrounds > 0 && fk && fk->side;
+        cudaStream_t sst = fork ? fk->side : st;
         if (fork) {
             CK(cudaEventRecord(fk->fork, st));
             CK(cudaStreamWaitEvent(fk->side, fk->fork, 0));
         }
-        if (v.sym_nblocks > 0) {
+        bt::SymGather64Args g;
+        g.nleaves = v.T_nleaves; g.leaf_node = v.d_tleaves; g.ibeg = d_tibeg; g.numpar = d_tnum;
+        g.in_off = v.d_sym_in_off; g.in_slot = v.d_sym_in_slot; g.partial = v.d_sym_partial64; g.pot = d_pot;
+        g.run = v.d_sym_run; g.nrounds = nrounds;
+        for (int r = 0; r < nrounds; r++) {
+            const SymRound &w = v.sym_rounds[r];       // FP64: one group of pairs
             bt::Sym64Args y;
-            y.nblocks = v.sym_nblocks; y.block = v.d_sym_blocks; y.pair = v.d_sym_pairs; y.slot = v.d_sym_slot; y.ibeg = d_sibeg; y.numpar = d_snum;
+            y.nblocks = (int)(w.far1 - w.far0); y.block = v.d_sym_blocks + w.far0;
+            y.pair = v.d_sym_pairs; y.slot = v.d_sym_slot; y.ibeg = d_sibeg; y.numpar = d_snum;
             y.x = d_sx; y.y = d_sy; y.z = d_sz; y.q = d_sq; y.partial = v.d_sym_partial64; y.kp = v.kp;
-            bt::launch_pp_sym64(v.kernel, y, fork ? fk->side : st);
+            bt::launch_pp_sym64(v.kernel, y, sst);
+            launches++;
+            if (r + 1 == nrounds) break;
+            g.round = r;
+            bt::launch_sym_gather64(g, sst);
             launches++;
         }
         bt::launch_eval_targets(v.kernel, herm, a, st);
@@ -1129,10 +1172,8 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
             CK(cudaEventRecord(fk->join, fk->side));
             CK(cudaStreamWaitEvent(st, fk->join, 0));
         }
-        if (v.sym_nblocks > 0) {
-            bt::SymGather64Args g;
-            g.nleaves = v.T_nleaves; g.leaf_node = v.d_tleaves; g.ibeg = d_tibeg; g.numpar = d_tnum;
-            g.in_off = v.d_sym_in_off; g.in_slot = v.d_sym_in_slot; g.partial = v.d_sym_partial64; g.pot = d_pot;
+        if (nrounds > 0) {
+            g.round = nrounds - 1;
             bt::launch_sym_gather64(g, st);
             launches++;
         }
@@ -1190,6 +1231,327 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
     CK(cudaGetLastError());
 done:
     return rc;
+}
+
+// Symmetric near-field pairs: with the targets being the sources and a
+// symmetric kernel, leaf pairs {A, B} (A != B) that hold each other as
+// near-field entries are evaluated once for both sides (bt_sym.cu,
+// bt_sym64.cu) and leave the per-target lists.  Every pass runs per unit in
+// parallel.  The pairs whose boxes are farther apart than the close-pair
+// distance come first, then the pairs within it (mixed: their own kernel);
+// each group is numbered by head unit (A < B), then by partner node, so the
+// numbering does not depend on the thread count.
+//
+// The pairs' slices are the call's largest work array.  They are bounded: the
+// head units are divided into rounds whose slices fit, each round's slices are
+// gathered before the next one reuses them, and a leaf's running sum goes on
+// from round to round.  A leaf's slices come in partner order, that is in the
+// order of the head units, so the sums, and their bits, do not depend on the
+// rounds.
+struct SymPairs {
+    const bt_plan &pl;
+    PhaseTimer &pt;
+    bool fp64 = false;
+    hvec<int> far, fent;                // per unit: partners sorted by node, the list entry of each
+    hvec<unsigned char> fnear;          // and whether the boxes are within the close-pair distance
+    std::vector<int64_t> far_end;
+    hvec<int64_t> rev, pid;             // the partner's entry for this leaf (-1: none), a head entry's pair
+    std::vector<int> sleaf, unit_of;
+    std::vector<unsigned char> owned;
+    std::vector<int64_t> poff0, poff1, ioff;    // pairs headed by each unit (the two groups), slices it gathers
+    std::vector<int64_t> size;          // values of the slices of the pairs that a unit heads
+    int64_t npaired = 0, npairs = 0, nblocks = 0, total = 0, max_size = 0;
+    // FP64: the units of systems that have pairs, whose near field is what is
+    // left of the leaf-expanded list.  The other systems of a batch keep the
+    // plan's list, as in a call of their own: the segments of the sums are cut
+    // by list entries, and cluster-cluster lists hold interior nodes.
+    std::vector<unsigned char> unit_expanded;
+    // placed:
+    bool taken = false;                 // the pairs have left the per-target lists
+    hvec<int2> pairs, blocks;
+    hvec<int64_t> slot, in_slot;
+    std::vector<int64_t> in_off;        // (rounds + 1) x units: where each round's slices of a unit begin
+    std::vector<SymRound> rounds;
+    int64_t round_values = 0;           // values of the largest round's slices
+
+    SymPairs(const bt_plan &p, PhaseTimer &t) : pl(p), pt(t) {}
+    // a pair belongs to the shard that owns its head (the lower leaf): that
+    // shard evaluates it and gathers both sides, the partner's side into
+    // targets another shard owns (the combining sum adds them)
+    bool evaluated(int head, int) const { return owned[head]; }
+    bool gathered(int, int head) const { return owned[head]; }
+    // values of the slices of pair {A, B}: A's once, B's per part of A
+    int64_t pair_values(int A, int B) const
+    {
+        return pl.st.numpar[A] + (int64_t)bt::sym_parts(pl.st.numpar[A]) * pl.st.numpar[B];
+    }
+
+    void find(bool fp64_path, const std::vector<int64_t> &doff, const hvec<int> &didx, const hvec<unsigned char> &dflag,
+              const std::vector<int> &leaf_count, int nshards);
+    int divide(int64_t values, std::vector<int> *start) const;
+    size_t bytes(int nrounds) const;
+    void place(int64_t values, std::vector<int64_t> &doff, hvec<int> &didx, hvec<unsigned char> &dflag);
+};
+
+// The pairs, their sizes and owners.  leaf_count: 0 for the leaves of other shards.
+void SymPairs::find(bool fp64_path, const std::vector<int64_t> &doff, const hvec<int> &didx,
+                    const hvec<unsigned char> &dflag, const std::vector<int> &leaf_count, int nshards)
+{
+    const bt_tree &S = pl.st, &T = pl.tt;
+    const int NU = T.nleaves;
+    fp64 = fp64_path;
+    auto leaf64 = [&](int v) { return S.numpar[v] >= bt::SYM64_MIN_LEAF && S.numpar[v] <= bt::SYM_MAX_LEAF; };
+    // the source node that a unit's leaf is: the trees are one, or (FP64,
+    // a batch) the trees of a system whose targets are its sources have
+    // the same nodes from their roots on
+    sleaf.resize(NU);
+    unit_of.assign(S.n, -1);
+    for (int k = 0; k < T.nroots; k++)
+        for (int u = T.leaf_off[k]; u < T.leaf_off[k + 1]; u++)
+            sleaf[u] = pl.same_tree ? T.leaves[u]
+                       : pl.sys_same[k] ? T.leaves[u] - T.roots[k] + S.roots[k] : -1;
+    for (int u = 0; u < NU; u++)
+        if (sleaf[u] >= 0) unit_of[sleaf[u]] = u;
+    owned.assign(NU, 1);
+    if (nshards > 1)
+        for (int u = 0; u < NU; u++) owned[u] = leaf_count[u] > 0;
+    const int64_t ne = doff[NU];
+    // per unit: its partners (other leaves), sorted by node, each with the
+    // list entry it came from and whether the boxes are within the
+    // close-pair distance (the same test from both sides)
+    far.resize(ne);
+    fent.resize(ne);
+    fnear.resize(ne);
+    far_end.resize(NU);
+#pragma omp parallel
+    {
+        std::vector<uint64_t> keys;
+#pragma omp for schedule(static)
+        for (int u = 0; u < NU; u++) {
+            const int A = sleaf[u];
+            keys.clear();
+            for (int64_t k = doff[u]; k < doff[u + 1]; k++) {
+                const int B = didx[k];
+                if (A < 0 || B == A || unit_of[B] < 0) continue;
+                if (fp64 && !(leaf64(A) && leaf64(B))) continue;
+                keys.push_back(((uint64_t)(uint32_t)B << 32) | (uint64_t)(k - doff[u]));
+            }
+            std::sort(keys.begin(), keys.end());
+            int64_t w = doff[u];
+            for (uint64_t key : keys) {
+                far[w] = (int)(key >> 32);
+                fent[w] = (int)(key & 0xffffffffu);
+                fnear[w] = dflag[doff[u] + fent[w]];
+                w++;
+            }
+            far_end[u] = w;
+        }
+    }
+    pt.mark("plan: symmetric: sorted partners");
+    // rev[j]: where the partner's sorted list holds this unit's leaf (-1:
+    // nowhere, the entry stays one-directional)
+    rev.resize(ne);
+#pragma omp parallel for schedule(static)
+    for (int u = 0; u < NU; u++)
+        for (int64_t j = doff[u]; j < far_end[u]; j++) rev[j] = -1;
+    // the head of each pair (A < B) looks itself up in B's list and links
+    // both entries; every entry is written by one head at most
+#pragma omp parallel for schedule(static)
+    for (int u = 0; u < NU; u++) {
+        const int A = sleaf[u];
+        for (int64_t j = doff[u]; j < far_end[u]; j++) {
+            const int B = far[j], ub = unit_of[B];
+            if (B < A) continue;
+            const int *b0 = far.data() + doff[ub], *b1 = far.data() + far_end[ub];
+            const int *it = std::lower_bound(b0, b1, A);
+            if (it != b1 && *it == A) {
+                const int64_t q = it - far.data();
+                rev[j] = q;
+                rev[q] = j;
+            }
+        }
+    }
+    poff0.assign(NU + 1, 0);
+    poff1.assign(NU + 1, 0);
+    ioff.assign(NU + 1, 0);
+    size.assign(NU, 0);
+    // npaired: entries in a pair, whichever shard evaluates it
+    int64_t paired = 0, blk = 0;
+#pragma omp parallel for schedule(static) reduction(+ : paired, blk)
+    for (int u = 0; u < NU; u++) {
+        const int A = sleaf[u];
+        int64_t heads[2] = {0, 0}, all = 0, values = 0;
+        for (int64_t j = doff[u]; j < far_end[u]; j++)
+            if (rev[j] >= 0) {
+                paired++;
+                const int B = far[j], ub = unit_of[B];
+                const bool head = A < B;
+                // one slice from a pair this leaf heads, one per part of a head's particles
+                if (gathered(u, head ? u : ub)) all += head ? 1 : bt::sym_parts(S.numpar[B]);
+                if (!head || !evaluated(u, ub)) continue;
+                heads[fnear[j]]++;
+                values += pair_values(A, B);
+                blk += bt::sym_parts(S.numpar[A]);
+            }
+        poff0[u + 1] = heads[0];
+        poff1[u + 1] = heads[1];
+        ioff[u + 1] = all;
+        size[u] = values;
+    }
+    npaired = paired;
+    nblocks = blk;
+    for (int u = 0; u < NU; u++) {
+        poff0[u + 1] += poff0[u];
+        ioff[u + 1] += ioff[u];
+        total += size[u];
+        max_size = std::max(max_size, size[u]);
+    }
+    poff1[0] = poff0[NU];
+    for (int u = 0; u < NU; u++) poff1[u + 1] += poff1[u];
+    npairs = poff1[NU];
+    if (fp64) {
+        unit_expanded.assign(NU, 0);
+        for (int k = 0; k < T.nroots; k++) {
+            bool has = false;
+            for (int u = T.leaf_off[k]; u < T.leaf_off[k + 1] && !has; u++)
+                for (int64_t j = doff[u]; j < far_end[u] && !has; j++) has = rev[j] >= 0;
+            if (has) std::fill(unit_expanded.begin() + T.leaf_off[k], unit_expanded.begin() + T.leaf_off[k + 1], 1);
+        }
+    }
+    pt.mark("plan: symmetric: reverse look-ups");
+}
+
+// Rounds of at most `values` slice values each: how many (-1: a unit alone has
+// more), and the first unit of each.
+int SymPairs::divide(int64_t values, std::vector<int> *start) const
+{
+    if (max_size > values) return -1;
+    int n = 0;
+    int64_t sum = values + 1;
+    for (size_t u = 0; u < size.size(); u++) {
+        if (n == 0 || sum + size[u] > values) {
+            n++;
+            sum = 0;
+            if (start) start->push_back((int)u);
+        }
+        sum += size[u];
+    }
+    return n;
+}
+
+// Device bytes of the pass besides the slices.
+size_t SymPairs::bytes(int nrounds) const
+{
+    const size_t NU = size.size(), run = nrounds > 1 ? sizeof(double) * (size_t)pl.tgt.n : 0;
+    return sizeof(int2) * (size_t)(nblocks + npairs) + sizeof(int64_t) * (size_t)(npairs + ioff[NU]) +
+           sizeof(int64_t) * NU * (size_t)(nrounds + 1) + run + (fp64 ? 0 : 6 * sizeof(double) * (size_t)pl.st.n) +
+           8 * 256;
+}
+
+// Takes the pairs out of the per-target lists and gives them their blocks and
+// slices, in rounds of at most `values` slice values.
+void SymPairs::place(int64_t values, std::vector<int64_t> &doff, hvec<int> &didx, hvec<unsigned char> &dflag)
+{
+    const bt_tree &S = pl.st;
+    const int NU = (int)size.size();
+    const int64_t ne = doff[NU];
+    std::vector<int> start;
+    const int nr = divide(values, &start);
+    taken = true;
+    // each unit's first slice value within its round: its pairs of the first
+    // group, then those of the second
+    std::vector<int64_t> base(NU);
+    std::vector<int> round_of(NU);
+    for (int r = 0; r < nr; r++) {
+        int64_t sum = 0;
+        for (int u = start[r]; u < (r + 1 < nr ? start[r + 1] : NU); u++) {
+            base[u] = sum;
+            round_of[u] = r;
+            sum += size[u];
+        }
+        round_values = std::max(round_values, sum);
+    }
+    // all pairs of a unit's group have the unit's leaf as A, so their blocks
+    // (one per part of A) are consecutive
+    std::vector<int64_t> boff0(NU + 1, 0), boff1(NU + 1, 0);
+    for (int u = 0; u < NU; u++) {
+        const int parts = sleaf[u] >= 0 ? bt::sym_parts(S.numpar[sleaf[u]]) : 0;
+        boff0[u + 1] = boff0[u] + (poff0[u + 1] - poff0[u]) * parts;
+        boff1[u + 1] = (poff1[u + 1] - poff1[u]) * parts;
+    }
+    boff1[0] = boff0[NU];
+    for (int u = 0; u < NU; u++) boff1[u + 1] += boff1[u];
+    for (int r = 0; r < nr; r++) {
+        const int u0 = start[r], u1 = r + 1 < nr ? start[r + 1] : NU;
+        rounds.push_back(SymRound{boff0[u0], boff0[u1], boff1[u0], boff1[u1]});
+    }
+    pairs.resize((size_t)npairs);
+    slot.resize((size_t)npairs);
+    blocks.resize((size_t)boff1[NU]);
+    pid.resize((size_t)ne);
+#pragma omp parallel for schedule(static)
+    for (int u = 0; u < NU; u++) {
+        const int A = sleaf[u], parts = A >= 0 ? bt::sym_parts(S.numpar[A]) : 0;
+        int64_t p[2] = {poff0[u], poff1[u]}, w[2] = {boff0[u], boff1[u]}, s = base[u];
+        for (int g = 0; g < 2; g++)
+            for (int64_t j = doff[u]; j < far_end[u]; j++)
+                if (rev[j] >= 0 && A < far[j] && fnear[j] == g && evaluated(u, unit_of[far[j]])) {
+                    pid[j] = p[g];
+                    pairs[p[g]] = make_int2(A, far[j]);
+                    slot[p[g]] = s;
+                    s += pair_values(A, far[j]);
+                    for (int k = 0; k < parts; k++) blocks[w[g]++] = make_int2((int)p[g], k);
+                    p[g]++;
+                }
+    }
+    // per leaf the slices addressed to it, in partner order: its own side of
+    // the pairs it heads, the B side of the pairs headed by a partner (found
+    // through the partner's entry for this leaf); both directions leave the
+    // lists
+    in_off.resize((size_t)(nr + 1) * NU);
+    in_slot.resize((size_t)ioff[NU]);
+    hvec<unsigned char> drop(ne);
+#pragma omp parallel for schedule(static)
+    for (int u = 0; u < NU; u++) {
+        const int A = sleaf[u];
+        int64_t w = ioff[u];
+        int next = 0;               // rounds whose begin is written
+        std::fill(drop.begin() + doff[u], drop.begin() + doff[u + 1], (unsigned char)0);
+        for (int64_t j = doff[u]; j < far_end[u]; j++) {
+            if (rev[j] < 0) continue;
+            const int B = far[j], ub = unit_of[B], head = A < B ? u : ub;
+            drop[doff[u] + fent[j]] = 1;
+            if (!gathered(u, head)) continue;
+            while (next <= round_of[head]) in_off[(size_t)next++ * NU + u] = w;
+            if (A < B) {
+                in_slot[w++] = slot[pid[j]];
+                continue;
+            }
+            for (int k = 0; k < bt::sym_parts(S.numpar[B]); k++)
+                in_slot[w++] = slot[pid[rev[j]]] + S.numpar[B] + (int64_t)k * S.numpar[A];
+        }
+        while (next <= nr) in_off[(size_t)next++ * NU + u] = w;
+    }
+    pt.mark("plan: symmetric: pairs and slots");
+    std::vector<int64_t> noff(NU + 1, 0);
+#pragma omp parallel for schedule(static)
+    for (int u = 0; u < NU; u++) {
+        int64_t kept = 0;
+        for (int64_t k = doff[u]; k < doff[u + 1]; k++) kept += !drop[k];
+        noff[u + 1] = kept;
+    }
+    for (int u = 0; u < NU; u++) noff[u + 1] += noff[u];
+    hvec<int> nidx((size_t)noff[NU]);
+    hvec<unsigned char> nflag((size_t)noff[NU]);
+#pragma omp parallel for schedule(static)
+    for (int u = 0; u < NU; u++) {
+        int64_t w = noff[u];
+        for (int64_t k = doff[u]; k < doff[u + 1]; k++)
+            if (!drop[k]) { nidx[w] = didx[k]; nflag[w] = dflag[k]; w++; }
+    }
+    doff.swap(noff);
+    didx.swap(nidx);
+    dflag.swap(nflag);
 }
 
 // Device evaluation of a built plan; writes potentials in caller order to out_host.
@@ -1375,12 +1737,11 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     // targets that are the sources, and a kernel that is symmetric in r: the
     // symmetric near-field pass.  FP64 takes it pair by pair (leaves of
     // SYM64_MIN_LEAF to SYM_MAX_LEAF particles); a shard in FP64 evaluates
-    // all of its targets' potentials itself, and the static scratch holds no
-    // partial sums.
+    // all of its targets' potentials itself.
     const bool sym_kernel = shape.sym && T.nleaves > 1 && o.kernel >= COULOMB && o.kernel <= REGULARIZED_COULOMB;
     const bool sym_ok = pl.same_tree && sym_kernel;
     const bool sym64 = (pl.same_tree || pl.sys_same) && sym_kernel && !mixed && !ssm && shape.nshards == 1 &&
-                       !arena.fixed && max_leaf >= bt::SYM64_MIN_LEAF;
+                       max_leaf >= bt::SYM64_MIN_LEAF;
     if (mixed || sym64) {
         std::vector<int> lf, lc;
         leaf_ranges(S, lf, lc);
@@ -1408,244 +1769,11 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     }
     if (sym64) std::fill(mx_dflag.begin(), mx_dflag.end(), (unsigned char)0);     // one group of pairs
     pt.mark("plan: work items and near-field lists");
-    // Symmetric near-field pairs: with the targets being the sources and a
-    // symmetric kernel, leaf pairs {A, B} (A != B) that hold each other as
-    // near-field entries are evaluated once for both sides (bt_sym.cu) and
-    // leave the per-target lists.  Every pass runs per unit in parallel.  The
-    // pairs whose boxes are farther apart than the close-pair distance come
-    // first, then the pairs within it (their own kernel); each group is
-    // numbered by head unit (A < B), then by partner node, so the numbering
-    // does not depend on the thread count.
-    hvec<int2> sym_pairs, sym_blocks;
-    int64_t sym_far_blocks = 0;
-    hvec<int64_t> sym_slot, sym_in_slot;
-    std::vector<int64_t> sym_in_off;
-    int64_t sym_total = 0, sym_far_pairs = 0;
-    bool sym_dropped = false;      // the pairs have left the per-target lists
-    // FP64: the units of systems that have pairs, whose near field is what is
-    // left of the leaf-expanded list.  The other systems of a batch keep the
-    // plan's list, as in a call of their own: the segments of the sums are cut
-    // by list entries, and cluster-cluster lists hold interior nodes.
-    std::vector<unsigned char> unit_expanded;
-    auto sym64_leaf = [&](int v) { return S.numpar[v] >= bt::SYM64_MIN_LEAF && S.numpar[v] <= bt::SYM_MAX_LEAF; };
-    if ((mixed && sym_ok && max_leaf <= bt::SYM_MAX_LEAF) || sym64) {
-        const int NU = T.nleaves;
-        // the source node that a unit's leaf is: the trees are one, or (FP64,
-        // a batch) the trees of a system whose targets are its sources have
-        // the same nodes from their roots on
-        std::vector<int> sleaf(NU), unit_of(S.n, -1);
-        for (int k = 0; k < T.nroots; k++)
-            for (int u = T.leaf_off[k]; u < T.leaf_off[k + 1]; u++)
-                sleaf[u] = pl.same_tree ? T.leaves[u]
-                           : pl.sys_same[k] ? T.leaves[u] - T.roots[k] + S.roots[k] : -1;
-        for (int u = 0; u < NU; u++)
-            if (sleaf[u] >= 0) unit_of[sleaf[u]] = u;
-        // a pair belongs to the shard that owns its head (the lower leaf):
-        // that shard evaluates it and gathers both sides, the partner's side
-        // into targets another shard owns (the combining sum adds them)
-        std::vector<unsigned char> owned(NU, 1);
-        if (shape.nshards > 1)
-            for (int u = 0; u < NU; u++) owned[u] = leaf_count[u] > 0;
-        const int64_t ne = mx_doff[NU];
-        // per unit: its partners (other leaves), sorted by node, each with the
-        // list entry it came from and whether the boxes are within the
-        // close-pair distance (the same test from both sides)
-        hvec<int> far(ne), fent(ne);
-        hvec<unsigned char> fnear(ne);
-        std::vector<int64_t> far_end(NU);
-#pragma omp parallel
-        {
-            std::vector<uint64_t> keys;
-#pragma omp for schedule(static)
-            for (int u = 0; u < NU; u++) {
-                const int A = sleaf[u];
-                keys.clear();
-                for (int64_t k = mx_doff[u]; k < mx_doff[u + 1]; k++) {
-                    const int B = mx_didx[k];
-                    if (A < 0 || B == A || unit_of[B] < 0) continue;
-                    if (sym64 && !(sym64_leaf(A) && sym64_leaf(B))) continue;
-                    keys.push_back(((uint64_t)(uint32_t)B << 32) | (uint64_t)(k - mx_doff[u]));
-                }
-                std::sort(keys.begin(), keys.end());
-                int64_t w = mx_doff[u];
-                for (uint64_t key : keys) {
-                    far[w] = (int)(key >> 32);
-                    fent[w] = (int)(key & 0xffffffffu);
-                    fnear[w] = mx_dflag[mx_doff[u] + fent[w]];
-                    w++;
-                }
-                far_end[u] = w;
-            }
-        }
-        pt.mark("plan: symmetric: sorted partners");
-        // rev[j]: where the partner's sorted list holds this unit's leaf (-1:
-        // nowhere, the entry stays one-directional)
-        hvec<int64_t> rev(ne);
-        std::vector<int64_t> poff0(NU + 1, 0), poff1(NU + 1, 0), ioff(NU + 1, 0);
-#pragma omp parallel for schedule(static)
-        for (int u = 0; u < NU; u++)
-            for (int64_t j = mx_doff[u]; j < far_end[u]; j++) rev[j] = -1;
-        // the head of each pair (A < B) looks itself up in B's list and links
-        // both entries; every entry is written by one head at most
-#pragma omp parallel for schedule(static)
-        for (int u = 0; u < NU; u++) {
-            const int A = sleaf[u];
-            for (int64_t j = mx_doff[u]; j < far_end[u]; j++) {
-                const int B = far[j], ub = unit_of[B];
-                if (B < A) continue;
-                const int *b0 = far.data() + mx_doff[ub], *b1 = far.data() + far_end[ub];
-                const int *it = std::lower_bound(b0, b1, A);
-                if (it != b1 && *it == A) {
-                    const int64_t q = it - far.data();
-                    rev[j] = q;
-                    rev[q] = j;
-                }
-            }
-        }
-        int64_t npaired = 0;       // entries in a pair, whichever shard evaluates it
-#pragma omp parallel for schedule(static) reduction(+ : npaired)
-        for (int u = 0; u < NU; u++) {
-            const int A = sleaf[u];
-            int64_t heads[2] = {0, 0}, all = 0;
-            for (int64_t j = mx_doff[u]; j < far_end[u]; j++)
-                if (rev[j] >= 0) {
-                    npaired++;
-                    const bool head = A < far[j];
-                    // one slice from a pair this leaf heads, one per part of a head's particles
-                    if (head ? owned[u] : owned[unit_of[far[j]]]) all += head ? 1 : bt::sym_parts(S.numpar[far[j]]);
-                    heads[fnear[j]] += head && owned[u] ? 1 : 0;
-                }
-            poff0[u + 1] = heads[0];
-            poff1[u + 1] = heads[1];
-            ioff[u + 1] = all;
-        }
-        for (int u = 0; u < NU; u++) {
-            poff0[u + 1] += poff0[u];
-            ioff[u + 1] += ioff[u];
-        }
-        sym_far_pairs = poff0[NU];
-        poff1[0] = sym_far_pairs;
-        for (int u = 0; u < NU; u++) poff1[u + 1] += poff1[u];
-        if (sym64) {
-            unit_expanded.assign(NU, 0);
-            for (int k = 0; k < T.nroots; k++) {
-                bool has = false;
-                for (int u = T.leaf_off[k]; u < T.leaf_off[k + 1] && !has; u++)
-                    for (int64_t j = mx_doff[u]; j < far_end[u] && !has; j++) has = rev[j] >= 0;
-                if (has) std::fill(unit_expanded.begin() + T.leaf_off[k], unit_expanded.begin() + T.leaf_off[k + 1], 1);
-            }
-        }
-        pt.mark("plan: symmetric: reverse look-ups");
-        const int64_t npairs = poff1[NU];
-        hvec<int64_t> pid;
-        std::vector<int64_t> usz0(NU + 1, 0), usz1(NU + 1, 0);
-        if (npaired > 0) {
-            // pairs headed by each unit, and the pair number of each head entry
-            sym_pairs.resize((size_t)npairs);
-            pid.resize((size_t)ne);
-#pragma omp parallel for schedule(static)
-            for (int u = 0; u < NU; u++) {
-                const int A = sleaf[u];
-                int64_t p[2] = {poff0[u], poff1[u]}, sz[2] = {0, 0};
-                for (int64_t j = mx_doff[u]; j < far_end[u]; j++)
-                    if (rev[j] >= 0 && A < far[j] && owned[u]) {
-                        const int g = fnear[j];
-                        pid[j] = p[g];
-                        sym_pairs[p[g]++] = make_int2(A, far[j]);
-                        sz[g] += S.numpar[A] + (int64_t)bt::sym_parts(S.numpar[A]) * S.numpar[far[j]];
-                    }
-                usz0[u + 1] = sz[0];
-                usz1[u + 1] = sz[1];
-            }
-            for (int u = 0; u < NU; u++) usz0[u + 1] += usz0[u];
-            usz1[0] = usz0[NU];
-            for (int u = 0; u < NU; u++) usz1[u + 1] += usz1[u];
-            sym_total = usz1[NU];
-            // Slices within 32 GB (FP64, some 70M particles) or 64 GB (mixed);
-            // a larger system evaluates every direction.  Shards of one
-            // system have to decide alike, so they always take the pairs.
-            sym_dropped = shape.nshards > 1 || sym_total <= (sym64 ? (int64_t)1 << 32 : (int64_t)1 << 34);
-        }
-        if (!sym_dropped) {
-            sym_pairs.clear();
-            sym_total = 0;
-        } else {
-            // each pair's partial sums: A's particles, then B's for every part
-            // of A; and its blocks, one per part.  All pairs of a unit's group
-            // have the unit's leaf as A, so their blocks are consecutive.
-            sym_slot.resize((size_t)npairs);
-            std::vector<int64_t> boff0(NU + 1, 0), boff1(NU + 1, 0);
-            for (int u = 0; u < NU; u++) {
-                const int parts = sleaf[u] >= 0 ? bt::sym_parts(S.numpar[sleaf[u]]) : 0;
-                boff0[u + 1] = boff0[u] + (poff0[u + 1] - poff0[u]) * parts;
-                boff1[u + 1] = (poff1[u + 1] - poff1[u]) * parts;
-            }
-            boff1[0] = sym_far_blocks = boff0[NU];
-            for (int u = 0; u < NU; u++) boff1[u + 1] += boff1[u];
-            sym_blocks.resize((size_t)boff1[NU]);
-#pragma omp parallel for schedule(static)
-            for (int u = 0; u < NU; u++) {
-                const int64_t pb[2] = {poff0[u], poff1[u]}, pe[2] = {poff0[u + 1], poff1[u + 1]};
-                const int64_t sb[2] = {usz0[u], usz1[u]}, bb[2] = {boff0[u], boff1[u]};
-                const int parts = sleaf[u] >= 0 ? bt::sym_parts(S.numpar[sleaf[u]]) : 0;
-                for (int g = 0; g < 2; g++) {
-                    int64_t s = sb[g], w = bb[g];
-                    for (int64_t p = pb[g]; p < pe[g]; p++) {
-                        sym_slot[p] = s;
-                        s += S.numpar[sym_pairs[p].x] + (int64_t)parts * S.numpar[sym_pairs[p].y];
-                        for (int k = 0; k < parts; k++) sym_blocks[w++] = make_int2((int)p, k);
-                    }
-                }
-            }
-            // per leaf the slices addressed to it, in partner order: its own
-            // side of the pairs it heads, the B side of the pairs headed by
-            // a partner (found through the partner's entry for this leaf)
-            sym_in_off = ioff;
-            sym_in_slot.resize((size_t)ioff[NU]);
-            hvec<unsigned char> drop(ne);
-#pragma omp parallel for schedule(static)
-            for (int u = 0; u < NU; u++) {
-                const int A = sleaf[u];
-                int64_t w = ioff[u];
-                std::fill(drop.begin() + mx_doff[u], drop.begin() + mx_doff[u + 1], (unsigned char)0);
-                for (int64_t j = mx_doff[u]; j < far_end[u]; j++) {
-                    if (rev[j] < 0) continue;
-                    const int B = far[j];
-                    // both directions leave the lists; only this shard's pairs are gathered
-                    drop[mx_doff[u] + fent[j]] = 1;
-                    if (!(A < B ? owned[u] : owned[unit_of[B]])) continue;
-                    if (A < B) {
-                        sym_in_slot[w++] = sym_slot[pid[j]];
-                        continue;
-                    }
-                    for (int k = 0; k < bt::sym_parts(S.numpar[B]); k++)
-                        sym_in_slot[w++] = sym_slot[pid[rev[j]]] + S.numpar[B] + (int64_t)k * S.numpar[A];
-                }
-            }
-            pt.mark("plan: symmetric: pairs and slots");
-            // both directions leave the per-target near-field lists
-            std::vector<int64_t> noff(NU + 1, 0);
-#pragma omp parallel for schedule(static)
-            for (int u = 0; u < NU; u++) {
-                int64_t kept = 0;
-                for (int64_t k = mx_doff[u]; k < mx_doff[u + 1]; k++) kept += !drop[k];
-                noff[u + 1] = kept;
-            }
-            for (int u = 0; u < NU; u++) noff[u + 1] += noff[u];
-            hvec<int> nidx((size_t)noff[NU]);
-            hvec<unsigned char> nflag((size_t)noff[NU]);
-#pragma omp parallel for schedule(static)
-            for (int u = 0; u < NU; u++) {
-                int64_t w = noff[u];
-                for (int64_t k = mx_doff[u]; k < mx_doff[u + 1]; k++)
-                    if (!drop[k]) { nidx[w] = mx_didx[k]; nflag[w] = mx_dflag[k]; w++; }
-            }
-            mx_doff.swap(noff);
-            mx_didx.swap(nidx);
-            mx_dflag.swap(nflag);
-        }
-    }
-    pt.mark("plan: symmetric near-field pairs");
+    // Symmetric near-field pairs (SymPairs): found here, placed once the rest of
+    // the call's device memory is known.
+    SymPairs sym(pl, pt);
+    if ((mixed && sym_ok && max_leaf <= bt::SYM_MAX_LEAF) || sym64)
+        sym.find(sym64, mx_doff, mx_didx, mx_dflag, leaf_count, shape.nshards);
     // Hermite upward pass: particle chunks of every source node
     std::vector<bt::HermChunk> hchunks;
     std::vector<int3> hred;
@@ -1654,36 +1782,6 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     bt::HermChunk *d_hchunks = nullptr;
     int3 *d_hred = nullptr;
     double *d_hpartial = nullptr;
-
-    // The near field of the FP64 kernels: what the symmetric pairs leave, or
-    // the plan's own list.  Entries whose box meets the target leaf's, the
-    // only ones where a source can coincide with a target, carry EV_MEETS.
-    const int64_t *near_off = pl.t_direct.off;
-    const int *near_idx = pl.t_direct.idx;
-    std::vector<int64_t> doff64;
-    hvec<int> didx64;
-    if (!mixed && !ssm) {
-        auto expanded = [&](int u) { return sym_dropped && unit_expanded[u]; };
-        doff64.assign((size_t)T.nleaves + 1, 0);
-        for (int u = 0; u < T.nleaves; u++) {
-            const int64_t *off = expanded(u) ? mx_doff.data() : pl.t_direct.off;
-            doff64[u + 1] = doff64[u] + (off[u + 1] - off[u]);
-        }
-        didx64.resize((size_t)doff64[T.nleaves]);
-#pragma omp parallel for schedule(static)
-        for (int u = 0; u < T.nleaves; u++) {
-            const int t = T.leaves[u];
-            const int *from = expanded(u) ? mx_didx.data() + mx_doff[u] : pl.t_direct.idx + pl.t_direct.off[u];
-            for (int64_t k = doff64[u]; k < doff64[u + 1]; k++) {
-                const int s = from[k - doff64[u]];
-                const bool meets = S.x0[s] <= T.x1[t] && T.x0[t] <= S.x1[s] && S.y0[s] <= T.y1[t] &&
-                                   T.y0[t] <= S.y1[s] && S.z0[s] <= T.z1[t] && T.z0[t] <= S.z1[s];
-                didx64[k] = meets ? s | bt::EV_MEETS : s;
-            }
-        }
-        near_off = doff64.data();
-        near_idx = didx64.data();
-    }
 
     // device layout
     double *d_sx, *d_sy, *d_sz, *d_sq, *d_tx, *d_ty, *d_tz, *d_pot, *d_sgrid, *d_tgrid, *d_slen, *d_tlen, *d_ww;
@@ -1714,7 +1812,10 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     L.add(&d_tibeg, T.n); L.add(&d_tnum, T.n); L.add(&d_tnch, T.n); L.add(&d_tch, 8 * (size_t)T.n);
     L.add(&d_tpar, T.n); L.add(&d_tleaves, T.nleaves); L.add(&d_tlvl, T.lvl_off ? T.lvl_off[T.max_depth] : 0);
     L.add(&d_aoff, pl.t_approx.rows + 1); L.add(&d_aidx, pl.t_approx.off[pl.t_approx.rows]);
-    L.add(&d_doff, pl.t_direct.rows + 1); L.add(&d_didx, near_off[pl.t_direct.rows]);
+    // (with the pairs still in the list: the longest it can be)
+    int64_t near_cap = pl.t_direct.off[pl.t_direct.rows];
+    if (sym64) near_cap = std::max(near_cap, mx_doff[T.nleaves]);
+    L.add(&d_doff, pl.t_direct.rows + 1); L.add(&d_didx, near_cap);
     L.add(&d_ccoff, pl.g_cc.rows + 1); L.add(&d_ccidx, pl.g_cc.off[pl.g_cc.rows]);
     L.add(&d_cpoff, pl.g_cp.rows + 1); L.add(&d_cpidx, pl.g_cp.off[pl.g_cp.rows]);
     L.add(&d_evitems, ev_items.size()); L.add(&d_griditems, grid_items.size()); L.add(&d_l2pitems, l2p_items.size());
@@ -1751,13 +1852,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     int64_t *d_sym_slot = nullptr, *d_sym_in_off = nullptr, *d_sym_in_slot = nullptr;
     float *d_sym_partial = nullptr;
     double *d_sbox = nullptr;
-    double *d_sym_partial64 = nullptr;
-    if (!sym_pairs.empty()) {
-        L.add(&d_sym_blocks, sym_blocks.size());
-        L.add(&d_sym_pairs, sym_pairs.size()); L.add(&d_sym_slot, sym_slot.size());
-        L.add(&d_sym_in_off, sym_in_off.size()); L.add(&d_sym_in_slot, sym_in_slot.size());
-        if (!mixed) W.add(&d_sym_partial64, (size_t)sym_total);
-    }
+    double *d_sym_partial64 = nullptr, *d_sym_run = nullptr;
     if (mixed) {
         W.add(&d_spos, ns); W.add(&d_tpos, nt);
         if (need_src_clusters) W.add(&d_Q32, (size_t)S.n * P * nq);
@@ -1766,8 +1861,6 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         L.add(&d_mxcpoff, mx_cpoff.size()); L.add(&d_mxcpidx, mx_cpidx.size());
         if (pl.a_deg) L.add(&d_adeg, n_approx);
         L.add(&d_srad, S.n); L.add(&d_trad, T.n);
-        if ((int64_t)sym_blocks.size() > sym_far_blocks) L.add(&d_sbox, 6 * (size_t)S.n);
-        if (!sym_pairs.empty()) W.add(&d_sym_partial, (size_t)sym_total);
         for (size_t i = 0; i < xdeg.size(); i++) {
             size_t Pd = (size_t)(xdeg[i] + 1) * (xdeg[i] + 1) * (xdeg[i] + 1);
             L.add(&d_xgrid[i], xgrid[i].size());
@@ -1778,26 +1871,109 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         }
     }
 
-    L.reqs.insert(L.reqs.end(), W.reqs.begin(), W.reqs.end());
-
     // Segment sums of the evaluation kernels, where their work items are
     // few (the results are the same without them): up to EV_SEGS doubles per
     // target, or per grid point within a fixed bound.
     double *d_evpart = nullptr, *d_gridpart = nullptr;
+    size_t ev_doubles = 0, grid_doubles = 0;
+    if (mixed ? bt::mixed_split(ev_items.size()) : bt::eval64_split(ev_items.size())) ev_doubles = (size_t)bt::EV_SEGS * nt;
+    if (!mixed && !ssm && need_tgt_grids && !herm && bt::eval64_split(grid_items.size()))
+        grid_doubles = (size_t)bt::EV_SEGS * T.n * P;
+    constexpr size_t SEG_BYTES = (size_t)1 << 30;
+    if (sizeof(double) * ev_doubles > SEG_BYTES) ev_doubles = 0;
+    if (sizeof(double) * (ev_doubles + grid_doubles) > SEG_BYTES) grid_doubles = 0;
+
+    // The device memory this call may use: the static scratch, or what the
+    // arena holds, or (asked for only where it has to grow) what is free.
+    const size_t rest = L.total() + W.total();
+    size_t room = arena.cap, grow = 0;
     {
-        const size_t room = arena.fixed ? (arena.cap > L.total() ? arena.cap - L.total() : 0) : (size_t)1 << 30;
-        size_t need = 0;
-        auto want = [&](double **p, size_t count) {
-            if (need + sizeof(double) * count + 512 > room) return;
-            need += sizeof(double) * count + 512;
-            L.add(p, count);
-        };
-        if (mixed ? bt::mixed_split(ev_items.size()) : bt::eval64_split(ev_items.size())) want(&d_evpart, (size_t)bt::EV_SEGS * nt);
-        if (!mixed && !ssm && need_tgt_grids && !herm && bt::eval64_split(grid_items.size()))
-            want(&d_gridpart, (size_t)bt::EV_SEGS * T.n * P);
+        const size_t slice = mixed ? sizeof(float) : sizeof(double);
+        size_t want = rest + sizeof(double) * (ev_doubles + grid_doubles) + 4 * 256;
+        if (sym.npaired > 0) want += sym.bytes(1) + std::min((size_t)sym.total * slice, SYM_SLICE_BYTES);
+        if (!arena.fixed && want > arena.cap) {
+            size_t free_bytes = 0, all_bytes = 0;
+            if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess) {
+                cudaGetLastError();
+                free_bytes = 0;
+            }
+            room = arena.cap + free_bytes - std::min(free_bytes, (size_t)256 << 20);
+        }
+        if (!arena.fixed && want <= room) grow = want;
+        // Slices within SYM_SLICE_BYTES and the room, in as few rounds as that
+        // gives; the pass is left out where its lists do not fit besides the
+        // rest.  Shards of one system have to decide alike, so they always
+        // take the pairs.
+        if (sym.npaired > 0) {
+            int64_t values = -1;
+            for (int guess = 1;;) {
+                const size_t fix = rest + sym.bytes(guess);
+                if (fix >= room) break;
+                const int64_t fits = (int64_t)(std::min(room - fix, SYM_SLICE_BYTES) / slice);
+                const int nr = sym.divide(fits, nullptr);
+                if (nr < 0) break;
+                if (nr <= guess) {
+                    values = fits;
+                    break;
+                }
+                guess = nr;
+            }
+            if (values < 0 && shape.nshards > 1) values = std::max<int64_t>(sym.max_size, 1);
+            if (values >= 0) sym.place(values, mx_doff, mx_didx, mx_dflag);
+        }
+        pt.mark("plan: symmetric near-field pairs");
     }
 
-    if (!arena.reserve(L.total())) {
+    // The near field of the FP64 kernels: what the symmetric pairs leave, or
+    // the plan's own list.  Entries whose box meets the target leaf's, the
+    // only ones where a source can coincide with a target, carry EV_MEETS.
+    const int64_t *near_off = pl.t_direct.off;
+    const int *near_idx = pl.t_direct.idx;
+    std::vector<int64_t> doff64;
+    hvec<int> didx64;
+    if (!mixed && !ssm) {
+        auto expanded = [&](int u) { return sym.taken && sym.unit_expanded[u]; };
+        doff64.assign((size_t)T.nleaves + 1, 0);
+        for (int u = 0; u < T.nleaves; u++) {
+            const int64_t *off = expanded(u) ? mx_doff.data() : pl.t_direct.off;
+            doff64[u + 1] = doff64[u] + (off[u + 1] - off[u]);
+        }
+        didx64.resize((size_t)doff64[T.nleaves]);
+#pragma omp parallel for schedule(static)
+        for (int u = 0; u < T.nleaves; u++) {
+            const int t = T.leaves[u];
+            const int *from = expanded(u) ? mx_didx.data() + mx_doff[u] : pl.t_direct.idx + pl.t_direct.off[u];
+            for (int64_t k = doff64[u]; k < doff64[u + 1]; k++) {
+                const int s = from[k - doff64[u]];
+                const bool meets = S.x0[s] <= T.x1[t] && T.x0[t] <= S.x1[s] && S.y0[s] <= T.y1[t] &&
+                                   T.y0[t] <= S.y1[s] && S.z0[s] <= T.z1[t] && T.z0[t] <= S.z1[s];
+                didx64[k] = meets ? s | bt::EV_MEETS : s;
+            }
+        }
+        near_off = doff64.data();
+        near_idx = didx64.data();
+    }
+
+    L.resize(&d_didx, near_off[pl.t_direct.rows]);
+    if (!sym.pairs.empty()) {
+        L.add(&d_sym_blocks, sym.blocks.size());
+        L.add(&d_sym_pairs, sym.pairs.size()); L.add(&d_sym_slot, sym.slot.size());
+        L.add(&d_sym_in_off, sym.in_off.size()); L.add(&d_sym_in_slot, sym.in_slot.size());
+        if (mixed) L.add(&d_sbox, 6 * (size_t)S.n);
+        if (mixed) W.add(&d_sym_partial, (size_t)sym.round_values);
+        else W.add(&d_sym_partial64, (size_t)sym.round_values);
+        if (sym.rounds.size() > 1) W.add(&d_sym_run, nt);
+    }
+    L.reqs.insert(L.reqs.end(), W.reqs.begin(), W.reqs.end());
+    {
+        auto want = [&](double **p, size_t count) {
+            if (count > 0 && L.total() + sizeof(double) * count + 512 <= room) L.add(p, count);
+        };
+        want(&d_evpart, ev_doubles);
+        want(&d_gridpart, grid_doubles);
+    }
+
+    if (!arena.reserve(std::max(L.total(), grow))) {
         if (arena.fixed) {
             set_err("this call needs %zu bytes of device scratch; the static scratch holds %zu", L.total(), arena.cap);
             return BT_ERR_PARAM;
@@ -1838,10 +2014,10 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         UP(d_griditems, grid_items.data(), grid_items.size());
         UP(d_l2pitems, l2p_items.data(), l2p_items.size());
         if (ssm && !dp) UP(d_sordh, pl.src.order, ns);
-        if (!sym_pairs.empty()) {
-            UP(d_sym_blocks, sym_blocks.data(), sym_blocks.size());
-            UP(d_sym_pairs, sym_pairs.data(), sym_pairs.size()); UP(d_sym_slot, sym_slot.data(), sym_slot.size());
-            UP(d_sym_in_off, sym_in_off.data(), sym_in_off.size()); UP(d_sym_in_slot, sym_in_slot.data(), sym_in_slot.size());
+        if (!sym.pairs.empty()) {
+            UP(d_sym_blocks, sym.blocks.data(), sym.blocks.size());
+            UP(d_sym_pairs, sym.pairs.data(), sym.pairs.size()); UP(d_sym_slot, sym.slot.data(), sym.slot.size());
+            UP(d_sym_in_off, sym.in_off.data(), sym.in_off.size()); UP(d_sym_in_slot, sym.in_slot.data(), sym.in_slot.size());
         }
         if (mixed) {
             UP(d_sctr, sctr.data(), sctr.size()); UP(d_tctr, tctr.data(), tctr.size());
@@ -1886,9 +2062,9 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         v.sharded = shape.nshards > 1;
         v.d_evpart = d_evpart; v.d_gridpart = d_gridpart;
         v.base_full = pl.a_deg == nullptr;
-        v.sym_nblocks = (int)sym_blocks.size();
-        v.sym_far_blocks = (int)sym_far_blocks;
+        if (!sym.pairs.empty()) v.sym_rounds = sym.rounds;
         v.d_sym_blocks = d_sym_blocks;
+        v.d_sym_run = d_sym_run;
         v.d_sbox = d_sbox;
         v.d_sym_pairs = d_sym_pairs; v.d_sym_slot = d_sym_slot; v.d_sym_in_off = d_sym_in_off;
         v.d_sym_in_slot = d_sym_in_slot; v.d_sym_partial = d_sym_partial; v.d_sym_partial64 = d_sym_partial64;
@@ -1997,7 +2173,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             rep->ms_eval_kernel = c;
             rep->kernel_launches = (int)launches;
             long long symw = 0;
-            for (const int2 &pr : sym_pairs) symw += 2LL * S.numpar[pr.x] * S.numpar[pr.y];
+            for (const int2 &pr : sym.pairs) symw += 2LL * S.numpar[pr.x] * S.numpar[pr.y];
             rep->sym_ptwise = symw;
             rep->source_nodes = S.n;
             rep->target_nodes = T.n;

@@ -307,15 +307,18 @@ __global__ void __launch_bounds__(SY_THREADS, BT_SYM_MIN_BLOCKS) k_pp_sym(const 
 
 // One block per leaf and GATHER_THREADS of its particles; the slices' offsets
 // go through shared memory, so that a thread's loads do not wait for them.
+// With several rounds the sum goes on from the round before and reaches the
+// potential in the last one: the same additions in the same order as in one.
 __global__ void __launch_bounds__(GATHER_THREADS) k_sym_gather(SymGatherArgs a)
 {
     __shared__ int64_t slot[GATHER_THREADS];
     const int u = blockIdx.x;
-    const int64_t k0 = a.in_off[u], k1 = a.in_off[u + 1];
+    const int64_t *off = a.in_off + u;
+    const int64_t k0 = off[(size_t)a.round * a.nleaves], k1 = off[(size_t)(a.round + 1) * a.nleaves];
     const int node = a.leaf_node[u];
     const int nb = a.numpar[node], j = blockIdx.y * GATHER_THREADS + threadIdx.x;
-    if (k0 == k1 || (int)blockIdx.y * GATHER_THREADS >= nb) return;
-    double s = 0.0;
+    if ((int)blockIdx.y * GATHER_THREADS >= nb || off[0] == off[(size_t)a.nrounds * a.nleaves]) return;
+    double s = a.round > 0 && j < nb ? a.run[a.ibeg[node] + j] : 0.0;
     for (int64_t b = k0; b < k1; b += GATHER_THREADS) {
         const int m = (int)min((int64_t)GATHER_THREADS, k1 - b);
         __syncthreads();
@@ -325,7 +328,9 @@ __global__ void __launch_bounds__(GATHER_THREADS) k_sym_gather(SymGatherArgs a)
 #pragma unroll 8
             for (int k = 0; k < m; k++) s += (double)a.partial[slot[k] + j];
     }
-    if (j < nb) a.pot[a.ibeg[node] + j] += s;
+    if (j >= nb) return;
+    if (a.round + 1 < a.nrounds) a.run[a.ibeg[node] + j] = s;
+    else a.pot[a.ibeg[node] + j] += s;
 }
 
 }  // namespace

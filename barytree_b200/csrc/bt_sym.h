@@ -47,10 +47,14 @@ struct SymGatherArgs {
     int nleaves;
     const int *leaf_node;
     const int *ibeg, *numpar;
-    const int64_t *in_off;        // per unit: partial vectors addressed to it, in pair order
+    // partial vectors addressed to each unit, in pair order: those of round r
+    // in_off[r * nleaves + unit] .. in_off[(r + 1) * nleaves + unit]
+    const int64_t *in_off;
     const int64_t *in_slot;
     const float *partial;
-    double *pot;                  // += the sum of the partial vectors, FP64, in that order
+    double *pot;                  // += the sum of all rounds' partial vectors, FP64, in that order
+    double *run = nullptr;        // the sum so far, between rounds (several rounds only)
+    int round = 0, nrounds = 1;
 };
 
 // Pairs whose leaf boxes are farther apart than the close-pair distance.
@@ -78,7 +82,8 @@ struct SymGather64Args {
     const int *ibeg, *numpar;
     const int64_t *in_off, *in_slot;
     const double *partial;
-    double *pot;
+    double *pot, *run = nullptr;
+    int round = 0, nrounds = 1;
 };
 
 void launch_pp_sym64(int kernel, const Sym64Args &a, cudaStream_t st);

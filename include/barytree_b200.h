@@ -268,7 +268,10 @@ int bt_tuning_get(int device, int kernel, int approximation, bt_tuning *tuning, 
  *
  * Arguments are those of bt_eval, except that all seven input arrays and
  * outputArray are DEVICE pointers (FP64) on `device`, and precision is a
- * BT_PRECISION_* value.  The result equals bt_eval with inputs_on_device.
+ * BT_PRECISION_* value.  The result equals bt_eval with
+ * inputs_on_device (the symmetric pass runs in as many rounds as its slices
+ * need in the room that is left; where not even its lists fit, every
+ * direction is evaluated separately and the result agrees to rounding).
  * A call whose scratch need exceeds the static array returns BT_ERR_PARAM
  * with a message giving both sizes (roughly up to 5e5 particles at degree 8).
  * The first call on a device looks up the array's device address

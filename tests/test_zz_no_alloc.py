@@ -131,6 +131,29 @@ def test_noalloc_mixed_symmetric_pass_matches_regular_entry_point():
     assert np.array_equal(outs[0], outs[1])      # deterministic in the shared array
 
 
+# Symmetric pairs whose slices are near or above what the static array holds
+# (mixed: about 58 and 77 MB; FP64 twice that), and one far below.
+@pytest.mark.parametrize("precision", [B.PRECISION_MIXED, B.PRECISION_FP64])
+@pytest.mark.parametrize("n,leaf,theta", [(44000, 800, 0.7), (120000, 2000, 0.5), (128000, 2048, 0.4)])
+def test_noalloc_symmetric_pass_in_bounded_scratch(precision, n, leaf, theta):
+    """The pairs' slices take what room there is, in several rounds where it
+    is small: the call is not refused for them and keeps bt_eval's bits."""
+    torch = pytest.importorskip("torch")
+    f = _noalloc_fn()
+    p = dict(_params(1), theta=theta, ls=leaf, lt=leaf)
+    d = _device_arrays(torch, uniform_inputs(104, n, "same"))
+    ref = torch.empty(n, dtype=torch.float64, device="cuda")
+    rep = _call_regular(d, ref, p, precision)
+    assert rep["sym_ptwise"] > 0
+    for _ in range(2):
+        out = torch.full((n,), 7.0, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        rc = _call_noalloc(f, d, out, p, precision)
+        assert rc == B.BT_OK, B.last_error()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+
+
 def test_noalloc_rejects_too_large():
     torch = pytest.importorskip("torch")
     f = _noalloc_fn()
