@@ -1275,11 +1275,15 @@ struct SymPairs {
     int64_t round_values = 0;           // values of the largest round's slices
 
     SymPairs(const bt_plan &p, PhaseTimer &t) : pl(p), pt(t) {}
-    // a pair belongs to the shard that owns its head (the lower leaf): that
-    // shard evaluates it and gathers both sides, the partner's side into
-    // targets another shard owns (the combining sum adds them)
-    bool evaluated(int head, int) const { return owned[head]; }
-    bool gathered(int, int head) const { return owned[head]; }
+    // Mixed shards: a pair belongs to the shard that owns its head (the lower
+    // leaf), which evaluates it and gathers both sides, the partner's side
+    // into targets another shard owns (the combining sum adds them).  FP64
+    // shards evaluate every pair that touches a leaf of theirs (13 FP64
+    // instructions for the two directions, 12 for the one that counts) and
+    // gather their own leaves, so that each potential is formed whole by one
+    // shard and the sum of the shards has the unsharded call's bits.
+    bool evaluated(int head, int partner) const { return owned[head] || (fp64 && owned[partner]); }
+    bool gathered(int unit, int head) const { return owned[fp64 ? unit : head]; }
     // values of the slices of pair {A, B}: A's once, B's per part of A
     int64_t pair_values(int A, int B) const
     {
@@ -1736,11 +1740,10 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     for (int u = 0; u < T.nleaves; u++) max_leaf = std::max(max_leaf, T.numpar[T.leaves[u]]);
     // targets that are the sources, and a kernel that is symmetric in r: the
     // symmetric near-field pass.  FP64 takes it pair by pair (leaves of
-    // SYM64_MIN_LEAF to SYM_MAX_LEAF particles); a shard in FP64 evaluates
-    // all of its targets' potentials itself.
+    // SYM64_MIN_LEAF to SYM_MAX_LEAF particles).
     const bool sym_kernel = shape.sym && T.nleaves > 1 && o.kernel >= COULOMB && o.kernel <= REGULARIZED_COULOMB;
     const bool sym_ok = pl.same_tree && sym_kernel;
-    const bool sym64 = (pl.same_tree || pl.sys_same) && sym_kernel && !mixed && !ssm && shape.nshards == 1 &&
+    const bool sym64 = (pl.same_tree || pl.sys_same) && sym_kernel && !mixed && !ssm &&
                        max_leaf >= bt::SYM64_MIN_LEAF;
     if (mixed || sym64) {
         std::vector<int> lf, lc;
@@ -2172,8 +2175,12 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
             rep->ms_downward = d;
             rep->ms_eval_kernel = c;
             rep->kernel_launches = (int)launches;
+            // a direction counts where it is used
             long long symw = 0;
-            for (const int2 &pr : sym.pairs) symw += 2LL * S.numpar[pr.x] * S.numpar[pr.y];
+            for (const int2 &pr : sym.pairs) {
+                const int ua = sym.unit_of[pr.x], ub = sym.unit_of[pr.y];
+                symw += (long long)(sym.gathered(ua, ua) + sym.gathered(ub, ua)) * S.numpar[pr.x] * S.numpar[pr.y];
+            }
             rep->sym_ptwise = symw;
             rep->source_nodes = S.n;
             rep->target_nodes = T.n;

@@ -106,25 +106,27 @@ typedef struct bt_options {
     /* Target sharding: with shard_count > 1 the call evaluates shard_index's
      * share of the target leaves (contiguous in tree order, equal estimated
      * cost) and leaves the other potentials 0; the sum of the outputs of all
-     * shards is the unsharded result, bit for bit without the symmetric
-     * pass.  With it, a pair of near-field leaves belongs to the shard that
-     * owns its lower leaf, which also adds the partner's side into targets
-     * another shard owns; the sum then agrees with the unsharded result to
-     * FP64 rounding (the slice sums are grouped by shard).  FP64 shards run
-     * without the symmetric pass.  Trees, lists and proxies
+     * shards is the unsharded result, bit for bit in FP64 and without the
+     * symmetric pass.  With it, in the mixed path, a pair of near-field leaves
+     * belongs to the shard that owns its lower leaf, which also adds the
+     * partner's side into targets another shard owns; the sum then agrees
+     * with the unsharded result to FP64 rounding (the slice sums are grouped
+     * by shard).  FP64 shards evaluate every pair that touches one of their
+     * leaves and keep their own leaves' side.  Trees, lists and proxies
      * are built in full by every shard; with target grids (cluster-particle,
      * cluster-cluster) a shard evaluates the grids of its leaves and their
      * ancestors only, so the grids of shared ancestors are evaluated by
      * every shard that holds a leaf under them.                            */
     int shard_index;
     int shard_count;
-    int symmetry;         /* targets = sources (all of a batch's systems), Coulomb, Yukawa or
-                             regularized Coulomb: BT_SYMMETRY_AUTO (default) evaluates each
-                             pair of near-field leaves that list each other once for both
-                             sides (mixed: leaves of at most 2048 particles throughout the
-                             call; FP64: pairs of leaves of 512 to 2048 particles, unsharded
-                             calls); BT_SYMMETRY_OFF evaluates every direction separately.
-                             Results agree to rounding and are deterministic.  */
+    int symmetry;         /* targets = sources, Coulomb, Yukawa or regularized Coulomb:
+                             BT_SYMMETRY_AUTO (default) evaluates each pair of near-field
+                             leaves that list each other once for both sides (mixed: all of
+                             a batch's systems their own targets and leaves of at most 2048
+                             particles throughout the call; FP64: system by system, pairs
+                             of leaves of 512 to 2048 particles); BT_SYMMETRY_OFF evaluates
+                             every direction separately.  Results agree to rounding and are
+                             deterministic.  */
 } bt_options;
 
 enum { BT_TREE_GPU = 0, BT_TREE_HOST = 1 };

@@ -71,6 +71,25 @@ def test_sharded_learned_degrees_and_sessions():
     assert np.array_equal(sparts[0], parts[0]) and np.array_equal(sparts[1], parts[1])
 
 
+@pytest.mark.parametrize("ctype", [B.ComputeType.PARTICLE_CLUSTER, B.ComputeType.CLUSTER_CLUSTER])
+@pytest.mark.parametrize("nshards", [2, 3])
+def test_fp64_shards_of_the_symmetric_pass_sum_bit_for_bit(ctype, nshards):
+    """FP64 shards evaluate every pair that touches one of their leaves and
+    gather their own leaves' sides only: the default unsharded result, bit for
+    bit, every target from one shard."""
+    x, y, z, q = _clustered(60000, 37)
+    kw = dict(compute_type=ctype, kernel=B.Kernel.YUKAWA, kernel_param=0.5, theta=0.8, degree=6,
+              max_source_leaf=1500, max_target_leaf=1500)
+    full, rep = B.treecode(x, y, z, x, y, z, q, return_report=True, **kw)
+    assert rep["sym_ptwise"] > 0
+    parts, reps = zip(*[B.treecode(x, y, z, x, y, z, q, shard=(k, nshards), return_report=True, **kw)
+                        for k in range(nshards)])
+    assert np.array_equal(np.sum(parts, axis=0), full)
+    assert np.all(np.sum([p != 0 for p in parts], axis=0) == 1)
+    assert all(r["sym_ptwise"] > 0 for r in reps)
+    assert sum(r["sym_ptwise"] for r in reps) == rep["sym_ptwise"]     # a direction is counted where it is used
+
+
 def test_one_shard_is_the_unsharded_call():
     tx, ty, tz, sx, sy, sz, sq = uniform_inputs(33, 50000)
     kw = dict(theta=0.7, degree=5, max_source_leaf=400, max_target_leaf=400, precision=B.PRECISION_MIXED)
