@@ -8,9 +8,10 @@
 //
 // What is left of the issue slots decides how much of that rate is reached, so
 // every thread evaluates two outputs against each value it reads from shared
-// memory, the near-field tiles are padded to the unrolled loop with sources of
-// no charge, and the skipping rule is tested only for source nodes whose box
-// meets the target leaf's.
+// memory, the near-field tiles are padded to the unrolled loop with their first
+// source without its charge (finite values wherever that source's are), and the
+// skipping rule is tested only for source nodes whose box meets the target
+// leaf's.
 //
 // A work item is a chunk of up to EV_CHUNK outputs (targets of a leaf, or
 // points of a target grid) and its block's threads are `lanes` pairs of
@@ -41,7 +42,7 @@ constexpr int EV_TILE = 512;        // sources per shared-memory tile
 struct Kern64 {
     double kp, kp2, eps2;
     Exp64 ex;
-    bool lib;               // Yukawa with kappa < 0 (or NaN): the library functions throughout
+    bool lib;               // Yukawa with a kappa that exp64 does not take: the library functions throughout
 };
 
 template <int KT>
@@ -53,7 +54,7 @@ __device__ __forceinline__ Kern64 kern64_make(double kp, double kp2, double2 *ta
     Kern64 k;
     k.kp = kp; k.kp2 = kp2;
     k.eps2 = KT == K_REGCOULOMB ? kp * kp : 0.0;
-    k.lib = KT == K_YUKAWA && !(kp >= 0.0);
+    k.lib = KT == K_YUKAWA && !exp64_takes(kp);
     if (KT == K_YUKAWA) {
         for (int i = threadIdx.x; i < EXP64_TAB; i += blockDim.x) tab[i] = exp64_table[i];
         k.ex = exp64_make(kp, tab);
@@ -228,9 +229,6 @@ struct Tile64 {
     double2 *xy, *zq;
 };
 
-// Padding sources: far away, no charge (r^2 about 1e300, a normal number).
-constexpr double PAD64 = 1.0e150;
-
 // Sources i0, i0 + step, ... < cm of a tile, the range a multiple of 4 * step
 // long.  TEST: with the skipping rule, else mn gets the smallest upper half of
 // the thread's r^2 (as an integer: r^2 is never negative).
@@ -300,9 +298,9 @@ __device__ __forceinline__ void near64_node(double *acc, const Tile64 &t, int sb
         const int cm = min(EV_TILE, sn - c0);
         const int pad = 4 * w.slices, cmp = fast64<KT>() ? (cm + pad - 1) & ~(pad - 1) : cm;   // EV_TILE is a multiple
         for (int i = threadIdx.x; i < cmp; i += EV_THREADS) {
-            const int j = sb + c0 + i;
-            t.xy[i] = i < cm ? make_double2(sx[j], sy[j]) : make_double2(PAD64, PAD64);
-            t.zq[i] = i < cm ? make_double2(sz[j], sq[j]) : make_double2(PAD64, 0.0);
+            const int j = sb + c0 + (i < cm ? i : 0);
+            t.xy[i] = make_double2(sx[j], sy[j]);
+            t.zq[i] = make_double2(sz[j], i < cm ? sq[j] : 0.0);
         }
         __syncthreads();
         if (w.active[0]) {

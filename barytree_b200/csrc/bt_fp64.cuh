@@ -87,25 +87,29 @@ __constant__ const double2 exp64_table[EXP64_TAB] = {      // {2^(j/64) rounded,
 
 struct Exp64 {
     double chi, clo;        // -kappa * 64 / ln2 in two parts
-    int rmax;               // upper half of the r where exp is 2^-1101
+    int rmax;               // upper half of the r where exp is 2^-1101 (kappa < 0: 2^1024.5)
     const double2 *tab;     // the table in shared memory
 };
 
-// kappa >= 0
+// |kappa| < 1e300 (a NaN or more than that: the library functions).
+__device__ __forceinline__ bool exp64_takes(double kappa) { return fabs(kappa) < 1.0e300; }
 __device__ __forceinline__ Exp64 exp64_make(double kappa, const double2 *tab)
 {
     constexpr double hi = 92.33248261689366, lo = 1.3027375194195861e-15;     // 64 / ln2
     Exp64 c;
     c.chi = -kappa * hi;
     c.clo = fma(-kappa, hi, -c.chi) - kappa * lo;
-    c.rmax = __double2hiint(1101.0 * 0.6931471805599453 / kappa);             // kappa 0: infinity
+    // kappa 0: infinity
+    c.rmax = __double2hiint((kappa < 0.0 ? 1024.5 : 1101.0) * 0.6931471805599453 / fabs(kappa));
     c.tab = tab;
     return c;
 }
 
 // r >= 0 (a NaN may give any value).  No branch, so that the compiler can
 // interleave several values: r is cut off where exp is below every normal
-// number, and a result below 2^-1021 is replaced by one below 2^-1021.
+// number, and a result below 2^-1021 is replaced by one below 2^-1021.  A
+// growing exponential (kappa < 0) is cut off within [2^1024, 2^1025), whose
+// exponent field is that of infinities and NaNs, so an overflow is not finite.
 __device__ __forceinline__ double exp64(double r, const Exp64 &c)
 {
     constexpr double magic = 6755399441055744.0;            // 1.5 * 2^52

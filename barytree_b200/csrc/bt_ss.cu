@@ -129,7 +129,7 @@ __device__ __forceinline__ void ss_grid(double dx, double dy, double dz, double 
 struct SsKern {
     double eps2;
     Exp64 ex;
-    bool lib;               // parameters outside exp64's range
+    bool lib;               // parameters that exp64 does not take
 };
 
 template <int KT>
@@ -138,7 +138,7 @@ __device__ __forceinline__ SsKern ss_kern(double kp, double kp2, double2 *tab)
     SsKern k;
     k.eps2 = KT == K_REGCOULOMB || KT == K_REGYUKAWA ? kp2 * kp2 : 0.0;
     const double kappa = KT == K_YUKAWA || KT == K_REGYUKAWA ? kp : 1.0 / (kp * kp);
-    k.lib = !(kappa >= 0.0 && kappa < 1.0e300);
+    k.lib = !exp64_takes(kappa);
     for (int i = threadIdx.x; i < EXP64_TAB; i += blockDim.x) tab[i] = exp64_table[i];
     k.ex = exp64_make(kappa, tab);
     return k;

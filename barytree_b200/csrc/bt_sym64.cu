@@ -84,9 +84,9 @@ __global__ void __launch_bounds__(S64_THREADS, BT_S64_MINB) k_pp_sym64(const __g
         const int cm = min(S64_TILE, nb - s0), groups = (cm + S64_SB - 1) / S64_SB;
         __syncthreads();                             // the previous tile is done with
         for (int i = threadIdx.x; i < groups * S64_SB; i += S64_THREADS) {
-            const int j = ib + s0 + i;
-            xy[i] = i < cm ? make_double2(a.x[j], a.y[j]) : make_double2(PAD64, PAD64);
-            zq[i] = i < cm ? make_double2(a.z[j], a.q[j]) : make_double2(PAD64, 0.0);
+            const int j = ib + s0 + (i < cm ? i : 0);
+            xy[i] = make_double2(a.x[j], a.y[j]);
+            zq[i] = make_double2(a.z[j], i < cm ? a.q[j] : 0.0);
         }
         __syncthreads();
         const int b0 = groups * warp / S64_WARPS * S64_SB, b1 = groups * (warp + 1) / S64_WARPS * S64_SB;

@@ -83,6 +83,27 @@ def test_few_items_and_many_items_give_the_same_bits(approx):
     assert np.array_equal(B.treecode_batch([sys_of(one), sys_of(big)], **kw)[0], alone)
 
 
+def test_growing_exponential_takes_the_short_forms():
+    """kappa < 0: the same kernels and pairs as a decaying one, at about their
+    time (the library's exp in every sum took four times as long)."""
+    x, y, z, q = _cube(5, 60000)
+    kw = dict(kernel=2, degree=6, theta=0.7, max_source_leaf=1000, max_target_leaf=1000)
+    ms = {}
+    for kp in (0.5, -0.5):
+        best = []
+        for _ in range(4):
+            _, rep = B.treecode(x, y, z, x, y, z, q, kernel_param=kp, return_report=True, **kw)
+            assert rep["sym_ptwise"] > 0
+            best.append(rep["ms_eval_kernel"])
+        ms[kp] = min(best[1:])
+    assert ms[-0.5] <= 2.0 * ms[0.5], ms
+    near = dict(kw, theta=1e-9, max_source_leaf=800, max_target_leaf=800)      # every pair of leaves direct
+    p = [a[:6000] for a in (x, y, z, q)]
+    got, rep = B.treecode(*p[:3], *p, kernel_param=-0.5, return_report=True, **near)
+    assert rep["sym_ptwise"] > 0
+    assert _rel(got, _direct(p[:3], p[:3], p[3], 2, -0.5)) <= TOL
+
+
 @pytest.mark.parametrize("kernel,kp,scale", [(1, 0.0, 1e160), (1, 0.0, 1e-160), (3, 0.0, 1e-160), (2, -0.4, 1.0),
                                               (2, 900.0, 1.0), (2, 0.0, 1.0), (2, 1e-3, 1e160)])
 def test_arguments_outside_the_short_forms(kernel, kp, scale):
