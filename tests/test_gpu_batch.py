@@ -83,6 +83,28 @@ def test_mixed_hermite_cluster_particle_batch_equals_separate_calls():
     assert np.array_equal(pots[0], B.treecode(*own, **kw))
 
 
+def test_fp64_batch_on_device_arrays_equals_separate_calls():
+    """The per-system comparison of targets and sources on the device."""
+    torch = pytest.importorskip("torch")
+    _, pairs, own = _kinds()
+    shifted = tuple(a.copy() for a in pairs)
+    shifted[2][-1] = np.nextafter(shifted[2][-1], 2.0)      # one target apart from its source by a bit
+    systems = [own, pairs, shifted]
+    kw = dict(kernel=1, compute_type=1, degree=5, theta=0.7, max_source_leaf=600, max_target_leaf=600)
+    d = [torch.from_numpy(np.concatenate([s[k] for s in systems])).cuda() for k in range(7)]
+    out = torch.empty_like(d[0])
+    torch.cuda.synchronize()
+    off = np.concatenate([[0], np.cumsum([len(s[0]) for s in systems])]).astype(np.int64)
+    rep = B.treecode_batch_ptr(len(systems), off, off, *[a.data_ptr() for a in d], out.data_ptr(),
+                               inputs_on_device=True, **kw)
+    got = np.split(out.cpu().numpy(), off[1:-1])
+    alone, reps = zip(*[B.treecode(*s, return_report=True, **kw) for s in systems])
+    assert [r["sym_ptwise"] > 0 for r in reps] == [False, True, False]
+    assert rep["sym_ptwise"] == reps[1]["sym_ptwise"]
+    for p, a in zip(got, alone):
+        assert np.array_equal(p, a)
+
+
 def test_batch_host_and_gpu_tree_builds_agree():
     systems = _systems(2, SIZES)
     kw = dict(kernel=1, degree=6, max_source_leaf=200, max_target_leaf=200, precision=B.PRECISION_MIXED)

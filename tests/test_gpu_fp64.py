@@ -105,11 +105,12 @@ def test_growing_exponential_takes_the_short_forms():
 
 
 @pytest.mark.parametrize("kernel,kp,scale", [(1, 0.0, 1e160), (1, 0.0, 1e-160), (3, 0.0, 1e-160), (2, -0.4, 1.0),
-                                              (2, 900.0, 1.0), (2, 0.0, 1.0), (2, 1e-3, 1e160)])
+                                              (2, 900.0, 1.0), (2, 0.0, 1.0), (2, 1e-3, 1e160), (2, -400.0, 1.0)])
 def test_arguments_outside_the_short_forms(kernel, kp, scale):
     """Squares that overflow or underflow, a growing exponential, one that
-    underflows: what the library functions give, term by term."""
-    x, y, z, q = _cube(3, 1500)
+    underflows: what the library functions give, term by term.  Leaves of
+    about 750 particles, so that the pair kernel meets them too."""
+    x, y, z, q = _cube(3, 6000)
     x, y, z = x * scale, y * scale, z * scale
     with np.errstate(all="ignore"):
         d2 = sum((a[:, None] - a[None, :]) ** 2 for a in (x, y, z))
@@ -121,13 +122,83 @@ def test_arguments_outside_the_short_forms(kernel, kp, scale):
         else:
             ref = np.where(d2 > np.finfo(float).tiny, 1.0 / np.sqrt(d2), 0.0) @ q
     got = [B.direct(x, y, z, x, y, z, q, kernel, kp)]
-    kw = dict(kernel=kernel, kernel_param=kp, degree=3, max_source_leaf=400, max_target_leaf=400, theta=1e-9)
-    got.append(B.treecode(x, y, z, x, y, z, q, **kw))                               # near field only, pairs
+    kw = dict(kernel=kernel, kernel_param=kp, degree=3, max_source_leaf=800, max_target_leaf=800, theta=1e-9)
+    pot, rep = B.treecode(x, y, z, x, y, z, q, return_report=True, **kw)            # near field only, pairs
+    assert rep["sym_ptwise"] > 0
+    got.append(pot)
     got.append(B.treecode(x, y, z, x, y, z, q, symmetry=B.SYMMETRY_OFF, **kw))
     for g in got:
         ok = np.isfinite(ref)
         assert np.array_equal(np.isfinite(g), ok)
-        if ok.any() and np.linalg.norm(ref[ok]) > 0:
-            assert _rel(g[ok], ref[ok]) <= 1e-12
+        top = np.max(np.abs(ref[ok]), initial=0.0)            # (the squares of the norm overflow at 1e300)
+        if top > 0:
+            assert _rel(g[ok] / top, ref[ok] / top) <= 1e-12
         else:
             assert np.all(g[ok] == ref[ok])
+
+
+def test_charge_that_is_not_finite_goes_through_the_pairs():
+    """A NaN charge reaches every potential but its own particle's (the pair
+    with itself is skipped), through the pair kernel's second route."""
+    x, y, z, q = _cube(4, 6000)
+    q[1234] = np.nan
+    ref = _direct((x[1234:1235], y[1234:1235], z[1234:1235]), tuple(np.delete(a, 1234) for a in (x, y, z)),
+                  np.delete(q, 1234), 1, 0.0)
+    pot, rep = B.treecode(x, y, z, x, y, z, q, degree=3, max_source_leaf=800, max_target_leaf=800, theta=1e-9,
+                          return_report=True)
+    assert rep["sym_ptwise"] > 0
+    assert np.array_equal(np.flatnonzero(~np.isnan(pot)), [1234])
+    assert abs(pot[1234] - ref[0]) <= TOL * abs(ref[0])
+
+
+# The short forms themselves, one kernel value per target: a unit charge at
+# the origin and targets on the x axis, so that r^2 is r * r rounded once and
+# the sum is the value.  Against extended precision (64 bits of mantissa).
+U = 2.0 ** -53
+
+
+def _values(r, kernel, kp):
+    o = np.zeros(1)
+    return B.direct(r, np.zeros_like(r), np.zeros_like(r), o, o, o, np.ones(1), kernel, kp)
+
+
+def _radii(lo, hi, n):
+    """Both exponent parities, and mantissas spread by an odd step."""
+    return np.exp(np.linspace(np.log(lo), np.log(hi), n))
+
+
+def test_reciprocal_root_to_the_last_place():
+    """rsqrt_n: the estimate's error e leaves (5/16)|e|^3 < 2^-64 after the
+    step, and the last rounding half a unit, at most 2^-53 of the value."""
+    r = np.concatenate([_radii(1e-153, 1e153, 200_001), _radii(0.5, 8.0, 100_001)])
+    r2 = r * r
+    exact = 1.0 / np.sqrt(r2.astype(np.longdouble))
+    assert np.max(np.abs(_values(r, 1, 0.0) - exact) / exact) <= 1.01 * U
+    # eps^2 in the square: one rounding more, halved by the root
+    r = _radii(1e-6, 1e3, 100_001).astype(np.float32).astype(np.float64)      # r * r exact
+    for eps in (1e-3, 2.0):
+        exact = 1.0 / np.sqrt(r.astype(np.longdouble) ** 2 + np.longdouble(eps * eps))
+        assert np.max(np.abs(_values(r, 3, eps) - exact) / exact) <= 1.52 * U
+
+
+@pytest.mark.parametrize("kappa", [0.0, 1e-9, 0.37, 1.0, 64.0, -0.37, -1.0, -64.0])
+def test_exponential_to_the_last_places(kappa):
+    """rsqrt_sqrt_n and exp64 in the Yukawa value: half a unit each for 1/r, for
+    the table entry plus polynomial (truncated below 0.36 of 2^-53) and for the
+    product, and the rounding of r times the exponent; every table entry, down
+    to the cut below 2^-1021 and, growing, up to the overflow."""
+    top = 700.0 / abs(kappa) if kappa else 1e100
+    r = np.concatenate([_radii(1e-12 * top, top, 200_001), np.linspace(0.001, 1.0, 100_001) * min(top, 1e3)])
+    s = np.sqrt((r * r).astype(np.longdouble))
+    exact = np.exp(-np.longdouble(kappa) * s) / s
+    normal = exact >= 2.0 ** -1021                          # (as doubles are rounded to 53 bits)
+    err = np.abs(_values(r, 2, kappa) - exact)[normal] / exact[normal]
+    r = r[normal]
+    assert np.max(err / (3.5 + 1.1 * np.abs(kappa) * r)) <= U
+    if kappa > 0:
+        far = np.linspace(1022.0, 4000.0, 1001) * np.log(2.0) / kappa
+        v = _values(far, 2, kappa) * far
+        assert np.all((v >= 0.0) & (v <= 2.0 ** -1021))
+    if kappa < 0:
+        far = np.linspace(1024.01, 4000.0, 1001) * np.log(2.0) / -kappa
+        assert np.all(np.isposinf(_values(far, 2, kappa)))

@@ -125,3 +125,18 @@ def test_mixed_single_particle_leaves(kernel):
     b = B.treecode(tx, ty, tz, sx, sy, sz, sq, precision=B.PRECISION_FP64, **kw)
     assert np.all(np.isfinite(a))
     assert np.linalg.norm(a - b) / np.linalg.norm(b) <= TOL_VS_FP64_TREE_YUKAWA
+
+
+@pytest.mark.parametrize("approx,ctype,kernel,kp", [(1, 1, 1, 0.0), (2, 1, 3, 1e-3), (1, 3, 2, 0.5)])
+def test_few_items_and_many_items_give_the_same_bits(approx, ctype, kernel, kp):
+    """A system evaluated alone (a block per list segment) and in a batch with
+    more than 3,552 work items (a block per item)."""
+    rng = np.random.default_rng(9)
+    system = lambda n: (*(rng.uniform(-1, 1, n) for _ in range(3)), rng.uniform(-1, 1, n))  # noqa: E731
+    one, big = system(20000), system(300000)
+    kw = dict(kernel=kernel, kernel_param=kp, approximation=approx, compute_type=ctype, degree=3, theta=0.8,
+              max_source_leaf=60, max_target_leaf=60, size_check=1.0 if approx == 1 else 4.0,
+              precision=B.PRECISION_MIXED)
+    sys_of = lambda p: (*p[:3], *(a.copy() for a in p[:3]), p[3])  # noqa: E731
+    alone = B.treecode(*sys_of(one), **kw)
+    assert np.array_equal(B.treecode_batch([sys_of(one), sys_of(big)], **kw)[0], alone)

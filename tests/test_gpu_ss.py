@@ -87,3 +87,55 @@ def test_subtraction_with_unit_weights_and_zero_target_charges_equals_skipping()
     ss = B.callTreedriver(*args, B.Singularity.SUBTRACTION, 1, 1, True, 0, **kw)
     sk = B.callTreedriver(*args, B.Singularity.SKIPPING, 1, 1, True, 0, **kw)
     assert np.linalg.norm(ss - sk) / np.linalg.norm(sk) <= 1e-13
+
+
+# The subtraction kernels' second route (parameters that the short exponential
+# does not take, sums that are not finite) and the direct sum split over its
+# sources: against the pair terms in numpy.
+def _pairs(t, tq, s, q, w, kernel, kp):
+    """sum_j (q_j - tq_i g) w_j K + c tq_i with the library's terms (bt_ss.cu)."""
+    with np.errstate(all="ignore"):
+        r2 = sum((a[:, None] - b[None, :]) ** 2 for a, b in zip(t, s))
+        r = np.sqrt(r2)
+        if kernel in (2, 4):
+            k = np.exp(-kp[0] * r) / (r if kernel == 2 else np.sqrt(r2 + kp[1] ** 2))
+            g, c = np.ones_like(r), 4.0 * np.pi / kp[0] / kp[0]
+        else:
+            k = 1.0 / (r if kernel == 1 else np.sqrt(r2 + kp[1] ** 2))
+            g, c = np.exp(-r2 / (kp[0] * kp[0])), 2.0 * np.pi * kp[0] * kp[0]
+        v = (q - tq[:, None] * g) * w * k
+        if kernel in (1, 2):
+            v[r <= np.finfo(float).tiny] = 0.0
+        return v.sum(axis=1) + c * tq
+
+
+@pytest.mark.parametrize("kernel,kp,scale,other", [
+    (1, [0.7], 1.0, True), (1, [0.0], 1.0, False), (1, [1e-200], 1.0, True), (1, [0.7], 1e160, False),
+    (2, [-0.4], 1.0, False), (2, [1e301], 1.0, True), (2, [0.5], 1e160, True),
+    (3, [0.7, 0.0], 1.0, False), (3, [0.0, 1e-2], 1.0, False), (3, [0.7, 0.0], 1.0, True),
+    (4, [0.5, 0.0], 1.0, False), (4, [0.5, 0.0], 1.0, True), (4, [-0.3, 1e-2], 1.0, False)])
+@pytest.mark.parametrize("nt,ns", [(1500, 1500), (200, 20000)])
+def test_subtraction_outside_the_short_forms(kernel, kp, scale, other, nt, ns):
+    tx, ty, tz, tq, sx, sy, sz, q, w = (a * (scale if i in (0, 1, 2, 4, 5, 6) else 1.0)
+                                        for i, a in enumerate(_inputs(11, ns, other)))
+    t, tq = [a[:nt].copy() for a in (tx, ty, tz)], tq[:nt].copy()
+    ref = _pairs(t, tq, (sx, sy, sz), q, w, kernel, kp)
+    got = [B.direct(*t, sx, sy, sz, q, kernel, kp, singularity=B.Singularity.SUBTRACTION, target_q=tq, source_w=w),
+           B.treecode(*t, sx, sy, sz, q, kernel=kernel, kernel_param=kp, degree=3, theta=1e-9, max_source_leaf=300,
+                      max_target_leaf=300, singularity=B.Singularity.SUBTRACTION, target_q=tq, source_w=w)]
+    ok = np.isfinite(ref)
+    for g in got:
+        assert np.array_equal(np.isfinite(g), ok)
+        assert np.linalg.norm((g - ref)[ok]) <= 1e-12 * np.linalg.norm(ref[ok])
+
+
+@pytest.mark.parametrize("ctype", [1, 2, 3])
+def test_subtraction_with_a_vanishing_factor_is_the_skipping_sum(ctype):
+    """alpha = 0: g = 0 away from r = 0, which the kernels form with the
+    library functions (clusters and grids included): the treecode of q w."""
+    tx, ty, tz, tq, sx, sy, sz, q, w = _inputs(12, 9000, other=True)
+    kw = dict(compute_type=ctype, degree=6, theta=0.8, max_source_leaf=200, max_target_leaf=200)
+    ss = B.treecode(tx, ty, tz, sx, sy, sz, q, kernel=1, kernel_param=[0.0], singularity=B.Singularity.SUBTRACTION,
+                    target_q=tq, source_w=w, **kw)
+    sk = B.treecode(tx, ty, tz, sx, sy, sz, q * w, kernel=1, **kw)
+    assert np.linalg.norm(ss - sk) <= 1e-12 * np.linalg.norm(sk)
