@@ -893,10 +893,10 @@ void launch_l2l(int n, int nparents, const int *parents, const int *nchild, cons
     k_l2l<<<KRON_CHILDREN * nparents, 256, sm, st>>>(n, parents, nchild, child, grid, Phi);
 }
 
-// With fewer items than about four waves of resident blocks (8 blocks of
-// EV_THREADS threads on each of 148 SMs) the last wave is a large part of the
-// whole; a block per segment then gives the scheduler 16 times as many.
-bool eval64_split(size_t items) { return items < (size_t)4 * 8 * 148; }
+// With fewer items than eight waves of resident blocks (EV_MINB = 4 blocks on
+// each of 148 SMs) the last wave is a large part of the whole; a block per
+// segment then gives the scheduler 16 times as many.
+bool eval64_split(size_t items) { return items < (size_t)8 * EV_MINB * 148; }
 
 // Kernels with Hermite forms: Coulomb, Yukawa, regularized Coulomb, sin-over-r.
 void launch_eval_targets(int kernel, bool hermite, const EvalTargetsArgs &a, cudaStream_t st)
@@ -979,12 +979,12 @@ void launch_l2p(int n, bool hermite, int nitems, const int2 *items, const int *l
     }
 }
 
-// Enough parts for about three waves of resident blocks, each of at least one
+// Enough parts for about six waves of resident blocks, each of at least one
 // source tile.
 int direct_parts(int nt, int ns)
 {
     const int blocks = std::max(1, (nt + EV_CHUNK - 1) / EV_CHUNK);
-    return std::max(1, std::min(3 * 8 * 148 / blocks, ns / 512));
+    return std::max(1, std::min(6 * EV_MINB * 148 / blocks, ns / 512));
 }
 
 void launch_direct(int kernel, int nt, int ns, const double *tx, const double *ty, const double *tz,

@@ -30,10 +30,6 @@
 #include "bt_fp64.cuh"
 #include "bt_kernels.cuh"
 
-#ifndef BT_EV_MINB
-#define BT_EV_MINB 4
-#endif
-
 namespace bt {
 
 constexpr int EV_TILE = 512;        // sources per shared-memory tile
@@ -359,7 +355,7 @@ __device__ __forceinline__ void sum_slices(double *acc, double *red, const Lanes
 // Particle outputs: PC (clusters) + PP (particles) onto a chunk of a target
 // leaf.  NP1 = n + 1 (Lagrange with a short form), else 0.
 template <int KT, int NP1, bool HERM>
-__global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB) k_eval_targets(const __grid_constant__ EvalTargetsArgs a)
+__global__ void __launch_bounds__(EV_THREADS, EV_MINB) k_eval_targets(const __grid_constant__ EvalTargetsArgs a)
 {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[2 * EV_THREADS];
@@ -433,7 +429,7 @@ __global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB) k_eval_targets(const _
 // Grid outputs: M2L (clusters, Lagrange) + CP (particles) onto a chunk of a
 // target node's grid points.
 template <int KT, int NP1>
-__global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB) k_eval_grids(const __grid_constant__ EvalGridsArgs a)
+__global__ void __launch_bounds__(EV_THREADS, EV_MINB) k_eval_grids(const __grid_constant__ EvalGridsArgs a)
 {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[2 * EV_THREADS];
@@ -497,7 +493,7 @@ __global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB) k_eval_grids(const __g
 // Direct sum: sources blockIdx.y of gridDim.y parts onto EV_CHUNK targets;
 // several parts go to `out` nt apart and are added by k_sum_parts.
 template <int KT>
-__global__ void __launch_bounds__(EV_THREADS, BT_EV_MINB)
+__global__ void __launch_bounds__(EV_THREADS, EV_MINB)
 k_direct(int nt, int ns, const double *__restrict__ tx, const double *__restrict__ ty, const double *__restrict__ tz,
          const double *__restrict__ sx, const double *__restrict__ sy, const double *__restrict__ sz,
          const double *__restrict__ sq, double kp, double kp2, double *__restrict__ out)

@@ -58,11 +58,7 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v)
 }
 
 constexpr int MX_THREADS = 128;                 // threads of the grid-output kernel
-// Register budget of the grid-output kernel: BT_MX_MIN_BLOCKS resident blocks per SM.
-#ifndef BT_MX_MIN_BLOCKS
-#define BT_MX_MIN_BLOCKS 6
-#endif
-#define BT_MX_BOUNDS __launch_bounds__(MX_THREADS, BT_MX_MIN_BLOCKS)
+constexpr int MX_MIN_BLOCKS = 6;                // its resident blocks per SM (8 measured the same)
 constexpr int MX_TILE = 1024;                   // sources per tile of the grid-output kernel
 // Register budget of the 2-targets-per-thread Lagrange particle-output
 // kernel (Coulomb, regularised Coulomb): room for 6 resident blocks per SM.
@@ -832,7 +828,7 @@ __device__ __forceinline__ void grids_item(const MixedGridsArgs &a, const int2 i
 }
 
 template <int KT>
-__global__ void BT_MX_BOUNDS
+__global__ void __launch_bounds__(MX_THREADS, MX_MIN_BLOCKS)
 k_eval_grids_mixed(MixedGridsArgs a)
 {
     extern __shared__ float smf[];

@@ -52,9 +52,10 @@ namespace {
 
 constexpr int SY_THREADS = 128;
 // targets of A per thread (packed in pairs) and the resident blocks per SM
-// the register budget is sized for; build-time choices.  Measured on the 16M
-// clustered step: 4 and 6 (856 ms) against 6 and 4 (872 ms), 8 and 4
-// (886 ms), 8 and 3 (894 ms)
+// the register budget is sized for; build-time choices.  Measured, evaluation
+// phase of 2M clustered Coulomb and of 1M cluster-cluster Yukawa, degree 8:
+// 4 and 6 91.0 and 16.4 ms, 4 and 5 91.1 and 16.9, 4 and 7 91.0 and 16.5,
+// 8 and 4 90.2 and 16.8, 8 and 3 90.9 and 16.5, 2 and 8 96.7 and 18.2
 #ifndef BT_SYM_TPT
 #define BT_SYM_TPT 4
 #endif
@@ -64,11 +65,13 @@ constexpr int SY_THREADS = 128;
 constexpr int SY_TPT = BT_SYM_TPT;
 constexpr int SY_NP = SY_TPT / 2;
 constexpr int SY_CHUNK = SY_TPT * 32;          // targets of A a warp holds at a time
+static_assert(SY_TPT % 2 == 0 && SYM_PART % SY_CHUNK == 0, "a part is whole chunks (accA), targets are packed in pairs");
 #ifndef BT_SYM_TILE
 #define BT_SYM_TILE 256
 #endif
 constexpr int SY_TILE = BT_SYM_TILE;                   // sources of B per shared-memory tile
 constexpr int SY_SB = 16;                      // sources per warp reduction
+static_assert(SY_TILE % SY_SB == 0, "a tile is whole groups of sources");
 constexpr int SY_WARPS = SY_THREADS / 32;
 constexpr float SY_PAD_POS = 1.0e18f;          // padding sources: far away, no charge
 

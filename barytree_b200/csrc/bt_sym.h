@@ -10,11 +10,12 @@ namespace bt {
 constexpr int SYM_MAX_LEAF = 2048;
 // Smallest leaf whose pairs the FP64 path's symmetric pass takes (a rule per
 // pair, so that a batch takes the pairs its systems take in separate calls).
-// Measured, uniform systems, whole calls without and with the pass: leaves of
-// 195 particles 5.7 and 6.0 ms (Yukawa 10.9 and 10.8 ms; the pairs' planning
-// eats the gain), of 390 particles 10.4 and 9.3 ms (26.2 and 22.6 ms), of 1560
-// particles 5.8 and 5.0 ms (13.4 and 10.3 ms).  Leaves below 512, where the
-// gain is small, keep the sums of every direction.
+// Measured with the line at 128, uniform systems, whole calls without and with
+// the pass, Coulomb (Yukawa): leaves of 195 particles 5.5 and 5.2 ms (13.1 and
+// 11.0), of 244 6.2 and 5.8 (14.9 and 12.6), of 312 8.9 and 8.1 (22.1 and
+// 17.9), of 400 14.0 and 11.5 (35.8 and 26.7); of 1560, above the line, 5.8 and
+// 5.0 (13.4 and 10.3).  So the line is higher than it need be: leaves below it
+// keep the sums of every direction.
 constexpr int SYM64_MIN_LEAF = 512;
 
 // Threads (particles) per block of the gathers.

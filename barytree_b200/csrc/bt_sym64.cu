@@ -25,15 +25,12 @@
 #include "bt_eval64.cuh"
 #include "bt_sym.h"
 
-#ifndef BT_S64_MINB
-#define BT_S64_MINB 3
-#endif
-
 namespace bt {
 
 namespace {
 
 constexpr int S64_THREADS = 128;
+constexpr int S64_MINB = 3;                      // resident blocks per SM (4 measured 1.5 % slower, 300k Yukawa)
 constexpr int S64_WARPS = S64_THREADS / 32;
 constexpr int S64_TPT = 4;                       // particles of A per thread
 constexpr int S64_CHUNK = 32 * S64_TPT;          // per warp
@@ -64,7 +61,7 @@ __device__ __noinline__ double leaf_again(const Sym64Args &a, int i, int jb, int
 }
 
 template <int KT>
-__global__ void __launch_bounds__(S64_THREADS, BT_S64_MINB) k_pp_sym64(const __grid_constant__ Sym64Args a)
+__global__ void __launch_bounds__(S64_THREADS, S64_MINB) k_pp_sym64(const __grid_constant__ Sym64Args a)
 {
     __shared__ double2 xy[S64_TILE], zq[S64_TILE];
     __shared__ double accB[SYM_MAX_LEAF];
