@@ -3564,7 +3564,7 @@ int bt_autotune(int numSystems, const long long *targetOffsets, const long long 
                         bt::launch_eval_targets_mixed(S->v.kernel, a, st);
                         cudaEventRecord(e1, st);
                         if (cudaEventSynchronize(e1) != cudaSuccess || cudaGetLastError() != cudaSuccess) { rc = BT_ERR_CUDA; break; }
-                        g_launches += 1;
+                        g_launches += a.partial ? 2 : 1;
                         float ms = 0.0f;
                         cudaEventElapsedTime(&ms, e0, e1);
                         if (r == 1 || (r == 2 && ms < bestms)) bestms = ms;
