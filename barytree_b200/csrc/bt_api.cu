@@ -741,7 +741,10 @@ int build_plan_gpu(DeviceCtx *ctx, Arena &tarena, bt_plan &pl, const Systems &sy
 struct SymRound {
     int64_t far0, far1, near0, near1;
 };
-// Device memory of the pairs' slices (a round's).
+// Device memory of the pairs' slices (a round's).  16M clustered particles have
+// 10 GB of them; evaluation in one round (16 GB) 815.9 ms, in two 816.2, with
+// 2 GB 817.7 (8.5 GB less memory), with 1 GB 819.2: a round costs little, so
+// the bound is what a call may take of the device, not what is fastest.
 constexpr size_t SYM_SLICE_BYTES = (size_t)8 << 30;
 
 // Everything the device sequence of one evaluation needs: the device arrays
