@@ -332,8 +332,8 @@ def cpu_baseline(cfg, config_id, cores):
 # committed ncu summaries that carry a DRAM traffic figure for a configuration,
 # and what that figure is
 PROFILE_FOR_CONFIG = {5: ("eval_traffic_blobs16M.md",
-                          "ncu capture (one pass per kernel) of the 16M evaluation's four kernels "
-                          "(k_eval_targets_mixed_rb, k_pp_sym x2, k_sym_gather), second evaluation of the process: "
+                          "ncu capture (one pass per kernel) of the 16M evaluation's kernels "
+                          "(k_eval_targets_mixed_rb, k_pp_sym x2, k_sym_gather), fifth evaluation of the process: "
                           "dram__bytes_read.sum + dram__bytes_write.sum summed")}
 
 
