@@ -756,6 +756,7 @@ struct DevPlan {
     bool base_full = true;      // proxies at the base degree for every node (else only the selected
                                 // degrees' marked subtrees, the base degree among them)
     bool tc_up = false;         // leaf P2M on the tensor cores (bt_tc.cu)
+    bool far_exp = false;       // FP64 Yukawa: exponentials outside exp64's range occur
     bool sharded = false;       // this call evaluates a share of the target leaves (others get 0)
     // symmetric near-field pairs (bt_sym.cu)
     std::vector<SymRound> sym_rounds;
@@ -1053,7 +1054,7 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         g.c_off = d_ccoff; g.c_idx = d_ccidx; g.p_off = d_cpoff; g.p_idx = d_cpidx;
         g.s_ibeg = d_sibeg; g.s_numpar = d_snum; g.s_grid = d_sgrid; g.Q = d_Q;
         g.sx = d_sx; g.sy = d_sy; g.sz = d_sz; g.sq = d_sq; g.kp = v.kp; g.kp2 = v.kp2; g.Phi = d_Phi;
-        g.partial = v.d_gridpart; g.pstride = (size_t)v.T_n * P;
+        g.partial = v.d_gridpart; g.pstride = (size_t)v.T_n * P; g.far_exp = v.far_exp;
         bt::launch_eval_grids(v.kernel, herm, g, st);
         launches += g.partial ? 2 : 1;
     }
@@ -1141,7 +1142,7 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
         a.s_ibeg = d_sibeg; a.s_numpar = d_snum; a.s_grid = d_sgrid; a.Q = d_Q;
         a.sx = d_sx; a.sy = d_sy; a.sz = d_sz; a.sq = d_sq; a.tx = d_tx; a.ty = d_ty; a.tz = d_tz;
         a.kp = v.kp; a.kp2 = v.kp2; a.pot = d_pot;
-        a.partial = v.d_evpart; a.pstride = (size_t)nt;
+        a.partial = v.d_evpart; a.pstride = (size_t)nt; a.far_exp = v.far_exp;
         // the symmetric pairs beside the particle-output kernel, joined before
         // the gather adds their slices
         const int nrounds = (int)v.sym_rounds.size();
@@ -1161,6 +1162,7 @@ int issue_plan(const DevPlan &v, cudaStream_t st, cudaEvent_t *ev, double *scatt
             y.nblocks = (int)(w.far1 - w.far0); y.block = v.d_sym_blocks + w.far0;
             y.pair = v.d_sym_pairs; y.slot = v.d_sym_slot; y.ibeg = d_sibeg; y.numpar = d_snum;
             y.x = d_sx; y.y = d_sy; y.z = d_sz; y.q = d_sq; y.partial = v.d_sym_partial64; y.kp = v.kp;
+            y.far_exp = v.far_exp;
             bt::launch_pp_sym64(v.kernel, y, sst);
             launches++;
             if (r + 1 == nrounds) break;
@@ -1559,6 +1561,26 @@ void SymPairs::place(int64_t values, std::vector<int64_t> &doff, hvec<int> &didx
     doff.swap(noff);
     didx.swap(nidx);
     dflag.swap(nflag);
+}
+
+// Whether a Yukawa call can meet exponentials outside exp64's range: kappa
+// times the diagonal of the box around a system's targets and sources.
+bool far_exponentials(const bt_plan &pl)
+{
+    if (pl.prm.kernel != YUKAWA) return false;
+    const bt_tree &S = pl.st, &T = pl.tt;
+    double extent = 0.0;
+    for (int k = 0; k < T.nroots; k++) {
+        const int s = S.roots[k], t = T.roots[k];
+        if (s < 0 || t < 0) continue;
+        const double dx = std::max(S.x1[s], T.x1[t]) - std::min(S.x0[s], T.x0[t]),
+                     dy = std::max(S.y1[s], T.y1[t]) - std::min(S.y0[s], T.y0[t]),
+                     dz = std::max(S.z1[s], T.z1[t]) - std::min(S.z0[s], T.z0[t]);
+        const double d = sqrt(dx * dx + dy * dy + dz * dz);
+        if (!(d <= extent)) extent = d;
+        if (std::isnan(extent)) break;
+    }
+    return !bt::exp64_range(pl.prm.kp, extent);
 }
 
 // Device evaluation of a built plan; writes potentials in caller order to out_host.
@@ -2066,6 +2088,7 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
         v.tile = shape.tile;
         v.tc_up = shape.tc_up && mixed;
         v.sharded = shape.nshards > 1;
+        v.far_exp = !mixed && !ssm && far_exponentials(pl);
         v.d_evpart = d_evpart; v.d_gridpart = d_gridpart;
         v.base_full = pl.a_deg == nullptr;
         if (!sym.pairs.empty()) v.sym_rounds = sym.rounds;

@@ -904,7 +904,10 @@ void launch_eval_targets(int kernel, bool hermite, const EvalTargetsArgs &a, cud
     if (a.nitems <= 0) return;
     switch (kernel) {
     case K_COULOMB: eval_targets_kt<K_COULOMB>(hermite, a, st); break;
-    case K_YUKAWA: eval_targets_kt<K_YUKAWA>(hermite, a, st); break;
+    case K_YUKAWA:
+        if (a.far_exp) eval_targets_kt<K_YUKAWA, true>(hermite, a, st);
+        else eval_targets_kt<K_YUKAWA>(hermite, a, st);
+        break;
     case K_REGCOULOMB: eval_targets_kt<K_REGCOULOMB>(hermite, a, st); break;
     case K_SINOVERR: eval_targets_kt<K_SINOVERR>(hermite, a, st); break;
     case K_REGYUKAWA: eval_targets_kt<K_REGYUKAWA>(false, a, st); break;
@@ -946,7 +949,10 @@ void launch_eval_grids(int kernel, bool hermite, const EvalGridsArgs &a, cudaStr
     }
     switch (kernel) {
     case K_COULOMB: eval_grids_kt<K_COULOMB>(a, st); break;
-    case K_YUKAWA: eval_grids_kt<K_YUKAWA>(a, st); break;
+    case K_YUKAWA:
+        if (a.far_exp) eval_grids_kt<K_YUKAWA, true>(a, st);
+        else eval_grids_kt<K_YUKAWA>(a, st);
+        break;
     case K_REGCOULOMB: eval_grids_kt<K_REGCOULOMB>(a, st); break;
     case K_SINOVERR: eval_grids_kt<K_SINOVERR>(a, st); break;
     case K_REGYUKAWA: eval_grids_kt<K_REGYUKAWA>(a, st); break;

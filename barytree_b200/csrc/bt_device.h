@@ -25,6 +25,10 @@ __host__ __device__ inline int64_t seg_begin(int64_t b, int64_t e, int s) { retu
 // a source can coincide with a target and the skipping rule is tested.
 constexpr int EV_MEETS = (int)0x80000000;
 
+// Whether exp(-kappa r) stays within 2^-1021.4 and 2^1021.4 for every r up to
+// `extent`, the range of the Yukawa kernels' short exponential.
+inline bool exp64_range(double kappa, double extent) { return (kappa < 0.0 ? -kappa : kappa) * extent < 708.0; }
+
 struct EvalTargetsArgs {
     int n, nitems;
     const int2 *items;            // (target leaf unit, chunk of EV_CHUNK targets), sorted by cost
@@ -40,6 +44,7 @@ struct EvalTargetsArgs {
     double *pot;
     double *partial = nullptr;
     size_t pstride = 0;
+    bool far_exp = false;         // Yukawa: exponentials beyond exp64's range occur
 };
 
 struct EvalGridsArgs {
@@ -55,6 +60,7 @@ struct EvalGridsArgs {
     double *Phi;
     double *partial = nullptr;                  // Lagrange only
     size_t pstride = 0;
+    bool far_exp = false;
 };
 
 void launch_p2m(int n, bool hermite, int nleaves, const int *leaves, int nnodes, const int *ibeg, const int *numpar,

@@ -34,7 +34,8 @@ namespace bt {
 
 constexpr int EV_TILE = 512;        // sources per shared-memory tile
 
-// What a kernel value needs besides r^2 and the charge.
+// What a kernel value needs besides r^2 and the charge.  FAR: exp64's.
+template <bool FAR>
 struct Kern64 {
     double kp, kp2, eps2;
     Exp64 ex;
@@ -44,10 +45,10 @@ struct Kern64 {
 template <int KT>
 __host__ __device__ constexpr bool fast64() { return KT <= K_REGCOULOMB; }
 
-template <int KT>
-__device__ __forceinline__ Kern64 kern64_make(double kp, double kp2, double2 *tab)
+template <int KT, bool FAR>
+__device__ __forceinline__ Kern64<FAR> kern64_make(double kp, double kp2, double2 *tab)
 {
-    Kern64 k;
+    Kern64<FAR> k;
     k.kp = kp; k.kp2 = kp2;
     k.eps2 = KT == K_REGCOULOMB ? kp * kp : 0.0;
     k.lib = KT == K_YUKAWA && !exp64_takes(kp);
@@ -59,18 +60,18 @@ __device__ __forceinline__ Kern64 kern64_make(double kp, double kp2, double2 *ta
 }
 
 // K(r), r2 the squared distance (plus eps^2 for the regularized kernel).
-template <int KT>
-__device__ __forceinline__ double value64(double r2, const Kern64 &k)
+template <int KT, bool FAR>
+__device__ __forceinline__ double value64(double r2, const Kern64<FAR> &k)
 {
     if (KT == K_YUKAWA) {
         double r;
         const double y = rsqrt_sqrt_n(r2, r);
-        return y * exp64(r, k.ex);
+        return y * exp64<FAR>(r, k.ex);
     }
     return rsqrt_n(r2);
 }
-template <int KT>
-__device__ __forceinline__ double add64(double acc, double r2, double q, const Kern64 &k)
+template <int KT, bool FAR>
+__device__ __forceinline__ double add64(double acc, double r2, double q, const Kern64<FAR> &k)
 {
     return fma(q, value64<KT>(r2, k), acc);
 }
@@ -109,9 +110,9 @@ struct Out2 {
 
 // Far field of one source cluster: grid rows slice, slice + slices, ...; g the
 // 3 (n+1) grid coordinates, q the proxy charges.
-template <int KT, int NP1>
+template <int KT, int NP1, bool FAR>
 __device__ __forceinline__ void far64(double *acc, const double *g, const double *q, const Out2 &o, const Lanes &w,
-                                      const Kern64 &k)
+                                      const Kern64<FAR> &k)
 {
     double gx[2][NP1];
 #pragma unroll
@@ -139,9 +140,9 @@ __device__ __forceinline__ void far64(double *acc, const double *g, const double
 }
 
 // The same for the kernels without a short form.
-template <int KT>
+template <int KT, bool FAR>
 __device__ __forceinline__ void far64_any(double *acc, int np1, const double *g, const double *q, const Out2 &o,
-                                          const Lanes &w, const Kern64 &k)
+                                          const Lanes &w, const Kern64<FAR> &k)
 {
     for (int row = w.slice; row < np1 * np1; row += w.slices) {
         const int k3 = row / np1, k2 = row - k3 * np1;
@@ -159,9 +160,9 @@ __device__ __forceinline__ void far64_any(double *acc, int np1, const double *g,
 //   1/r [ q + u (qx dx + qy dy + qz dz) + u^2 (qxy dx dy + qyz dy dz + qxz dx dz) + u^3 qxyz dx dy dz ]
 // sorted by powers of dx (b, c below): 15 FP64 instructions besides 1/r.
 // Yukawa has its polynomials in kappa r beside each power of u.
-template <int KT>
+template <int KT, bool FAR>
 __device__ __forceinline__ void herm64(double *acc, int np1, const double *g, const double *q, const Out2 &o,
-                                       const Lanes &w, const Kern64 &k)
+                                       const Lanes &w, const Kern64<FAR> &k)
 {
     for (int row = w.slice; row < np1 * np1; row += w.slices) {
         const int k3 = row / np1, k2 = row - k3 * np1;
@@ -189,7 +190,7 @@ __device__ __forceinline__ void herm64(double *acc, int np1, const double *g, co
                     const double e = fma(u * p2, m[5] * dydz[b], p1 * fma(m[3], dz[b], m[2] * dy[b]));
                     const double c = fma(u * p3, m[7] * dydz[b], p2 * fma(m[6], dz[b], m[4] * dy[b]));
                     const double v = fma(dx * u, fma(u, c, p1 * m[1]), fma(u, e, m[0]));
-                    acc[b] = fma(rinv * v, exp64(r, k.ex), acc[b]);
+                    acc[b] = fma(rinv * v, exp64<FAR>(r, k.ex), acc[b]);
                 } else {
                     const double rinv = rsqrt_n(r2), u = rinv * rinv, v = u * dydz[b];
                     const double e = fma(m[5], v, fma(m[3], dz[b], m[2] * dy[b]));
@@ -202,9 +203,9 @@ __device__ __forceinline__ void herm64(double *acc, int np1, const double *g, co
 }
 
 // sin-over-r Hermite: the library form.
-template <int KT>
+template <int KT, bool FAR>
 __device__ __forceinline__ void herm64_any(double *acc, int np1, const double *g, const double *q, const Out2 &o,
-                                           const Lanes &w, const Kern64 &k)
+                                           const Lanes &w, const Kern64<FAR> &k)
 {
     const int P = np1 * np1 * np1;
     for (int row = w.slice; row < np1 * np1; row += w.slices) {
@@ -228,9 +229,9 @@ struct Tile64 {
 // Sources i0, i0 + step, ... < cm of a tile, the range a multiple of 4 * step
 // long.  TEST: with the skipping rule, else mn gets the smallest upper half of
 // the thread's r^2 (as an integer: r^2 is never negative).
-template <int KT, bool TEST>
+template <int KT, bool TEST, bool FAR>
 __device__ __forceinline__ void near64(double *acc, const Tile64 &t, int i0, int step, int cm, const Out2 &o,
-                                       const Kern64 &k, int &mn)
+                                       const Kern64<FAR> &k, int &mn)
 {
     for (int c = i0; c < cm; c += 4 * step)
 #pragma unroll
@@ -252,9 +253,9 @@ __device__ __forceinline__ void near64(double *acc, const Tile64 &t, int i0, int
 // is at the rule's limit or below (a target that coincides with a source: one
 // group in hundreds).  The test in every term took 24 instructions per value
 // instead of 15, 5.1 ms for 10,000 x 500,000 pairs.
-template <int KT>
+template <int KT, bool FAR>
 __device__ __forceinline__ void near64_skip(double *acc, const Tile64 &t, int i0, int step, int cm, const Out2 &o,
-                                            const Kern64 &k)
+                                            const Kern64<FAR> &k)
 {
     for (int c = i0; c < cm; c += 32 * step) {
         const int ce = min(cm, c + 32 * step);
@@ -270,9 +271,9 @@ __device__ __forceinline__ void near64_skip(double *acc, const Tile64 &t, int i0
     }
 }
 
-template <int KT, bool PP>
+template <int KT, bool PP, bool FAR>
 __device__ __forceinline__ void near64_any(double *acc, const Tile64 &t, int i0, int step, int cm, const Out2 &o,
-                                           const Kern64 &k)
+                                           const Kern64<FAR> &k)
 {
     for (int i = i0; i < cm; i += step) {
         const double2 p = t.xy[i], s = t.zq[i];
@@ -284,11 +285,11 @@ __device__ __forceinline__ void near64_any(double *acc, const Tile64 &t, int i0,
 
 // Sources sb .. sb + sn - 1 for every thread of the block (tiles staged by
 // all).  test: some pair may coincide.
-template <int KT, bool PP>
+template <int KT, bool PP, bool FAR>
 __device__ __forceinline__ void near64_node(double *acc, const Tile64 &t, int sb, int sn, const double *__restrict__ sx,
                                             const double *__restrict__ sy, const double *__restrict__ sz,
                                             const double *__restrict__ sq, bool test, const Out2 &o, const Lanes &w,
-                                            const Kern64 &k)
+                                            const Kern64<FAR> &k)
 {
     for (int c0 = 0; c0 < sn; c0 += EV_TILE) {
         const int cm = min(EV_TILE, sn - c0);
@@ -354,13 +355,13 @@ __device__ __forceinline__ void sum_slices(double *acc, double *red, const Lanes
 
 // Particle outputs: PC (clusters) + PP (particles) onto a chunk of a target
 // leaf.  NP1 = n + 1 (Lagrange with a short form), else 0.
-template <int KT, int NP1, bool HERM>
+template <int KT, int NP1, bool HERM, bool FAR>
 __global__ void __launch_bounds__(EV_THREADS, EV_MINB) k_eval_targets(const __grid_constant__ EvalTargetsArgs a)
 {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[2 * EV_THREADS];
     __shared__ double2 tab[KT == K_YUKAWA ? EXP64_TAB : 1];
-    const Kern64 k = kern64_make<KT>(a.kp, a.kp2, tab);
+    const Kern64<FAR> k = kern64_make<KT, FAR>(a.kp, a.kp2, tab);
     const int2 it = a.items[blockIdx.x];
     const int u = it.x, tnode = a.leaf_node[u];
     const Lanes w(min(EV_CHUNK, a.t_numpar[tnode] - it.y * EV_CHUNK));
@@ -428,13 +429,13 @@ __global__ void __launch_bounds__(EV_THREADS, EV_MINB) k_eval_targets(const __gr
 
 // Grid outputs: M2L (clusters, Lagrange) + CP (particles) onto a chunk of a
 // target node's grid points.
-template <int KT, int NP1>
+template <int KT, int NP1, bool FAR>
 __global__ void __launch_bounds__(EV_THREADS, EV_MINB) k_eval_grids(const __grid_constant__ EvalGridsArgs a)
 {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[2 * EV_THREADS];
     __shared__ double2 tab[KT == K_YUKAWA ? EXP64_TAB : 1];
-    const Kern64 k = kern64_make<KT>(a.kp, a.kp2, tab);
+    const Kern64<FAR> k = kern64_make<KT, FAR>(a.kp, a.kp2, tab);
     const int2 it = a.items[blockIdx.x];
     const int T = it.x, np1 = NP1 ? NP1 : a.n + 1, P = np1 * np1 * np1;
     const Lanes w(min(EV_CHUNK, P - it.y * EV_CHUNK));
@@ -501,7 +502,7 @@ k_direct(int nt, int ns, const double *__restrict__ tx, const double *__restrict
     __shared__ double2 xy[EV_TILE], zq[EV_TILE];
     __shared__ double red[2 * EV_THREADS];
     __shared__ double2 tab[KT == K_YUKAWA ? EXP64_TAB : 1];
-    const Kern64 k = kern64_make<KT>(kp, kp2, tab);
+    const Kern64<true> k = kern64_make<KT, true>(kp, kp2, tab);      // the extent is not known
     const int t0 = blockIdx.x * EV_CHUNK;
     const Lanes w(min(EV_CHUNK, nt - t0));
     Out2 o;
@@ -541,40 +542,40 @@ void eval64_launch(K kernel, const A &a, size_t far_doubles, cudaStream_t st)
     kernel<<<dim3(a.nitems, a.partial ? EV_SEGS : 1), EV_THREADS, sm, st>>>(a);
 }
 
-template <int KT>
+template <int KT, bool FAR>
 void eval_targets_kt(bool hermite, const EvalTargetsArgs &a, cudaStream_t st)
 {
     const size_t np1 = a.n + 1, P = np1 * np1 * np1;
     if constexpr (fast64<KT>() || KT == K_SINOVERR)
         if (hermite) {
-            eval64_launch(k_eval_targets<KT, 0, true>, a, 3 * np1 + 1 + 8 * P, st);
+            eval64_launch(k_eval_targets<KT, 0, true, FAR>, a, 3 * np1 + 1 + 8 * P, st);
             return;
         }
     if constexpr (fast64<KT>()) {
         switch (np1) {
-#define BT_EV(N) case N: eval64_launch(k_eval_targets<KT, N, false>, a, 3 * np1 + P, st); return;
+#define BT_EV(N) case N: eval64_launch(k_eval_targets<KT, N, false, FAR>, a, 3 * np1 + P, st); return;
             BT_EV(2) BT_EV(3) BT_EV(4) BT_EV(5) BT_EV(6) BT_EV(7) BT_EV(8) BT_EV(9) BT_EV(10) BT_EV(11) BT_EV(12)
             BT_EV(13)
 #undef BT_EV
         }
     } else {
-        eval64_launch(k_eval_targets<KT, 0, false>, a, 3 * np1 + P, st);
+        eval64_launch(k_eval_targets<KT, 0, false, FAR>, a, 3 * np1 + P, st);
     }
 }
 
-template <int KT>
+template <int KT, bool FAR>
 void eval_grids_kt(const EvalGridsArgs &a, cudaStream_t st)
 {
     const size_t np1 = a.n + 1, P = np1 * np1 * np1;
     if constexpr (fast64<KT>()) {
         switch (np1) {
-#define BT_EV(N) case N: eval64_launch(k_eval_grids<KT, N>, a, 3 * np1 + P, st); return;
+#define BT_EV(N) case N: eval64_launch(k_eval_grids<KT, N, FAR>, a, 3 * np1 + P, st); return;
             BT_EV(2) BT_EV(3) BT_EV(4) BT_EV(5) BT_EV(6) BT_EV(7) BT_EV(8) BT_EV(9) BT_EV(10) BT_EV(11) BT_EV(12)
             BT_EV(13)
 #undef BT_EV
         }
     } else {
-        eval64_launch(k_eval_grids<KT, 0>, a, 3 * np1 + P, st);
+        eval64_launch(k_eval_grids<KT, 0, FAR>, a, 3 * np1 + P, st);
     }
 }
 
@@ -586,9 +587,10 @@ void direct_kt(int nt, int ns, int parts, const double *tx, const double *ty, co
                                                                                      kp, kp2, out);
 }
 
-#define BT_EVAL64_INSTANTIATE(KT)                                                                                    \
-    template void eval_targets_kt<KT>(bool, const EvalTargetsArgs &, cudaStream_t);                                  \
-    template void eval_grids_kt<KT>(const EvalGridsArgs &, cudaStream_t);                                            \
+#define BT_EVAL64_INSTANTIATE(KT, FAR)                                                                               \
+    template void eval_targets_kt<KT, FAR>(bool, const EvalTargetsArgs &, cudaStream_t);                             \
+    template void eval_grids_kt<KT, FAR>(const EvalGridsArgs &, cudaStream_t);
+#define BT_EVAL64_INSTANTIATE_DIRECT(KT)                                                                             \
     template void direct_kt<KT>(int, int, int, const double *, const double *, const double *, const double *,        \
                                 const double *, const double *, const double *, double, double, double *, cudaStream_t);
 

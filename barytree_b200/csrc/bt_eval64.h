@@ -8,9 +8,10 @@
 
 namespace bt {
 
-template <int KT>
+// FAR: Yukawa calls whose exponentials can leave the short form's range.
+template <int KT, bool FAR = false>
 void eval_targets_kt(bool hermite, const EvalTargetsArgs &a, cudaStream_t st);
-template <int KT>
+template <int KT, bool FAR = false>
 void eval_grids_kt(const EvalGridsArgs &a, cudaStream_t st);
 template <int KT>
 void direct_kt(int nt, int ns, int parts, const double *tx, const double *ty, const double *tz, const double *sx,

@@ -3,6 +3,7 @@
 
 namespace bt {
 
-BT_EVAL64_INSTANTIATE(K_COULOMB)
+BT_EVAL64_INSTANTIATE(K_COULOMB, false)
+BT_EVAL64_INSTANTIATE_DIRECT(K_COULOMB)
 
 }  // namespace bt

@@ -3,6 +3,7 @@
 
 namespace bt {
 
-BT_EVAL64_INSTANTIATE(K_REGCOULOMB)
+BT_EVAL64_INSTANTIATE(K_REGCOULOMB, false)
+BT_EVAL64_INSTANTIATE_DIRECT(K_REGCOULOMB)
 
 }  // namespace bt

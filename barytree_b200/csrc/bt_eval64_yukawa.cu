@@ -3,6 +3,7 @@
 
 namespace bt {
 
-BT_EVAL64_INSTANTIATE(K_YUKAWA)
+BT_EVAL64_INSTANTIATE(K_YUKAWA, false)
+BT_EVAL64_INSTANTIATE_DIRECT(K_YUKAWA)
 
 }  // namespace bt

@@ -152,18 +152,18 @@ __device__ __forceinline__ void ss_values(double r2, const SsKern &k, double &kv
     if (KT == K_YUKAWA) {
         double r;
         const double y = rsqrt_sqrt_n(r2, r);
-        kv = y * exp64(r, k.ex);
+        kv = y * exp64<true>(r, k.ex);
         g = 1.0;
     } else if (KT == K_REGYUKAWA) {
         // r of a coincident pair from a tiny r^2 instead of zero
         const double c = __hiloint2double(max(__double2hiint(r2), 0x01a00000), __double2loint(r2));
         double r;
         rsqrt_sqrt_n(c, r);
-        kv = rsqrt_n(r2 + k.eps2) * exp64(r, k.ex);
+        kv = rsqrt_n(r2 + k.eps2) * exp64<true>(r, k.ex);
         g = 1.0;
     } else {
         kv = rsqrt_n(KT == K_REGCOULOMB ? r2 + k.eps2 : r2);
-        g = exp64(r2, k.ex);
+        g = exp64<true>(r2, k.ex);
     }
 }
 

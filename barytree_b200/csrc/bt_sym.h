@@ -75,6 +75,7 @@ struct Sym64Args {
     const double *x, *y, *z, *q;  // particles in tree order
     double *partial;
     double kp;
+    bool far_exp = false;         // Yukawa: exponentials beyond exp64's range occur
 };
 
 struct SymGather64Args {

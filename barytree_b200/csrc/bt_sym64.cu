@@ -60,14 +60,14 @@ __device__ __noinline__ double leaf_again(const Sym64Args &a, int i, int jb, int
     return s;
 }
 
-template <int KT>
+template <int KT, bool FAR>
 __global__ void __launch_bounds__(S64_THREADS, S64_MINB) k_pp_sym64(const __grid_constant__ Sym64Args a)
 {
     __shared__ double2 xy[S64_TILE], zq[S64_TILE];
     __shared__ double accB[SYM_MAX_LEAF];
     __shared__ double accA[S64_WARPS][SYM_PART];
     __shared__ double2 tab[KT == K_YUKAWA ? EXP64_TAB : 1];
-    const Kern64 k = kern64_make<KT>(a.kp, 0.0, tab);
+    const Kern64<FAR> k = kern64_make<KT, FAR>(a.kp, 0.0, tab);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int2 work = a.block[blockIdx.x];
     const int2 pr = a.pair[work.x];
@@ -174,9 +174,10 @@ __global__ void __launch_bounds__(GATHER_THREADS) k_sym_gather64(SymGather64Args
 void launch_pp_sym64(int kernel, const Sym64Args &a, cudaStream_t st)
 {
     if (a.nblocks <= 0) return;
-    if (kernel == K_REGCOULOMB) k_pp_sym64<K_REGCOULOMB><<<a.nblocks, S64_THREADS, 0, st>>>(a);
-    else if (kernel == K_YUKAWA) k_pp_sym64<K_YUKAWA><<<a.nblocks, S64_THREADS, 0, st>>>(a);
-    else k_pp_sym64<K_COULOMB><<<a.nblocks, S64_THREADS, 0, st>>>(a);
+    if (kernel == K_REGCOULOMB) k_pp_sym64<K_REGCOULOMB, false><<<a.nblocks, S64_THREADS, 0, st>>>(a);
+    else if (kernel == K_YUKAWA && a.far_exp) k_pp_sym64<K_YUKAWA, true><<<a.nblocks, S64_THREADS, 0, st>>>(a);
+    else if (kernel == K_YUKAWA) k_pp_sym64<K_YUKAWA, false><<<a.nblocks, S64_THREADS, 0, st>>>(a);
+    else k_pp_sym64<K_COULOMB, false><<<a.nblocks, S64_THREADS, 0, st>>>(a);
 }
 
 void launch_sym_gather64(const SymGather64Args &a, cudaStream_t st)

@@ -83,6 +83,40 @@ def test_few_items_and_many_items_give_the_same_bits(approx):
     assert np.array_equal(B.treecode_batch([sys_of(one), sys_of(big)], **kw)[0], alone)
 
 
+@pytest.mark.parametrize("ctype", [1, 2, 3])
+@pytest.mark.parametrize("approx", [1, 2])
+def test_exponentials_that_all_underflow_sum_to_zero(ctype, approx):
+    """Clouds four apart at kappa = 200: every exp(-kappa r) is zero in FP64."""
+    if (ctype, approx) == (3, 2):
+        pytest.skip("cluster-cluster Hermite is not provided")
+    x, y, z, q = _cube(6, 4000)
+    kw = dict(kernel=2, kernel_param=200.0, compute_type=ctype, approximation=approx, degree=4, theta=0.7,
+              max_source_leaf=100, max_target_leaf=100, size_check=1.0 if approx == 1 else 4.0)
+    assert np.all(B.treecode(x + 6.0, y, z, x, y, z, q, **kw) == 0.0)
+    assert np.all(B.direct(x + 6.0, y, z, x, y, z, q, 2, 200.0) == 0.0)
+    # subtraction: the correction alone is left
+    tq = np.abs(q)
+    c = 4.0 * np.pi / 200.0 / 200.0
+    ss = B.direct(x + 6.0, y, z, x, y, z, q, 2, 200.0, singularity=B.Singularity.SUBTRACTION, target_q=tq,
+                  source_w=np.ones_like(q))
+    assert np.array_equal(ss, c * tq)
+
+
+@pytest.mark.parametrize("ctype,approx", [(1, 1), (1, 2), (2, 1), (3, 1)])
+def test_range_of_exponentials_does_not_change_a_system(ctype, approx):
+    """A system within the short exponential's range keeps its bits in a batch
+    beside one beyond it (which runs the whole batch on the other kernels)."""
+    one, wide = _cube(8, 9000), _cube(9, 3000)
+    sys_of = lambda p, s: (*(a * s for a in p[:3]), *(a * s for a in p[:3]), p[3])  # noqa: E731
+    kw = dict(kernel=2, kernel_param=50.0, compute_type=ctype, approximation=approx, degree=5, theta=0.8,
+              max_source_leaf=1200, max_target_leaf=1200, size_check=1.0 if approx == 1 else 4.0)
+    alone = B.treecode(*sys_of(one, 1.0), **kw)                  # 50 * 2 sqrt(3) = 173
+    pots = B.treecode_batch([sys_of(one, 1.0), sys_of(wide, 20.0)], **kw)
+    assert np.array_equal(pots[0], alone)
+    x, y, z, q = sys_of(wide, 20.0)[3:]
+    assert _rel(pots[1], _direct((x, y, z), (x, y, z), q, 2, 50.0)) <= 1e-8
+
+
 def test_growing_exponential_takes_the_short_forms():
     """kappa < 0: the same kernels and pairs as a decaying one, at about their
     time (the library's exp in every sum took four times as long)."""
@@ -186,7 +220,7 @@ def test_exponential_to_the_last_places(kappa):
     """rsqrt_sqrt_n and exp64 in the Yukawa value: half a unit each for 1/r, for
     the table entry plus polynomial (truncated below 0.36 of 2^-53) and for the
     product, and the rounding of r times the exponent; every table entry, down
-    to the cut below 2^-1021 and, growing, up to the overflow."""
+    to 2^-1021, zero below 2^-1022 and, growing, up to the overflow."""
     top = 700.0 / abs(kappa) if kappa else 1e100
     r = np.concatenate([_radii(1e-12 * top, top, 200_001), np.linspace(0.001, 1.0, 100_001) * min(top, 1e3)])
     s = np.sqrt((r * r).astype(np.longdouble))
@@ -196,9 +230,8 @@ def test_exponential_to_the_last_places(kappa):
     r = r[normal]
     assert np.max(err / (3.5 + 1.1 * np.abs(kappa) * r)) <= U
     if kappa > 0:
-        far = np.linspace(1022.0, 4000.0, 1001) * np.log(2.0) / kappa
-        v = _values(far, 2, kappa) * far
-        assert np.all((v >= 0.0) & (v <= 2.0 ** -1021))
+        far = np.linspace(1022.01, 4000.0, 1001) * np.log(2.0) / kappa
+        assert np.all(_values(far, 2, kappa) == 0.0)
     if kappa < 0:
         far = np.linspace(1024.01, 4000.0, 1001) * np.log(2.0) / -kappa
         assert np.all(np.isposinf(_values(far, 2, kappa)))
