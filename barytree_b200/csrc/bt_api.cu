@@ -1960,26 +1960,29 @@ int run_plan(DeviceCtx *ctx, Arena &arena, bt_plan &pl, double *out, bool out_on
     std::vector<int64_t> doff64;
     hvec<int> didx64;
     if (!mixed && !ssm) {
-        auto expanded = [&](int u) { return sym.taken && sym.unit_expanded[u]; };
-        doff64.assign((size_t)T.nleaves + 1, 0);
-        for (int u = 0; u < T.nleaves; u++) {
-            const int64_t *off = expanded(u) ? mx_doff.data() : pl.t_direct.off;
-            doff64[u + 1] = doff64[u] + (off[u + 1] - off[u]);
+        int *flagged = pl.t_direct.idx;      // marked in place: its last use
+        if (sym.taken) {
+            doff64.assign((size_t)T.nleaves + 1, 0);
+            for (int u = 0; u < T.nleaves; u++) {
+                const int64_t *off = sym.unit_expanded[u] ? mx_doff.data() : pl.t_direct.off;
+                doff64[u + 1] = doff64[u] + (off[u + 1] - off[u]);
+            }
+            didx64.resize((size_t)doff64[T.nleaves]);
+            near_off = doff64.data();
+            near_idx = flagged = didx64.data();
         }
-        didx64.resize((size_t)doff64[T.nleaves]);
 #pragma omp parallel for schedule(static)
         for (int u = 0; u < T.nleaves; u++) {
             const int t = T.leaves[u];
-            const int *from = expanded(u) ? mx_didx.data() + mx_doff[u] : pl.t_direct.idx + pl.t_direct.off[u];
-            for (int64_t k = doff64[u]; k < doff64[u + 1]; k++) {
-                const int s = from[k - doff64[u]];
+            const int *from = sym.taken && sym.unit_expanded[u] ? mx_didx.data() + mx_doff[u]
+                                                                : pl.t_direct.idx + pl.t_direct.off[u];
+            for (int64_t k = near_off[u]; k < near_off[u + 1]; k++) {
+                const int s = from[k - near_off[u]];
                 const bool meets = S.x0[s] <= T.x1[t] && T.x0[t] <= S.x1[s] && S.y0[s] <= T.y1[t] &&
                                    T.y0[t] <= S.y1[s] && S.z0[s] <= T.z1[t] && T.z0[t] <= S.z1[s];
-                didx64[k] = meets ? s | bt::EV_MEETS : s;
+                flagged[k] = meets ? s | bt::EV_MEETS : s;
             }
         }
-        near_off = doff64.data();
-        near_idx = didx64.data();
     }
 
     L.resize(&d_didx, near_off[pl.t_direct.rows]);

@@ -52,6 +52,15 @@ def test_every_degree(ctype, degree):
 
 
 @pytest.mark.parametrize("kernel,kp", [(1, 0.0), (2, 0.7), (3, 1e-2)])
+@pytest.mark.parametrize("ctype,sleaf,tleaf", [(1, 3, 3), (1, 10, 10), (1, 70, 10), (2, 10, 40), (3, 10, 10), (1, 40, 130)])
+def test_source_nodes_smaller_than_a_group_of_four_per_thread(kernel, kp, ctype, sleaf, tleaf):
+    x, y, z, q = _cube(sleaf + tleaf, 3000)
+    kw = dict(compute_type=ctype, degree=3, theta=0.7, max_source_leaf=sleaf, max_target_leaf=tleaf)
+    ref = O.treecode(x, y, z, None, x, y, z, q, None, kernel, [kp], 1, 1, ctype, 0.7, 3, sleaf, tleaf, 1.0, -1.0, 0)
+    assert _rel(B.treecode(x, y, z, x, y, z, q, kernel=kernel, kernel_param=kp, **kw), ref) <= TOL
+
+
+@pytest.mark.parametrize("kernel,kp", [(1, 0.0), (2, 0.7), (3, 1e-2)])
 @pytest.mark.parametrize("n,leaf", [(4200, 600), (6000, 800), (9000, 1200), (14000, 2048)])
 def test_symmetric_pairs(kernel, kp, n, leaf):
     """Leaves of 512 to 2048 particles in pairs; the rest direction by direction."""
